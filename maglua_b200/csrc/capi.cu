@@ -166,6 +166,7 @@ struct ConvPlan {
     DBuf<char> ten6;     // TEN6[kx][kz][ky][6] (real)
     DBuf<char> ten9;     // TEN9[kx][kz][ky][9] (complex)
     DBuf<char> spec2;    // split passes: S2[kx][ky][c][z] (complex)
+    MxPlan mx;           // any-length passes (k.mx): ten6 then holds TZ[kx][dz][6][ky]
     double max_imag = 0; // largest |Im| of the FP64 tensor transform (6-component)
     int device = -1;     // CUDA device the arrays above live on
     // SPEC holds the forward x transform of the spins of the system whose
@@ -669,6 +670,31 @@ bool is_conv(int kind)
            kind == MLB_OP_MAGNETOSTATIC;
 }
 
+// Strength over the transform's normalisation (the any-length passes do not
+// transform z).
+double conv_scale(const mlb_op* op, const ConvK& k)
+{
+    return op->g * op->gs / ((double)k.Px * k.Py * (k.mx ? 1 : k.Pz));
+}
+
+// The field h of the spins sp by the plan's passes (k: P.k or a copy with
+// its own g or run_if), through the spectrum buffer spec.
+void launch_field(const ConvPlan& P, const ConvK& k, const void* const sp[3], void* spec, void* const h[3],
+                  cudaStream_t st)
+{
+    if (k.mx) {
+        CK(mlb::launch_mx_conv(k, P.mx, P.L, P.tw.p, sp, spec, P.ten6.p, h, true, true, P.rb, st));
+    } else if (P.rb == 4 && mlb::conv_fast_ok(k)) {
+        const float* s[3] = {static_cast<const float*>(sp[0]), static_cast<const float*>(sp[1]),
+                             static_cast<const float*>(sp[2])};
+        float* hf[3] = {static_cast<float*>(h[0]), static_cast<float*>(h[1]), static_cast<float*>(h[2])};
+        CK(mlb::launch_conv_fast(k, P.L, reinterpret_cast<const float2*>(P.tw.p), s, static_cast<float2*>(spec),
+                                 reinterpret_cast<const float*>(P.ten6.p), hf, st));
+    } else {
+        CK(mlb::launch_conv(k, P.L[0], P.L[1], P.L[2], P.tw.p, sp, spec, P.ten6.p, P.ten9.p, h, P.rb, st));
+    }
+}
+
 void plan_sizes(mlb_op* op, ConvPlan& P)
 {
     ConvK& k = P.k;
@@ -1015,8 +1041,24 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
             }
         CK(cudaMemcpy(W.p, h.data(), sizeof(double2) * h.size(), cudaMemcpyHostToDevice));
     }
-    CK(mlb::launch_fft3d_d(W.p, ncomp, Px, Py, Pz, P->L, twdd.p, -1, st));
-    if (k.general) {
+    // edges of any length: x and y transforms, the layer tensor if it has the
+    // parities the layer sum relies on (to 1e-10 of its largest element)
+    CK(mlb::launch_fft3d_d(W.p, ncomp, Px, Py, Pz, P->L, twdd.p, -1, 0, 2, st));
+    if (!(rb == 4 && mlb::conv_fast_ok(k)) && mlb::mx_plan(k, rb, P->mx)) {
+        DBuf<unsigned long long> stat;
+        stat.alloc(2);
+        CK(cudaMemsetAsync(stat.p, 0, 2 * sizeof(unsigned long long), st));
+        P->ten6.alloc(mlb::mx_tensor_bytes(k, rb));
+        CK(mlb::launch_mx_pack(W.p, k, P->ten6.p, stat.p, rb, st));
+        double hs[2];
+        CK(cudaMemcpyAsync(hs, stat.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        k.mx = hs[1] <= 1e-10 * hs[0];
+    }
+    if (!k.mx) CK(mlb::launch_fft3d_d(W.p, ncomp, Px, Py, Pz, P->L, twdd.p, -1, 2, 3, st));
+    if (k.mx) {
+        k.split = 0;
+    } else if (k.general) {
         P->ten9.alloc((size_t)k.Kx * Py * Pz * 9 * 2 * rb);
         CK(mlb::launch_tensor_pack9(W.p, Px, Py, Pz, k.Kx, P->ten9.p, rb, k.split, st));
     } else if ((quarter_ok(k, rb) || (rb == 4 && mlb::yz_col3_ok(k))) && tensor_has_parities(W.p, k, st)) {
@@ -1320,7 +1362,7 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
         const int np = std::min(bp, npair - p0);
         for (size_t i = 0; i < plane * 9 * np; i++) h[i] = make_double2(op->t2[(size_t)p0 * 9 * plane + i], 0.0);
         CK(cudaMemcpyAsync(W.p, h.data(), sizeof(double2) * plane * 9 * np, cudaMemcpyHostToDevice, st));
-        CK(mlb::launch_fft3d_d(W.p, 9 * np, nx, ny, 1, P->L, twdd.p, -1, st));
+        CK(mlb::launch_fft3d_d(W.p, 9 * np, nx, ny, 1, P->L, twdd.p, -1, 0, 2, st));
         CK(mlb::launch_lr2d_pack(W.p, nx, ny, nz, p0, np, P->Q.p, rb, st));
         CK(cudaStreamSynchronize(st));
     }
@@ -1698,14 +1740,14 @@ void op_apply(mlb_op* op, mlb_system* s)
         sl.base_data = false;
         slot_alloc(s, sl);
         ConvPlan& P = *op->plan;
-        P.k.g = op->g * op->gs / ((double)P.k.Px * P.k.Py * P.k.Pz);
+        P.k.g = conv_scale(op, P.k);
         sl.state = ST_DATA;
         if (s->dry) return;
         if (s->sur && sur_hook(op, s, sl)) return;
-        if (s->rb == 4 && mlb::conv_fast_ok(P.k)) {
+        const void* spv[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
+        if (!P.k.mx && s->rb == 4 && mlb::conv_fast_ok(P.k)) {
             const float* sp[3] = {static_cast<const float*>(s->sp[s->cur][0]), static_cast<const float*>(s->sp[s->cur][1]),
                                   static_cast<const float*>(s->sp[s->cur][2])};
-            float* h[3] = {static_cast<float*>(sl.h[0]), static_cast<float*>(sl.h[1]), static_cast<float*>(sl.h[2])};
             if (s->defer_x && P.k.nrep == 1 && !P.k.general) {
                 // forward x pass only when SPEC does not already hold it
                 const bool carry = s->capturing ? s->cap_carry
@@ -1720,16 +1762,9 @@ void op_apply(mlb_op* op, mlb_system* s)
                 s->pend_si = si;
                 return;
             }
-            if (!s->capturing) P.spec_token = 0;
-            CK(mlb::launch_conv_fast(P.k, P.L, reinterpret_cast<const float2*>(P.tw.p), sp,
-                                     reinterpret_cast<float2*>(P.spec.p), reinterpret_cast<const float*>(P.ten6.p), h,
-                                     s->st));
-        } else {
-            if (!s->capturing) P.spec_token = 0;
-            const void* sp[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
-            CK(mlb::launch_conv(P.k, P.L[0], P.L[1], P.L[2], P.tw.p, sp, P.spec.p, P.ten6.p, P.ten9.p, sl.h, s->rb,
-                                s->st));
         }
+        if (!s->capturing) P.spec_token = 0;
+        launch_field(P, P.k, spv, P.spec.p, sl.h, s->st);
         sl.state = ST_DATA;
         return;
     }
@@ -2670,7 +2705,7 @@ void ens_class_conv(mlb_ensemble* e, EnsClass& c, const float* const s[3], cudaS
         const long long o = c.base + r * n;
         const void* cs[3] = {s[0] + o, s[1] + o, s[2] + o};
         void* ch[3] = {e->H[0] + o, e->H[1] + o, e->H[2] + o};
-        CK(mlb::launch_conv(k, P.L[0], P.L[1], P.L[2], P.tw.p, cs, P.spec.p, P.ten6.p, P.ten9.p, ch, 4, st));
+        launch_field(P, k, cs, P.spec.p, ch, st);
     }
 }
 
@@ -2923,7 +2958,7 @@ void ens_prepare(mlb_ensemble* e)
             build_plan(k.dip, e->st, 4);
             ConvPlan& P = *k.dip->plan;
             k.fast = mlb::conv_fast_ok(P.k) && !P.k.split;
-            P.k.g = c.g / ((double)P.k.Px * P.k.Py * P.k.Pz);
+            P.k.g = c.g / ((double)P.k.Px * P.k.Py * (P.k.mx ? 1 : P.k.Pz));
             P.k.nrep = k.fast ? k.nrep : 1;
             P.spec.alloc((size_t)P.k.Kx * 3 * k.nz * k.ny * P.k.nrep * sizeof(float2));
         }
@@ -2986,6 +3021,7 @@ int mlb_init(int device)
         CK(mlb::conv_configure());
         CK(mlb::fftreg_init());
         CK(mlb::conv_fast_configure());
+        CK(mlb::mx_configure());
         CK(mlb::sur_configure());
     });
 }
@@ -5852,15 +5888,9 @@ bool sur_hook(mlb_op* op, mlb_system* s, Slot& sl)
     if (!s->capturing) P.spec_token = 0;
     ConvK kk = P.k;
     kk.run_if = &d->exact;
-    if (mlb::conv_fast_ok(kk)) {
-        CK(mlb::launch_conv_fast(kk, P.L, reinterpret_cast<const float2*>(P.tw.p), a,
-                                 reinterpret_cast<float2*>(P.spec.p), reinterpret_cast<const float*>(P.ten6.p), out,
-                                 s->st));
-    } else {
-        const void* av[3] = {a[0], a[1], a[2]};
-        void* ov[3] = {out[0], out[1], out[2]};
-        CK(mlb::launch_conv(kk, P.L[0], P.L[1], P.L[2], P.tw.p, av, P.spec.p, P.ten6.p, P.ten9.p, ov, 4, s->st));
-    }
+    const void* av[3] = {a[0], a[1], a[2]};
+    void* ov[3] = {out[0], out[1], out[2]};
+    launch_field(P, kk, av, P.spec.p, ov, s->st);
     const float* hc[3] = {out[0], out[1], out[2]};
     float* sm[3] = {S->m0[0].p, S->m0[1].p, S->m0[2].p};
     float* sh[3] = {S->h0[0].p, S->h0[1].p, S->h0[2].p};
@@ -6323,18 +6353,10 @@ extern "C" int mlb_dipole_field_noalloc(mlb_op* op, const float* sx, const float
         const ConvPlan& P = *op->plan;
         ConvK k = P.k;
         k.nrep = 1;
-        k.g = op->g * op->gs / ((double)k.Px * k.Py * k.Pz);
-        cudaStream_t st = (cudaStream_t)stream;
-        const float* sp[3] = {sx, sy, sz};
-        float* h[3] = {hx, hy, hz};
-        if (mlb::conv_fast_ok(k)) {
-            CK(mlb::launch_conv_fast(k, P.L, reinterpret_cast<const float2*>(P.tw.p), sp,
-                                     static_cast<float2*>(scratch), reinterpret_cast<const float*>(P.ten6.p), h, st));
-        } else {
-            const void* spv[3] = {sx, sy, sz};
-            void* hv[3] = {hx, hy, hz};
-            CK(mlb::launch_conv(k, P.L[0], P.L[1], P.L[2], P.tw.p, spv, scratch, P.ten6.p, P.ten9.p, hv, 4, st));
-        }
+        k.g = conv_scale(op, k);
+        const void* spv[3] = {sx, sy, sz};
+        void* hv[3] = {hx, hy, hz};
+        launch_field(P, k, spv, scratch, hv, (cudaStream_t)stream);
     });
 }
 

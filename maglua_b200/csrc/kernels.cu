@@ -1499,10 +1499,10 @@ cudaError_t launch_tensor_open(int nx, int ny, int nz, const double ABC[9], int 
 }
 
 cudaError_t launch_fft3d_d(double2* W, int ncomp, int Px, int Py, int Pz, const FftLen L[3],
-                           const double2* tw, int sign, cudaStream_t st)
+                           const double2* tw, int sign, int ax0, int ax1, cudaStream_t st)
 {
     const int P[3] = {Px, Py, Pz};
-    for (int ax = 0; ax < 3; ax++) {
+    for (int ax = ax0; ax < ax1; ax++) {
         if (P[ax] == 1) continue;
         const long long nlines = (long long)Px * Py * Pz / P[ax];
         dim3 g((unsigned)nlines, ncomp);

@@ -121,6 +121,7 @@ struct ConvK {
     int general;             // 0: 6 real tensor entries per k, 1: 9 complex
     double g;                // strength * global_scale / (Px*Py*Pz)
     int fx, fy, fz;          // FftLen indices
+    int mx = 0;              // 1: the any-length passes of mx.cu with the layer tensor T(kx, ky, dz)
     int nrep;                // replicas of this size packed back to back (1 for a system)
     const int* run_if;       // when set, the passes run only while *run_if != 0
     int yz_variant = 0;      // (y,z) pass of the fast path: 0 automatic, 1 shared-memory Stockham, 2 register
@@ -141,6 +142,37 @@ struct ConvK {
     // wait, tl[1] = last CTA finished; the fused x pass tl[2], tl[3]
     // (%globaltimer, ns)
     unsigned long long* tl = nullptr;
+};
+
+// Lattice edges of any length (mx.cu): the Stockham stages of one axis, a
+// radix-R butterfly each (nb per line; Ns points already combined; twiddle
+// step tws; mnb, mNs the multipliers of the divisions by nb and Ns).
+#define MX_MAX_STAGES 10
+struct MxStage {
+    int R, nb, Ns, tws;
+    unsigned mnb, mNs;
+};
+struct MxAxis {
+    int n, LS, nst;          // points, line stride in shared memory, stages
+    MxStage s[MX_MAX_STAGES];
+};
+struct MxX {
+    int nx, ny, nz, nr, Kx;  // nr = nz ny rows
+    int rows, r2sh;          // rows per CTA, log2(rows / 2)
+    unsigned m3r2, mPx, mnx; // divisions by 3 rows / 2, Px, nx
+    const int* run_if;
+    MxAxis ax;
+};
+struct MxYZ {
+    int ny, nz, threads;
+    unsigned mPy, mny;
+    double g;
+    const int* run_if;
+    MxAxis ax;
+};
+struct MxPlan {
+    MxX x;
+    MxYZ yz;
 };
 
 // LongRange2D layer scales (spinoperationlongrange2d.cpp:430-530): the

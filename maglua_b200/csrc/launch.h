@@ -132,6 +132,18 @@ cudaError_t conv_configure();
 cudaError_t launch_conv(const ConvK& c, const FftLen& Lx, const FftLen& Ly, const FftLen& Lz, const void* tw,
                         const void* const s[3], void* spec, const void* ten6, const void* ten9, void* const h[3],
                         int rb, cudaStream_t st);
+// Any-length passes (mx.cu): the plan of a convolution (false: not a size or
+// tensor they take), the bytes of its layer tensor, its packing from the
+// six components transformed over x and y (stat2: largest |W| and largest
+// deviation from the parities, as double bits; zero them first), and the
+// forward x (fx), (y,z) and inverse x (ix) passes.
+bool mx_plan(const ConvK& c, int rb, MxPlan& p);
+size_t mx_tensor_bytes(const ConvK& c, int rb);
+cudaError_t launch_mx_pack(const double2* W, const ConvK& c, void* tz, unsigned long long* stat2, int rb,
+                           cudaStream_t st);
+cudaError_t launch_mx_conv(const ConvK& c, const MxPlan& p, const FftLen L[3], const void* tw, const void* const s[3],
+                           void* spec, const void* tz, void* const h[3], bool fx, bool ix, int rb, cudaStream_t st);
+cudaError_t mx_configure();
 cudaError_t launch_tensor_lattice(int nx, int ny, int nz, const int gmax[4], const double ABC[9], int Px,
                                   int Py, int Pz, int zsign, double2* W, cudaStream_t st);
 cudaError_t launch_tensor_rings(int nx, int ny, int nz, int nrings, int lstep, const double ABC[9], int Px, int Py,
@@ -149,8 +161,9 @@ cudaError_t launch_lr2d(const ConvK& c, const FftLen L[3], const void* tw, const
                         const void* Q, const LR2DScale& sc, void* const h[3], int rb, cudaStream_t st);
 cudaError_t launch_lr2d_pack(const double2* W, int nx, int ny, int nz, int p0, int np, void* Q, int rb,
                              cudaStream_t st);
+// FP64 transforms along axes ax0 .. ax1 - 1
 cudaError_t launch_fft3d_d(double2* W, int ncomp, int Px, int Py, int Pz, const FftLen L[3],
-                           const double2* tw, int sign, cudaStream_t st);
+                           const double2* tw, int sign, int ax0, int ax1, cudaStream_t st);
 // Parity check of the FP64 transformed six-component tensor (out3: max |W|,
 // largest ky- and kz-parity deviations, as double bits; zero them first)
 // and the FP32 quarter tensor of the split passes (ConvK::quarter).

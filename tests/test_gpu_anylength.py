@@ -1,0 +1,62 @@
+"""Dipole field on lattices whose edges are not powers of two (and of FP64
+state), against the oracle's lattice sum: every butterfly radix the transforms
+use, single rows and columns, odd row counts, one layer to more than are
+unrolled, and a unit cell without the tensor parities the layer sum needs.
+
+Tolerances: a transform of N points loses about log2(N) rounding errors of
+its precision, so fields agree to well within 1e-5 (FP32, unit roundoff
+6e-8) and 1e-11 (FP64) of their norm."""
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import random_spins, rel_err
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"f32": 1e-5, "f64": 1e-11}
+
+
+@pytest.fixture(scope="module")
+def M():
+    import maglua_b200 as M
+    M.init(0)
+    return M
+
+
+def _compare(M, dims, precision, trunc=12, cell=None):
+    n = int(np.prod(dims))
+    s = random_spins(n, 91, lengths=True)
+    ss = M.SpinSystem(*dims, precision=precision)
+    ss.setSpinArrays(*s)
+    dip = M.Dipole(ss)
+    dip.setStrength(0.3)
+    dip.setTruncation(trunc)
+    kw = {}
+    if cell is not None:
+        dip.setUnitCell(cell[0:3], cell[3:6], cell[6:9])
+        kw["ABC"] = cell
+    dip.apply(ss)
+    h = np.stack(ss.fieldArrays("Dipole"))
+    o = O.SpinSystem(*dims)
+    o.set_spins(*s)
+    O.LongRange(*dims, O.dipole_tensor(*dims, gmax=(trunc,) * 4, **kw)).apply(o, 0.3)
+    assert rel_err(h, o.field("Dipole")) <= TOL[precision]
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("dims", [(9, 10, 1), (11, 13, 2), (17, 19, 3), (23, 29, 1), (31, 62, 2), (30, 25, 4),
+                                  (84, 45, 5), (36, 14, 6), (49, 22, 7), (200, 26, 8), (12, 10, 9), (6, 15, 33),
+                                  (2, 3, 2), (1, 6, 2), (6, 1, 1), (1, 1, 3), (5, 241 - 1, 1)])
+def test_periodic_field(M, dims, precision):
+    _compare(M, dims, precision)
+
+
+@pytest.mark.parametrize("dims", [(32, 32, 1), (64, 128, 4), (256, 16, 8)])
+def test_periodic_field_powers_of_two_fp64(M, dims):
+    _compare(M, dims, "f64")
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_sheared_cell_keeps_the_full_tensor(M, precision):
+    _compare(M, (12, 10, 3), precision, cell=(1, 0, 0, 0.3, 1, 0, 0.2, 0.1, 1))
