@@ -166,7 +166,8 @@ struct ConvPlan {
     DBuf<char> ten6;     // TEN6[kx][kz][ky][6] (real)
     DBuf<char> ten9;     // TEN9[kx][kz][ky][9] (complex)
     DBuf<char> spec2;    // split passes: S2[kx][ky][c][z] (complex)
-    MxPlan mx;           // any-length passes (k.mx): ten6 then holds TZ[kx][dz][6][ky]
+    MxPlan mx{};         // any-length passes (k.mx): ten6 then holds TZ[kx][dz][6][ky]
+    DBuf<int> at;        // their tables: places of the x, then of the y frequencies
     double max_imag = 0; // largest |Im| of the FP64 tensor transform (6-component)
     int device = -1;     // CUDA device the arrays above live on
     // SPEC holds the forward x transform of the spins of the system whose
@@ -1044,12 +1045,17 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
     // edges of any length: x and y transforms, the layer tensor if it has the
     // parities the layer sum relies on (to 1e-10 of its largest element)
     CK(mlb::launch_fft3d_d(W.p, ncomp, Px, Py, Pz, P->L, twdd.p, -1, 0, 2, st));
-    if (!(rb == 4 && mlb::conv_fast_ok(k)) && mlb::mx_plan(k, rb, P->mx)) {
+    std::vector<int> at, at_y;
+    if (!(rb == 4 && mlb::conv_fast_ok(k)) && mlb::mx_plan(k, rb, P->mx, at, at_y)) {
+        at.insert(at.end(), at_y.begin(), at_y.end());
+        P->at.alloc(at.size());
+        CK(cudaMemcpy(P->at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice));
+        P->mx.x.at = P->at.p;
         DBuf<unsigned long long> stat;
         stat.alloc(2);
         CK(cudaMemsetAsync(stat.p, 0, 2 * sizeof(unsigned long long), st));
         P->ten6.alloc(mlb::mx_tensor_bytes(k, rb));
-        CK(mlb::launch_mx_pack(W.p, k, P->ten6.p, stat.p, rb, st));
+        CK(mlb::launch_mx_pack(W.p, k, P->at.p + Px, P->ten6.p, stat.p, rb, st));
         double hs[2];
         CK(cudaMemcpyAsync(hs, stat.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -1622,6 +1628,10 @@ void flush_pending(mlb_system* s)
     s->pend_op = nullptr;
     s->pend_si = -1;
     ConvPlan& P = *op->plan;
+    if (P.k.mx) {
+        CK(mlb::launch_mx_ix(P.mx.x, P.L, P.tw.p, P.spec.p, sl.h, P.rb, s->st));
+        return;
+    }
     float* h[3] = {static_cast<float*>(sl.h[0]), static_cast<float*>(sl.h[1]), static_cast<float*>(sl.h[2])};
     CK(mlb::launch_conv_fast_ix(P.k, P.L, reinterpret_cast<const float2*>(P.tw.p), reinterpret_cast<float2*>(P.spec.p),
                                 h, s->st));
@@ -1745,23 +1755,25 @@ void op_apply(mlb_op* op, mlb_system* s)
         if (s->dry) return;
         if (s->sur && sur_hook(op, s, sl)) return;
         const void* spv[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
-        if (!P.k.mx && s->rb == 4 && mlb::conv_fast_ok(P.k)) {
-            const float* sp[3] = {static_cast<const float*>(s->sp[s->cur][0]), static_cast<const float*>(s->sp[s->cur][1]),
-                                  static_cast<const float*>(s->sp[s->cur][2])};
-            if (s->defer_x && P.k.nrep == 1 && !P.k.general) {
-                // forward x pass only when SPEC does not already hold it
-                const bool carry = s->capturing ? s->cap_carry
-                                                : (s->spec_token != 0 && s->spec_token == P.spec_token);
-                ConvK kk = P.k;
-                kk.tl = s->capturing ? s->cap_tl : nullptr;
+        if (s->defer_x && P.k.nrep == 1 && !P.k.general && (P.k.mx || (s->rb == 4 && mlb::conv_fast_ok(P.k)))) {
+            // forward x pass only when SPEC does not already hold it
+            const bool carry = s->capturing ? s->cap_carry : (s->spec_token != 0 && s->spec_token == P.spec_token);
+            ConvK kk = P.k;
+            kk.tl = s->capturing ? s->cap_tl : nullptr;
+            if (P.k.mx) {
+                CK(mlb::launch_mx_conv(kk, P.mx, P.L, P.tw.p, spv, P.spec.p, P.ten6.p, sl.h, !carry, false, s->rb,
+                                       s->st));
+            } else {
+                const float* sp[3] = {static_cast<const float*>(spv[0]), static_cast<const float*>(spv[1]),
+                                      static_cast<const float*>(spv[2])};
                 CK(mlb::launch_conv_fast_fyz(kk, P.L, reinterpret_cast<const float2*>(P.tw.p), sp,
                                              reinterpret_cast<float2*>(P.spec.p),
                                              reinterpret_cast<const float*>(P.ten6.p), !carry, s->st));
-                if (!s->capturing) P.spec_token = 0;
-                s->pend_op = op;
-                s->pend_si = si;
-                return;
             }
+            if (!s->capturing) P.spec_token = 0;
+            s->pend_op = op;
+            s->pend_si = si;
+            return;
         }
         if (!s->capturing) P.spec_token = 0;
         launch_field(P, P.k, spv, P.spec.p, sl.h, s->st);
@@ -1854,6 +1866,59 @@ bool fast_fused(mlb_system* s, const TermsK& T, const mlb_llg* l, double dt, dou
     return fast_fused_t<float>(s, T, l, dt, dt_sys, F);
 }
 
+cudaError_t launch_fused_uniform(const FastKT<float>& F, const float* s[3], const float* a[3], float* o[3],
+                                 cudaStream_t st)
+{
+    return mlb::launch_fused_fast(F, s, a, o, st);
+}
+cudaError_t launch_fused_uniform(const FastKT<double>& F, const double* s[3], const double* a[3], double* o[3],
+                                 cudaStream_t st)
+{
+    return mlb::launch_fused_fast_f64(F, s, a, o, st);
+}
+
+// A step with uniform parameters into spin buffer nb: with a deferred
+// convolution CP, fused with its x passes (power-of-two FP32 lines of 32 to
+// 512 points: k_xstep; else the any-length kernel), else on its own.
+template <typename R, class Take>
+void fast_step(mlb_system* s, int nb, const TermsK& T, FastKT<R>& F, ConvPlan* CP, DevStep* cur, DevStep* next,
+               Take&& take_pending)
+{
+    const R* sp[3];
+    const R* ad[3] = {nullptr, nullptr, nullptr};
+    R* out[3];
+    for (int c = 0; c < 3; c++) {
+        sp[c] = static_cast<const R*>(s->sp[s->cur][c]);
+        out[c] = static_cast<R*>(s->sp[nb][c]);
+        if (T.nadd == 1) ad[c] = static_cast<const R*>(T.add[0][c]);
+    }
+    if constexpr (sizeof(R) == 4) {
+        if (CP && !CP->k.mx && mlb::xstep_ok(CP->k, F)) {
+            void* hv[3];
+            take_pending(hv);
+            float* h[3] = {static_cast<float*>(hv[0]), static_cast<float*>(hv[1]), static_cast<float*>(hv[2])};
+            ConvK kx = CP->k;
+            kx.tl = s->capturing ? s->cap_tl : nullptr;
+            F.adv_cur = cur;
+            F.adv_next = next;
+            CK(mlb::launch_xstep(kx, CP->L, reinterpret_cast<const float2*>(CP->tw.p),
+                                 reinterpret_cast<float2*>(CP->spec.p), F, true, sp, h, out, s->st));
+            return;
+        }
+    }
+    if (CP && CP->k.mx) {
+        void* hv[3];
+        take_pending(hv);
+        R* h[3] = {static_cast<R*>(hv[0]), static_cast<R*>(hv[1]), static_cast<R*>(hv[2])};
+        F.adv_cur = cur;
+        F.adv_next = next;
+        CK(mlb::launch_mx_step<R>(CP->mx.x, CP->L, CP->tw.p, CP->spec.p, F, sp, h, out, s->st));
+        return;
+    }
+    flush_pending(s);
+    CK(launch_fused_uniform(F, sp, ad, out, s->st));
+}
+
 // Fused in-place step when Total is lazily defined; returns false when the
 // caller must take the general path.
 bool llg_fused(mlb_llg* l, mlb_system* s, double dt)
@@ -1892,65 +1957,56 @@ bool llg_fused(mlb_llg* l, mlb_system* s, double dt)
     FastKT<double> Fd;
     bool carried = false;   // SPEC ends holding the new spins' x transform
     bool advanced = false;  // a kernel of the step wrote the next step's block
+    // a deferred convolution whose field is the last addend: its inverse x
+    // pass runs in the step's kernel
+    ConvPlan* CP = s->pend_op && T.nadd > 0 && T.add[T.nadd - 1][0] == s->slots[s->pend_si].h[0] &&
+                           !T.add_is_thermal[T.nadd - 1]
+                       ? s->pend_op->plan.get()
+                       : nullptr;
+    DevStep* cur = s->capturing ? s->dstep + s->cur : nullptr;
+    DevStep* next = s->capturing ? s->dstep + (1 - s->cur) : nullptr;
+    auto take_pending = [&](void* h[3]) {
+        for (int c = 0; c < 3; c++) h[c] = s->slots[s->pend_si].h[c];
+        carried = true;
+        advanced = s->capturing;
+        if (s->capturing) {
+            s->cap_xstep = s->pend_op;
+        } else {
+            CP->spec_token = ++g_spec_token;
+            s->spec_token = CP->spec_token;
+        }
+        s->pend_op = nullptr;
+        s->pend_si = -1;
+    };
     if (s->dry) {
         // bookkeeping only: the kernels of this step ran in a captured graph
     } else if (fast_fused(s, T, l, dt, dt_sys, F)) {
-        const float* sp[3];
-        const float* ad[3] = {nullptr, nullptr, nullptr};
-        float* out[3];
-        for (int c = 0; c < 3; c++) {
-            sp[c] = static_cast<const float*>(s->sp[s->cur][c]);
-            out[c] = static_cast<float*>(s->sp[nb][c]);
-            if (T.nadd == 1) ad[c] = static_cast<const float*>(T.add[0][c]);
-        }
-        ConvPlan* CP = s->pend_op ? s->pend_op->plan.get() : nullptr;
-        mlb_op* pend_op_was = s->pend_op;
-        if (CP && T.nadd == 1 && T.add[0][0] == s->slots[s->pend_si].h[0] && mlb::xstep_ok(CP->k, F)) {
-            float* h[3] = {static_cast<float*>(s->slots[s->pend_si].h[0]),
-                           static_cast<float*>(s->slots[s->pend_si].h[1]),
-                           static_cast<float*>(s->slots[s->pend_si].h[2])};
-            s->pend_op = nullptr;
-            s->pend_si = -1;
-            ConvK kx = CP->k;
-            kx.tl = s->capturing ? s->cap_tl : nullptr;
-            if (s->capturing) {
-                F.adv_cur = s->dstep + s->cur;
-                F.adv_next = s->dstep + (1 - s->cur);
-                advanced = true;
-            }
-            CK(mlb::launch_xstep(kx, CP->L, reinterpret_cast<const float2*>(CP->tw.p),
-                                 reinterpret_cast<float2*>(CP->spec.p), F, true, sp, h, out, s->st));
-            carried = true;
-            if (s->capturing) {
-                s->cap_xstep = pend_op_was;
-            } else {
-                CP->spec_token = ++g_spec_token;
-                s->spec_token = CP->spec_token;
-            }
-        } else {
-            flush_pending(s);
-            CK(mlb::launch_fused_fast(F, sp, ad, out, s->st));
-        }
+        fast_step<float>(s, nb, T, F, CP, cur, next, take_pending);
     } else if (s->rb == 8 && fast_fused_t<double>(s, T, l, dt, dt_sys, Fd)) {
-        // FP64 state with uniform parameters: the fast kernel in double
-        flush_pending(s);
-        const double* sp[3];
-        const double* ad[3] = {nullptr, nullptr, nullptr};
-        double* out[3];
-        for (int c = 0; c < 3; c++) {
-            sp[c] = static_cast<const double*>(s->sp[s->cur][c]);
-            out[c] = static_cast<double*>(s->sp[nb][c]);
-            if (T.nadd == 1) ad[c] = static_cast<const double*>(T.add[0][c]);
-        }
-        CK(mlb::launch_fused_fast_f64(Fd, sp, ad, out, s->st));
+        // FP64 state with uniform parameters: the fast kernels in double
+        fast_step<double>(s, nb, T, Fd, CP, cur, next, take_pending);
     } else {
-        flush_pending(s);
         FusedK P;
         P.sys = sysk(s, s->cur);
         P.terms = T;
         P.llg = llgk(l, dt, s->status);
         P.ox = s->sp[nb][0]; P.oy = s->sp[nb][1]; P.oz = s->sp[nb][2];
-        CK(mlb::launch_fused(P, dt_sys, s->rb, s->st));
+        if (CP && (CP->k.mx || mlb::xgstep_ok(CP->k))) {
+            void* h[3];
+            take_pending(h);
+            P.terms.nadd--;
+            const double w = T.addw[T.nadd - 1];
+            if (CP->k.mx) {
+                CK(mlb::launch_mx_gstep(CP->mx.x, CP->L, CP->tw.p, CP->spec.p, P, w, dt_sys, cur, next, h, s->rb, s->st));
+            } else {
+                float* hf[3] = {static_cast<float*>(h[0]), static_cast<float*>(h[1]), static_cast<float*>(h[2])};
+                CK(mlb::launch_xgstep(CP->k, CP->L, reinterpret_cast<const float2*>(CP->tw.p),
+                                      reinterpret_cast<float2*>(CP->spec.p), P, w, dt_sys, cur, next, hf, s->st));
+            }
+        } else {
+            flush_pending(s);
+            CK(mlb::launch_fused(P, dt_sys, s->rb, s->st));
+        }
     }
     if (s->capturing && !advanced) CK(mlb::launch_advance_step(s->dstep + s->cur, s->dstep + (1 - s->cur), s->st));
     if (!carried && !s->capturing && !s->dry) s->spec_token = 0;

@@ -16,6 +16,7 @@
 #include "fused.cuh"
 #include "kparams.h"
 #include "launch.h"
+#include "terms.cuh"
 
 #include <cuda_runtime.h>
 #include <math.h>
@@ -1047,17 +1048,20 @@ __global__ void __launch_bounds__(256) k_fused_fast(FastKT<R> F0, const R* __res
 // The spectrum rows a CTA reads in 1 and writes in 3 are its own.  Every
 // arithmetic step repeats k_ix_fast, fused_site and k_fx_fast operation for
 // operation, so the result is bitwise that of the three separate kernels.
-// 32- to 256-point lines (register transforms, a line per T-lane group)
-// take 512 threads: the transforms occupy the same L T lanes, and the site
-// step has two items per thread (384 threads left a third of them idle in
-// the last of three rounds); two CTAs per SM at 64 registers.  512-point
-// lines (shared-memory Stockham, TPL threads per line) take 384.
-template <int PX, bool TH = false>
+// SZ: the CTA's share.  0: 2048 sites (512-point lines 4096) on 512 threads
+// (384 for the shared-memory Stockham lines of 512 points), two CTAs per SM at
+// 64 registers, for lattices that fill the chip with such CTAs; 1: 512 sites on
+// 256 threads, 2: 128 sites on 128 threads (two rows at least), for smaller
+// ones (xs_size): a lattice of 128 x 128 x 4 is 32 CTAs of share 0, and the
+// step is one CTA's chain.  Lines are transformed alike at every share, so
+// results do not depend on it.
+template <int PX, bool TH = false, int SZ = 0>
 struct XSCfg {
-    static constexpr int NT = XReg<PX>::OK ? 512 : 384;
+    static constexpr int NT = SZ == 0 ? (XReg<PX>::OK ? 512 : 384) : (SZ == 1 ? 256 : 128);
     static constexpr int TPL = fr::Tpl<PX>::V;
-    static constexpr int L = 384 / TPL;                 // complex lines = 3 ROWS / 2
-    static constexpr int ROWS = 2 * L / 3;
+    static constexpr int SMALL = (SZ == 1 ? 512 : 128) / PX;
+    static constexpr int ROWS = SZ == 0 ? 2 * (384 / TPL) / 3 : (SMALL < 2 ? 2 : SMALL);
+    static constexpr int L = 3 * ROWS / 2;              // complex lines
     static constexpr int R2 = ROWS / 2;
     static constexpr int KX = PX / 2 + 1;
     // line stride in shared memory: one complex past the line, so that the
@@ -1073,26 +1077,33 @@ struct XSCfg {
     // 32- to 256-point lines: register four-step transforms, one exchange buffer per line
     static constexpr int EX = XReg<PX>::OK ? L * XReg<PX>::EX : 0;
     static constexpr int SMEM = (PX + 2 * BUF + EX) * 8 + NOISE * 4;
-    static_assert(L % 3 == 0 && ROWS % 2 == 0, "line layout");
-    static_assert(XReg<PX>::OK ? L * XReg<PX>::T <= NT : L * TPL == NT, "lines per CTA");
+    static_assert(ROWS % 2 == 0, "line layout");
+    static_assert(XReg<PX>::OK ? L * XReg<PX>::T <= NT : L * TPL <= NT, "lines per CTA");
+    // CTAs per SM: 64 registers per thread; the general form's 96 or so
+    static constexpr int OCC = SZ == 0 ? 2 : (SZ == 1 ? 4 : 8);
+    static constexpr int GOCC = SZ == 0 ? 1 : (SZ == 1 ? 2 : 4);
 };
 
-template <int PX, int LT, bool EXS, bool ANI, bool TH>
-__global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F0, int fwd, const float2* __restrict__ tw,
-                                                  float2* __restrict__ spec, const float* __restrict__ sx,
-                                                  const float* __restrict__ sy, const float* __restrict__ sz,
-                                                  float* __restrict__ hx, float* __restrict__ hy,
-                                                  float* __restrict__ hz, float* __restrict__ ox,
-                                                  float* __restrict__ oy, float* __restrict__ oz)
+// The body of the fused x pass: begin() runs once the previous kernel's
+// writes are visible, pre(row, x, i) is called for every site of the
+// CTA while the spectrum loads are in flight, site(i, row, x, y, z, A) gives
+// the new spin of site i in the dipole field A.
+template <int PX, bool TH, int SZ, int HU, class Begin, class Pre, class Site>
+__device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cur, DevStep* adv_next, int fwd,
+                                           const float2* __restrict__ tw, float2* __restrict__ spec,
+                                           const float* __restrict__ sx, const float* __restrict__ sy,
+                                           const float* __restrict__ sz, float* __restrict__ hx,
+                                           float* __restrict__ hy, float* __restrict__ hz, float* __restrict__ ox,
+                                           float* __restrict__ oy, float* __restrict__ oz, Begin&& begin, Pre&& pre,
+                                           Site&& site)
 {
-    using X = XSCfg<PX, TH>;
+    using X = XSCfg<PX, TH, SZ>;
     constexpr int KX = X::KX, NT = X::NT, ROWS = X::ROWS, R2 = X::R2, LS = X::LS;
     extern __shared__ float2 sm[];
     float2* twl = sm;               // [PX]
     float2* A = twl + PX;           // [L][LS] lines
     float2* B = A + X::BUF;         // [L][LS] scratch
     float2* EXB = B + X::BUF;       // [L][XReg<PX>::EX] exchange buffers (XReg<PX>::OK)
-    float* noise = reinterpret_cast<float*>(EXB + X::EX);   // [3][ROWS][PX] (X::PRE)
     const int nx = c.nx, ny = c.ny, nz = c.nz;
     const int nr = nz * ny;                     // rows (z, y), flattened
     const int row0 = blockIdx.x * ROWS;
@@ -1104,9 +1115,9 @@ __global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F
     tl_start(tls);
     // captured steps: the next step's block (the other of the pair; no
     // kernel of this step reads it)
-    if (F0.adv_next && blockIdx.x == 0 && threadIdx.x == 0) {
-        const DevStep* cu = F0.adv_cur;
-        DevStep* nx_ = F0.adv_next;
+    if (adv_next && blockIdx.x == 0 && threadIdx.x == 0) {
+        const DevStep* cu = adv_cur;
+        DevStep* nx_ = adv_next;
         nx_->th_counter = cu->th_counter + 1ull;
         for (int a = 0; a < 3; a++) {
             nx_->B[a] = cu->B[a] + cu->dB[a];
@@ -1127,7 +1138,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F
                 asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
         }
     }
-    const FastK F = fastk_resolved(F0);
+    begin();
     // 1. line l = comp R2 + p: Z[k] = S_row(2p)[k] + i S_row(2p+1)[k] for
     // k < KX, Hermitian completion Z[PX - k] from the conjugates; one item
     // per (kx, comp, p), the row pair's two spectrum values (adjacent in
@@ -1166,11 +1177,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int row = 2 * p + h;
-                    if (row < rows_here && x < nx) {
-                        const float3 g = thermal_normal3(F, (row0 + row) * nx + x);
-                        float* q = noise + row * PX + x;
-                        q[0] = g.x; q[ROWS * PX] = g.y; q[2 * ROWS * PX] = g.z;
-                    }
+                    if (row < rows_here && x < nx) pre(row, x, (row0 + row) * nx + x);
                 }
             }
         }
@@ -1195,7 +1202,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F
         xreg_lines<PX, +1>(A, LS, X::L, EXB, twl);
         R = A;
     } else {
-        R = fr::sm_fft<PX, +1, X::TPL, float2, LS>(A, B, l, tl, twl, true);
+        R = fr::sm_fft<PX, +1, X::TPL, float2, LS>(A, B, l, tl, twl, l < X::L);
     }
     float2* W = (R == A) ? B : A;   // free buffer: the new spins' lines (FWD)
     // 2. field of the rows to the slot, then the step of every site: one
@@ -1212,7 +1219,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F
         const int p = idx / PX, x = idx % PX;
         const float2 Ax2 = R[(0 * R2 + p) * LS + x], Ay2 = R[(1 * R2 + p) * LS + x], Az2 = R[(2 * R2 + p) * LS + x];
         float2 o0 = make_float2(0.f, 0.f), o1 = o0, o2 = o0;
-#pragma unroll
+#pragma unroll HU
         for (int h = 0; h < 2; h++) {
             const int row = 2 * p + h;
             if (row < rows_here && x < nx) {
@@ -1223,13 +1230,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F
                 const size_t i = (size_t)r * nx + x;
                 hx[i] = Ax; hy[i] = Ay; hz[i] = Az;
                 float rx, ry, rz;
-                float3 g;
-                if (X::PRE) {
-                    const float* q = noise + row * PX + x;
-                    g = make_float3(q[0], q[ROWS * PX], q[2 * ROWS * PX]);
-                }
-                fused_site_v<LT, EXS, ANI, TH, true>(F, nx, ny, nz, x, y, zz, (int)i, sx, sy, sz, Ax, Ay, Az, rx, ry,
-                                                     rz, X::PRE ? &g : nullptr);
+                site((int)i, row, x, y, zz, Ax, Ay, Az, rx, ry, rz);
                 ox[i] = rx; oy[i] = ry; oz[i] = rz;
                 if (h) { o0.y = rx; o1.y = ry; o2.y = rz; }
                 else { o0.x = rx; o1.x = ry; o2.x = rz; }
@@ -1248,7 +1249,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F
         xreg_lines<PX, -1>(W, LS, X::L, EXB, twl);
         Q = W;
     } else {
-        Q = fr::sm_fft<PX, -1, X::TPL, float2, LS>(W, const_cast<float2*>(R), l, tl, twl, true);
+        Q = fr::sm_fft<PX, -1, X::TPL, float2, LS>(W, const_cast<float2*>(R), l, tl, twl, l < X::L);
     }
     constexpr int IQ = (X::SPEC + NT - 1) / NT;
 #pragma unroll
@@ -1265,6 +1266,65 @@ __global__ void __launch_bounds__(XSCfg<PX, TH>::NT, 2) k_xstep(ConvK c, FastK F
         spec[((size_t)kx * 3 + comp) * nr + row0 + row] = o;
     }
     tl_end(tls);
+}
+
+template <int PX, int LT, bool EXS, bool ANI, bool TH, int SZ>
+__global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC) k_xstep(ConvK c, FastK F0, int fwd, const float2* __restrict__ tw,
+                                                  float2* __restrict__ spec, const float* __restrict__ sx,
+                                                  const float* __restrict__ sy, const float* __restrict__ sz,
+                                                  float* __restrict__ hx, float* __restrict__ hy,
+                                                  float* __restrict__ hz, float* __restrict__ ox,
+                                                  float* __restrict__ oy, float* __restrict__ oz)
+{
+    using X = XSCfg<PX, TH, SZ>;
+    constexpr int NP = X::ROWS * PX;
+    extern __shared__ float2 sm[];
+    float* noise = reinterpret_cast<float*>(sm + PX + 2 * X::BUF + X::EX);   // [3][ROWS][PX] (X::PRE)
+    // the step block's values are the previous kernel's: resolved after the wait
+    FastK F;
+    xstep_body<PX, TH, SZ, 2>(
+        c, F0.adv_cur, F0.adv_next, fwd, tw, spec, sx, sy, sz, hx, hy, hz, ox, oy, oz, [&] { F = fastk_resolved(F0); },
+        [&](int row, int x, int i) {
+            const float3 g = thermal_normal3(F, i);
+            float* q = noise + row * PX + x;
+            q[0] = g.x; q[NP] = g.y; q[2 * NP] = g.z;
+        },
+        [&](int i, int row, int x, int y, int z, float Ax, float Ay, float Az, float& rx, float& ry, float& rz) {
+            float3 g;
+            if (X::PRE) {
+                const float* q = noise + row * PX + x;
+                g = make_float3(q[0], q[NP], q[2 * NP]);
+            }
+            fused_site_v<LT, EXS, ANI, TH, true>(F, c.nx, c.ny, c.nz, x, y, z, i, sx, sy, sz, Ax, Ay, Az, rx, ry, rz,
+                                                 X::PRE ? &g : nullptr);
+        });
+}
+
+// The same pass for per-site parameters, pathway lists and further addends
+// (FusedK): P.terms without the dipole addend, whose weight is addw.  Every
+// site step repeats k_fused_step's arithmetic, so fused and separate steps
+// agree bit for bit.
+template <int PX, int SZ>
+__global__ void __launch_bounds__(XSCfg<PX, false, SZ>::NT, XSCfg<PX, false, SZ>::GOCC) k_xgstep(ConvK c, const __grid_constant__ FusedK P, double addw,
+                                                            double dt_sys, const DevStep* cur, DevStep* next,
+                                                            const float2* __restrict__ tw, float2* __restrict__ spec,
+                                                            float* __restrict__ hx, float* __restrict__ hy,
+                                                            float* __restrict__ hz)
+{
+    xstep_body<PX, false, SZ, 1>(
+        c, cur, next, 1, tw, spec, static_cast<const float*>(P.sys.x), static_cast<const float*>(P.sys.y),
+        static_cast<const float*>(P.sys.z), hx, hy, hz, static_cast<float*>(P.ox), static_cast<float*>(P.oy),
+        static_cast<float*>(P.oz), [] {}, [](int, int, int) {},
+        [&](int i, int, int, int, int, float Ax, float Ay, float Az, float& rx, float& ry, float& rz) {
+            const float ms = ms_at<float>(P.sys, i);
+            Fields<float> F;
+            if (ms > 0.f) {
+                F = eval_terms<float>(P.terms, P.sys, (float)dt_sys, i);
+                F.H = fma3((float)addw, v3<float>(Ax, Ay, Az), F.H);
+            }
+            const V3<float> o = step_site<float>(P, F, spin_at<float>(P.sys, i), ms, i);
+            rx = o.x; ry = o.y; rz = o.z;
+        });
 }
 
 // Packed ensemble: tile b covers sites [bstart[b], bstart[b] + blockDim) of
@@ -1706,14 +1766,37 @@ bool xstep_ok(const ConvK& c, const FastK& F)
     return c.nrep == 1 && F.ex && (c.Px == 32 || c.Px == 64 || c.Px == 128 || c.Px == 256 || c.Px == 512);
 }
 
+// Share of a CTA (XSCfg): the largest that gives at least about as many CTAs as
+// SMs.  A step alone, share 0 / the one taken: 32x32x1 13.3 / 9.0 us, 64x64x2
+// 15.0 / 9.0, 128x128x4 19.3 / 13.0, 256x256x1 22.9 / 17.1, 64x512x4 25.7 / 20.2,
+// 512x512x1 60.6 / 41.2; 256x256x4 (128 CTAs of share 0) 26.1 at either.
+template <int PX>
+static int xs_size(const ConvK& c)
+{
+    const int nr = c.nz * c.ny;
+    if (nr >= 120 * XSCfg<PX>::ROWS) return 0;
+    if (PX > 128 || nr >= 120 * XSCfg<PX, false, 1>::ROWS) return 1;
+    return 2;
+}
+
+template <int PX, int LT, bool ANI, bool TH, int SZ>
+static cudaError_t xstep_sz(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
+                            const float* s[3], float* h[3], float* o[3], cudaStream_t st)
+{
+    using X = XSCfg<PX, TH, SZ>;
+    dim3 grid((c.nz * c.ny + X::ROWS - 1) / X::ROWS, 1, 1);
+    return launch_pdl(k_xstep<PX, LT, true, ANI, TH, SZ>, grid, dim3(X::NT), (size_t)X::SMEM, st, c, F, fwd, tw, spec,
+                      s[0], s[1], s[2], h[0], h[1], h[2], o[0], o[1], o[2]);
+}
 template <int PX, int LT, bool ANI, bool TH>
 static cudaError_t xstep_t(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
                            const float* s[3], float* h[3], float* o[3], cudaStream_t st)
 {
-    using X = XSCfg<PX, TH>;
-    dim3 grid((c.nz * c.ny + X::ROWS - 1) / X::ROWS, 1, 1);
-    return launch_pdl(k_xstep<PX, LT, true, ANI, TH>, grid, dim3(X::NT), (size_t)X::SMEM, st, c, F, fwd, tw, spec,
-                      s[0], s[1], s[2], h[0], h[1], h[2], o[0], o[1], o[2]);
+    const int sz = xs_size<PX>(c);
+    if (sz == 0) return xstep_sz<PX, LT, ANI, TH, 0>(c, F, fwd, tw, spec, s, h, o, st);
+    if constexpr (PX <= 128)
+        if (sz == 2) return xstep_sz<PX, LT, ANI, TH, 2>(c, F, fwd, tw, spec, s, h, o, st);
+    return xstep_sz<PX, LT, ANI, TH, 1>(c, F, fwd, tw, spec, s, h, o, st);
 }
 template <int PX, int LT>
 static cudaError_t xstep_lt(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
@@ -1749,24 +1832,74 @@ cudaError_t launch_xstep(const ConvK& c, const FftLen L[3], const float2* tw, fl
     return cudaErrorInvalidValue;
 }
 
-template <int PX, int LT, bool ANI, bool TH>
+bool xgstep_ok(const ConvK& c)
+{
+    return c.nrep == 1 && (c.Px == 32 || c.Px == 64 || c.Px == 128 || c.Px == 256 || c.Px == 512);
+}
+
+template <int PX, int SZ>
+static cudaError_t xgstep_sz(const ConvK& c, const FusedK& P, double addw, double dt_sys, const DevStep* cur,
+                             DevStep* next, const float2* tw, float2* spec, float* const h[3], cudaStream_t st)
+{
+    using X = XSCfg<PX, false, SZ>;
+    return launch_pdl(k_xgstep<PX, SZ>, dim3((c.nz * c.ny + X::ROWS - 1) / X::ROWS), dim3(X::NT), (size_t)X::SMEM, st, c,
+                      P, addw, dt_sys, cur, next, tw, spec, h[0], h[1], h[2]);
+}
+template <int PX>
+static cudaError_t xgstep_px(const ConvK& c, const FusedK& P, double addw, double dt_sys, const DevStep* cur,
+                             DevStep* next, const float2* tw, float2* spec, float* const h[3], cudaStream_t st)
+{
+    const int sz = xs_size<PX>(c);
+    if (sz == 0) return xgstep_sz<PX, 0>(c, P, addw, dt_sys, cur, next, tw, spec, h, st);
+    if constexpr (PX <= 128)
+        if (sz == 2) return xgstep_sz<PX, 2>(c, P, addw, dt_sys, cur, next, tw, spec, h, st);
+    return xgstep_sz<PX, 1>(c, P, addw, dt_sys, cur, next, tw, spec, h, st);
+}
+
+cudaError_t launch_xgstep(const ConvK& c, const FftLen L[3], const float2* tw, float2* spec, const FusedK& P,
+                          double addw, double dt_sys, const DevStep* cur, DevStep* next, float* const h[3],
+                          cudaStream_t st)
+{
+    Prof pf("k_xstep", st);
+    const float2* t = tw + L[0].tw_off;
+    switch (c.Px) {
+    case 32: return xgstep_px<32>(c, P, addw, dt_sys, cur, next, t, spec, h, st);
+    case 64: return xgstep_px<64>(c, P, addw, dt_sys, cur, next, t, spec, h, st);
+    case 128: return xgstep_px<128>(c, P, addw, dt_sys, cur, next, t, spec, h, st);
+    case 256: return xgstep_px<256>(c, P, addw, dt_sys, cur, next, t, spec, h, st);
+    case 512: return xgstep_px<512>(c, P, addw, dt_sys, cur, next, t, spec, h, st);
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <int PX, int LT, bool ANI, bool TH, int SZ>
 static cudaError_t cfg_xs1()
 {
-    cudaError_t e = cudaFuncSetAttribute(k_xstep<PX, LT, true, ANI, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         XSCfg<PX, TH>::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(k_xstep<PX, LT, true, ANI, TH, SZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         XSCfg<PX, TH, SZ>::SMEM);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_xstep<PX, LT, true, ANI, TH>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    return cudaFuncSetAttribute(k_xstep<PX, LT, true, ANI, TH, SZ>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 (int)cudaSharedmemCarveoutMaxShared);
+}
+template <int PX, int SZ>
+static cudaError_t cfg_xs_sz()
+{
+    cudaError_t e =
+        cudaFuncSetAttribute(k_xgstep<PX, SZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, XSCfg<PX, false, SZ>::SMEM);
+    if (e != cudaSuccess) return e;
+    if ((e = cfg_xs1<PX, LLG_CART, false, false, SZ>()) || (e = cfg_xs1<PX, LLG_CART, false, true, SZ>()) ||
+        (e = cfg_xs1<PX, LLG_CART, true, false, SZ>()) || (e = cfg_xs1<PX, LLG_CART, true, true, SZ>()) ||
+        (e = cfg_xs1<PX, LLG_QUAT, false, false, SZ>()) || (e = cfg_xs1<PX, LLG_QUAT, false, true, SZ>()) ||
+        (e = cfg_xs1<PX, LLG_QUAT, true, false, SZ>()) || (e = cfg_xs1<PX, LLG_QUAT, true, true, SZ>()))
+        return e;
+    return cudaSuccess;
 }
 template <int PX>
 static cudaError_t cfg_xs()
 {
     cudaError_t e;
-    if ((e = cfg_xs1<PX, LLG_CART, false, false>()) || (e = cfg_xs1<PX, LLG_CART, false, true>()) ||
-        (e = cfg_xs1<PX, LLG_CART, true, false>()) || (e = cfg_xs1<PX, LLG_CART, true, true>()) ||
-        (e = cfg_xs1<PX, LLG_QUAT, false, false>()) || (e = cfg_xs1<PX, LLG_QUAT, false, true>()) ||
-        (e = cfg_xs1<PX, LLG_QUAT, true, false>()) || (e = cfg_xs1<PX, LLG_QUAT, true, true>()))
-        return e;
+    if ((e = cfg_xs_sz<PX, 0>()) != cudaSuccess || (e = cfg_xs_sz<PX, 1>()) != cudaSuccess) return e;
+    if constexpr (PX <= 128) return cfg_xs_sz<PX, 2>();
     return cudaSuccess;
 }
 

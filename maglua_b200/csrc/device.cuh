@@ -99,6 +99,23 @@ __device__ __forceinline__ float3 philox_normal3(uint64_t seed, uint64_t counter
     return make_float3(ra * ca, ra * sa, rb * cb);
 }
 
+// --------------------------------------------------------------- fixed roundings
+// The site arithmetic of a step is compiled into several kernels (separate
+// calls, fused passes) whose results must agree bit for bit, so which products
+// fuse into additions is written out instead of left to the compiler.
+__device__ __forceinline__ float fm(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float ml(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double ml(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float ad(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double ad(double a, double b) { return __dadd_rn(a, b); }
+// a b - c d and a0 b0 + a1 b1 + a2 b2
+template <typename R> __device__ __forceinline__ R crs(R a, R b, R c, R d) { return fm(a, b, -ml(c, d)); }
+template <typename R> __device__ __forceinline__ R dot3(R a0, R b0, R a1, R b1, R a2, R b2)
+{
+    return fm(a0, b0, fm(a1, b1, ml(a2, b2)));
+}
+
 // --------------------------------------------------------------- complex
 template <typename R> struct CT;
 template <> struct CT<float> { typedef float2 T; };

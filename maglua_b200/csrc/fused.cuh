@@ -32,20 +32,22 @@ template <typename R>
 __device__ __forceinline__ void cubic_field(R sx, R sy, R sz, const R* n, const R* K, int quirk, R& hx, R& hy,
                                             R& hz)
 {
-    const R n1s = n[0] * sx + n[1] * sy + n[2] * sz;
-    const R n2s = n[3] * sx + n[4] * sy + n[5] * sz;
-    const R n3s = n[6] * sx + n[7] * sy + n[8] * sz;
-    const R n1s2 = n1s * n1s, n2s2 = n2s * n2s, n3s2 = n3s * n3s;
-    const R n1s3 = n1s2 * n1s, n2s3 = n2s2 * n2s, n3s3 = n3s2 * n3s;
-    const R n1s4 = n1s2 * n1s2, n2s4 = n2s2 * n2s2, n3s4 = n3s2 * n3s2;
+    const R n1s = dot3(n[0], sx, n[1], sy, n[2], sz);
+    const R n2s = dot3(n[3], sx, n[4], sy, n[5], sz);
+    const R n3s = dot3(n[6], sx, n[7], sy, n[8], sz);
+    const R n1s2 = ml(n1s, n1s), n2s2 = ml(n2s, n2s), n3s2 = ml(n3s, n3s);
+    const R n1s3 = ml(n1s2, n1s), n2s3 = ml(n2s2, n2s), n3s3 = ml(n3s2, n3s);
+    const R n1s4 = ml(n1s2, n1s2), n2s4 = ml(n2s2, n2s2), n3s4 = ml(n3s2, n3s2);
     const R q = quirk ? n3s3 : n3s2;
-    const R a1 = (R)2 * K[0] * n1s * (n2s2 + q), a2 = (R)2 * K[0] * n2s * (n1s2 + n3s2), a3 = (R)2 * K[0] * n3s * (n1s2 + n2s2);
-    const R p = n1s * n2s * n3s;
-    const R b1 = (R)2 * K[1] * p * n2s * n3s, b2 = (R)2 * K[1] * p * n1s * n3s, b3 = (R)2 * K[1] * p * n1s * n2s;
-    const R c1 = (R)4 * K[2] * n1s3 * (n2s4 + n3s4), c2 = (R)4 * K[2] * n2s3 * (n1s4 + n3s4), c3 = (R)4 * K[2] * n3s3 * (n1s4 + n2s4);
-    hx = (n[0] * a1 + n[3] * a2 + n[6] * a3) + (n[0] * b1 + n[3] * b2 + n[6] * b3) + (n[0] * c1 + n[3] * c2 + n[6] * c3);
-    hy = (n[1] * a1 + n[4] * a2 + n[7] * a3) + (n[1] * b1 + n[4] * b2 + n[7] * b3) + (n[1] * c1 + n[4] * c2 + n[7] * c3);
-    hz = (n[2] * a1 + n[5] * a2 + n[8] * a3) + (n[2] * b1 + n[5] * b2 + n[8] * b3) + (n[2] * c1 + n[5] * c2 + n[8] * c3);
+    const R k1 = ml((R)2, K[0]), k2 = ml((R)2, K[1]), k3 = ml((R)4, K[2]);
+    const R a1 = ml(ml(k1, n1s), ad(n2s2, q)), a2 = ml(ml(k1, n2s), ad(n1s2, n3s2)), a3 = ml(ml(k1, n3s), ad(n1s2, n2s2));
+    const R p = ml(k2, ml(ml(n1s, n2s), n3s));
+    const R b1 = ml(p, ml(n2s, n3s)), b2 = ml(p, ml(n1s, n3s)), b3 = ml(p, ml(n1s, n2s));
+    const R c1 = ml(ml(k3, n1s3), ad(n2s4, n3s4)), c2 = ml(ml(k3, n2s3), ad(n1s4, n3s4)), c3 = ml(ml(k3, n3s3), ad(n1s4, n2s4));
+    const R s1 = ad(ad(a1, b1), c1), s2 = ad(ad(a2, b2), c2), s3 = ad(ad(a3, b3), c3);
+    hx = dot3(n[0], s1, n[3], s2, n[6], s3);
+    hy = dot3(n[1], s1, n[4], s2, n[7], s3);
+    hz = dot3(n[2], s1, n[5], s2, n[8], s3);
 }
 
 // ------------------------------------------------------------------ fused step
@@ -114,88 +116,92 @@ __device__ __forceinline__ void fused_site_ld(const FastKT<R>& F, int NX, int NY
         for (int k = 0; k < 6; k++) {
             const R J = F.J[k];
             if (J != (R)0 && f[k] >= 0) {
-                ex += J * nb[k][0]; ey += J * nb[k][1]; ez += J * nb[k][2];
+                ex = fm(J, nb[k][0], ex); ey = fm(J, nb[k][1], ey); ez = fm(J, nb[k][2], ez);
             }
         }
-        Hx += ex; Hy += ey; Hz += ez;
+        Hx = ad(Hx, ex); Hy = ad(Hy, ey); Hz = ad(Hz, ez);
     }
     if (ANI) {
         if (F.ani == 2) {
             // one uniform cubic axis set
             R cx, cy, cz;
-            cubic_field<R>(Sx * F.cub_ims, Sy * F.cub_ims, Sz * F.cub_ims, F.cub_n, F.cub_K, F.cub_quirk, cx, cy,
-                           cz);
-            Hx += cx; Hy += cy; Hz += cz;
+            cubic_field<R>(ml(Sx, F.cub_ims), ml(Sy, F.cub_ims), ml(Sz, F.cub_ims), F.cub_n, F.cub_K, F.cub_quirk, cx,
+                           cy, cz);
+            Hx = ad(Hx, cx); Hy = ad(Hy, cy); Hz = ad(Hz, cz);
         } else {
-            const R v = F.ani_c * (Sx * F.axis[0] + Sy * F.axis[1] + Sz * F.axis[2]);
-            Hx += v * F.axis[0]; Hy += v * F.axis[1]; Hz += v * F.axis[2];
+            const R v = ml(F.ani_c, dot3(Sx, F.axis[0], Sy, F.axis[1], Sz, F.axis[2]));
+            Hx = fm(v, F.axis[0], Hx); Hy = fm(v, F.axis[1], Hy); Hz = fm(v, F.axis[2], Hz);
         }
     }
     R Tx = 0, Ty = 0, Tz = 0;
     if (TH) {
         const float3 nrm = pre ? *pre : thermal_normal3(F, i);
-        Tx = F.sigma * nrm.x; Ty = F.sigma * nrm.y; Tz = F.sigma * nrm.z;
-        Hx += Tx; Hy += Ty; Hz += Tz;
+        Tx = ml(F.sigma, (R)nrm.x); Ty = ml(F.sigma, (R)nrm.y); Tz = ml(F.sigma, (R)nrm.z);
+        Hx = ad(Hx, Tx); Hy = ad(Hy, Ty); Hz = ad(Hz, Tz);
     }
     if (ADD) {
-        Hx += F.addw * Ax; Hy += F.addw * Ay; Hz += F.addw * Az;
+        Hx = fm(F.addw, Ax, Hx); Hy = fm(F.addw, Ay, Hy); Hz = fm(F.addw, Az, Hz);
     }
     R nx_, ny_, nz_;
     if (LT == LLG_CART) {
         if (F.dt_zero) { nx_ = Sx; ny_ = Sy; nz_ = Sz; }
         else {
             // h = H - Hth; dM = -p gaa M x H - d (a/ms) gaa M x (M x h)
-            const R hx = F.tof ? Hx - Tx : Hx, hy = F.tof ? Hy - Ty : Hy, hz = F.tof ? Hz - Tz : Hz;
-            const R mhx = Sy * hz - Sz * hy, mhy = Sz * hx - Sx * hz, mhz = Sx * hy - Sy * hx;
-            const R mmx = Sy * mhz - Sz * mhy, mmy = Sz * mhx - Sx * mhz, mmz = Sx * mhy - Sy * mhx;
-            const R MHx = Sy * Hz - Sz * Hy, MHy = Sz * Hx - Sx * Hz, MHz = Sx * Hy - Sy * Hx;
-            nx_ = Sx + F.dt * (F.c_prec * MHx - F.c_damp * mmx);
-            ny_ = Sy + F.dt * (F.c_prec * MHy - F.c_damp * mmy);
-            nz_ = Sz + F.dt * (F.c_prec * MHz - F.c_damp * mmz);
+            const R hx = F.tof ? ad(Hx, -Tx) : Hx, hy = F.tof ? ad(Hy, -Ty) : Hy, hz = F.tof ? ad(Hz, -Tz) : Hz;
+            const R mhx = crs(Sy, hz, Sz, hy), mhy = crs(Sz, hx, Sx, hz), mhz = crs(Sx, hy, Sy, hx);
+            const R mmx = crs(Sy, mhz, Sz, mhy), mmy = crs(Sz, mhx, Sx, mhz), mmz = crs(Sx, mhy, Sy, mhx);
+            const R MHx = crs(Sy, Hz, Sz, Hy), MHy = crs(Sz, Hx, Sx, Hz), MHz = crs(Sx, Hy, Sy, Hx);
+            nx_ = fm(F.dt, crs(F.c_prec, MHx, F.c_damp, mmx), Sx);
+            ny_ = fm(F.dt, crs(F.c_prec, MHy, F.c_damp, mmy), Sy);
+            nz_ = fm(F.dt, crs(F.c_prec, MHz, F.c_damp, mmz), Sz);
         }
     } else {
         R Hpx, Hpy, Hpz;
         if (F.tof) {
-            const R hx = Hx - Tx, hy = Hy - Ty, hz = Hz - Tz;
-            const R shx = Sy * hz - Sz * hy, shy = Sz * hx - Sx * hz, shz = Sx * hy - Sy * hx;
-            Hpx = F.precess * Hx + F.c_damp * shx;
-            Hpy = F.precess * Hy + F.c_damp * shy;
-            Hpz = F.precess * Hz + F.c_damp * shz;
+            const R hx = ad(Hx, -Tx), hy = ad(Hy, -Ty), hz = ad(Hz, -Tz);
+            const R shx = crs(Sy, hz, Sz, hy), shy = crs(Sz, hx, Sx, hz), shz = crs(Sx, hy, Sy, hx);
+            Hpx = fm(F.precess, Hx, ml(F.c_damp, shx));
+            Hpy = fm(F.precess, Hy, ml(F.c_damp, shy));
+            Hpz = fm(F.precess, Hz, ml(F.c_damp, shz));
         } else {
-            const R shx = Sy * Hz - Sz * Hy, shy = Sz * Hx - Sx * Hz, shz = Sx * Hy - Sy * Hx;
-            Hpx = Hx + F.c_damp * shx; Hpy = Hy + F.c_damp * shy; Hpz = Hz + F.c_damp * shz;
+            const R shx = crs(Sy, Hz, Sz, Hy), shy = crs(Sz, Hx, Sx, Hz), shz = crs(Sx, Hy, Sy, Hx);
+            Hpx = fm(F.c_damp, shx, Hx); Hpy = fm(F.c_damp, shy, Hy); Hpz = fm(F.c_damp, shz, Hz);
         }
-        const R HL2 = Hpx * Hpx + Hpy * Hpy + Hpz * Hpz;
+        const R HL2 = dot3(Hpx, Hpx, Hpy, Hpy, Hpz, Hpz);
         if (HL2 > (R)0) {
             const R iHL = fs_rsqrt(HL2);
-            const R HL = HL2 * iHL;
+            const R HL = ml(HL2, iHL);
             // half rotation angle; in FP32 small angles by their Taylor
             // series (|th| <= 0.1: truncation below 1e-10, under FP32
             // rounding), else (and always in FP64) sine and cosine
-            const R th = F.c_rot * HL;
+            const R th = ml(F.c_rot, HL);
             R sn, cs;
             if (sizeof(R) == 4 && fabs(th) <= (R)0.1) {
-                const R t2 = th * th;
-                sn = th * (1.0f - t2 * (1.0f / 6.0f) * (1.0f - t2 * (1.0f / 20.0f) * (1.0f - t2 * (1.0f / 42.0f))));
-                cs = 1.0f - t2 * 0.5f * (1.0f - t2 * (1.0f / 12.0f) * (1.0f - t2 * (1.0f / 30.0f) * (1.0f - t2 * (1.0f / 56.0f))));
+                const R t2 = ml(th, th);
+                const R a = fm(-t2, (R)(1.0f / 42.0f), (R)1), b = fm(ml(-t2, (R)(1.0f / 20.0f)), a, (R)1);
+                sn = ml(th, fm(ml(-t2, (R)(1.0f / 6.0f)), b, (R)1));
+                const R c = fm(-t2, (R)(1.0f / 56.0f), (R)1), d = fm(ml(-t2, (R)(1.0f / 30.0f)), c, (R)1);
+                const R e = fm(ml(-t2, (R)(1.0f / 12.0f)), d, (R)1);
+                cs = fm(ml(-t2, (R)0.5f), e, (R)1);
             } else {
                 fs_sincos(th, &sn, &cs);
             }
-            const R qw = cs, qx = sn * Hpx * iHL, qy = sn * Hpy * iHL, qz = sn * Hpz * iHL;
-            const R tw = -qx * Sx - qy * Sy - qz * Sz;
-            const R tx = qw * Sx + qy * Sz - qz * Sy;
-            const R ty = qw * Sy + qz * Sx - qx * Sz;
-            const R tz = qw * Sz + qx * Sy - qy * Sx;
-            nx_ = -tw * qx + qw * tx - ty * qz + tz * qy;
-            ny_ = -tw * qy + qw * ty - tz * qx + tx * qz;
-            nz_ = -tw * qz + qw * tz - tx * qy + ty * qx;
+            const R k = ml(sn, iHL);
+            const R qw = cs, qx = ml(k, Hpx), qy = ml(k, Hpy), qz = ml(k, Hpz);
+            const R tw = -dot3(qx, Sx, qy, Sy, qz, Sz);
+            const R tx = fm(qw, Sx, crs(qy, Sz, qz, Sy));
+            const R ty = fm(qw, Sy, crs(qz, Sx, qx, Sz));
+            const R tz = fm(qw, Sz, crs(qx, Sy, qy, Sx));
+            nx_ = fm(qw, tx, fm(-tw, qx, crs(tz, qy, ty, qz)));
+            ny_ = fm(qw, ty, fm(-tw, qy, crs(tx, qz, tz, qx)));
+            nz_ = fm(qw, tz, fm(-tw, qz, crs(ty, qx, tx, qy)));
         } else { nx_ = Sx; ny_ = Sy; nz_ = Sz; }
     }
     if (F.renorm) {
-        const R mm = nx_ * nx_ + ny_ * ny_ + nz_ * nz_;
+        const R mm = dot3(nx_, nx_, ny_, ny_, nz_, nz_);
         if (mm != (R)0) {
-            const R inv = F.ms * fs_rsqrt(mm);
-            nx_ *= inv; ny_ *= inv; nz_ *= inv;
+            const R inv = ml(F.ms, fs_rsqrt(mm));
+            nx_ = ml(nx_, inv); ny_ = ml(ny_, inv); nz_ = ml(nz_, inv);
         }
     }
     rx = nx_; ry = ny_; rz = nz_;

@@ -17,6 +17,7 @@
 #include "fused.cuh"
 #include "kparams.h"
 #include "launch.h"
+#include "terms.cuh"
 
 #include <cuda_runtime.h>
 #include <math.h>
@@ -24,289 +25,6 @@
 #include <algorithm>
 #include <stdint.h>
 #include <stdio.h>
-
-// ------------------------------------------------------------ helpers
-template <typename R>
-struct V3 {
-    R x, y, z;
-};
-template <typename R> __device__ __forceinline__ V3<R> v3(R a, R b, R c) { V3<R> v; v.x = a; v.y = b; v.z = c; return v; }
-template <typename R> __device__ __forceinline__ V3<R> add3(V3<R> a, V3<R> b) { return v3<R>(a.x + b.x, a.y + b.y, a.z + b.z); }
-template <typename R> __device__ __forceinline__ V3<R> sub3(V3<R> a, V3<R> b) { return v3<R>(a.x - b.x, a.y - b.y, a.z - b.z); }
-template <typename R> __device__ __forceinline__ V3<R> scl3(R a, V3<R> b) { return v3<R>(a * b.x, a * b.y, a * b.z); }
-template <typename R> __device__ __forceinline__ V3<R> cross3(V3<R> a, V3<R> b)
-{
-    return v3<R>(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-}
-template <typename R> __device__ __forceinline__ R ldr(const void* p, int i) { return __ldg(static_cast<const R*>(p) + i); }
-template <typename R> __device__ __forceinline__ R ms_at(const SysK& s, int i) { return s.ms_uniform ? (R)s.ms_u : ldr<R>(s.ms, i); }
-template <typename R> __device__ __forceinline__ R alpha_at(const SysK& s, int i) { return s.site_alpha ? ldr<R>(s.site_alpha, i) : (R)s.alpha; }
-template <typename R> __device__ __forceinline__ R gamma_at(const SysK& s, int i) { return s.site_gamma ? ldr<R>(s.site_gamma, i) : (R)s.gamma; }
-template <typename R> __device__ __forceinline__ V3<R> spin_at(const SysK& s, int i)
-{
-    return v3<R>(ldr<R>(s.x, i), ldr<R>(s.y, i), ldr<R>(s.z, i));
-}
-template <typename R> __device__ __forceinline__ R rsq(R v);
-template <> __device__ __forceinline__ float rsq<float>(float v) { return sqrtf(v); }
-template <> __device__ __forceinline__ double rsq<double>(double v) { return sqrt(v); }
-__device__ __forceinline__ void sincos_r(float v, float* s, float* c) { sincosf(v, s, c); }
-__device__ __forceinline__ void sincos_r(double v, double* s, double* c) { sincos(v, s, c); }
-
-// ------------------------------------------------------------ field terms
-// Exchange: h_t += J s_f / (m_f m_t) (normalised) or J s_f / m_f, only for
-// m_f != 0 (M/cpu/exchange/spinoperationexchange.cpp:134-213).
-template <typename R>
-__device__ __forceinline__ V3<R> ex_term(const ExchangeK& e, const SysK& s, int i, R mt)
-{
-    V3<R> h = v3<R>(0, 0, 0);
-    if (e.mode == EX_STENCIL) {
-        const int ix = i % s.nx;
-        const int iy = (i / s.nx) % s.ny;
-        const int iz = i / (s.nx * s.ny);
-        const int nxy = s.nx * s.ny;
-#pragma unroll
-        for (int d = 0; d < 6; d++) {
-            const R J = (R)e.J[d];
-            if (J == (R)0) continue;
-            const int ax = d >> 1;
-            const int sg = (d & 1) ? -1 : 1;
-            int c = ax == 0 ? ix : (ax == 1 ? iy : iz);
-            const int n = ax == 0 ? s.nx : (ax == 1 ? s.ny : s.nz);
-            c += sg;
-            if (c < 0 || c >= n) {
-                if (!e.pbc[ax]) continue;
-                c = c < 0 ? c + n : c - n;
-            }
-            const int f = ax == 0 ? (i - ix + c) : (ax == 1 ? (i + (c - iy) * s.nx) : (i + (c - iz) * nxy));
-            const R mf = ms_at<R>(s, f);
-            if (mf != (R)0) {
-                const V3<R> sf = spin_at<R>(s, f);
-                const R w = J / (e.normalize ? mf * mt : mf);   // one division per neighbour
-                h = add3(h, v3<R>(sf.x * w, sf.y * w, sf.z * w));
-            }
-        }
-    } else if (e.mode == EX_CSR) {
-        const int p0 = __ldg(e.ptr + i), p1 = __ldg(e.ptr + i + 1);
-        for (int p = p0; p < p1; p++) {
-            const int f = __ldg(e.col + p);
-            const R J = (R)__ldg(e.val + p);
-            const R mf = ms_at<R>(s, f);
-            if (mf != (R)0) {
-                const V3<R> sf = spin_at<R>(s, f);
-                const R den = e.normalize ? mf * mt : mf;
-                h = add3(h, v3<R>(sf.x * J / den, sf.y * J / den, sf.z * J / den));
-            }
-        }
-    }
-    return h;
-}
-
-// Anisotropy: H = 2K (s.n)/ms^2 n for ms > 0
-// (M/cpu/anisotropy/spinoperationanisotropy.cpp:247-283).
-template <typename R>
-__device__ __forceinline__ V3<R> ani_one(V3<R> sp, R ms, R n0, R n1, R n2, R K)
-{
-    const R sda = sp.x * n0 + sp.y * n1 + sp.z * n2;
-    const R v = (R)2 * K * sda / (ms * ms);
-    return v3<R>(n0 * v, n1 * v, n2 * v);
-}
-template <typename R>
-__device__ __forceinline__ V3<R> ani_term(const AniK& a, V3<R> sp, R ms, int i)
-{
-    V3<R> h = v3<R>(0, 0, 0);
-    if (!(ms > (R)0)) return h;
-    if (a.mode == ANI_UNIFORM) return ani_one<R>(sp, ms, (R)a.axis[0], (R)a.axis[1], (R)a.axis[2], (R)a.K);
-    if (a.mode == ANI_CSR) {
-        const int p0 = __ldg(a.ptr + i), p1 = __ldg(a.ptr + i + 1);
-        for (int p = p0; p < p1; p++)
-            h = add3(h, ani_one<R>(sp, ms, (R)__ldg(a.axes + 3 * p), (R)__ldg(a.axes + 3 * p + 1),
-                                   (R)__ldg(a.axes + 3 * p + 2), (R)__ldg(a.Ks + p)));
-    }
-    return h;
-}
-
-// Uniaxial: [2K1 u + 4K2 u^3] n with u = s.n of the unit spin; quirk keeps
-// the reference's sz*nx (..._uniaxial.cpp:250-298, :287).
-template <typename R>
-__device__ __forceinline__ V3<R> uni_one(V3<R> u3, R n0, R n1, R n2, R K1, R K2, int quirk)
-{
-    const R u = u3.x * n0 + u3.y * n1 + u3.z * (quirk ? n0 : n2);
-    const R mag = (R)2 * K1 * u + (R)4 * K2 * (u * u * u);
-    return v3<R>(n0 * mag, n1 * mag, n2 * mag);
-}
-template <typename R>
-__device__ __forceinline__ V3<R> uni_term(const UniK& a, V3<R> sp, R ms, int i)
-{
-    V3<R> h = v3<R>(0, 0, 0);
-    if (!(ms > (R)0) || a.mode == ANI_NONE) return h;
-    const V3<R> u = v3<R>(sp.x / ms, sp.y / ms, sp.z / ms);
-    if (a.mode == ANI_UNIFORM)
-        return uni_one<R>(u, (R)a.axis[0], (R)a.axis[1], (R)a.axis[2], (R)a.K1, (R)a.K2, a.quirk);
-    const int p0 = __ldg(a.ptr + i), p1 = __ldg(a.ptr + i + 1);
-    for (int p = p0; p < p1; p++)
-        h = add3(h, uni_one<R>(u, (R)__ldg(a.axes + 3 * p), (R)__ldg(a.axes + 3 * p + 1), (R)__ldg(a.axes + 3 * p + 2),
-                               (R)__ldg(a.K12 + 2 * p), (R)__ldg(a.K12 + 2 * p + 1), a.quirk));
-    return h;
-}
-
-// Cubic (..._cubic.cpp:308-390): cubic_field (fused.cuh) on a V3.
-template <typename R>
-__device__ __forceinline__ V3<R> cub_one(V3<R> s, const R* n, const R* K, int quirk)
-{
-    V3<R> h;
-    cubic_field<R>(s.x, s.y, s.z, n, K, quirk, h.x, h.y, h.z);
-    return h;
-}
-template <typename R>
-__device__ __forceinline__ V3<R> cub_term(const CubK& a, V3<R> sp, R ms, int i)
-{
-    V3<R> h = v3<R>(0, 0, 0);
-    if (!(ms > (R)0) || a.mode == ANI_NONE) return h;
-    const V3<R> u = v3<R>(sp.x / ms, sp.y / ms, sp.z / ms);
-    R n[9], K[3];
-    if (a.mode == ANI_UNIFORM) {
-#pragma unroll
-        for (int q = 0; q < 9; q++) n[q] = (R)a.axes[q];
-#pragma unroll
-        for (int q = 0; q < 3; q++) K[q] = (R)a.K[q];
-        return cub_one<R>(u, n, K, a.quirk);
-    }
-    const int p0 = __ldg(a.ptr + i), p1 = __ldg(a.ptr + i + 1);
-    for (int p = p0; p < p1; p++) {
-#pragma unroll
-        for (int q = 0; q < 9; q++) n[q] = (R)__ldg(a.axs + 9 * p + q);
-#pragma unroll
-        for (int q = 0; q < 3; q++) K[q] = (R)__ldg(a.Ks + 3 * p + q);
-        h = add3(h, cub_one<R>(u, n, K, a.quirk));
-    }
-    return h;
-}
-
-// Thermal: sigma = sqrt(2 alpha T scale / (ms dt gamma)) times N(0,1) per
-// component, zero where ms == 0, T == 0 or gamma <= 0
-// (M/cpu/thermal/spinoperationthermal.cpp:135-191).
-template <typename R>
-__device__ __forceinline__ V3<R> th_term(const ThermalK& t, const SysK& s, R dt_sys, int i, R ms)
-{
-    V3<R> h = v3<R>(0, 0, 0);
-    if (t.mode == TH_NONE || ms == (R)0 || t.T == 0.0) return h;
-    const R a = alpha_at<R>(s, i), g = gamma_at<R>(s, i);
-    if (!(g > (R)0)) return h;
-    const R sc = t.scale ? (R)__ldg(t.scale + i) : (R)1;
-    const R sd = rsq<R>(((R)2 * a * (R)t.T * sc) / (ms * dt_sys * g));
-    V3<R> n;
-    if (t.mode == TH_PHILOX) {
-        const uint64_t ctr = t.counter + (t.dctr ? *t.dctr : 0ull);
-        const float3 f = philox_normal3(t.seed, ctr, (uint32_t)i, 0x6d6c6232u);
-        n = v3<R>((R)f.x, (R)f.y, (R)f.z);
-    } else {
-        n = v3<R>((R)__ldg(t.nx + i), (R)__ldg(t.ny + i), (R)__ldg(t.nz + i));
-    }
-    return v3<R>(sd * n.x, sd * n.y, sd * n.z);
-}
-
-template <typename R>
-struct Fields {
-    V3<R> H;
-    V3<R> Hth;
-};
-
-// Every term of TermsK at site i.  H is the would-be "Total" slot, Hth the
-// "Thermal" slot that LLG subtracts (llgcartesian.cpp:160-172).
-template <typename R>
-__device__ __forceinline__ Fields<R> eval_terms(const TermsK& T, const SysK& s, R dt_sys, int i)
-{
-    const R ms = ms_at<R>(s, i);
-    const V3<R> sp = spin_at<R>(s, i);
-    V3<R> H = v3<R>(0, 0, 0);
-    V3<R> Hth = v3<R>(0, 0, 0);
-    if (T.ex.mode != EX_NONE) H = add3(H, scl3((R)T.ex_gs, ex_term<R>(T.ex, s, i, ms)));
-    if (T.ani.mode != ANI_NONE) H = add3(H, ani_term<R>(T.ani, sp, ms, i));
-    if (T.uni.mode != ANI_NONE) H = add3(H, uni_term<R>(T.uni, sp, ms, i));
-    if (T.cub.mode != ANI_NONE) H = add3(H, cub_term<R>(T.cub, sp, ms, i));
-    if (T.th.mode != TH_NONE) { Hth = th_term<R>(T.th, s, dt_sys, i, ms); H = add3(H, Hth); }
-    if (T.zee.on) {
-        const V3<R> B = T.zee.Bdev ? v3<R>((R)T.zee.Bdev[0], (R)T.zee.Bdev[1], (R)T.zee.Bdev[2])
-                                   : v3<R>((R)T.zee.B[0], (R)T.zee.B[1], (R)T.zee.B[2]);
-        H = add3(H, B);
-    }
-    for (int a = 0; a < T.nadd; a++) {
-        const V3<R> v = v3<R>(ldr<R>(T.add[a][0], i), ldr<R>(T.add[a][1], i), ldr<R>(T.add[a][2], i));
-        const R w = (R)T.addw[a];
-        H = add3(H, v3<R>(w * v.x, w * v.y, w * v.z));
-        if (T.add_is_thermal[a]) Hth = add3(Hth, v);
-    }
-    Fields<R> f;
-    f.H = H;
-    f.Hth = Hth;
-    return f;
-}
-
-// ------------------------------------------------------------ LLG
-// Cartesian Euler step (M/cpu/llg/llgcartesian.cpp:90-278) or quaternion
-// rotation (M/cpu/llg/llgquat.cpp:126-378) for one site with ms > 0.
-// S: from-spin, M: dmdt-spin, H: Total, Hth: Thermal.
-template <typename R>
-__device__ __forceinline__ V3<R> llg_site(const LlgK& L, V3<R> S, V3<R> M, V3<R> H, V3<R> Hth, R ms, R a, R g)
-{
-    const R dt = (R)L.dt, p = (R)L.precess, d = (R)L.damp;
-    if (L.type == LLG_CART) {
-        if (L.dt_zero) return S;
-        const R gaa = g / ((R)1 + a * a);
-        if (L.thermal_only_first_term) {
-            const V3<R> h = sub3(H, Hth);
-            const V3<R> Mh = cross3(M, h);
-            const V3<R> MMH = cross3(M, Mh);
-            const V3<R> MH = cross3(M, H);
-            const V3<R> dM = sub3(scl3(p * -gaa, MH), scl3(d * (a / ms) * gaa, MMH));
-            return add3(S, scl3(dt, dM));
-        }
-        const V3<R> MH = cross3(M, H);
-        const V3<R> MMH = cross3(M, MH);
-        const V3<R> dM = sub3(scl3(-gaa, MH), scl3((a / ms) * gaa, MMH));
-        return add3(S, scl3(dt, dM));
-    }
-    // quaternion
-    const R inv = (R)1 / ms;
-    V3<R> Hp;
-    if (L.thermal_only_first_term) {
-        const V3<R> h = sub3(H, Hth);
-        const V3<R> Sh = cross3(M, h);
-        Hp = add3(scl3(p, H), scl3(d * a * inv, Sh));
-    } else {
-        const V3<R> SH = cross3(S, H);
-        Hp = add3(H, scl3(a * inv, SH));
-    }
-    const R HLen = rsq<R>(Hp.x * Hp.x + Hp.y * Hp.y + Hp.z * Hp.z);
-    if (!(HLen > (R)0)) return S;
-    const R iHLen = (R)1 / HLen;
-    const R ra = (R)1 * g * HLen / ((R)1 + a * a);
-    R sint, cost;
-    sincos_r(((R)0.5) * ra * dt, &sint, &cost);
-    // qRot = (cost, sint * Hp/|Hp|); qRes = qRot * (0,S) * conj(qRot)
-    const R qw = cost, qx = sint * Hp.x * iHLen, qy = sint * Hp.y * iHLen, qz = sint * Hp.z * iHLen;
-    const R tw = -qx * S.x - qy * S.y - qz * S.z;
-    const R tx = qw * S.x + qy * S.z - qz * S.y;
-    const R ty = qw * S.y + qz * S.x - qx * S.z;
-    const R tz = qw * S.z + qx * S.y - qy * S.x;
-    const R cx = -qx, cy = -qy, cz = -qz;
-    V3<R> r;
-    r.x = tw * cx + qw * tx + ty * cz - tz * cy;
-    r.y = tw * cy + qw * ty + tz * cx - tx * cz;
-    r.z = tw * cz + qw * tz + tx * cy - ty * cx;
-    return r;
-}
-
-template <typename R>
-__device__ __forceinline__ V3<R> renorm(V3<R> v, R ms)
-{
-    const R mm = v.x * v.x + v.y * v.y + v.z * v.z;
-    if (mm != (R)0) {
-        const R inv = ms / rsq<R>(mm);
-        return v3<R>(v.x * inv, v.y * inv, v.z * inv);
-    }
-    return v;
-}
 
 // ------------------------------------------------------------ kernels
 template <typename R>
@@ -316,13 +34,9 @@ __global__ void __launch_bounds__(256) k_fused_step(FusedK P, double dt_sys)
     if (i >= P.sys.n) return;
     const R ms = ms_at<R>(P.sys, i);
     const V3<R> S = spin_at<R>(P.sys, i);
-    V3<R> out = S;
-    if (ms > (R)0) {
-        const Fields<R> F = eval_terms<R>(P.terms, P.sys, (R)dt_sys, i);
-        out = llg_site<R>(P.llg, S, S, F.H, F.Hth, ms, alpha_at<R>(P.sys, i), gamma_at<R>(P.sys, i));
-    }
-    if (P.llg.renorm) out = renorm<R>(out, ms);
-    if (P.llg.status && !(isfinite(out.x) && isfinite(out.y) && isfinite(out.z))) atomicOr(P.llg.status, 1u);
+    Fields<R> F;
+    if (ms > (R)0) F = eval_terms<R>(P.terms, P.sys, (R)dt_sys, i);
+    const V3<R> out = step_site<R>(P, F, S, ms, i);
     static_cast<R*>(P.ox)[i] = out.x;
     static_cast<R*>(P.oy)[i] = out.y;
     static_cast<R*>(P.oz)[i] = out.z;

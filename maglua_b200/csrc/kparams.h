@@ -144,28 +144,31 @@ struct ConvK {
     unsigned long long* tl = nullptr;
 };
 
-// Lattice edges of any length (mx.cu): the Stockham stages of one axis, a
-// radix-R butterfly each (nb per line; Ns points already combined; twiddle
-// step tws; mnb, mNs the multipliers of the divisions by nb and Ns).
+// Lattice edges of any length (mx.cu): the stages of one axis, radix-R
+// butterflies in place (nb per line, of the points j + r m of a block of R m;
+// twiddle step tws; mnb, mm the multipliers of the divisions by nb and m).
 #define MX_MAX_STAGES 10
 struct MxStage {
-    int R, nb, Ns, tws;
-    unsigned mnb, mNs;
+    int R, nb, m, tws;
+    unsigned mnb, mm;
 };
 struct MxAxis {
-    int n, LS, nst;          // points, line stride in shared memory, stages
+    int n, nst;              // points, stages
+    int sh, LS;              // padding (element i at i + (i >> sh)), line stride in shared memory
+    int big;                 // a stage of radix above 16
     MxStage s[MX_MAX_STAGES];
 };
 struct MxX {
     int nx, ny, nz, nr, Kx;  // nr = nz ny rows
-    int rows, r2sh;          // rows per CTA, log2(rows / 2)
-    unsigned m3r2, mPx, mnx; // divisions by 3 rows / 2, Px, nx
+    int rows;                // rows per CTA (even)
+    unsigned m3r2, mr2, mPx, mnx;   // divisions by 3 rows / 2, rows / 2, Px, nx
+    const int* at;           // places of frequencies k and n - k in a transformed line
     const int* run_if;
     MxAxis ax;
 };
 struct MxYZ {
     int ny, nz, threads;
-    unsigned mPy, mny;
+    unsigned mPy, mny, mcols; // divisions by Py, ny and the columns a CTA takes at a time
     double g;
     const int* run_if;
     MxAxis ax;

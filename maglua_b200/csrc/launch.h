@@ -96,6 +96,11 @@ bool xstep_ok(const ConvK& c, const FastK& F);
 // Inverse x pass + fused step (+ forward x pass of the new spins when fwd).
 cudaError_t launch_xstep(const ConvK& c, const FftLen L[3], const float2* tw, float2* spec, const FastK& F,
                          bool fwd, const float* s[3], float* h[3], float* o[3], cudaStream_t st);
+// The same for the general form of a step (launch_mx_gstep's arguments).
+bool xgstep_ok(const ConvK& c);
+cudaError_t launch_xgstep(const ConvK& c, const FftLen L[3], const float2* tw, float2* spec, const FusedK& P,
+                          double addw, double dt_sys, const DevStep* cur, DevStep* next, float* const h[3],
+                          cudaStream_t st);
 cudaError_t launch_fused_fast(const FastK& F, const float* s[3], const float* a[3], float* o[3], cudaStream_t st);
 // the same for FP64 state (constants in double)
 cudaError_t launch_fused_fast_f64(const FastKT<double>& F, const double* s[3], const double* a[3], double* o[3],
@@ -133,16 +138,26 @@ cudaError_t launch_conv(const ConvK& c, const FftLen& Lx, const FftLen& Ly, cons
                         const void* const s[3], void* spec, const void* ten6, const void* ten9, void* const h[3],
                         int rb, cudaStream_t st);
 // Any-length passes (mx.cu): the plan of a convolution (false: not a size or
-// tensor they take), the bytes of its layer tensor, its packing from the
+// tensor they take) with the places of its x and y frequencies, the bytes of its layer tensor, its packing from the
 // six components transformed over x and y (stat2: largest |W| and largest
 // deviation from the parities, as double bits; zero them first), and the
 // forward x (fx), (y,z) and inverse x (ix) passes.
-bool mx_plan(const ConvK& c, int rb, MxPlan& p);
+bool mx_plan(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vector<int>& at_y);
 size_t mx_tensor_bytes(const ConvK& c, int rb);
-cudaError_t launch_mx_pack(const double2* W, const ConvK& c, void* tz, unsigned long long* stat2, int rb,
+cudaError_t launch_mx_pack(const double2* W, const ConvK& c, const int* at, void* tz, unsigned long long* stat2, int rb,
                            cudaStream_t st);
 cudaError_t launch_mx_conv(const ConvK& c, const MxPlan& p, const FftLen L[3], const void* tw, const void* const s[3],
                            void* spec, const void* tz, void* const h[3], bool fx, bool ix, int rb, cudaStream_t st);
+cudaError_t launch_mx_ix(const MxX& x, const FftLen L[3], const void* tw, const void* spec, void* const h[3], int rb,
+                         cudaStream_t st);
+// Inverse x pass + step + forward x pass of the new spins: uniform
+// parameters, or the general form (P.terms without the dipole addend of
+// weight addw; cur -> next advance the device step block of a captured step).
+template <typename R>
+cudaError_t launch_mx_step(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FastKT<R>& F,
+                           const R* const s[3], R* const h[3], R* const o[3], cudaStream_t st);
+cudaError_t launch_mx_gstep(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FusedK& P, double addw,
+                            double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], int rb, cudaStream_t st);
 cudaError_t mx_configure();
 cudaError_t launch_tensor_lattice(int nx, int ny, int nz, const int gmax[4], const double ABC[9], int Px,
                                   int Py, int Pz, int zsign, double2* W, cudaStream_t st);

@@ -10,13 +10,16 @@
 //                       transform of the new spins in one pass.
 //
 // Transforms.  A CTA's lines lie in shared memory and go through two or three
-// Stockham stages of radix 2..31 (one butterfly per thread and turn, in
-// registers).  The stages a length takes are chosen on the host from the
-// number of lines that share the CTA (mx_axis): few large butterflies leave
-// threads idle, many small ones cost a barrier each.  Indices use
-// multiply-shift division; lines are padded (one element per 128 bytes) so
-// that stride-R stores spread over the banks.  An inverse transform is the
-// forward one with real and imaginary parts swapped on the way in and out.
+// stages of radix 2..31 butterflies, each held in one thread's registers and
+// written back to the places it was read from: decimation in frequency
+// forward (natural order in, digit-reversed out), decimation in time back.
+// Nothing is reordered: the layer tensor is stored in the digit-reversed order
+// of ky, and the x spectra are read and written through a table of kx places.
+// So a line needs one buffer and a stage one barrier.  The stages a length
+// takes are chosen on the host from the number of lines that share the CTA
+// (mx_axis): few large butterflies leave threads idle, many small ones cost a
+// barrier each; so is the padding of the lines against bank conflicts.  An
+// inverse transform is the conjugate of the forward one of the conjugate.
 //
 // Layers.  The z direction is not transformed: with the point-dipole parities
 // (checked on the FP64 tensor) T(kx, ky, dz) of XX, XY, YY, ZZ is real and
@@ -24,16 +27,19 @@
 // component pair replace the zero-padded transforms, nothing is padded, and
 // the plane stays at 3 nz rows.
 //
-// What bounds them: at 100 to 200 CTAs of one wave each, a CTA's own chain of
-// loads, stages and barriers (DRAM sees the tensor only).  Measured, one step
-// alone, before (mixed-radix stages with runtime divisions, three components
-// in turn, zero-padded z transforms) and after: 200x150x5 FP32 122 -> 33 us,
-// 128x128x4 FP64 37.5 -> 31 us, 32x95x3 FP64 173 -> 29 us, 128x58x3 (prime
-// factor 29) 381 -> 29 us.
+// What bounds them: at 100 to 300 CTAs of one wave each, a CTA's own chain of
+// loads, stages and barriers (DRAM sees the tensor only); at a million sites
+// instruction issue (400x500x5: 830 instructions per site in k_mx_step).
+// Measured, one step alone, before (mixed-radix stages with runtime divisions,
+// three components in turn, zero-padded z transforms, five kernels) and after:
+// 200x150x5 FP32 122 -> 23 us, 128x128x4 FP64 37.5 -> 24 us, 32x95x3 FP64 173 ->
+// 19 us, 128x58x3 with per-site anisotropy (prime factor 29) 381 -> 24 us,
+// 32x32x1 FP64 25 -> 13 us.
 #include "device.cuh"
 #include "fused.cuh"
 #include "kparams.h"
 #include "launch.h"
+#include "terms.cuh"
 
 #include <cuda_runtime.h>
 #include <math.h>
@@ -143,87 +149,170 @@ __device__ __forceinline__ void dft(C* v)
 // n d < 2^32
 __device__ __forceinline__ int qdiv(int n, unsigned m) { return m ? (int)__umulhi((unsigned)n, m) : n; }
 
-template <typename C> struct Pad { static constexpr int SH = sizeof(C) == 8 ? 4 : 3; };
-template <typename C> __device__ __forceinline__ int pd(int i) { return i + (i >> Pad<C>::SH); }
+// place of element i of a line
+__device__ __forceinline__ int pd(const MxAxis& ax, int i) { return i + (i >> ax.sh); }
 
 extern __shared__ __align__(16) unsigned char mx_sm[];
 
-// One radix-R stage of `total` butterflies (nb per line) from the lines at
-// element src to those at dst; the axis' twiddle table lies at element 0.
-template <int R, typename C>
-__device__ __noinline__ void stage(int src, int dst, int total, const MxStage s, int LS)
+// One radix-R stage of `total` butterflies (nb per line), in place on the
+// lines at element A; the axis' twiddle table lies at element 0.  Butterfly j
+// of a block of R m points takes its points j, j + m, ...
+template <int R, typename C, bool DIT>
+__device__ __noinline__ void stage(int A, int total, const MxStage s, int LS, int sh)
 {
     C* sm = reinterpret_cast<C*>(mx_sm);
     for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        const int l = qdiv(idx, s.mnb), j = idx - l * s.nb;
-        const C* a = sm + src + l * LS;
+        const int l = qdiv(idx, s.mnb), i = idx - l * s.nb;
+        const int blk = qdiv(i, s.mm), j = i - blk * s.m;
+        const int o = blk * s.m * R + j;
+        C* a = sm + A + l * LS;
         C v[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = a[pd<C>(j + r * s.nb)];
-        const int q = qdiv(j, s.mNs), jm = j - q * s.Ns;
-        if (s.Ns > 1) {
-            const int e = jm * s.tws;
+        for (int r = 0; r < R; r++) {
+            const int p = o + r * s.m;
+            v[r] = a[p + (p >> sh)];
+        }
+        const int e = j * s.tws;   // twiddles w^{j r} of the block length
+        if (DIT && s.m > 1) {
             int t = e;
 #pragma unroll
             for (int r = 1; r < R; r++, t += e) v[r] = cmul(v[r], sm[t]);
         }
-        C* b = sm + dst + l * LS;
-        const int o = q * s.Ns * R + jm;
         if constexpr (first_factor(R) == 0 && R > 7) {
-            dft_prime<R>(v, [&](int k, C x) { b[pd<C>(o + k * s.Ns)] = x; });
+            dft_prime<R>(v, [&](int k, C x) {
+                if (!DIT && k > 0) x = cmul(x, sm[e * k]);
+                const int p = o + k * s.m;
+                a[p + (p >> sh)] = x;
+            });
         } else {
             dft<R>(v);
+            if (!DIT && s.m > 1) {
+                int t = e;
 #pragma unroll
-            for (int r = 0; r < R; r++) b[pd<C>(o + r * s.Ns)] = v[r];
+                for (int r = 1; r < R; r++, t += e) v[r] = cmul(v[r], sm[t]);
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int p = o + r * s.m;
+                a[p + (p >> sh)] = v[r];
+            }
         }
     }
 }
 
-// Forward transforms of the nl lines at element a (line stride ax.LS), b a
-// buffer of the same size; every thread of the CTA calls it, and the CTA is
-// synchronised after each stage.  Returns the element where the result lies.
-template <typename C>
-__device__ __forceinline__ int fft(int a, int b, int nl, const MxAxis& ax)
+// The same for a prime radix when there are few butterflies: H + 1 threads
+// per butterfly, thread k forming the outputs k and R - k from all inputs, so
+// that a stage is R long and not R^2 / 2 (R = 31, 18 butterflies: the chain of
+// one thread takes 3.5 us).  A turn's inputs are read before its outputs are
+// written; the points of other turns are not touched.
+template <int R, typename C, bool DIT>
+__device__ __noinline__ void stage_split(int A, int total, const MxStage s, int LS, int sh)
 {
-    for (int i = 0; i < ax.nst; i++) {
-        const MxStage s = ax.s[i];
-        const int total = nl * s.nb;
-        switch (s.R) {
-        case 2: stage<2, C>(a, b, total, s, ax.LS); break;
-        case 3: stage<3, C>(a, b, total, s, ax.LS); break;
-        case 4: stage<4, C>(a, b, total, s, ax.LS); break;
-        case 5: stage<5, C>(a, b, total, s, ax.LS); break;
-        case 6: stage<6, C>(a, b, total, s, ax.LS); break;
-        case 7: stage<7, C>(a, b, total, s, ax.LS); break;
-        case 8: stage<8, C>(a, b, total, s, ax.LS); break;
-        case 9: stage<9, C>(a, b, total, s, ax.LS); break;
-        case 10: stage<10, C>(a, b, total, s, ax.LS); break;
-        case 11: stage<11, C>(a, b, total, s, ax.LS); break;
-        case 12: stage<12, C>(a, b, total, s, ax.LS); break;
-        case 13: stage<13, C>(a, b, total, s, ax.LS); break;
-        case 15: stage<15, C>(a, b, total, s, ax.LS); break;
-        case 16: stage<16, C>(a, b, total, s, ax.LS); break;
-        case 17: stage<17, C>(a, b, total, s, ax.LS); break;
-        case 19: stage<19, C>(a, b, total, s, ax.LS); break;
-        case 23: stage<23, C>(a, b, total, s, ax.LS); break;
-        case 29: stage<29, C>(a, b, total, s, ax.LS); break;
-        case 31: stage<31, C>(a, b, total, s, ax.LS); break;
+    typedef decltype(C().x) T;
+    constexpr int H = (R - 1) / 2;
+    C* sm = reinterpret_cast<C*>(mx_sm);
+    const int per = blockDim.x / (H + 1);   // butterflies of a turn
+    const int b = threadIdx.x / (H + 1), k = threadIdx.x - b * (H + 1);
+    const int wst = s.nb;                   // n / R: w_R^1 in the axis' table
+    for (int b0 = 0; b0 < total; b0 += per) {
+        const int idx = b0 + b;
+        const bool act = b < per && idx < total;
+        C x0 = cmk<C>(0, 0), x1 = x0;
+        C* a = sm;
+        int o = 0, e = 0;
+        if (act) {
+            const int l = qdiv(idx, s.mnb), i = idx - l * s.nb;
+            const int blk = qdiv(i, s.mm), j = i - blk * s.m;
+            o = blk * s.m * R + j;
+            e = j * s.tws;
+            a = sm + A + l * LS;
+            const C v0 = a[o + (o >> sh)];
+            T ax = v0.x, ay = v0.y, bx = 0, by = 0;
+            int q = 0;
+#pragma unroll 5
+            for (int r = 1; r <= H; r++) {
+                const int p = o + r * s.m, u = o + (R - r) * s.m;
+                C f = a[p + (p >> sh)], g = a[u + (u >> sh)];
+                if (DIT && s.m > 1) {
+                    f = cmul(f, sm[e * r]);
+                    g = cmul(g, sm[e * (R - r)]);
+                }
+                q += k;
+                if (q >= R) q -= R;
+                const C w = sm[q * wst];   // w_R^{r k}
+                ax += w.x * (f.x + g.x); ay += w.x * (f.y + g.y);
+                bx += w.y * (f.x - g.x); by += w.y * (f.y - g.y);
+            }
+            x0 = cmk<C>(ax - by, ay + bx);
+            x1 = cmk<C>(ax + by, ay - bx);
+            if (!DIT && s.m > 1) {
+                x0 = cmul(x0, sm[e * k]);
+                if (k > 0) x1 = cmul(x1, sm[e * (R - k)]);
+            }
         }
         __syncthreads();
-        const int t = a;
-        a = b;
-        b = t;
+        if (act) {
+            const int p = o + k * s.m, u = o + (R - k) * s.m;
+            a[p + (p >> sh)] = x0;
+            if (k > 0) a[u + (u >> sh)] = x1;
+        }
     }
-    return a;
 }
 
-template <typename C>
-__device__ __forceinline__ C swp(C a) { return cmk<C>(a.y, a.x); }
+template <int R, typename C, bool DIT>
+__device__ __forceinline__ void stage_prime(int A, int total, const MxStage s, int LS, int sh)
+{
+    // the split butterfly does about three times the arithmetic: taken while
+    // the CTA's threads hold all of it in two turns
+    if (total * ((R + 1) / 2) <= 2 * (int)blockDim.x) stage_split<R, C, DIT>(A, total, s, LS, sh);
+    else stage<R, C, DIT>(A, total, s, LS, sh);
+}
+
+// Forward transforms of the nl lines at element A, in place: natural order to
+// digit-reversed (DIT: back).  Every thread of the CTA calls it, and the CTA is
+// synchronised after each stage.  BIG: the axis has a prime radix above 13,
+// whose butterflies take twice the registers of the others.
+template <typename C, bool DIT, bool BIG>
+__device__ __forceinline__ void fft(int A, int nl, const MxAxis& ax)
+{
+    for (int i = 0; i < ax.nst; i++) {
+        const MxStage s = ax.s[DIT ? ax.nst - 1 - i : i];
+        const int total = nl * s.nb;
+        switch (s.R) {
+        case 2: stage<2, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 3: stage<3, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 4: stage<4, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 5: stage<5, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 6: stage<6, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 7: stage<7, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 8: stage<8, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 9: stage<9, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 10: stage<10, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 11: stage_prime<11, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 12: stage<12, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 13: stage_prime<13, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 15: stage<15, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        case 16: stage<16, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+        default:
+            if constexpr (BIG) {
+                switch (s.R) {
+                case 17: stage_prime<17, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+                case 19: stage_prime<19, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+                case 23: stage_prime<23, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+                case 29: stage_prime<29, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+                case 31: stage_prime<31, C, DIT>(A, total, s, ax.LS, ax.sh); break;
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
 
 // ------------------------------------------------------------------ x passes
-// A CTA owns `rows` (a power of two) consecutive rows r = z ny + y of all
-// three components: 3 rows/2 complex lines, line comp R2 + p holding rows
-// 2p and 2p + 1 as real and imaginary parts.
+// A CTA owns `rows` (even) consecutive rows r = z ny + y of all three
+// components: 3 R2 complex lines (R2 = rows / 2), line comp R2 + p holding
+// rows 2p and 2p + 1 as real and imaginary parts.  Shared memory: twiddles
+// [n], the places of kx (low half) and n - kx (high half) [n / 2 + 1], lines.
 struct RowCta {
     int row0, here;   // first row, rows that exist
 };
@@ -234,12 +323,22 @@ __device__ __forceinline__ RowCta row_cta(const MxX& m)
     c.here = min(m.rows, m.nr - c.row0);
     return c;
 }
+template <typename C> __device__ __forceinline__ int* places(const MxAxis& ax)
+{
+    return reinterpret_cast<int*>(reinterpret_cast<C*>(mx_sm) + ax.n);
+}
+// element where the lines start (the table of places before them)
+template <typename C> __device__ __forceinline__ int lines_at(const MxAxis& ax)
+{
+    return ax.n + ((ax.n / 2 + 1) * (int)sizeof(int) + (int)sizeof(C) - 1) / (int)sizeof(C);
+}
 
-// SPEC rows -> Hermitian lines, parts swapped for the inverse transform
+// SPEC rows -> the conjugates of Hermitian lines
 template <typename C>
 __device__ __forceinline__ void load_lines(const MxX& m, const RowCta& rc, const C* __restrict__ spec, int A)
 {
     C* sm = reinterpret_cast<C*>(mx_sm);
+    const int* at = places<C>(m.ax);
     const int R2 = m.rows >> 1, n3 = 3 * R2, total = m.Kx * n3;
     constexpr int U = 4;   // row pairs in flight per thread
     for (int i0 = threadIdx.x; i0 < total; i0 += U * blockDim.x) {
@@ -250,7 +349,7 @@ __device__ __forceinline__ void load_lines(const MxX& m, const RowCta& rc, const
             a[u] = b[u] = cmk<C>(0, 0);
             if (idx < total) {
                 const int kx = qdiv(idx, m.m3r2), rem = idx - kx * n3;
-                const int comp = rem >> m.r2sh, p = rem & (R2 - 1);
+                const int comp = qdiv(rem, m.mr2), p = rem - comp * R2;
                 const C* src = spec + ((size_t)kx * 3 + comp) * m.nr + rc.row0 + 2 * p;
                 if (2 * p < rc.here) a[u] = src[0];
                 if (2 * p + 1 < rc.here) b[u] = src[1];
@@ -262,55 +361,70 @@ __device__ __forceinline__ void load_lines(const MxX& m, const RowCta& rc, const
             if (idx >= total) break;
             const int kx = qdiv(idx, m.m3r2), l = idx - kx * n3;
             C* Z = sm + A + l * m.ax.LS;
-            // Z[k] = S_2p[k] + i S_2p+1[k], Z[Px - k] from the conjugates
-            Z[pd<C>(kx)] = cmk<C>(a[u].y + b[u].x, a[u].x - b[u].y);
-            if (kx > 0 && 2 * kx < m.ax.n) Z[pd<C>(m.ax.n - kx)] = cmk<C>(b[u].x - a[u].y, a[u].x + b[u].y);
+            // conj of Z[k] = S_2p[k] + i S_2p+1[k]; Z[n - k] from the
+            // conjugate spectra
+            const int pp = at[kx];
+            Z[pp & 0xffff] = cmk<C>(a[u].x - b[u].y, -(a[u].y + b[u].x));
+            if (kx > 0 && 2 * kx < m.ax.n) Z[pp >> 16] = cmk<C>(a[u].x + b[u].y, a[u].y - b[u].x);
         }
     }
 }
 
 // Transformed lines -> the two rows' spectra to SPEC
 template <typename C>
-__device__ __forceinline__ void store_spec(const MxX& m, const RowCta& rc, int Q, C* __restrict__ spec)
+__device__ __forceinline__ void store_spec(const MxX& m, const RowCta& rc, int A, C* __restrict__ spec)
 {
     typedef decltype(C().x) R;
     const C* sm = reinterpret_cast<const C*>(mx_sm);
+    const int* at = places<C>(m.ax);
     const int R2 = m.rows >> 1, n3 = 3 * R2, total = m.Kx * n3;
     for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
         const int kx = qdiv(idx, m.m3r2), l = idx - kx * n3;
-        const int comp = l >> m.r2sh, p = l & (R2 - 1);
-        const C* Z = sm + Q + l * m.ax.LS;
-        const C zk = Z[pd<C>(kx)], zn = Z[pd<C>(kx ? m.ax.n - kx : 0)];
+        const int comp = qdiv(l, m.mr2), p = l - comp * R2;
+        const C* Z = sm + A + l * m.ax.LS;
+        const int pp = at[kx];
+        const C zk = Z[pp & 0xffff], zn = Z[pp >> 16];
         C* dst = spec + ((size_t)kx * 3 + comp) * m.nr + rc.row0 + 2 * p;
         if (2 * p < rc.here) dst[0] = cmk<C>((R)0.5 * (zk.x + zn.x), (R)0.5 * (zk.y - zn.y));
         if (2 * p + 1 < rc.here) dst[1] = cmk<C>((R)0.5 * (zk.y + zn.y), (R)0.5 * (zn.x - zk.x));
     }
 }
 
+// twiddles and (at: global) the places of an axis to shared memory
 template <typename C>
-__device__ __forceinline__ void load_twiddles(const MxAxis& ax, const C* __restrict__ tw)
+__device__ __forceinline__ void load_tables(const MxAxis& ax, const C* __restrict__ tw, const int* __restrict__ at)
 {
     C* sm = reinterpret_cast<C*>(mx_sm);
-    for (int k = threadIdx.x; k < ax.n; k += blockDim.x) sm[k] = tw[k];
+    for (int k = threadIdx.x; k < ax.n; k += blockDim.x) {
+        sm[k] = tw[k];
+        if (at && k <= ax.n / 2) places<C>(ax)[k] = at[k];
+    }
 }
 
 } // namespace mx
 
+// CTAs of 256 threads per SM the registers allow
+// (x passes), and the threads of a (y,z) CTA
+template <typename R, bool BIG> struct Occ {
+    static constexpr int X = sizeof(R) == 4 ? (BIG ? 2 : 3) : (BIG ? 1 : 2);
+    static constexpr int YZ = sizeof(R) == 8 && BIG ? 256 : 512;
+};
+
 // Forward x transform of the spins to SPEC.
-template <typename R>
-__global__ void __launch_bounds__(256, 2) k_mx_fx(const __grid_constant__ MxX m, const typename CT<R>::T* __restrict__ tw,
+template <typename R, bool BIG>
+__global__ void __launch_bounds__(256, Occ<R, BIG>::X) k_mx_fx(const __grid_constant__ MxX m, const typename CT<R>::T* __restrict__ tw,
                                                   const R* __restrict__ sx, const R* __restrict__ sy,
                                                   const R* __restrict__ sz, typename CT<R>::T* __restrict__ spec)
 {
     typedef typename CT<R>::T C;
     using namespace mx;
-    load_twiddles<C>(m.ax, tw);
+    load_tables<C>(m.ax, tw, m.at);
     pdl_trigger();
     pdl_wait();
     if (m.run_if && *m.run_if == 0) return;
     C* sm = reinterpret_cast<C*>(mx_sm);
     const RowCta rc = row_cta(m);
-    const int R2 = m.rows >> 1, A = m.ax.n, B = A + 3 * R2 * m.ax.LS;
+    const int R2 = m.rows >> 1, A = lines_at<C>(m.ax);
     const int total = m.rows * m.ax.n;
     for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
         const int row = qdiv(idx, m.mPx), x = idx - row * m.ax.n;
@@ -321,39 +435,147 @@ __global__ void __launch_bounds__(256, 2) k_mx_fx(const __grid_constant__ MxX m,
         }
 #pragma unroll
         for (int c = 0; c < 3; c++)
-            reinterpret_cast<R*>(sm + A + (c * R2 + (row >> 1)) * m.ax.LS + pd<C>(x))[row & 1] = v[c];
+            reinterpret_cast<R*>(sm + A + (c * R2 + (row >> 1)) * m.ax.LS + pd(m.ax, x))[row & 1] = v[c];
     }
     __syncthreads();
-    const int Q = fft<C>(A, B, 3 * R2, m.ax);
-    store_spec<C>(m, rc, Q, spec);
+    fft<C, false, BIG>(A, 3 * R2, m.ax);
+    store_spec<C>(m, rc, A, spec);
 }
 
 // Inverse x transform of SPEC to the field.
-template <typename R>
-__global__ void __launch_bounds__(256, 2) k_mx_ix(const __grid_constant__ MxX m, const typename CT<R>::T* __restrict__ tw,
+template <typename R, bool BIG>
+__global__ void __launch_bounds__(256, Occ<R, BIG>::X) k_mx_ix(const __grid_constant__ MxX m, const typename CT<R>::T* __restrict__ tw,
                                                   const typename CT<R>::T* __restrict__ spec, R* __restrict__ hx,
                                                   R* __restrict__ hy, R* __restrict__ hz)
 {
     typedef typename CT<R>::T C;
     using namespace mx;
-    load_twiddles<C>(m.ax, tw);
+    load_tables<C>(m.ax, tw, m.at);
     pdl_trigger();
     pdl_wait();
     if (m.run_if && *m.run_if == 0) return;
     const C* sm = reinterpret_cast<const C*>(mx_sm);
     const RowCta rc = row_cta(m);
-    const int R2 = m.rows >> 1, A = m.ax.n, B = A + 3 * R2 * m.ax.LS;
+    const int R2 = m.rows >> 1, A = lines_at<C>(m.ax);
+    __syncthreads();
     load_lines<C>(m, rc, spec, A);
     __syncthreads();
-    const int Q = fft<C>(A, B, 3 * R2, m.ax);
-    const int total = rc.here * m.nx;
+    fft<C, true, BIG>(A, 3 * R2, m.ax);
+    const int total = rc.here * m.nx, cs = 2 * R2 * m.ax.LS;
     for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
         const int row = qdiv(idx, m.mnx), x = idx - row * m.nx;
         const size_t i = (size_t)(rc.row0 + row) * m.nx + x;
-        const R* z = reinterpret_cast<const R*>(sm + Q + (row >> 1) * m.ax.LS + pd<C>(x)) + ((row & 1) ^ 1);
-        const int cs = 2 * R2 * m.ax.LS;
-        hx[i] = z[0]; hy[i] = z[cs]; hz[i] = z[2 * cs];
+        const R* z = reinterpret_cast<const R*>(sm + A + (row >> 1) * m.ax.LS + pd(m.ax, x)) + (row & 1);
+        const R s = (row & 1) ? (R)-1 : (R)1;   // conjugate
+        hx[i] = s * z[0]; hy[i] = s * z[cs]; hz[i] = s * z[2 * cs];
     }
+}
+
+// ------------------------------------------------------------------ fused x pass of a step
+// The CTA's rows through the inverse x transform (-> their dipole field,
+// written to its slot), the field terms and LLG update of their sites (-> the
+// new spins; neighbours read from the current spin arrays, which no CTA
+// writes) and the forward x transform of the new spins (-> the next step's
+// spectrum rows, the ones the CTA itself read).  site(i, x, y, z, A) returns
+// the new spin of site i in the dipole field A.
+namespace mx {
+// captured steps: the next step's block (the other of the pair; no kernel
+// of this step reads it)
+__device__ __forceinline__ void next_block(const DevStep* cu, DevStep* nx)
+{
+    if (nx && blockIdx.x == 0 && threadIdx.x == 0) {
+        nx->th_counter = cu->th_counter + 1ull;
+        for (int a = 0; a < 3; a++) {
+            nx->B[a] = cu->B[a] + cu->dB[a];
+            nx->dB[a] = cu->dB[a];
+        }
+    }
+}
+
+template <typename R, bool BIG, class F>
+__device__ __forceinline__ void step_rows(const MxX& m, typename CT<R>::T* __restrict__ spec, R* __restrict__ hx,
+                                          R* __restrict__ hy, R* __restrict__ hz, R* __restrict__ ox,
+                                          R* __restrict__ oy, R* __restrict__ oz, F&& site)
+{
+    typedef typename CT<R>::T C;
+    C* sm = reinterpret_cast<C*>(mx_sm);
+    const RowCta rc = row_cta(m);
+    const int R2 = m.rows >> 1, LS = m.ax.LS, A = lines_at<C>(m.ax);
+    __syncthreads();
+    load_lines<C>(m, rc, spec, A);
+    __syncthreads();
+    fft<C, true, BIG>(A, 3 * R2, m.ax);
+    const int zr0 = rc.row0 / m.ny, yr0 = rc.row0 - zr0 * m.ny;
+    const int total = m.rows * m.ax.n, cs = 2 * R2 * LS;
+    // a thread reads the field of its row and x and puts the new spin in the
+    // same places
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+        const int row = qdiv(idx, m.mPx), x = idx - row * m.ax.n;
+        R* q = reinterpret_cast<R*>(sm + A + (row >> 1) * LS + pd(m.ax, x)) + (row & 1);
+        V3<R> o = v3<R>(0, 0, 0);
+        if (x < m.nx && row < rc.here) {
+            const R s = (row & 1) ? (R)-1 : (R)1;   // conjugate
+            const V3<R> Ad = v3<R>(s * q[0], s * q[cs], s * q[2 * cs]);
+            int z = zr0, y = yr0 + row;
+            while (y >= m.ny) { y -= m.ny; z++; }
+            const int i = (rc.row0 + row) * m.nx + x;
+            hx[i] = Ad.x; hy[i] = Ad.y; hz[i] = Ad.z;
+            o = site(i, x, y, z, Ad);
+            ox[i] = o.x; oy[i] = o.y; oz[i] = o.z;
+        }
+        q[0] = o.x; q[cs] = o.y; q[2 * cs] = o.z;
+    }
+    __syncthreads();
+    fft<C, false, BIG>(A, 3 * R2, m.ax);
+    store_spec<C>(m, rc, A, spec);
+}
+} // namespace mx
+
+// Uniform parameters (FastKT).
+template <typename R, int LT, bool ANI, bool TH, bool BIG>
+__global__ void __launch_bounds__(256, Occ<R, BIG>::X) k_mx_step(const __grid_constant__ MxX m, const __grid_constant__ FastKT<R> F,
+                                                    const typename CT<R>::T* __restrict__ tw,
+                                                    typename CT<R>::T* __restrict__ spec, const R* __restrict__ sx,
+                                                    const R* __restrict__ sy, const R* __restrict__ sz,
+                                                    R* __restrict__ hx, R* __restrict__ hy, R* __restrict__ hz,
+                                                    R* __restrict__ ox, R* __restrict__ oy, R* __restrict__ oz)
+{
+    mx::load_tables<typename CT<R>::T>(m.ax, tw, m.at);
+    pdl_trigger();
+    pdl_wait();
+    mx::next_block(F.adv_cur, F.adv_next);
+    mx::step_rows<R, BIG>(m, spec, hx, hy, hz, ox, oy, oz, [&](int i, int x, int y, int z, V3<R> A) {
+        V3<R> o;
+        fused_site_v<LT, true, ANI, TH, true, R>(F, m.nx, m.ny, m.nz, x, y, z, i, sx, sy, sz, A.x, A.y, A.z, o.x, o.y,
+                                                 o.z);
+        return o;
+    });
+}
+
+// Per-site parameters, pathway lists, further addends (FusedK): P.terms
+// without the dipole addend, whose weight is addw.
+template <typename R, bool BIG>
+__global__ void __launch_bounds__(256, BIG && sizeof(R) == 8 ? 1 : 2) k_mx_gstep(const __grid_constant__ MxX m, const __grid_constant__ FusedK P,
+                                                     double addw, double dt_sys, const DevStep* cur, DevStep* next,
+                                                     const typename CT<R>::T* __restrict__ tw,
+                                                     typename CT<R>::T* __restrict__ spec, R* __restrict__ hx,
+                                                     R* __restrict__ hy, R* __restrict__ hz)
+{
+    mx::load_tables<typename CT<R>::T>(m.ax, tw, m.at);
+    pdl_trigger();
+    pdl_wait();
+    mx::next_block(cur, next);
+    mx::step_rows<R, BIG>(m, spec, hx, hy, hz, static_cast<R*>(P.ox), static_cast<R*>(P.oy), static_cast<R*>(P.oz),
+                     [&](int i, int, int, int, V3<R> A) {
+                         const R ms = ms_at<R>(P.sys, i);
+                         Fields<R> F;
+                         if (ms > (R)0) {
+                             F = eval_terms<R>(P.terms, P.sys, (R)dt_sys, i);
+                             F.H = fma3((R)addw, A, F.H);
+                         }
+                         return step_site<R>(P, F, spin_at<R>(P.sys, i), ms, i);
+                     });
 }
 
 // ------------------------------------------------------------------ (y,z) pass
@@ -362,9 +584,10 @@ __global__ void __launch_bounds__(256, 2) k_mx_ix(const __grid_constant__ MxX m,
 // T_ab(dz) real and even in dz, or (exactly one of a, b is z) i times a real
 // odd function.  tz: [kx][dz][6][ky].  One thread per (a, ky) keeps all NZ
 // sums in registers (each spectrum value is read once per component, each
-// tensor value once per thread); NZ = 0: one thread per (a, zt, ky).
-template <typename R, int NZ>
-__global__ void __launch_bounds__(512, 1) k_mx_yz(const __grid_constant__ MxYZ m, const typename CT<R>::T* __restrict__ tw,
+// tensor value once per thread); NZ = 0: one thread per (a, zt, ky).  ky: the
+// digit-reversed places the transforms leave, in which tz is stored.
+template <typename R, int NZ, bool BIG>
+__global__ void __launch_bounds__(Occ<R, BIG>::YZ, 1) k_mx_yz(const __grid_constant__ MxYZ m, const typename CT<R>::T* __restrict__ tw,
                                                   typename CT<R>::T* __restrict__ spec, const R* __restrict__ tz)
 {
     typedef typename CT<R>::T C;
@@ -378,104 +601,114 @@ __global__ void __launch_bounds__(512, 1) k_mx_yz(const __grid_constant__ MxYZ m
         if ((((uintptr_t)T) & 15) == 0 && (bytes & 15) == 0)
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(T), "r"(bytes) : "memory");
     }
-    load_twiddles<C>(m.ax, tw);
+    load_tables<C>(m.ax, tw, nullptr);
     pdl_trigger();
     pdl_wait();
     if (m.run_if && *m.run_if == 0) return;
     C* sm = reinterpret_cast<C*>(mx_sm);
-    const int A = Py, B = A + nl * LS;
+    const int A = Py;
     C* sp = spec + (size_t)kx * nl * ny;
     constexpr int U = 4;
     {
         const int total = nl * Py;
         for (int i0 = threadIdx.x; i0 < total; i0 += U * blockDim.x) {
             C v[U];
+            int at[U];
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const int idx = i0 + u * blockDim.x;
                 const int l = qdiv(idx, m.mPy), y = idx - l * Py;
                 v[u] = idx < total && y < ny ? sp[l * ny + y] : cmk<C>(0, 0);
+                at[u] = A + l * LS + pd(m.ax, y);
             }
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int idx = i0 + u * blockDim.x;
-                const int l = qdiv(idx, m.mPy), y = idx - l * Py;
-                if (idx < total) sm[A + l * LS + pd<C>(y)] = v[u];
-            }
+            for (int u = 0; u < U; u++)
+                if (i0 + u * blockDim.x < total) sm[at[u]] = v[u];
         }
     }
     __syncthreads();
-    const int P = fft<C>(A, B, nl, m.ax);
-    const int Hb = P == A ? B : A;
+    fft<C, false, BIG>(A, nl, m.ax);
+    // columns (places of the digit-reversed ky), as many at a time as the
+    // CTA's threads cover whole: all of them are read before any is written
     const R g = (R)m.g;
-    if constexpr (NZ > 0) {
-        for (int idx = threadIdx.x; idx < 3 * Py; idx += blockDim.x) {
-            const int a = idx >= 2 * Py ? 2 : (idx >= Py ? 1 : 0), ky = idx - a * Py, kp = pd<C>(ky);
+    const int per = NZ > 0 ? 3 : nl, cols = blockDim.x / per;
+    const int w = qdiv(threadIdx.x, m.mcols), c = threadIdx.x - w * cols;   // component (and layer), column
+    for (int k0 = 0; k0 < Py; k0 += cols) {
+        const int ky = k0 + c, kp = pd(m.ax, ky);
+        const bool act = w < per && ky < Py;
+        if constexpr (NZ > 0) {
+            const int a = w;
             C acc[NZ];
 #pragma unroll
             for (int z = 0; z < NZ; z++) acc[z] = cmk<C>(0, 0);
+            if (act) {
 #pragma unroll
-            for (int b = 0; b < 3; b++) {
-                const int lo = min(a, b), hi = max(a, b);
-                const int q = lo == 0 ? hi : lo + hi + 1;   // XX XY XZ YY YZ ZZ
-                const bool odd = (a == 2) != (b == 2);
-                R t[NZ], tn[NZ];
+                for (int b = 0; b < 3; b++) {
+                    const int lo = min(a, b), hi = max(a, b);
+                    const int q = lo == 0 ? hi : lo + hi + 1;   // XX XY XZ YY YZ ZZ
+                    const bool odd = (a == 2) != (b == 2);
+                    R t[NZ], tn[NZ];
 #pragma unroll
-                for (int d = 0; d < NZ; d++) {
-                    t[d] = __ldg(T + (d * 6 + q) * Py + ky);
-                    tn[d] = odd ? -t[d] : t[d];
-                }
+                    for (int d = 0; d < NZ; d++) {
+                        t[d] = __ldg(T + (d * 6 + q) * Py + ky);
+                        tn[d] = odd ? -t[d] : t[d];
+                    }
 #pragma unroll
-                for (int zs = 0; zs < NZ; zs++) {
-                    const C v = sm[P + (b * NZ + zs) * LS + kp];
-                    const C s = odd ? cmk<C>(-v.y, v.x) : v;
+                    for (int zs = 0; zs < NZ; zs++) {
+                        const C v = sm[A + (b * NZ + zs) * LS + kp];
+                        const C s = odd ? cmk<C>(-v.y, v.x) : v;
 #pragma unroll
-                    for (int zt = 0; zt < NZ; zt++) {
-                        const R w = zt >= zs ? t[zt - zs] : tn[zs - zt];
-                        acc[zt].x += w * s.x;
-                        acc[zt].y += w * s.y;
+                        for (int zt = 0; zt < NZ; zt++) {
+                            const R u = zt >= zs ? t[zt - zs] : tn[zs - zt];
+                            acc[zt].x += u * s.x;
+                            acc[zt].y += u * s.y;
+                        }
                     }
                 }
             }
+            __syncthreads();
+            if (act) {
 #pragma unroll
-            for (int z = 0; z < NZ; z++) sm[Hb + (a * NZ + z) * LS + kp] = cmk<C>(g * acc[z].y, g * acc[z].x);
-        }
-    } else {
-        for (int idx = threadIdx.x; idx < nl * Py; idx += blockDim.x) {
-            const int l = qdiv(idx, m.mPy), ky = idx - l * Py, kp = pd<C>(ky);
-            const int a = l / nz, zt = l - a * nz;
+                for (int z = 0; z < NZ; z++) sm[A + (a * NZ + z) * LS + kp] = cmk<C>(g * acc[z].x, -(g * acc[z].y));
+            }
+        } else {
+            const int a = w / nz, zt = w - a * nz;
             C acc = cmk<C>(0, 0);
-            for (int b = 0; b < 3; b++) {
-                const int lo = min(a, b), hi = max(a, b);
-                const int q = lo == 0 ? hi : lo + hi + 1;
-                const bool odd = (a == 2) != (b == 2);
-                for (int zs = 0; zs < nz; zs++) {
-                    const int dz = zt - zs;
-                    R w = __ldg(T + (abs(dz) * 6 + q) * Py + ky);
-                    if (odd && dz < 0) w = -w;
-                    const C v = sm[P + (b * nz + zs) * LS + kp];
-                    acc.x += w * (odd ? -v.y : v.x);
-                    acc.y += w * (odd ? v.x : v.y);
+            if (act) {
+                for (int b = 0; b < 3; b++) {
+                    const int lo = min(a, b), hi = max(a, b);
+                    const int q = lo == 0 ? hi : lo + hi + 1;
+                    const bool odd = (a == 2) != (b == 2);
+                    for (int zs = 0; zs < nz; zs++) {
+                        const int dz = zt - zs;
+                        R u = __ldg(T + (abs(dz) * 6 + q) * Py + ky);
+                        if (odd && dz < 0) u = -u;
+                        const C v = sm[A + (b * nz + zs) * LS + kp];
+                        acc.x += u * (odd ? -v.y : v.x);
+                        acc.y += u * (odd ? v.x : v.y);
+                    }
                 }
             }
-            sm[Hb + l * LS + kp] = cmk<C>(g * acc.y, g * acc.x);
+            __syncthreads();
+            if (act) sm[A + w * LS + kp] = cmk<C>(g * acc.x, -(g * acc.y));
         }
     }
     __syncthreads();
-    const int Q = fft<C>(Hb, P, nl, m.ax);
+    fft<C, true, BIG>(A, nl, m.ax);
     for (int idx = threadIdx.x; idx < nl * ny; idx += blockDim.x) {
         const int l = qdiv(idx, m.mny), y = idx - l * ny;
-        sp[idx] = swp(sm[Q + l * LS + pd<C>(y)]);
+        sp[idx] = cconj(sm[A + l * LS + pd(m.ax, y)]);
     }
 }
 
 // ------------------------------------------------------------------ tensor
 // T(kx, ky, dz) of six components from their FP64 transforms over x and y,
-// W[q][z][ky][kx] (z = dz mod Pz): tz[kx][dz][q][ky], the real part or (XZ,
-// YZ) the imaginary part.  stat: bits of the largest |W| and of the largest
+// W[q][z][ky][kx] (z = dz mod Pz): tz[kx][dz][q][at[ky]], the real part or (XZ,
+// YZ) the imaginary part, ky at its place after the y transform.  stat: bits of the largest |W| and of the largest
 // deviation from the parities the layer sum relies on.
 template <typename R>
-__global__ void k_mx_pack(const double2* W, int Px, int Py, int Pz, int nz, int Kx, R* tz, unsigned long long* stat)
+__global__ void k_mx_pack(const double2* W, int Px, int Py, int Pz, int nz, int Kx, const int* at, R* tz,
+                          unsigned long long* stat)
 {
     const long long total = (long long)Kx * nz * 6 * Py;
     double big = 0, dev = 0;
@@ -491,7 +724,7 @@ __global__ void k_mx_pack(const double2* W, int Px, int Py, int Pz, int nz, int 
         const double2 v = Wq[((size_t)dz * Py + ky) * Px + kx];
         const double2 u = Wq[((size_t)((Pz - dz) % Pz) * Py + ky) * Px + kx];
         const bool odd = q == 2 || q == 4;
-        tz[(((size_t)kx * nz + dz) * 6 + q) * Py + ky] = (R)(odd ? v.y : v.x);
+        tz[(((size_t)kx * nz + dz) * 6 + q) * Py + at[ky]] = (R)(odd ? v.y : v.x);
         big = fmax(big, fmax(fabs(v.x), fabs(v.y)));
         dev = fmax(dev, odd ? fmax(fmax(fabs(v.x), fabs(u.x)), fabs(v.y + u.y))
                             : fmax(fmax(fabs(v.y), fabs(u.y)), fabs(v.x - u.x)));
@@ -556,88 +789,166 @@ static double mx_best(int n, int total, bool f64, std::vector<int>& out)
     return best;
 }
 
-// The stages of an axis of n points of which a CTA holds nl lines; false when
-// n has a prime factor above 31.
-static bool mx_axis(int n, int nl, bool f64, MxAxis& ax)
+// Wavefronts of the axis' shared-memory accesses with padding shift sh: the
+// first warps of every stage, elements of eb bytes.
+static int mx_conflicts(const MxAxis& ax, int sh, int nl, int eb)
+{
+    const int lanes = 128 / eb, LS = ax.n + (ax.n >> sh);
+    int sum = 0;
+    for (int i = 0; i < ax.nst; i++) {
+        const MxStage& s = ax.s[i];
+        const int total = std::min(nl * s.nb, 128);
+        for (int w = 0; w < total; w += lanes)
+            for (int r = 0; r < s.R; r++) {
+                int hit[16] = {0}, worst = 0;
+                for (int t = w; t < std::min(w + lanes, total); t++) {
+                    const int l = t / s.nb, q = t % s.nb, p = (q / s.m) * s.m * s.R + q % s.m + r * s.m;
+                    worst = std::max(worst, ++hit[(l * (LS | 1) + p + (p >> sh)) % lanes]);
+                }
+                sum += worst;
+            }
+    }
+    return sum;
+}
+
+// The stages of an axis of n points of which a CTA holds nl lines, their
+// padding, and the place of each frequency after the forward transform (into
+// *at); false when n has a prime factor above 31.
+static bool mx_axis(int n, int nl, bool f64, MxAxis& ax, std::vector<int>* at)
 {
     std::vector<int> r;
     if (mx_best(n, nl * n, f64, r) >= 1e300 || (int)r.size() > MX_MAX_STAGES) return false;
+    memset(&ax, 0, sizeof(ax));
     ax.n = n;
     ax.nst = (int)r.size();
-    const int sh = f64 ? 3 : 4;
-    ax.LS = n + (n >> sh) + 1;
-    int Ns = 1;
-    for (int i = 0; i < ax.nst; i++) {
-        MxStage& s = ax.s[i];
-        s.R = r[i];
-        s.nb = n / r[i];
-        s.Ns = Ns;
-        s.tws = n / (Ns * r[i]);
-        s.mnb = qmagic(s.nb);
-        s.mNs = qmagic(Ns);
-        Ns *= r[i];
+    ax.sh = 4;
+    ax.big = std::any_of(r.begin(), r.end(), [](int R) { return R > 16; });
+    // order and padding with the fewest bank conflicts; a large prime comes
+    // last, where its butterflies need no twiddles
+    std::sort(r.begin(), r.end());
+    int best = 1 << 30;
+    MxAxis t = ax;
+    do {
+        if (ax.big && r.back() <= 16) continue;
+        int len = n;   // points of a block
+        for (int i = 0; i < t.nst; i++) {
+            MxStage& s = t.s[i];
+            s.R = r[i];
+            s.nb = n / r[i];
+            s.m = len / r[i];
+            s.tws = n / len;
+            s.mnb = qmagic(s.nb);
+            s.mm = qmagic(s.m);
+            len = s.m;
+        }
+        for (int sh : {3, 4, 5, 30}) {
+            const int c = mx_conflicts(t, sh, nl, f64 ? 16 : 8);
+            if (c < best) {
+                best = c;
+                ax = t;
+                ax.sh = sh;
+            }
+        }
+    } while (std::next_permutation(r.begin(), r.end()));
+    ax.LS = (n + (n >> ax.sh)) | 1;   // odd: the same place of consecutive lines in different banks
+    if (at) {
+        at->resize(n);
+        for (int k = 0; k < n; k++) {
+            int q = k, p = 0;
+            for (int i = 0; i < ax.nst; i++) {
+                p += (q % ax.s[i].R) * ax.s[i].m;
+                q /= ax.s[i].R;
+            }
+            (*at)[k] = p;
+        }
     }
     return true;
 }
 
-static size_t mx_smem(const MxAxis& ax, int nl, int rb) { return ((size_t)ax.n + 2 * (size_t)nl * ax.LS) * 2 * rb; }
+static size_t mx_smem_x(const MxAxis& ax, int nl, int rb)
+{
+    const size_t cb = 2 * rb;
+    return ((size_t)ax.n + ((size_t)(ax.n / 2 + 1) * sizeof(int) + cb - 1) / cb + (size_t)nl * ax.LS) * cb;
+}
+static size_t mx_smem_y(const MxAxis& ax, int nl, int rb) { return ((size_t)ax.n + (size_t)nl * ax.LS) * 2 * rb; }
 
 constexpr size_t MX_SMEM = 227 * 1024;
 
-// Rows per CTA of the x passes: as few as keep the 148 SMs supplied (more
-// rows make longer contiguous runs of SPEC), within shared memory.
-bool mx_plan(const ConvK& c, int rb, MxPlan& p)
+// The x passes' plan.  Rows per CTA: the estimated time of the busiest SM,
+// waves of the CTAs it holds (a chain of latencies each) plus its share of the
+// work, in cycles; sizes near a multiple of 148 CTAs differ by a whole wave.
+static bool mx_plan_x(const ConvK& c, int rb, MxX& x, std::vector<int>& at)
 {
-    if (c.general || c.nrep != 1 || c.nz > 32) return false;
+    memset(&x, 0, sizeof(x));
+    if (c.nrep != 1 || c.Px > 8192) return false;
     const bool f64 = rb == 8;
-    memset(&p, 0, sizeof(p));
     const int nr = c.nz * c.ny;
-    if ((long long)c.Px * c.Py > (1 << 22) || c.Px > 8192 || c.Py > 8192) return false;
-    MxX& x = p.x;
-    if (!mx_axis(c.Py, 3 * c.nz, f64, p.yz.ax) || mx_smem(p.yz.ax, 3 * c.nz, rb) > MX_SMEM) return false;
-    int rows = 2;
-    while (rows < 16 && (nr + 2 * rows - 1) / (2 * rows) >= 148) rows *= 2;
-    for (;; rows /= 2) {
-        if (rows < 2) return false;
-        if (!mx_axis(c.Px, 3 * rows / 2, f64, x.ax)) return false;
-        if (mx_smem(x.ax, 3 * rows / 2, rb) <= MX_SMEM / (rows > 2 ? 2 : 1)) break;
+    double best = 1e300;
+    int rows = 0;
+    for (int r = 2; r <= 32; r += 2) {
+        MxAxis ax;
+        if (!mx_axis(c.Px, 3 * r / 2, f64, ax, nullptr)) return false;
+        const size_t sm = mx_smem_x(ax, 3 * r / 2, rb);
+        if (sm > MX_SMEM) break;
+        const int regs = f64 ? (ax.big ? 1 : 2) : (ax.big ? 2 : 3);
+        const int occ = std::max(1, std::min(regs, (int)(MX_SMEM / (sm + 1024))));
+        const int per_sm = ((nr + r - 1) / r + 147) / 148, sites = r * c.Px;
+        const double t = (double)((per_sm + occ - 1) / occ) * (5000.0 + 6.0 * sites) + 10.0 * per_sm * sites;
+        if (t < best) { best = t; rows = r; }
+        if (r >= nr) break;
     }
+    if (!rows) return false;
+    mx_axis(c.Px, 3 * rows / 2, f64, x.ax, &at);
+    for (int& p : at) p += p >> x.ax.sh;
+    for (int k = 0; k <= c.Px / 2; k++) at[k] |= (k ? at[c.Px - k] : at[0]) << 16;
     x.nx = c.nx; x.ny = c.ny; x.nz = c.nz; x.nr = nr; x.Kx = c.Kx;
     x.rows = rows;
-    x.r2sh = rows == 2 ? 0 : (rows == 4 ? 1 : (rows == 8 ? 2 : 3));
     x.m3r2 = qmagic(3 * rows / 2);
+    x.mr2 = qmagic(rows / 2);
     x.mPx = qmagic(c.Px);
     x.mnx = qmagic(c.nx);
+    return true;
+}
+
+bool mx_plan(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vector<int>& at_y)
+{
+    memset(&p.yz, 0, sizeof(p.yz));
+    if (c.general || c.nrep != 1 || c.nz > 32 || c.Py > 8192) return false;
     MxYZ& y = p.yz;
+    const int nl = 3 * c.nz, pts = nl * c.Py;
+    if (!mx_axis(c.Py, nl, rb == 8, y.ax, &at_y) || mx_smem_y(y.ax, nl, rb) > MX_SMEM) return false;
+    if (!mx_plan_x(c, rb, p.x, at_x)) return false;
     y.ny = c.ny; y.nz = c.nz;
     y.mPy = qmagic(c.Py);
     y.mny = qmagic(c.ny);
-    const int pts = 3 * c.nz * c.Py;
-    y.threads = pts >= 4096 ? 512 : (pts >= 1024 ? 256 : 128);
+    y.threads = pts >= 4096 && !(rb == 8 && y.ax.big) ? 512 : (pts >= 1024 ? 256 : 128);
+    y.mcols = qmagic(y.threads / (c.nz <= 8 ? 3 : nl));
     return true;
 }
 
 size_t mx_tensor_bytes(const ConvK& c, int rb) { return (size_t)c.Kx * c.nz * 6 * c.Py * rb; }
 
-cudaError_t launch_mx_pack(const double2* W, const ConvK& c, void* tz, unsigned long long* stat2, int rb,
+cudaError_t launch_mx_pack(const double2* W, const ConvK& c, const int* at, void* tz, unsigned long long* stat2, int rb,
                            cudaStream_t st)
 {
     const long long total = (long long)c.Kx * c.nz * 6 * c.Py;
     const unsigned nb = (unsigned)std::min<long long>((total + 255) / 256, 148 * 8);
     if (rb == 8)
-        k_mx_pack<double><<<nb, 256, 0, st>>>(W, c.Px, c.Py, c.Pz, c.nz, c.Kx, static_cast<double*>(tz), stat2);
+        k_mx_pack<double><<<nb, 256, 0, st>>>(W, c.Px, c.Py, c.Pz, c.nz, c.Kx, at, static_cast<double*>(tz),
+                                              stat2);
     else
-        k_mx_pack<float><<<nb, 256, 0, st>>>(W, c.Px, c.Py, c.Pz, c.nz, c.Kx, static_cast<float*>(tz), stat2);
+        k_mx_pack<float><<<nb, 256, 0, st>>>(W, c.Px, c.Py, c.Pz, c.nz, c.Kx, at, static_cast<float*>(tz),
+                                             stat2);
     return cudaGetLastError();
 }
 
 template <typename R>
-static cudaError_t mx_fx(const MxX& x, const MxPlan& p, const typename CT<R>::T* tw, const void* const s[3],
+static cudaError_t mx_fx(const MxX& x, const typename CT<R>::T* tw, const void* const s[3],
                          typename CT<R>::T* spec, cudaStream_t st)
 {
     Prof pf("k_conv_fx", st);
-    return launch_pdl(k_mx_fx<R>, dim3((x.nr + x.rows - 1) / x.rows), dim3(256),
-                      mx_smem(x.ax, 3 * x.rows / 2, sizeof(R)), st, x, tw, static_cast<const R*>(s[0]),
+    return launch_pdl(x.ax.big ? k_mx_fx<R, true> : k_mx_fx<R, false>, dim3((x.nr + x.rows - 1) / x.rows), dim3(256),
+                      mx_smem_x(x.ax, 3 * x.rows / 2, sizeof(R)), st, x, tw, static_cast<const R*>(s[0]),
                       static_cast<const R*>(s[1]), static_cast<const R*>(s[2]), spec);
 }
 
@@ -646,33 +957,35 @@ static cudaError_t mx_ix(const MxX& x, const typename CT<R>::T* tw, const typena
                          cudaStream_t st)
 {
     Prof pf("k_conv_ix", st);
-    return launch_pdl(k_mx_ix<R>, dim3((x.nr + x.rows - 1) / x.rows), dim3(256),
-                      mx_smem(x.ax, 3 * x.rows / 2, sizeof(R)), st, x, tw, spec, static_cast<R*>(h[0]),
+    return launch_pdl(x.ax.big ? k_mx_ix<R, true> : k_mx_ix<R, false>, dim3((x.nr + x.rows - 1) / x.rows), dim3(256),
+                      mx_smem_x(x.ax, 3 * x.rows / 2, sizeof(R)), st, x, tw, spec, static_cast<R*>(h[0]),
                       static_cast<R*>(h[1]), static_cast<R*>(h[2]));
 }
 
-template <typename R>
-static void (*yz_kernel(int nz))(MxYZ, const typename CT<R>::T*, typename CT<R>::T*, const R*)
+template <typename R, bool BIG>
+static void (*yz_kernel_b(int nz))(MxYZ, const typename CT<R>::T*, typename CT<R>::T*, const R*)
 {
     switch (nz) {
-    case 1: return k_mx_yz<R, 1>;
-    case 2: return k_mx_yz<R, 2>;
-    case 3: return k_mx_yz<R, 3>;
-    case 4: return k_mx_yz<R, 4>;
-    case 5: return k_mx_yz<R, 5>;
-    case 6: return k_mx_yz<R, 6>;
-    case 7: return k_mx_yz<R, 7>;
-    case 8: return k_mx_yz<R, 8>;
+    case 1: return k_mx_yz<R, 1, BIG>;
+    case 2: return k_mx_yz<R, 2, BIG>;
+    case 3: return k_mx_yz<R, 3, BIG>;
+    case 4: return k_mx_yz<R, 4, BIG>;
+    case 5: return k_mx_yz<R, 5, BIG>;
+    case 6: return k_mx_yz<R, 6, BIG>;
+    case 7: return k_mx_yz<R, 7, BIG>;
+    case 8: return k_mx_yz<R, 8, BIG>;
     }
-    return k_mx_yz<R, 0>;
+    return k_mx_yz<R, 0, BIG>;
 }
+template <typename R>
+static auto yz_kernel(int nz, bool big) { return big ? yz_kernel_b<R, true>(nz) : yz_kernel_b<R, false>(nz); }
 
 template <typename R>
 static cudaError_t mx_yz(const ConvK& c, const MxYZ& y, const typename CT<R>::T* tw, typename CT<R>::T* spec,
                          const R* tz, cudaStream_t st)
 {
     Prof pf("k_conv_yz", st);
-    return launch_pdl(yz_kernel<R>(c.nz), dim3(c.Kx), dim3(y.threads), mx_smem(y.ax, 3 * c.nz, sizeof(R)), st, y, tw,
+    return launch_pdl(yz_kernel<R>(c.nz, y.ax.big), dim3(c.Kx), dim3(y.threads), mx_smem_y(y.ax, 3 * c.nz, sizeof(R)), st, y, tw,
                       spec, tz);
 }
 
@@ -688,7 +1001,7 @@ static cudaError_t mx_conv_t(const ConvK& c, const MxPlan& p, const FftLen L[3],
     x.run_if = y.run_if = c.run_if;
     y.g = c.g;
     cudaError_t e = cudaSuccess;
-    if (fx && (e = mx_fx<R>(x, p, tw + L[0].tw_off, s, spec, st)) != cudaSuccess) return e;
+    if (fx && (e = mx_fx<R>(x, tw + L[0].tw_off, s, spec, st)) != cudaSuccess) return e;
     if ((e = mx_yz<R>(c, y, tw + L[1].tw_off, spec, static_cast<const R*>(tz), st)) != cudaSuccess) return e;
     if (ix) e = mx_ix<R>(x, tw + L[0].tw_off, spec, h, st);
     return e;
@@ -701,20 +1014,84 @@ cudaError_t launch_mx_conv(const ConvK& c, const MxPlan& p, const FftLen L[3], c
     return mx_conv_t<float>(c, p, L, tw, s, spec, tz, h, fx, ix, st);
 }
 
+template <typename R>
+using StepKernel = void (*)(MxX, FastKT<R>, const typename CT<R>::T*, typename CT<R>::T*, const R*, const R*, const R*,
+                            R*, R*, R*, R*, R*, R*);
+
+template <typename R, bool BIG>
+static StepKernel<R> step_kernel_b(int llg, bool ani, bool th)
+{
+    if (llg == LLG_CART) {
+        if (ani) return th ? k_mx_step<R, LLG_CART, true, true, BIG> : k_mx_step<R, LLG_CART, true, false, BIG>;
+        return th ? k_mx_step<R, LLG_CART, false, true, BIG> : k_mx_step<R, LLG_CART, false, false, BIG>;
+    }
+    if (ani) return th ? k_mx_step<R, LLG_QUAT, true, true, BIG> : k_mx_step<R, LLG_QUAT, true, false, BIG>;
+    return th ? k_mx_step<R, LLG_QUAT, false, true, BIG> : k_mx_step<R, LLG_QUAT, false, false, BIG>;
+}
+template <typename R>
+static StepKernel<R> step_kernel(int llg, bool ani, bool th, bool big)
+{
+    return big ? step_kernel_b<R, true>(llg, ani, th) : step_kernel_b<R, false>(llg, ani, th);
+}
+
+template <typename R>
+cudaError_t launch_mx_step(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FastKT<R>& F,
+                           const R* const s[3], R* const h[3], R* const o[3], cudaStream_t st)
+{
+    typedef typename CT<R>::T C;
+    Prof pf("k_xstep", st);
+    return launch_pdl(step_kernel<R>(F.llg_type, F.ani != 0, F.th != 0, x.ax.big), dim3((x.nr + x.rows - 1) / x.rows), dim3(256),
+                      mx_smem_x(x.ax, 3 * x.rows / 2, sizeof(R)), st, x, F, static_cast<const C*>(tw) + L[0].tw_off,
+                      static_cast<C*>(spec), s[0], s[1], s[2], h[0], h[1], h[2], o[0], o[1], o[2]);
+}
+template cudaError_t launch_mx_step<float>(const MxX&, const FftLen[3], const void*, void*, const FastKT<float>&,
+                                           const float* const[3], float* const[3], float* const[3], cudaStream_t);
+template cudaError_t launch_mx_step<double>(const MxX&, const FftLen[3], const void*, void*, const FastKT<double>&,
+                                            const double* const[3], double* const[3], double* const[3], cudaStream_t);
+
+template <typename R>
+static cudaError_t mx_gstep_t(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FusedK& P, double addw,
+                              double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], cudaStream_t st)
+{
+    typedef typename CT<R>::T C;
+    Prof pf("k_xstep", st);
+    return launch_pdl(x.ax.big ? k_mx_gstep<R, true> : k_mx_gstep<R, false>, dim3((x.nr + x.rows - 1) / x.rows), dim3(256),
+                      mx_smem_x(x.ax, 3 * x.rows / 2, sizeof(R)), st, x, P, addw, dt_sys, cur, next,
+                      static_cast<const C*>(tw) + L[0].tw_off, static_cast<C*>(spec), static_cast<R*>(h[0]),
+                      static_cast<R*>(h[1]), static_cast<R*>(h[2]));
+}
+
+cudaError_t launch_mx_gstep(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FusedK& P, double addw,
+                            double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], int rb, cudaStream_t st)
+{
+    if (rb == 8) return mx_gstep_t<double>(x, L, tw, spec, P, addw, dt_sys, cur, next, h, st);
+    return mx_gstep_t<float>(x, L, tw, spec, P, addw, dt_sys, cur, next, h, st);
+}
+
+cudaError_t launch_mx_ix(const MxX& x, const FftLen L[3], const void* tw, const void* spec, void* const h[3], int rb,
+                         cudaStream_t st)
+{
+    if (rb == 8)
+        return mx_ix<double>(x, static_cast<const double2*>(tw) + L[0].tw_off, static_cast<const double2*>(spec), h, st);
+    return mx_ix<float>(x, static_cast<const float2*>(tw) + L[0].tw_off, static_cast<const float2*>(spec), h, st);
+}
+
 template <typename K>
 static cudaError_t mx_max_smem(K kern)
 {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MX_SMEM);
 }
 
-template <typename R>
+template <typename R, bool BIG>
 static cudaError_t mx_configure_t()
 {
     cudaError_t e;
-    if ((e = mx_max_smem(k_mx_fx<R>)) != cudaSuccess || (e = mx_max_smem(k_mx_ix<R>)) != cudaSuccess) return e;
+    if ((e = mx_max_smem(k_mx_fx<R, BIG>)) != cudaSuccess || (e = mx_max_smem(k_mx_ix<R, BIG>)) != cudaSuccess) return e;
     for (int nz = 0; nz <= 8; nz++)
-        if ((e = mx_max_smem(yz_kernel<R>(nz))) != cudaSuccess) return e;
-    return cudaSuccess;
+        if ((e = mx_max_smem(yz_kernel_b<R, BIG>(nz))) != cudaSuccess) return e;
+    for (int q = 0; q < 8; q++)
+        if ((e = mx_max_smem(step_kernel_b<R, BIG>(q & 1 ? LLG_CART : LLG_QUAT, q & 2, q & 4))) != cudaSuccess) return e;
+    return mx_max_smem(k_mx_gstep<R, BIG>);
 }
 
 cudaError_t mx_configure()
@@ -730,8 +1107,9 @@ cudaError_t mx_configure()
     cudaError_t e;
     if ((e = cudaMemcpyToSymbol(mx::c_wf, hf, sizeof(hf))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(mx::c_wd, hd, sizeof(hd))) != cudaSuccess) return e;
-    if ((e = mx_configure_t<float>()) != cudaSuccess) return e;
-    return mx_configure_t<double>();
+    if ((e = mx_configure_t<float, false>()) != cudaSuccess || (e = mx_configure_t<float, true>()) != cudaSuccess) return e;
+    if ((e = mx_configure_t<double, false>()) != cudaSuccess) return e;
+    return mx_configure_t<double, true>();
 }
 
 } // namespace mlb
