@@ -39,17 +39,20 @@ def build(force=False, verbose=False):
     """Compile every .cu into one shared library (static cudart)."""
     if not force and not _stale():
         return LIB
-    objs = []
+    objs, running = [], []
     bdir = os.path.join(HERE, "_build")
     os.makedirs(bdir, exist_ok=True)
-    for src in SOURCES:
+    for src in SOURCES:   # the sources compile side by side
         obj = os.path.join(bdir, src.replace(".cu", ".o"))
         cmd = [nvcc()] + ARCH + FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
             print(" ".join(cmd))
-        subprocess.check_call(cmd)
+        running.append((cmd, subprocess.Popen(cmd)))
         objs.append(obj)
+    failed = [cmd for cmd, p in running if p.wait() != 0]
+    if failed:
+        raise subprocess.CalledProcessError(1, failed[0])
     tmp = LIB + ".tmp"
     subprocess.check_call([nvcc()] + ARCH + ["-shared", "-o", tmp] + objs + ["-lcudart_static", "-lrt", "-ldl", "-lpthread"])
     os.replace(tmp, LIB)

@@ -168,6 +168,7 @@ struct ConvPlan {
     DBuf<char> spec2;    // split passes: S2[kx][ky][c][z] (complex)
     MxPlan mx{};         // any-length passes (k.mx): ten6 then holds TZ[kx][dz][6][ky]
     DBuf<int> at;        // their tables: places of the x, then of the y frequencies
+    bool x_mx = false;   // the x passes are mx.cu's too
     double max_imag = 0; // largest |Im| of the FP64 tensor transform (6-component)
     int device = -1;     // CUDA device the arrays above live on
     // SPEC holds the forward x transform of the spins of the system whose
@@ -176,14 +177,10 @@ struct ConvPlan {
 };
 
 // LongRange2D / Dipole2D: the per-kx layer-mixing convolution and its
-// tensor spectrum Q[kx][ky][s][d][9] (complex, state precision).
-struct LR2DPlan {
-    ConvK k;
-    FftLen L[3];
-    int rb = 4;
-    DBuf<char> tw;
-    DBuf<char> spec;
-    DBuf<char> spec2;    // S2[kx][ky][c][z] for the FP32 register y passes
+// tensor spectrum (complex, state precision): Q[kx][ky][s][d][9], or with the
+// any-length (y,z) pass (k.mx) Q[kx][s][d][9][ky], ky at its place after the
+// y transform.
+struct LR2DPlan : ConvPlan {
     DBuf<char> Q;
 };
 
@@ -1059,7 +1056,7 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
         double hs[2];
         CK(cudaMemcpyAsync(hs, stat.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        k.mx = hs[1] <= 1e-10 * hs[0];
+        k.mx = P->x_mx = hs[1] <= 1e-10 * hs[0];
     }
     if (!k.mx) CK(mlb::launch_fft3d_d(W.p, ncomp, Px, Py, Pz, P->L, twdd.p, -1, 2, 3, st));
     if (k.mx) {
@@ -1358,6 +1355,17 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
     const size_t plane = (size_t)nx * ny;
     const int npair = nz * nz;
     P->Q.alloc((size_t)k.Kx * ny * npair * 9 * cb);
+    // the x passes: the power-of-two FP32 kernels, or the any-length ones; the
+    // any-length (y,z) pass wherever a kx' layers and their field fit
+    std::vector<int> at, at_y;
+    if (mlb::mx_plan_lr2d(k, rb, P->mx, at, at_y)) {
+        at.insert(at.end(), at_y.begin(), at_y.end());
+        P->at.alloc(at.size());
+        CK(cudaMemcpy(P->at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice));
+        P->mx.x.at = P->at.p;
+        k.mx = 1;
+        P->x_mx = !(rb == 4 && nx >= 32 && mlb::x_fast_ok(k));
+    }
     // batch of layer pairs whose FP64 transforms fit 256 MB
     int bp = (int)std::max<size_t>(1, ((size_t)256 << 20) / (plane * 9 * sizeof(double2)));
     bp = std::min(bp, npair);
@@ -1369,11 +1377,11 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
         for (size_t i = 0; i < plane * 9 * np; i++) h[i] = make_double2(op->t2[(size_t)p0 * 9 * plane + i], 0.0);
         CK(cudaMemcpyAsync(W.p, h.data(), sizeof(double2) * plane * 9 * np, cudaMemcpyHostToDevice, st));
         CK(mlb::launch_fft3d_d(W.p, 9 * np, nx, ny, 1, P->L, twdd.p, -1, 0, 2, st));
-        CK(mlb::launch_lr2d_pack(W.p, nx, ny, nz, p0, np, P->Q.p, rb, st));
+        CK(mlb::launch_lr2d_pack(W.p, nx, ny, nz, p0, np, k.mx ? P->at.p + nx : nullptr, P->Q.p, rb, st));
         CK(cudaStreamSynchronize(st));
     }
     P->spec.alloc((size_t)k.Kx * 3 * nz * ny * cb);
-    if (rb == 4 && mlb::x_fast_ok(k) && mlb::split_y_fast_ok(k)) {
+    if (!k.mx && rb == 4 && mlb::x_fast_ok(k) && mlb::split_y_fast_ok(k)) {
         // FP32 power-of-two planes: y transforms through a second spectrum
         P->spec2.alloc((size_t)k.Kx * ny * 3 * nz * cb);
         P->k.spec2 = P->spec2.p;
@@ -1619,6 +1627,9 @@ void check_dims(const mlb_op* op, const mlb_system* s)
 bool sur_hook(mlb_op* op, mlb_system* s, Slot& sl);
 void sur_advance(mlb_system* s);
 
+// The plan of a convolution operator (built).
+ConvPlan* conv_of(mlb_op* op) { return is_lr2d(op->kind) ? static_cast<ConvPlan*>(op->lr2.get()) : op->plan.get(); }
+
 // Run a deferred inverse x pass on its own (the step took another path).
 void flush_pending(mlb_system* s)
 {
@@ -1627,8 +1638,8 @@ void flush_pending(mlb_system* s)
     Slot& sl = s->slots[s->pend_si];
     s->pend_op = nullptr;
     s->pend_si = -1;
-    ConvPlan& P = *op->plan;
-    if (P.k.mx) {
+    ConvPlan& P = *conv_of(op);
+    if (P.x_mx) {
         CK(mlb::launch_mx_ix(P.mx.x, P.L, P.tw.p, P.spec.p, sl.h, P.rb, s->st));
         return;
     }
@@ -1735,7 +1746,35 @@ void op_apply(mlb_op* op, mlb_system* s)
             sc.dst[z] = op->lr2_dst[z] * op->gs;
         }
         const void* sp[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
-        CK(mlb::launch_lr2d(P.k, P.L, P.tw.p, sp, P.spec.p, P.Q.p, sc, sl.h, s->rb, s->st));
+        if (!P.k.mx) {
+            CK(mlb::launch_lr2d(P.k, P.L, P.tw.p, sp, P.spec.p, P.Q.p, sc, sl.h, s->rb, s->st));
+            return;
+        }
+        // inside a whole step: the inverse x pass waits for the LLG update,
+        // the forward one ran in the step before
+        const bool defer = s->defer_x;
+        const bool carry = defer && (s->capturing ? s->cap_carry : (s->spec_token != 0 && s->spec_token == P.spec_token));
+        auto x_pass = [&](bool fwd) {
+            if (P.x_mx) {
+                if (fwd) CK(mlb::launch_mx_fx(P.mx.x, P.L, P.tw.p, sp, P.spec.p, s->rb, s->st));
+                else CK(mlb::launch_mx_ix(P.mx.x, P.L, P.tw.p, P.spec.p, sl.h, s->rb, s->st));
+                return;
+            }
+            const float* sf[3] = {static_cast<const float*>(sp[0]), static_cast<const float*>(sp[1]),
+                                  static_cast<const float*>(sp[2])};
+            float* hf[3] = {static_cast<float*>(sl.h[0]), static_cast<float*>(sl.h[1]), static_cast<float*>(sl.h[2])};
+            CK(mlb::launch_x_pass_fast(P.k, P.L, reinterpret_cast<const float2*>(P.tw.p), sf,
+                                       reinterpret_cast<float2*>(P.spec.p), hf, fwd, s->st));
+        };
+        if (!carry) x_pass(true);
+        CK(mlb::launch_mx_lr2d(P.k, P.mx.yz, P.L, P.tw.p, P.spec.p, P.Q.p, sc, s->rb, s->st));
+        if (!s->capturing) P.spec_token = 0;
+        if (defer) {
+            s->pend_op = op;
+            s->pend_si = si;
+        } else {
+            x_pass(false);
+        }
         return;
     }
     case MLB_OP_DIPOLE:
@@ -1893,7 +1932,7 @@ void fast_step(mlb_system* s, int nb, const TermsK& T, FastKT<R>& F, ConvPlan* C
         if (T.nadd == 1) ad[c] = static_cast<const R*>(T.add[0][c]);
     }
     if constexpr (sizeof(R) == 4) {
-        if (CP && !CP->k.mx && mlb::xstep_ok(CP->k, F)) {
+        if (CP && !CP->x_mx && mlb::xstep_ok(CP->k, F)) {
             void* hv[3];
             take_pending(hv);
             float* h[3] = {static_cast<float*>(hv[0]), static_cast<float*>(hv[1]), static_cast<float*>(hv[2])};
@@ -1906,7 +1945,7 @@ void fast_step(mlb_system* s, int nb, const TermsK& T, FastKT<R>& F, ConvPlan* C
             return;
         }
     }
-    if (CP && CP->k.mx) {
+    if (CP && CP->x_mx) {
         void* hv[3];
         take_pending(hv);
         R* h[3] = {static_cast<R*>(hv[0]), static_cast<R*>(hv[1]), static_cast<R*>(hv[2])};
@@ -1961,7 +2000,7 @@ bool llg_fused(mlb_llg* l, mlb_system* s, double dt)
     // pass runs in the step's kernel
     ConvPlan* CP = s->pend_op && T.nadd > 0 && T.add[T.nadd - 1][0] == s->slots[s->pend_si].h[0] &&
                            !T.add_is_thermal[T.nadd - 1]
-                       ? s->pend_op->plan.get()
+                       ? conv_of(s->pend_op)
                        : nullptr;
     DevStep* cur = s->capturing ? s->dstep + s->cur : nullptr;
     DevStep* next = s->capturing ? s->dstep + (1 - s->cur) : nullptr;
@@ -1991,12 +2030,12 @@ bool llg_fused(mlb_llg* l, mlb_system* s, double dt)
         P.terms = T;
         P.llg = llgk(l, dt, s->status);
         P.ox = s->sp[nb][0]; P.oy = s->sp[nb][1]; P.oz = s->sp[nb][2];
-        if (CP && (CP->k.mx || mlb::xgstep_ok(CP->k))) {
+        if (CP && (CP->x_mx || mlb::xgstep_ok(CP->k))) {
             void* h[3];
             take_pending(h);
             P.terms.nadd--;
             const double w = T.addw[T.nadd - 1];
-            if (CP->k.mx) {
+            if (CP->x_mx) {
                 CK(mlb::launch_mx_gstep(CP->mx.x, CP->L, CP->tw.p, CP->spec.p, P, w, dt_sys, cur, next, h, s->rb, s->st));
             } else {
                 float* hf[3] = {static_cast<float*>(h[0]), static_cast<float*>(h[1]), static_cast<float*>(h[2])};
@@ -2525,7 +2564,7 @@ void plan_launch(mlb_plan* p, int nsteps)
         for (int a = 0; a < 3; a++) s->dstep_mirror.B[a] += s->dstep_mirror.dB[a];
     }
     s->dstep_known = true;
-    ConvPlan* CP = p->carry_op ? p->carry_op->plan.get() : nullptr;
+    ConvPlan* CP = p->carry_op ? conv_of(p->carry_op) : nullptr;
     for (int k = 0; k < nsteps; k++) {
         const bool carry = CP && s->spec_token != 0 && s->spec_token == CP->spec_token;
         if (carry && p->multi[s->cur] && nsteps - k >= kMultiSteps) {

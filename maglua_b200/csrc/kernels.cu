@@ -1230,9 +1230,10 @@ cudaError_t launch_fft3d_d(double2* W, int ncomp, int Px, int Py, int Pz, const 
 
 // LongRange2D tensor: Q[kx][ky][s][d][ab] = W_{(s d ab)}(kx, ky) / (nx ny) for
 // the layer pairs p0 .. p0 + np - 1 (p = s nz + d), W holding their
-// transforms [(p - p0) 9 + ab][ky][kx] over the full x length.
+// transforms [(p - p0) 9 + ab][ky][kx] over the full x length.  at (not null):
+// Q[kx][s][d][ab][at[ky]].
 template <typename R>
-__global__ void k_lr2d_pack(const double2* W, int nx, int ny, int nz, int Kx, int p0, int np,
+__global__ void k_lr2d_pack(const double2* W, int nx, int ny, int nz, int Kx, int p0, int np, const int* at,
                             typename CT<R>::T* Q)
 {
     const long long total = (long long)Kx * ny * np * 9;
@@ -1245,19 +1246,22 @@ __global__ void k_lr2d_pack(const double2* W, int nx, int ny, int nz, int Kx, in
     const int ky = (int)(r % ny), kx = (int)(r / ny);
     const double inv = 1.0 / ((double)nx * ny);
     const double2 v = W[((size_t)pl * 9 + ab) * nx * ny + (size_t)ky * nx + kx];
-    const size_t o = (((size_t)kx * ny + ky) * nz * nz + p0 + pl) * 9 + ab;
+    const size_t o = at ? (((size_t)kx * nz * nz + p0 + pl) * 9 + ab) * ny + at[ky]
+                        : (((size_t)kx * ny + ky) * nz * nz + p0 + pl) * 9 + ab;
     Q[o] = cmk<typename CT<R>::T>((R)(v.x * inv), (R)(v.y * inv));
 }
 
-cudaError_t launch_lr2d_pack(const double2* W, int nx, int ny, int nz, int p0, int np, void* Q, int rb,
+cudaError_t launch_lr2d_pack(const double2* W, int nx, int ny, int nz, int p0, int np, const int* at, void* Q, int rb,
                              cudaStream_t st)
 {
     const int Kx = nx / 2 + 1;
     const long long total = (long long)Kx * ny * np * 9;
     if (rb == 8)
-        k_lr2d_pack<double><<<blocks_for(total, 256), 256, 0, st>>>(W, nx, ny, nz, Kx, p0, np, static_cast<double2*>(Q));
+        k_lr2d_pack<double><<<blocks_for(total, 256), 256, 0, st>>>(W, nx, ny, nz, Kx, p0, np, at,
+                                                                static_cast<double2*>(Q));
     else
-        k_lr2d_pack<float><<<blocks_for(total, 256), 256, 0, st>>>(W, nx, ny, nz, Kx, p0, np, static_cast<float2*>(Q));
+        k_lr2d_pack<float><<<blocks_for(total, 256), 256, 0, st>>>(W, nx, ny, nz, Kx, p0, np, at,
+                                                               static_cast<float2*>(Q));
     return cudaGetLastError();
 }
 

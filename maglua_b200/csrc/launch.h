@@ -148,6 +148,13 @@ cudaError_t launch_mx_pack(const double2* W, const ConvK& c, const int* at, void
                            cudaStream_t st);
 cudaError_t launch_mx_conv(const ConvK& c, const MxPlan& p, const FftLen L[3], const void* tw, const void* const s[3],
                            void* spec, const void* tz, void* const h[3], bool fx, bool ix, int rb, cudaStream_t st);
+cudaError_t launch_mx_fx(const MxX& x, const FftLen L[3], const void* tw, const void* const s[3], void* spec, int rb,
+                         cudaStream_t st);
+// LongRange2D: the plan (false: a kx' layers and their field do not fit shared
+// memory), and the y transforms with the layer mixing in place on SPEC.
+bool mx_plan_lr2d(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vector<int>& at_y);
+cudaError_t launch_mx_lr2d(const ConvK& c, const MxYZ& y, const FftLen L[3], const void* tw, void* spec, const void* Q,
+                           const LR2DScale& sc, int rb, cudaStream_t st);
 cudaError_t launch_mx_ix(const MxX& x, const FftLen L[3], const void* tw, const void* spec, void* const h[3], int rb,
                          cudaStream_t st);
 // Inverse x pass + step + forward x pass of the new spins: uniform
@@ -174,7 +181,7 @@ cudaError_t launch_tensor_open(int nx, int ny, int nz, const double ABC[9], int 
 size_t lr2d_smem(const ConvK& c, int rb);
 cudaError_t launch_lr2d(const ConvK& c, const FftLen L[3], const void* tw, const void* const s[3], void* spec,
                         const void* Q, const LR2DScale& sc, void* const h[3], int rb, cudaStream_t st);
-cudaError_t launch_lr2d_pack(const double2* W, int nx, int ny, int nz, int p0, int np, void* Q, int rb,
+cudaError_t launch_lr2d_pack(const double2* W, int nx, int ny, int nz, int p0, int np, const int* at, void* Q, int rb,
                              cudaStream_t st);
 // FP64 transforms along axes ax0 .. ax1 - 1
 cudaError_t launch_fft3d_d(double2* W, int ncomp, int Px, int Py, int Pz, const FftLen L[3],

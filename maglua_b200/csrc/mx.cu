@@ -701,6 +701,82 @@ __global__ void __launch_bounds__(Occ<R, BIG>::YZ, 1) k_mx_yz(const __grid_const
     }
 }
 
+// ------------------------------------------------------------------ LongRange2D
+// One CTA per kx: y transforms of the 3 nz rows, for every column the layer
+// mixing
+//   H_a[d] = dst[d] sum_s src[s] sum_b Q[s][d][ab] M_b[s]
+// into a second buffer (no column waits for another), inverse y transforms.
+// Q: [kx][s][d][9][ky], read once, one thread per (a, d, ky): consecutive
+// threads take consecutive ky, three tensor values per source layer each, U
+// layers in flight.  stream: Q is larger than the L2 keeps; its lines are
+// evicted first.  Bound by one CTA's chain up to some 10 MB of Q, by its
+// stream above (256x256x8: 151 MB).  A step of a film with these layers alone,
+// before (y transforms, mixing and inverse y transforms as three passes, x
+// passes apart: seven kernels) and after: 128x128x4 28.0 -> 19.4 us, 100x60x3
+// 68.3 -> 15.0, 58x62x3 1334 -> 17.4, 256x256x8 75.4 -> 67.6.
+template <typename R, bool BIG>
+__global__ void __launch_bounds__(Occ<R, BIG>::YZ, 1) k_mx_lr2d(const __grid_constant__ MxYZ m,
+                                                                const __grid_constant__ LR2DScale sc, int stream,
+                                                                const typename CT<R>::T* __restrict__ tw,
+                                                                typename CT<R>::T* __restrict__ spec,
+                                                                const typename CT<R>::T* __restrict__ Q)
+{
+    typedef typename CT<R>::T C;
+    using namespace mx;
+    const int kx = blockIdx.x, nz = m.nz, ny = m.ny, LS = m.ax.LS, nl = 3 * nz;
+    __shared__ R src[MLB_LR2D_MAXZ], dst[MLB_LR2D_MAXZ];
+    if (threadIdx.x < nz) {
+        src[threadIdx.x] = (R)sc.src[threadIdx.x];
+        dst[threadIdx.x] = (R)sc.dst[threadIdx.x];
+    }
+    load_tables<C>(m.ax, tw, nullptr);
+    pdl_trigger();
+    pdl_wait();
+    C* sm = reinterpret_cast<C*>(mx_sm);
+    const int A = ny, B = A + nl * LS;
+    C* sp = spec + (size_t)kx * nl * ny;
+    for (int idx = threadIdx.x; idx < nl * ny; idx += blockDim.x) {
+        const int l = qdiv(idx, m.mny), y = idx - l * ny;
+        sm[A + l * LS + pd(m.ax, y)] = sp[idx];
+    }
+    __syncthreads();
+    fft<C, false, BIG>(A, nl, m.ax);
+    const C* Qk = Q + (size_t)kx * nz * nz * 9 * ny;
+    constexpr int U = 4;
+    for (int idx = threadIdx.x; idx < nl * ny; idx += blockDim.x) {
+        const int w = qdiv(idx, m.mny), ky = idx - w * ny, kp = pd(m.ax, ky);
+        const int a = w / nz, d = w - a * nz;
+        C acc = cmk<C>(0, 0);
+        for (int s0 = 0; s0 < nz; s0 += U) {
+            C q[U][3];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const C* p = Qk + (((size_t)min(s0 + u, nz - 1) * nz + d) * 9 + 3 * a) * ny + ky;
+#pragma unroll
+                for (int b = 0; b < 3; b++) q[u][b] = stream ? __ldcs(p + (size_t)b * ny) : __ldg(p + (size_t)b * ny);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (s0 + u >= nz) break;
+                const R v = src[s0 + u];
+#pragma unroll
+                for (int b = 0; b < 3; b++) {
+                    const C M = sm[A + (b * nz + s0 + u) * LS + kp];
+                    acc = cadd(acc, cmul(cmk<C>(v * q[u][b].x, v * q[u][b].y), M));
+                }
+            }
+        }
+        const R g = dst[d];
+        sm[B + w * LS + kp] = cmk<C>(g * acc.x, -(g * acc.y));   // conjugate, for the inverse transform
+    }
+    __syncthreads();
+    fft<C, true, BIG>(B, nl, m.ax);
+    for (int idx = threadIdx.x; idx < nl * ny; idx += blockDim.x) {
+        const int l = qdiv(idx, m.mny), y = idx - l * ny;
+        sp[idx] = cconj(sm[B + l * LS + pd(m.ax, y)]);
+    }
+}
+
 // ------------------------------------------------------------------ tensor
 // T(kx, ky, dz) of six components from their FP64 transforms over x and y,
 // W[q][z][ky][kx] (z = dz mod Pz): tz[kx][dz][q][at[ky]], the real part or (XZ,
@@ -926,6 +1002,25 @@ bool mx_plan(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vec
     return true;
 }
 
+static size_t mx_smem_lr2d(const MxAxis& ax, int nl, int rb)
+{
+    return ((size_t)ax.n + 2 * (size_t)nl * ax.LS) * 2 * rb;
+}
+
+bool mx_plan_lr2d(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vector<int>& at_y)
+{
+    memset(&p.yz, 0, sizeof(p.yz));
+    if (c.ny > 8192) return false;
+    MxYZ& y = p.yz;
+    const int nl = 3 * c.nz;
+    if (!mx_axis(c.ny, nl, rb == 8, y.ax, &at_y) || mx_smem_lr2d(y.ax, nl, rb) > MX_SMEM - 1024) return false;
+    if (!mx_plan_x(c, rb, p.x, at_x)) return false;
+    y.ny = c.ny; y.nz = c.nz;
+    y.mny = qmagic(c.ny);
+    y.threads = rb == 8 && y.ax.big ? 256 : (nl * c.ny >= 512 ? 512 : 256);
+    return true;
+}
+
 size_t mx_tensor_bytes(const ConvK& c, int rb) { return (size_t)c.Kx * c.nz * 6 * c.Py * rb; }
 
 cudaError_t launch_mx_pack(const double2* W, const ConvK& c, const int* at, void* tz, unsigned long long* stat2, int rb,
@@ -1015,6 +1110,32 @@ cudaError_t launch_mx_conv(const ConvK& c, const MxPlan& p, const FftLen L[3], c
 }
 
 template <typename R>
+static cudaError_t mx_lr2d_t(const ConvK& c, const MxYZ& y, const FftLen L[3], const void* tw, void* spec,
+                             const void* Q, const LR2DScale& sc, cudaStream_t st)
+{
+    typedef typename CT<R>::T C;
+    Prof pf("k_lr2d_yz", st);
+    const size_t qb = (size_t)c.Kx * c.ny * c.nz * c.nz * 9 * sizeof(C);
+    return launch_pdl(y.ax.big ? k_mx_lr2d<R, true> : k_mx_lr2d<R, false>, dim3(c.Kx), dim3(y.threads),
+                      mx_smem_lr2d(y.ax, 3 * c.nz, sizeof(R)), st, y, sc, qb > ((size_t)64 << 20) ? 1 : 0,
+                      static_cast<const C*>(tw) + L[1].tw_off, static_cast<C*>(spec), static_cast<const C*>(Q));
+}
+
+cudaError_t launch_mx_lr2d(const ConvK& c, const MxYZ& y, const FftLen L[3], const void* tw, void* spec, const void* Q,
+                           const LR2DScale& sc, int rb, cudaStream_t st)
+{
+    if (rb == 8) return mx_lr2d_t<double>(c, y, L, tw, spec, Q, sc, st);
+    return mx_lr2d_t<float>(c, y, L, tw, spec, Q, sc, st);
+}
+
+cudaError_t launch_mx_fx(const MxX& x, const FftLen L[3], const void* tw, const void* const s[3], void* spec, int rb,
+                         cudaStream_t st)
+{
+    if (rb == 8) return mx_fx<double>(x, static_cast<const double2*>(tw) + L[0].tw_off, s, static_cast<double2*>(spec), st);
+    return mx_fx<float>(x, static_cast<const float2*>(tw) + L[0].tw_off, s, static_cast<float2*>(spec), st);
+}
+
+template <typename R>
 using StepKernel = void (*)(MxX, FastKT<R>, const typename CT<R>::T*, typename CT<R>::T*, const R*, const R*, const R*,
                             R*, R*, R*, R*, R*, R*);
 
@@ -1079,7 +1200,10 @@ cudaError_t launch_mx_ix(const MxX& x, const FftLen L[3], const void* tw, const 
 template <typename K>
 static cudaError_t mx_max_smem(K kern)
 {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MX_SMEM);
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MX_SMEM - a.sharedSizeBytes));
 }
 
 template <typename R, bool BIG>
@@ -1091,6 +1215,7 @@ static cudaError_t mx_configure_t()
         if ((e = mx_max_smem(yz_kernel_b<R, BIG>(nz))) != cudaSuccess) return e;
     for (int q = 0; q < 8; q++)
         if ((e = mx_max_smem(step_kernel_b<R, BIG>(q & 1 ? LLG_CART : LLG_QUAT, q & 2, q & 4))) != cudaSuccess) return e;
+    if ((e = mx_max_smem(k_mx_lr2d<R, BIG>)) != cudaSuccess) return e;
     return mx_max_smem(k_mx_gstep<R, BIG>);
 }
 

@@ -60,3 +60,50 @@ def test_periodic_field_powers_of_two_fp64(M, dims):
 @pytest.mark.parametrize("precision", ["f32", "f64"])
 def test_sheared_cell_keeps_the_full_tensor(M, precision):
     _compare(M, (12, 10, 3), precision, cell=(1, 0, 0, 0.3, 1, 0, 0.2, 0.1, 1))
+
+
+@pytest.mark.parametrize("dims,precision", [((9, 31, 5), "f32"), ((30, 13, 1), "f32"), ((16, 6, 9), "f32"),
+                                            ((128, 58, 4), "f32"), ((12, 17, 3), "f64"), ((7, 64, 6), "f64")])
+def test_layer_tensors(M, dims, precision):
+    """LongRange2D over the same passes: prime rows, one layer, layer counts
+    off the four that are loaded together; the field on its own and inside
+    captured steps (whose inverse x pass runs in the step)."""
+    nx, ny, nz = dims
+    r = np.random.default_rng(92)
+    T = r.normal(size=(nz, nz, 9, ny, nx)) / (nx * ny)
+    src, dst = r.uniform(0.5, 1.5, nz), r.uniform(0.5, 1.5, nz)
+    s = random_spins(nx * ny * nz, 93)
+    res = []
+    for captured in (False, True):
+        ss = M.SpinSystem(*dims, precision=precision)
+        ss.setSpinArrays(*s, np.ones(nx * ny * nz))
+        ss.setAlpha(0.1)
+        ss.setTimeStep(0.01)
+        ex = M.Exchange(ss)
+        ex.addPaths(*O.nn_paths(*dims, pbc=(1, 1, 0)))
+        op = M.LongRange2D(ss)
+        op.setNewDataRequired(False)
+        for i in range(nz):
+            for j in range(nz):
+                for q, ab in enumerate(("XX", "XY", "XZ", "YX", "YY", "YZ", "ZX", "ZY", "ZZ")):
+                    op.setTensorArray(i + 1, j + 1, ab, T[i, j, q].reshape(-1))
+        for z in range(nz):
+            op.setSourceMomentScale(z + 1, src[z])
+            op.setDestinationFieldScale(z + 1, dst[z])
+        op.setCompileRequired(True)
+        op.apply(ss)
+        h = np.stack(ss.fieldArrays("LongRange2D"))
+        ref = O.longrange2d_apply(s.reshape(3, nz, ny, nx), T, src, dst)
+        assert rel_err(h, np.asarray(ref).reshape(3, -1)) <= TOL[precision]
+        llg = M.LLG.new("Quaternion")
+        if captured:
+            M.run(ss, [ex, op], llg, 5)
+        else:
+            for _ in range(5):
+                ss.resetFields()
+                ex.apply(ss)
+                op.apply(ss)
+                ss.sumFields()
+                llg.apply(ss)
+        res.append(np.stack(ss.spinArrays()[:3]))
+    np.testing.assert_array_equal(res[0], res[1])
