@@ -675,13 +675,42 @@ double conv_scale(const mlb_op* op, const ConvK& k)
     return op->g * op->gs / ((double)k.Px * k.Py * (k.mx ? 1 : k.Pz));
 }
 
+// Forward x pass of the spins sp (fwd) or inverse to the field h of a plan
+// with a layer tensor.
+void launch_x(const ConvPlan& P, const ConvK& k, const void* const sp[3], void* spec, void* const h[3], bool fwd,
+              cudaStream_t st)
+{
+    if (P.x_mx) {
+        if (fwd) CK(mlb::launch_mx_fx(P.mx.x, P.L, P.tw.p, sp, spec, k.run_if, P.rb, st));
+        else CK(mlb::launch_mx_ix(P.mx.x, P.L, P.tw.p, spec, h, k.run_if, P.rb, st));
+        return;
+    }
+    const float* s[3] = {nullptr, nullptr, nullptr};
+    float* hf[3] = {nullptr, nullptr, nullptr};
+    for (int c = 0; c < 3; c++) {
+        if (fwd) s[c] = static_cast<const float*>(sp[c]);
+        else hf[c] = static_cast<float*>(h[c]);
+    }
+    CK(mlb::launch_x_pass_fast(k, P.L, reinterpret_cast<const float2*>(P.tw.p), s, static_cast<float2*>(spec), hf, fwd,
+                               st));
+}
+
+// (y,z) pass of a plan with a layer tensor
+void launch_yz(const ConvPlan& P, const ConvK& k, void* spec, cudaStream_t st)
+{
+    if (k.ls) CK(mlb::launch_yz_ls(k, P.L, P.tw.p, spec, P.ten6.p, P.rb, st));
+    else CK(mlb::launch_mx_yz(k, P.mx.yz, P.L, P.tw.p, spec, P.ten6.p, P.rb, st));
+}
+
 // The field h of the spins sp by the plan's passes (k: P.k or a copy with
-// its own g or run_if), through the spectrum buffer spec.
+// its own g, run_if or replicas), through the spectrum buffer spec.
 void launch_field(const ConvPlan& P, const ConvK& k, const void* const sp[3], void* spec, void* const h[3],
                   cudaStream_t st)
 {
     if (k.mx) {
-        CK(mlb::launch_mx_conv(k, P.mx, P.L, P.tw.p, sp, spec, P.ten6.p, h, true, true, P.rb, st));
+        launch_x(P, k, sp, spec, h, true, st);
+        launch_yz(P, k, spec, st);
+        launch_x(P, k, sp, spec, h, false, st);
     } else if (P.rb == 4 && mlb::conv_fast_ok(k)) {
         const float* s[3] = {static_cast<const float*>(sp[0]), static_cast<const float*>(sp[1]),
                              static_cast<const float*>(sp[2])};
@@ -692,6 +721,10 @@ void launch_field(const ConvPlan& P, const ConvK& k, const void* const sp[3], vo
         CK(mlb::launch_conv(k, P.L[0], P.L[1], P.L[2], P.tw.p, sp, spec, P.ten6.p, P.ten9.p, h, P.rb, st));
     }
 }
+
+// Whether k_xstep's lines (power-of-two FP32, 32 to 512 points) take the x
+// passes of a plan with a layer tensor.
+bool x_pow2(const ConvK& k, int rb, int lo) { return rb == 4 && k.Px >= lo && mlb::x_fast_ok(k); }
 
 void plan_sizes(mlb_op* op, ConvPlan& P)
 {
@@ -1039,11 +1072,16 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
             }
         CK(cudaMemcpy(W.p, h.data(), sizeof(double2) * h.size(), cudaMemcpyHostToDevice));
     }
-    // edges of any length: x and y transforms, the layer tensor if it has the
-    // parities the layer sum relies on (to 1e-10 of its largest element)
+    // x and y transforms; then the layer tensor, if a pass that sums over the
+    // layers takes the size and the tensor has the parities it relies on (to
+    // 1e-10 of its largest element), else the transform in z
     CK(mlb::launch_fft3d_d(W.p, ncomp, Px, Py, Pz, P->L, twdd.p, -1, 0, 2, st));
     std::vector<int> at, at_y;
-    if (!(rb == 4 && mlb::conv_fast_ok(k)) && mlb::mx_plan(k, rb, P->mx, at, at_y)) {
+    const bool ls = mlb::yz_ls_plan(k, rb, at_y);
+    P->x_mx = !x_pow2(k, rb, 32);
+    if ((ls || (!(rb == 4 && mlb::conv_fast_ok(k)) && mlb::mx_plan_yz(k, rb, P->mx.yz, at_y))) && !k.general &&
+        (!P->x_mx || mlb::mx_plan_x(k, rb, P->mx.x, at))) {
+        at.resize(Px, 0);
         at.insert(at.end(), at_y.begin(), at_y.end());
         P->at.alloc(at.size());
         CK(cudaMemcpy(P->at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice));
@@ -1056,23 +1094,21 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
         double hs[2];
         CK(cudaMemcpyAsync(hs, stat.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        k.mx = P->x_mx = hs[1] <= 1e-10 * hs[0];
+        k.mx = hs[1] <= 1e-10 * hs[0];
+        k.ls = k.mx && ls;
     }
+    P->x_mx = P->x_mx && k.mx;
     if (!k.mx) CK(mlb::launch_fft3d_d(W.p, ncomp, Px, Py, Pz, P->L, twdd.p, -1, 2, 3, st));
     if (k.mx) {
         k.split = 0;
     } else if (k.general) {
         P->ten9.alloc((size_t)k.Kx * Py * Pz * 9 * 2 * rb);
         CK(mlb::launch_tensor_pack9(W.p, Px, Py, Pz, k.Kx, P->ten9.p, rb, k.split, st));
-    } else if ((quarter_ok(k, rb) || (rb == 4 && mlb::yz_col3_ok(k))) && tensor_has_parities(W.p, k, st)) {
-        // the split FP32 passes and the single-CTA-plane (y,z) kernel read a
-        // quarter of the tensor (ky <= Py/2, kz <= Pz/2)
+    } else if (quarter_ok(k, rb) && tensor_has_parities(W.p, k, st)) {
+        // the split FP32 passes read a quarter of the tensor (ky <= Py/2, kz <= Pz/2)
         k.quarter = 1;
-        const size_t q6 = (size_t)(Py / 2 + 1) * (Pz / 2 + 1) * 6;
-        const size_t per_kx = k.split ? q6 : ((q6 + 3) & ~(size_t)3);
-        P->ten6.alloc((size_t)k.Kx * per_kx * rb);
-        CK(cudaMemsetAsync(P->ten6.p, 0, (size_t)k.Kx * per_kx * rb, st));
-        CK(mlb::launch_tensor_pack6q(W.p, Px, Py, Pz, k.Kx, reinterpret_cast<float*>(P->ten6.p), k.split ? 0 : 1, st));
+        P->ten6.alloc((size_t)k.Kx * (Py / 2 + 1) * (Pz / 2 + 1) * 6 * rb);
+        CK(mlb::launch_tensor_pack6q(W.p, Px, Py, Pz, k.Kx, reinterpret_cast<float*>(P->ten6.p), st));
     } else {
         P->ten6.alloc((size_t)k.Kx * Py * Pz * 6 * rb);
         DBuf<double> mi;
@@ -1358,14 +1394,16 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
     // the x passes: the power-of-two FP32 kernels, or the any-length ones; the
     // any-length (y,z) pass wherever a kx' layers and their field fit
     std::vector<int> at, at_y;
-    if (mlb::mx_plan_lr2d(k, rb, P->mx, at, at_y)) {
+    P->x_mx = !x_pow2(k, rb, 32);
+    if (mlb::mx_plan_lr2d(k, rb, P->mx.yz, at_y) && (!P->x_mx || mlb::mx_plan_x(k, rb, P->mx.x, at))) {
+        at.resize(nx, 0);
         at.insert(at.end(), at_y.begin(), at_y.end());
         P->at.alloc(at.size());
         CK(cudaMemcpy(P->at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice));
         P->mx.x.at = P->at.p;
         k.mx = 1;
-        P->x_mx = !(rb == 4 && nx >= 32 && mlb::x_fast_ok(k));
     }
+    P->x_mx = P->x_mx && k.mx;
     // batch of layer pairs whose FP64 transforms fit 256 MB
     int bp = (int)std::max<size_t>(1, ((size_t)256 << 20) / (plane * 9 * sizeof(double2)));
     bp = std::min(bp, npair);
@@ -1639,8 +1677,8 @@ void flush_pending(mlb_system* s)
     s->pend_op = nullptr;
     s->pend_si = -1;
     ConvPlan& P = *conv_of(op);
-    if (P.x_mx) {
-        CK(mlb::launch_mx_ix(P.mx.x, P.L, P.tw.p, P.spec.p, sl.h, P.rb, s->st));
+    if (P.k.mx) {
+        launch_x(P, P.k, nullptr, P.spec.p, sl.h, false, s->st);
         return;
     }
     float* h[3] = {static_cast<float*>(sl.h[0]), static_cast<float*>(sl.h[1]), static_cast<float*>(sl.h[2])};
@@ -1754,26 +1792,14 @@ void op_apply(mlb_op* op, mlb_system* s)
         // the forward one ran in the step before
         const bool defer = s->defer_x;
         const bool carry = defer && (s->capturing ? s->cap_carry : (s->spec_token != 0 && s->spec_token == P.spec_token));
-        auto x_pass = [&](bool fwd) {
-            if (P.x_mx) {
-                if (fwd) CK(mlb::launch_mx_fx(P.mx.x, P.L, P.tw.p, sp, P.spec.p, s->rb, s->st));
-                else CK(mlb::launch_mx_ix(P.mx.x, P.L, P.tw.p, P.spec.p, sl.h, s->rb, s->st));
-                return;
-            }
-            const float* sf[3] = {static_cast<const float*>(sp[0]), static_cast<const float*>(sp[1]),
-                                  static_cast<const float*>(sp[2])};
-            float* hf[3] = {static_cast<float*>(sl.h[0]), static_cast<float*>(sl.h[1]), static_cast<float*>(sl.h[2])};
-            CK(mlb::launch_x_pass_fast(P.k, P.L, reinterpret_cast<const float2*>(P.tw.p), sf,
-                                       reinterpret_cast<float2*>(P.spec.p), hf, fwd, s->st));
-        };
-        if (!carry) x_pass(true);
+        if (!carry) launch_x(P, P.k, sp, P.spec.p, sl.h, true, s->st);
         CK(mlb::launch_mx_lr2d(P.k, P.mx.yz, P.L, P.tw.p, P.spec.p, P.Q.p, sc, s->rb, s->st));
         if (!s->capturing) P.spec_token = 0;
         if (defer) {
             s->pend_op = op;
             s->pend_si = si;
         } else {
-            x_pass(false);
+            launch_x(P, P.k, sp, P.spec.p, sl.h, false, s->st);
         }
         return;
     }
@@ -1800,8 +1826,8 @@ void op_apply(mlb_op* op, mlb_system* s)
             ConvK kk = P.k;
             kk.tl = s->capturing ? s->cap_tl : nullptr;
             if (P.k.mx) {
-                CK(mlb::launch_mx_conv(kk, P.mx, P.L, P.tw.p, spv, P.spec.p, P.ten6.p, sl.h, !carry, false, s->rb,
-                                       s->st));
+                if (!carry) launch_x(P, kk, spv, P.spec.p, sl.h, true, s->st);
+                launch_yz(P, kk, P.spec.p, s->st);
             } else {
                 const float* sp[3] = {static_cast<const float*>(spv[0]), static_cast<const float*>(spv[1]),
                                       static_cast<const float*>(spv[2])};
@@ -2787,11 +2813,9 @@ void ens_class_conv(mlb_ensemble* e, EnsClass& c, const float* const s[3], cudaS
     if (c.fast) {
         ConvK k = P.k;
         k.yz_variant = c.yz_variant;
-        const float* cs[3] = {s[0] + c.base, s[1] + c.base, s[2] + c.base};
-        float* ch[3] = {e->H[0] + c.base, e->H[1] + c.base, e->H[2] + c.base};
-        CK(mlb::launch_conv_fast(k, P.L, reinterpret_cast<const float2*>(P.tw.p), cs,
-                                 reinterpret_cast<float2*>(P.spec.p), reinterpret_cast<const float*>(P.ten6.p), ch,
-                                 st));
+        const void* cs[3] = {s[0] + c.base, s[1] + c.base, s[2] + c.base};
+        void* ch[3] = {e->H[0] + c.base, e->H[1] + c.base, e->H[2] + c.base};
+        launch_field(P, k, cs, P.spec.p, ch, st);
         return;
     }
     ConvK k = P.k;
@@ -2970,7 +2994,7 @@ void ens_autotune(mlb_ensemble* e)
             if (e->cfg.g != 0.0 && c.fast) {
                 float best = 1e30f;
                 // 2 (the 384-thread register kernel) differs from 0 only for 256-wide planes
-                const int nv = c.dip->plan->k.Py == 256 ? 3 : 2;
+                const int nv = c.dip->plan->k.mx ? 1 : (c.dip->plan->k.Py == 256 ? 3 : 2);
                 for (int v = 0; v < nv; v++) {
                     c.yz_variant = v;
                     const float ms = ens_time(e, [&] { ens_class_conv(e, c, s, e->st); }, 10);
@@ -3052,7 +3076,9 @@ void ens_prepare(mlb_ensemble* e)
             k.dip->plan_dirty = true;
             build_plan(k.dip, e->st, 4);
             ConvPlan& P = *k.dip->plan;
-            k.fast = mlb::conv_fast_ok(P.k) && !P.k.split;
+            // all replicas per launch: the power-of-two passes
+            if (P.k.ls && x_pow2(P.k, 4, 16)) P.x_mx = false;
+            k.fast = P.k.mx ? P.k.ls && !P.x_mx : mlb::conv_fast_ok(P.k) && !P.k.split;
             P.k.g = c.g / ((double)P.k.Px * P.k.Py * (P.k.mx ? 1 : P.k.Pz));
             P.k.nrep = k.fast ? k.nrep : 1;
             P.spec.alloc((size_t)P.k.Kx * 3 * k.nz * k.ny * P.k.nrep * sizeof(float2));
@@ -3117,6 +3143,7 @@ int mlb_init(int device)
         CK(mlb::fftreg_init());
         CK(mlb::conv_fast_configure());
         CK(mlb::mx_configure());
+        CK(mlb::yz_ls_configure());
         CK(mlb::sur_configure());
     });
 }

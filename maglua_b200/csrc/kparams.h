@@ -121,7 +121,8 @@ struct ConvK {
     int general;             // 0: 6 real tensor entries per k, 1: 9 complex
     double g;                // strength * global_scale / (Px*Py*Pz)
     int fx, fy, fz;          // FftLen indices
-    int mx = 0;              // 1: the any-length passes of mx.cu with the layer tensor T(kx, ky, dz)
+    int mx = 0;              // 1: z is not transformed, the layer tensor T(kx, ky, dz) is summed over
+    int ls = 0;              // with mx: the power-of-two (y,z) pass of yzls.cu, else that of mx.cu
     int nrep;                // replicas of this size packed back to back (1 for a system)
     const int* run_if;       // when set, the passes run only while *run_if != 0
     int yz_variant = 0;      // (y,z) pass of the fast path: 0 automatic, 1 shared-memory Stockham, 2 register

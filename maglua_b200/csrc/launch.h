@@ -63,10 +63,8 @@ struct Prof {
 cudaError_t fftreg_init();
 cudaError_t conv_fast_configure();
 bool conv_fast_ok(const ConvK& c);
-// the 256-wide single-CTA-plane (y,z) kernel runs this pass (it can read a quarter tensor)
-bool yz_col3_ok(const ConvK& c);
-// FP32 x passes alone (power-of-two periodic x, 16..512): the forward
-// transform of the spins to SPEC (fwd) or the inverse to the field h.
+// FP32 x passes alone (power-of-two Px 16..512): the forward transform of the
+// spins to SPEC (fwd) or the inverse to the field h.
 bool x_fast_ok(const ConvK& c);
 // The fast x passes for FP64 state (power-of-two Px 16..512).
 bool x_fast_ok_f64(const ConvK& c);
@@ -137,26 +135,35 @@ cudaError_t conv_configure();
 cudaError_t launch_conv(const ConvK& c, const FftLen& Lx, const FftLen& Ly, const FftLen& Lz, const void* tw,
                         const void* const s[3], void* spec, const void* ten6, const void* ten9, void* const h[3],
                         int rb, cudaStream_t st);
-// Any-length passes (mx.cu): the plan of a convolution (false: not a size or
-// tensor they take) with the places of its x and y frequencies, the bytes of its layer tensor, its packing from the
-// six components transformed over x and y (stat2: largest |W| and largest
-// deviation from the parities, as double bits; zero them first), and the
-// forward x (fx), (y,z) and inverse x (ix) passes.
-bool mx_plan(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vector<int>& at_y);
+// Layer tensor T(kx, ky, dz) of the passes that sum over the layers instead of
+// transforming z (ConvK::mx): its bytes, and its packing from the six components
+// transformed over x and y, ky stored at at[ky] (stat2: largest |W| and largest
+// deviation from the parities, as double bits; zero them first).
 size_t mx_tensor_bytes(const ConvK& c, int rb);
 cudaError_t launch_mx_pack(const double2* W, const ConvK& c, const int* at, void* tz, unsigned long long* stat2, int rb,
                            cudaStream_t st);
-cudaError_t launch_mx_conv(const ConvK& c, const MxPlan& p, const FftLen L[3], const void* tw, const void* const s[3],
-                           void* spec, const void* tz, void* const h[3], bool fx, bool ix, int rb, cudaStream_t st);
-cudaError_t launch_mx_fx(const MxX& x, const FftLen L[3], const void* tw, const void* const s[3], void* spec, int rb,
+// Its (y,z) pass for power-of-two Py (yzls.cu; ConvK::ls): whether it takes the
+// size, with the places of the y frequencies, and the pass.
+bool yz_ls_plan(const ConvK& c, int rb, std::vector<int>& at);
+cudaError_t launch_yz_ls(const ConvK& c, const FftLen L[3], const void* tw, void* spec, const void* tz, int rb,
                          cudaStream_t st);
+cudaError_t yz_ls_configure();
+// Any-length passes (mx.cu): the plans of the x passes and of the (y,z) pass
+// (false: not a size they take) with the places of their frequencies, and the
+// passes.
+bool mx_plan_x(const ConvK& c, int rb, MxX& x, std::vector<int>& at);
+bool mx_plan_yz(const ConvK& c, int rb, MxYZ& y, std::vector<int>& at);
+cudaError_t launch_mx_yz(const ConvK& c, const MxYZ& plan, const FftLen L[3], const void* tw, void* spec, const void* tz,
+                         int rb, cudaStream_t st);
+cudaError_t launch_mx_fx(const MxX& plan, const FftLen L[3], const void* tw, const void* const s[3], void* spec,
+                         const int* run_if, int rb, cudaStream_t st);
+cudaError_t launch_mx_ix(const MxX& plan, const FftLen L[3], const void* tw, const void* spec, void* const h[3],
+                         const int* run_if, int rb, cudaStream_t st);
 // LongRange2D: the plan (false: a kx' layers and their field do not fit shared
 // memory), and the y transforms with the layer mixing in place on SPEC.
-bool mx_plan_lr2d(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vector<int>& at_y);
+bool mx_plan_lr2d(const ConvK& c, int rb, MxYZ& y, std::vector<int>& at);
 cudaError_t launch_mx_lr2d(const ConvK& c, const MxYZ& y, const FftLen L[3], const void* tw, void* spec, const void* Q,
                            const LR2DScale& sc, int rb, cudaStream_t st);
-cudaError_t launch_mx_ix(const MxX& x, const FftLen L[3], const void* tw, const void* spec, void* const h[3], int rb,
-                         cudaStream_t st);
 // Inverse x pass + step + forward x pass of the new spins: uniform
 // parameters, or the general form (P.terms without the dipole addend of
 // weight addw; cur -> next advance the device step block of a captured step).
@@ -191,8 +198,7 @@ cudaError_t launch_fft3d_d(double2* W, int ncomp, int Px, int Py, int Pz, const 
 // and the FP32 quarter tensor of the split passes (ConvK::quarter).
 cudaError_t launch_tensor_symcheck(const double2* W, int Px, int Py, int Pz, int Kx, unsigned long long* out3,
                                    cudaStream_t st);
-cudaError_t launch_tensor_pack6q(const double2* W, int Px, int Py, int Pz, int Kx, float* ten, int zmaj,
-                                cudaStream_t st);
+cudaError_t launch_tensor_pack6q(const double2* W, int Px, int Py, int Pz, int Kx, float* ten, cudaStream_t st);
 cudaError_t launch_tensor_pack6(const double2* W, int Px, int Py, int Pz, int Kx, void* ten6, double* maxim,
                                 int rb, int kmaj, cudaStream_t st);
 cudaError_t launch_tensor_pack9(const double2* W, int Px, int Py, int Pz, int Kx, void* ten9, int rb, int kmaj,

@@ -953,7 +953,7 @@ constexpr size_t MX_SMEM = 227 * 1024;
 // The x passes' plan.  Rows per CTA: the estimated time of the busiest SM,
 // waves of the CTAs it holds (a chain of latencies each) plus its share of the
 // work, in cycles; sizes near a multiple of 148 CTAs differ by a whole wave.
-static bool mx_plan_x(const ConvK& c, int rb, MxX& x, std::vector<int>& at)
+bool mx_plan_x(const ConvK& c, int rb, MxX& x, std::vector<int>& at)
 {
     memset(&x, 0, sizeof(x));
     if (c.nrep != 1 || c.Px > 8192) return false;
@@ -986,14 +986,12 @@ static bool mx_plan_x(const ConvK& c, int rb, MxX& x, std::vector<int>& at)
     return true;
 }
 
-bool mx_plan(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vector<int>& at_y)
+bool mx_plan_yz(const ConvK& c, int rb, MxYZ& y, std::vector<int>& at)
 {
-    memset(&p.yz, 0, sizeof(p.yz));
+    memset(&y, 0, sizeof(y));
     if (c.general || c.nrep != 1 || c.nz > 32 || c.Py > 8192) return false;
-    MxYZ& y = p.yz;
     const int nl = 3 * c.nz, pts = nl * c.Py;
-    if (!mx_axis(c.Py, nl, rb == 8, y.ax, &at_y) || mx_smem_y(y.ax, nl, rb) > MX_SMEM) return false;
-    if (!mx_plan_x(c, rb, p.x, at_x)) return false;
+    if (!mx_axis(c.Py, nl, rb == 8, y.ax, &at) || mx_smem_y(y.ax, nl, rb) > MX_SMEM) return false;
     y.ny = c.ny; y.nz = c.nz;
     y.mPy = qmagic(c.Py);
     y.mny = qmagic(c.ny);
@@ -1007,14 +1005,12 @@ static size_t mx_smem_lr2d(const MxAxis& ax, int nl, int rb)
     return ((size_t)ax.n + 2 * (size_t)nl * ax.LS) * 2 * rb;
 }
 
-bool mx_plan_lr2d(const ConvK& c, int rb, MxPlan& p, std::vector<int>& at_x, std::vector<int>& at_y)
+bool mx_plan_lr2d(const ConvK& c, int rb, MxYZ& y, std::vector<int>& at)
 {
-    memset(&p.yz, 0, sizeof(p.yz));
+    memset(&y, 0, sizeof(y));
     if (c.ny > 8192) return false;
-    MxYZ& y = p.yz;
     const int nl = 3 * c.nz;
-    if (!mx_axis(c.ny, nl, rb == 8, y.ax, &at_y) || mx_smem_lr2d(y.ax, nl, rb) > MX_SMEM - 1024) return false;
-    if (!mx_plan_x(c, rb, p.x, at_x)) return false;
+    if (!mx_axis(c.ny, nl, rb == 8, y.ax, &at) || mx_smem_lr2d(y.ax, nl, rb) > MX_SMEM - 1024) return false;
     y.ny = c.ny; y.nz = c.nz;
     y.mny = qmagic(c.ny);
     y.threads = rb == 8 && y.ax.big ? 256 : (nl * c.ny >= 512 ? 512 : 256);
@@ -1084,29 +1080,17 @@ static cudaError_t mx_yz(const ConvK& c, const MxYZ& y, const typename CT<R>::T*
                       spec, tz);
 }
 
-template <typename R>
-static cudaError_t mx_conv_t(const ConvK& c, const MxPlan& p, const FftLen L[3], const void* tw_, const void* const s[3],
-                             void* spec_, const void* tz, void* const h[3], bool fx, bool ix, cudaStream_t st)
+cudaError_t launch_mx_yz(const ConvK& c, const MxYZ& plan, const FftLen L[3], const void* tw, void* spec, const void* tz,
+                         int rb, cudaStream_t st)
 {
-    typedef typename CT<R>::T C;
-    const C* tw = static_cast<const C*>(tw_);
-    C* spec = static_cast<C*>(spec_);
-    MxX x = p.x;
-    MxYZ y = p.yz;
-    x.run_if = y.run_if = c.run_if;
+    MxYZ y = plan;
+    y.run_if = c.run_if;
     y.g = c.g;
-    cudaError_t e = cudaSuccess;
-    if (fx && (e = mx_fx<R>(x, tw + L[0].tw_off, s, spec, st)) != cudaSuccess) return e;
-    if ((e = mx_yz<R>(c, y, tw + L[1].tw_off, spec, static_cast<const R*>(tz), st)) != cudaSuccess) return e;
-    if (ix) e = mx_ix<R>(x, tw + L[0].tw_off, spec, h, st);
-    return e;
-}
-
-cudaError_t launch_mx_conv(const ConvK& c, const MxPlan& p, const FftLen L[3], const void* tw, const void* const s[3],
-                           void* spec, const void* tz, void* const h[3], bool fx, bool ix, int rb, cudaStream_t st)
-{
-    if (rb == 8) return mx_conv_t<double>(c, p, L, tw, s, spec, tz, h, fx, ix, st);
-    return mx_conv_t<float>(c, p, L, tw, s, spec, tz, h, fx, ix, st);
+    if (rb == 8)
+        return mx_yz<double>(c, y, static_cast<const double2*>(tw) + L[1].tw_off, static_cast<double2*>(spec),
+                             static_cast<const double*>(tz), st);
+    return mx_yz<float>(c, y, static_cast<const float2*>(tw) + L[1].tw_off, static_cast<float2*>(spec),
+                        static_cast<const float*>(tz), st);
 }
 
 template <typename R>
@@ -1128,9 +1112,11 @@ cudaError_t launch_mx_lr2d(const ConvK& c, const MxYZ& y, const FftLen L[3], con
     return mx_lr2d_t<float>(c, y, L, tw, spec, Q, sc, st);
 }
 
-cudaError_t launch_mx_fx(const MxX& x, const FftLen L[3], const void* tw, const void* const s[3], void* spec, int rb,
-                         cudaStream_t st)
+cudaError_t launch_mx_fx(const MxX& plan, const FftLen L[3], const void* tw, const void* const s[3], void* spec,
+                         const int* run_if, int rb, cudaStream_t st)
 {
+    MxX x = plan;
+    x.run_if = run_if;
     if (rb == 8) return mx_fx<double>(x, static_cast<const double2*>(tw) + L[0].tw_off, s, static_cast<double2*>(spec), st);
     return mx_fx<float>(x, static_cast<const float2*>(tw) + L[0].tw_off, s, static_cast<float2*>(spec), st);
 }
@@ -1189,9 +1175,11 @@ cudaError_t launch_mx_gstep(const MxX& x, const FftLen L[3], const void* tw, voi
     return mx_gstep_t<float>(x, L, tw, spec, P, addw, dt_sys, cur, next, h, st);
 }
 
-cudaError_t launch_mx_ix(const MxX& x, const FftLen L[3], const void* tw, const void* spec, void* const h[3], int rb,
-                         cudaStream_t st)
+cudaError_t launch_mx_ix(const MxX& plan, const FftLen L[3], const void* tw, const void* spec, void* const h[3],
+                         const int* run_if, int rb, cudaStream_t st)
 {
+    MxX x = plan;
+    x.run_if = run_if;
     if (rb == 8)
         return mx_ix<double>(x, static_cast<const double2*>(tw) + L[0].tw_off, static_cast<const double2*>(spec), h, st);
     return mx_ix<float>(x, static_cast<const float2*>(tw) + L[0].tw_off, static_cast<const float2*>(spec), h, st);

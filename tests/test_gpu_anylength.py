@@ -58,6 +58,15 @@ def test_periodic_field_powers_of_two_fp64(M, dims):
 
 
 @pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("dims", [(20, 16, 8), (9, 16, 16), (33, 32, 1), (16, 32, 16), (40, 64, 3), (8, 64, 7),
+                                  (64, 128, 5), (300, 128, 2), (12, 256, 6), (7, 512, 4), (2, 512, 8)])
+def test_power_of_two_rows_of_y(M, dims, precision):
+    """The (y,z) pass for power-of-two Py: every width, layer counts in turn,
+    few and many CTAs (few: large CTAs of several items per thread)."""
+    _compare(M, dims, precision)
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
 def test_sheared_cell_keeps_the_full_tensor(M, precision):
     _compare(M, (12, 10, 3), precision, cell=(1, 0, 0, 0.3, 1, 0, 0.2, 0.1, 1))
 
