@@ -279,6 +279,7 @@ struct mlb_system {
     mlb_op* pend_op = nullptr;      // operator whose inverse x pass is pending
     int pend_si = -1;               // and its slot
     bool cap_carry = false;         // capture: assume SPEC holds the current spins' x transform
+    bool cap_inner = false;         // capture: not the last step of its graph
     mlb_op* cap_xstep = nullptr;    // capture: the convolution whose x pass the captured step fused
     unsigned long long* cap_tl = nullptr;   // capture: device timeline stamps of a timing plan
     unsigned long long spec_token = 0;   // matches ConvPlan::spec_token while that holds
@@ -722,9 +723,12 @@ void launch_field(const ConvPlan& P, const ConvK& k, const void* const sp[3], vo
     }
 }
 
-// Whether k_xstep's lines (power-of-two FP32, 32 to 512 points) take the x
-// passes of a plan with a layer tensor.
-bool x_pow2(const ConvK& k, int rb, int lo) { return rb == 4 && k.Px >= lo && mlb::x_fast_ok(k); }
+// Whether the power-of-two FP32 x passes take a plan with a layer tensor: lines
+// of lo to 512 points (k_xstep: from 32, its rows in pairs).
+bool x_pow2(const ConvK& k, int rb, int lo)
+{
+    return rb == 4 && k.Px >= lo && mlb::x_fast_ok(k) && (lo < 32 || mlb::xstep_pairs(k));
+}
 
 void plan_sizes(mlb_op* op, ConvPlan& P)
 {
@@ -2031,7 +2035,9 @@ bool llg_fused(mlb_llg* l, mlb_system* s, double dt)
     DevStep* cur = s->capturing ? s->dstep + s->cur : nullptr;
     DevStep* next = s->capturing ? s->dstep + (1 - s->cur) : nullptr;
     auto take_pending = [&](void* h[3]) {
-        for (int c = 0; c < 3; c++) h[c] = s->slots[s->pend_si].h[c];
+        // a captured step that another follows in the same graph leaves the
+        // field to it
+        for (int c = 0; c < 3; c++) h[c] = s->cap_inner ? nullptr : s->slots[s->pend_si].h[c];
         carried = true;
         advanced = s->capturing;
         if (s->capturing) {
@@ -2512,6 +2518,7 @@ void plan_capture(mlb_plan* p)
                 try {
                     for (int j = 0; j < kMultiSteps && ok; j++) {
                         s->cap_carry = true;
+                        s->cap_inner = j < kMultiSteps - 1;
                         s->cap_xstep = nullptr;
                         do_step(s, p->ops.data(), nops, p->l);
                         ok = s->cap_xstep == p->carry_op;
@@ -2522,6 +2529,7 @@ void plan_capture(mlb_plan* p)
                 }
                 s->capturing = false;
                 s->cap_carry = false;
+                s->cap_inner = false;
                 cudaError_t e = cudaStreamEndCapture(s->st, &graph);
                 if (ok && e == cudaSuccess) e = cudaGraphInstantiate(&p->multi[q], graph, 0);
                 if (graph) cudaGraphDestroy(graph);
@@ -2542,6 +2550,7 @@ void plan_capture(mlb_plan* p)
         s->dry = false;
         s->capturing = false;
         s->cap_carry = false;
+        s->cap_inner = false;
         s->cap_tl = nullptr;
         mlb::prof_set_capture_sink(nullptr);
         load_state(s, p->ops, h0);

@@ -1068,10 +1068,11 @@ struct XSCfg {
 };
 
 // The body of the fused x pass: begin() runs once the previous kernel's
-// writes are visible, pre(row, x, i) is called for every site of the
-// CTA while the spectrum loads are in flight, site(i, row, x, y, z, A) gives
-// the new spin of site i in the dipole field A.
-template <int PX, bool TH, int SZ, int HU, class Begin, class Pre, class Site>
+// writes are visible; pre(p, x, i, both) is called for every row pair p and x
+// of the CTA (sites i and, if both, i + nx) while the spectrum loads are in
+// flight; site(i, row, x, y, z, A..., r...) gives the new spin of site i in the
+// dipole field A, or with PAIR site(i, p, ...) those of i and i + nx.
+template <int PX, bool TH, int SZ, bool PAIR, class Begin, class Pre, class Site>
 __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cur, DevStep* adv_next, int fwd,
                                            const float2* __restrict__ tw, float2* __restrict__ spec,
                                            const float* __restrict__ sx, const float* __restrict__ sy,
@@ -1157,11 +1158,7 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
                 const int idx = threadIdx.x + it * NT;
                 if (idx >= R2 * PX) break;
                 const int p = idx / PX, x = idx % PX;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int row = 2 * p + h;
-                    if (row < rows_here && x < nx) pre(row, x, (row0 + row) * nx + x);
-                }
+                if (2 * p < rows_here && x < nx) pre(p, x, (row0 + 2 * p) * nx + x, 2 * p + 1 < rows_here);
             }
         }
 #pragma unroll
@@ -1188,9 +1185,10 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
         R = fr::sm_fft<PX, +1, X::TPL, float2, LS>(A, B, l, tl, twl, l < X::L);
     }
     float2* W = (R == A) ? B : A;   // free buffer: the new spins' lines (FWD)
-    // 2. field of the rows to the slot, then the step of every site: one
-    // (row pair, x) per item, the pair's two rows the real and imaginary
-    // parts of one line element
+    // 2. field of the rows to the slot (unless a later step of the same launch
+    // overwrites it: hx null), then the step of every site: one (row pair, x)
+    // per item, the pair's two rows the real and imaginary parts of one line
+    // element
     constexpr int IP = (R2 * PX + NT - 1) / NT;
     // (z, y) of the CTA's first row; a later row's by counting forward (no
     // division per site)
@@ -1202,21 +1200,35 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
         const int p = idx / PX, x = idx % PX;
         const float2 Ax2 = R[(0 * R2 + p) * LS + x], Ay2 = R[(1 * R2 + p) * LS + x], Az2 = R[(2 * R2 + p) * LS + x];
         float2 o0 = make_float2(0.f, 0.f), o1 = o0, o2 = o0;
-#pragma unroll HU
-        for (int h = 0; h < 2; h++) {
-            const int row = 2 * p + h;
-            if (row < rows_here && x < nx) {
-                const float Ax = h ? Ax2.y : Ax2.x, Ay = h ? Ay2.y : Ay2.x, Az = h ? Az2.y : Az2.x;
-                const int r = row0 + row;
-                int zz = zr0, y = yr0 + row;
-                while (y >= ny) { y -= ny; zz++; }
-                const size_t i = (size_t)r * nx + x;
-                hx[i] = Ax; hy[i] = Ay; hz[i] = Az;
-                float rx, ry, rz;
-                site((int)i, row, x, y, zz, Ax, Ay, Az, rx, ry, rz);
-                ox[i] = rx; oy[i] = ry; oz[i] = rz;
-                if (h) { o0.y = rx; o1.y = ry; o2.y = rz; }
-                else { o0.x = rx; o1.x = ry; o2.x = rz; }
+        int zz = zr0, y = yr0 + 2 * p;
+        while (y >= ny) { y -= ny; zz++; }
+        if constexpr (PAIR) {
+            // ny is even: the pair lies in one layer, and both rows exist
+            if (2 * p < rows_here && x < nx) {
+                const int i = (row0 + 2 * p) * nx + x;
+                if (hx) {
+                    hx[i] = Ax2.x; hy[i] = Ay2.x; hz[i] = Az2.x;
+                    hx[i + nx] = Ax2.y; hy[i + nx] = Ay2.y; hz[i + nx] = Az2.y;
+                }
+                site(i, p, x, y, zz, Ax2, Ay2, Az2, o0, o1, o2);
+                ox[i] = o0.x; oy[i] = o1.x; oz[i] = o2.x;
+                ox[i + nx] = o0.y; oy[i + nx] = o1.y; oz[i + nx] = o2.y;
+            }
+        } else {
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                const int row = 2 * p + h;
+                if (h && ++y >= ny) { y -= ny; zz++; }
+                if (row < rows_here && x < nx) {
+                    const float Ax = h ? Ax2.y : Ax2.x, Ay = h ? Ay2.y : Ay2.x, Az = h ? Az2.y : Az2.x;
+                    const size_t i = (size_t)(row0 + row) * nx + x;
+                    if (hx) { hx[i] = Ax; hy[i] = Ay; hz[i] = Az; }
+                    float rx, ry, rz;
+                    site((int)i, row, x, y, zz, Ax, Ay, Az, rx, ry, rz);
+                    ox[i] = rx; oy[i] = ry; oz[i] = rz;
+                    if (h) { o0.y = rx; o1.y = ry; o2.y = rz; }
+                    else { o0.x = rx; o1.x = ry; o2.x = rz; }
+                }
             }
         }
         if (fwd) { W[(0 * R2 + p) * LS + x] = o0; W[(1 * R2 + p) * LS + x] = o1; W[(2 * R2 + p) * LS + x] = o2; }
@@ -1251,8 +1263,11 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
     tl_end(tls);
 }
 
-template <int PX, int LT, bool EXS, bool ANI, bool TH, int SZ>
-__global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC) k_xstep(ConvK c, FastK F0, int fwd, const float2* __restrict__ tw,
+// PAIR: two sites at a time (fused_pair), for an even number of rows per layer
+// and at most 2^30 sites.
+template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR>
+__global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC) k_xstep(ConvK c, FastK F0,
+                                                  int fwd, const float2* __restrict__ tw,
                                                   float2* __restrict__ spec, const float* __restrict__ sx,
                                                   const float* __restrict__ sy, const float* __restrict__ sz,
                                                   float* __restrict__ hx, float* __restrict__ hy,
@@ -1260,27 +1275,48 @@ __global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC)
                                                   float* __restrict__ oy, float* __restrict__ oz)
 {
     using X = XSCfg<PX, TH, SZ>;
-    constexpr int NP = X::ROWS * PX;
+    constexpr int NP = X::R2 * PX;
     extern __shared__ float2 sm[];
-    float* noise = reinterpret_cast<float*>(sm + PX + 2 * X::BUF + X::EX);   // [3][ROWS][PX] (X::PRE)
+    float2* noise = sm + PX + 2 * X::BUF + X::EX;   // [3][R2][PX] row pairs (X::PRE)
     // the step block's values are the previous kernel's: resolved after the wait
     FastK F;
-    xstep_body<PX, TH, SZ, 2>(
-        c, F0.adv_cur, F0.adv_next, fwd, tw, spec, sx, sy, sz, hx, hy, hz, ox, oy, oz, [&] { F = fastk_resolved(F0); },
-        [&](int row, int x, int i) {
-            const float3 g = thermal_normal3(F, i);
-            float* q = noise + row * PX + x;
-            q[0] = g.x; q[NP] = g.y; q[2 * NP] = g.z;
-        },
-        [&](int i, int row, int x, int y, int z, float Ax, float Ay, float Az, float& rx, float& ry, float& rz) {
-            float3 g;
-            if (X::PRE) {
-                const float* q = noise + row * PX + x;
-                g = make_float3(q[0], q[NP], q[2 * NP]);
-            }
-            fused_site_v<LT, EXS, ANI, TH, true>(F, c.nx, c.ny, c.nz, x, y, z, i, sx, sy, sz, Ax, Ay, Az, rx, ry, rz,
-                                                 X::PRE ? &g : nullptr);
-        });
+    const auto begin = [&] { F = fastk_resolved(F0); };
+    const auto pre = [&](int p, int x, int i, bool both) {
+        const float3 g = thermal_normal3(F, i);
+        float3 k = make_float3(0.f, 0.f, 0.f);
+        if (PAIR || both) k = thermal_normal3(F, i + c.nx);
+        float2* q = noise + p * PX + x;
+        q[0] = make_float2(g.x, k.x); q[NP] = make_float2(g.y, k.y); q[2 * NP] = make_float2(g.z, k.z);
+    };
+    if constexpr (PAIR) {
+        xstep_body<PX, TH, SZ, true>(
+            c, F0.adv_cur, F0.adv_next, fwd, tw, spec, sx, sy, sz, hx, hy, hz, ox, oy, oz, begin, pre,
+            [&](int i, int p, int x, int y, int z, float2 Ax, float2 Ay, float2 Az, float2& rx, float2& ry, float2& rz) {
+                const p2 A[3] = {pk(Ax.x, Ax.y), pk(Ay.x, Ay.y), pk(Az.x, Az.y)};
+                p2 n[3] = {pk(0.f, 0.f), pk(0.f, 0.f), pk(0.f, 0.f)}, r[3];
+                if (X::PRE) {
+                    const float2* q = noise + p * PX + x;
+                    n[0] = pk(q[0].x, q[0].y); n[1] = pk(q[NP].x, q[NP].y); n[2] = pk(q[2 * NP].x, q[2 * NP].y);
+                } else if (TH) {
+                    const float3 g = thermal_normal3(F, i), k = thermal_normal3(F, i + c.nx);
+                    n[0] = pk(g.x, k.x); n[1] = pk(g.y, k.y); n[2] = pk(g.z, k.z);
+                }
+                fused_pair<LT, ANI, TH>(F, c.nx, c.ny, c.nz, x, y, z, i, sx, sy, sz, A, n, r);
+                rx = up(r[0]); ry = up(r[1]); rz = up(r[2]);
+            });
+    } else {
+        xstep_body<PX, TH, SZ, false>(
+            c, F0.adv_cur, F0.adv_next, fwd, tw, spec, sx, sy, sz, hx, hy, hz, ox, oy, oz, begin, pre,
+            [&](int i, int row, int x, int y, int z, float Ax, float Ay, float Az, float& rx, float& ry, float& rz) {
+                float3 g;
+                if (X::PRE) {
+                    const float* q = reinterpret_cast<const float*>(noise + (row >> 1) * PX + x) + (row & 1);
+                    g = make_float3(q[0], q[2 * NP], q[4 * NP]);
+                }
+                fused_site_v<LT, true, ANI, TH, true>(F, c.nx, c.ny, c.nz, x, y, z, i, sx, sy, sz, Ax, Ay, Az, rx, ry,
+                                                      rz, X::PRE ? &g : nullptr);
+            });
+    }
 }
 
 // The same pass for per-site parameters, pathway lists and further addends
@@ -1294,10 +1330,10 @@ __global__ void __launch_bounds__(XSCfg<PX, false, SZ>::NT, XSCfg<PX, false, SZ>
                                                             float* __restrict__ hx, float* __restrict__ hy,
                                                             float* __restrict__ hz)
 {
-    xstep_body<PX, false, SZ, 1>(
+    xstep_body<PX, false, SZ, false>(
         c, cur, next, 1, tw, spec, static_cast<const float*>(P.sys.x), static_cast<const float*>(P.sys.y),
         static_cast<const float*>(P.sys.z), hx, hy, hz, static_cast<float*>(P.ox), static_cast<float*>(P.oy),
-        static_cast<float*>(P.oz), [] {}, [](int, int, int) {},
+        static_cast<float*>(P.oz), [] {}, [](int, int, int, bool) {},
         [&](int i, int, int, int, int, float Ax, float Ay, float Az, float& rx, float& ry, float& rz) {
             const float ms = ms_at<float>(P.sys, i);
             Fields<float> F;
@@ -1719,6 +1755,12 @@ bool xstep_ok(const ConvK& c, const FastK& F)
     return c.nrep == 1 && F.ex && (c.Px == 32 || c.Px == 64 || c.Px == 128 || c.Px == 256 || c.Px == 512);
 }
 
+// Whether the rows of a layer come in pairs (k_xstep's two sites at a time).
+bool xstep_pairs(const ConvK& c)
+{
+    return c.ny % 2 == 0 && (long long)c.nx * c.ny * c.nz <= (1ll << 30);
+}
+
 // Share of a CTA (XSCfg): the largest that gives at least about as many CTAs as
 // SMs.  A step alone, share 0 / the one taken: 32x32x1 13.3 / 9.0 us, 64x64x2
 // 15.0 / 9.0, 128x128x4 19.3 / 13.0, 256x256x1 22.9 / 17.1, 64x512x4 25.7 / 20.2,
@@ -1732,24 +1774,25 @@ static int xs_size(const ConvK& c)
     return 2;
 }
 
-template <int PX, int LT, bool ANI, bool TH, int SZ>
+template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR>
 static cudaError_t xstep_sz(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
                             const float* s[3], float* h[3], float* o[3], cudaStream_t st)
 {
     using X = XSCfg<PX, TH, SZ>;
     dim3 grid((c.nz * c.ny + X::ROWS - 1) / X::ROWS, 1, 1);
-    return launch_pdl(k_xstep<PX, LT, true, ANI, TH, SZ>, grid, dim3(X::NT), (size_t)X::SMEM, st, c, F, fwd, tw, spec,
+    return launch_pdl(k_xstep<PX, LT, ANI, TH, SZ, PAIR>, grid, dim3(X::NT), (size_t)X::SMEM, st, c, F, fwd, tw, spec,
                       s[0], s[1], s[2], h[0], h[1], h[2], o[0], o[1], o[2]);
 }
 template <int PX, int LT, bool ANI, bool TH>
 static cudaError_t xstep_t(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
                            const float* s[3], float* h[3], float* o[3], cudaStream_t st)
 {
+    if (!xstep_pairs(c)) return xstep_sz<PX, LT, ANI, TH, 0, false>(c, F, fwd, tw, spec, s, h, o, st);
     const int sz = xs_size<PX>(c);
-    if (sz == 0) return xstep_sz<PX, LT, ANI, TH, 0>(c, F, fwd, tw, spec, s, h, o, st);
+    if (sz == 0) return xstep_sz<PX, LT, ANI, TH, 0, true>(c, F, fwd, tw, spec, s, h, o, st);
     if constexpr (PX <= 128)
-        if (sz == 2) return xstep_sz<PX, LT, ANI, TH, 2>(c, F, fwd, tw, spec, s, h, o, st);
-    return xstep_sz<PX, LT, ANI, TH, 1>(c, F, fwd, tw, spec, s, h, o, st);
+        if (sz == 2) return xstep_sz<PX, LT, ANI, TH, 2, true>(c, F, fwd, tw, spec, s, h, o, st);
+    return xstep_sz<PX, LT, ANI, TH, 1, true>(c, F, fwd, tw, spec, s, h, o, st);
 }
 template <int PX, int LT>
 static cudaError_t xstep_lt(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
@@ -1825,25 +1868,24 @@ cudaError_t launch_xgstep(const ConvK& c, const FftLen L[3], const float2* tw, f
     return cudaErrorInvalidValue;
 }
 
-template <int PX, int LT, bool ANI, bool TH, int SZ>
+template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR>
 static cudaError_t cfg_xs1()
 {
-    cudaError_t e = cudaFuncSetAttribute(k_xstep<PX, LT, true, ANI, TH, SZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         XSCfg<PX, TH, SZ>::SMEM);
+    const auto k = k_xstep<PX, LT, ANI, TH, SZ, PAIR>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, XSCfg<PX, TH, SZ>::SMEM);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_xstep<PX, LT, true, ANI, TH, SZ>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                (int)cudaSharedmemCarveoutMaxShared);
+    return cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
 }
-template <int PX, int SZ>
+template <int PX, int SZ, bool PAIR>
 static cudaError_t cfg_xs_sz()
 {
     cudaError_t e =
         cudaFuncSetAttribute(k_xgstep<PX, SZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, XSCfg<PX, false, SZ>::SMEM);
     if (e != cudaSuccess) return e;
-    if ((e = cfg_xs1<PX, LLG_CART, false, false, SZ>()) || (e = cfg_xs1<PX, LLG_CART, false, true, SZ>()) ||
-        (e = cfg_xs1<PX, LLG_CART, true, false, SZ>()) || (e = cfg_xs1<PX, LLG_CART, true, true, SZ>()) ||
-        (e = cfg_xs1<PX, LLG_QUAT, false, false, SZ>()) || (e = cfg_xs1<PX, LLG_QUAT, false, true, SZ>()) ||
-        (e = cfg_xs1<PX, LLG_QUAT, true, false, SZ>()) || (e = cfg_xs1<PX, LLG_QUAT, true, true, SZ>()))
+    if ((e = cfg_xs1<PX, LLG_CART, false, false, SZ, PAIR>()) || (e = cfg_xs1<PX, LLG_CART, false, true, SZ, PAIR>()) ||
+        (e = cfg_xs1<PX, LLG_CART, true, false, SZ, PAIR>()) || (e = cfg_xs1<PX, LLG_CART, true, true, SZ, PAIR>()) ||
+        (e = cfg_xs1<PX, LLG_QUAT, false, false, SZ, PAIR>()) || (e = cfg_xs1<PX, LLG_QUAT, false, true, SZ, PAIR>()) ||
+        (e = cfg_xs1<PX, LLG_QUAT, true, false, SZ, PAIR>()) || (e = cfg_xs1<PX, LLG_QUAT, true, true, SZ, PAIR>()))
         return e;
     return cudaSuccess;
 }
@@ -1851,8 +1893,9 @@ template <int PX>
 static cudaError_t cfg_xs()
 {
     cudaError_t e;
-    if ((e = cfg_xs_sz<PX, 0>()) != cudaSuccess || (e = cfg_xs_sz<PX, 1>()) != cudaSuccess) return e;
-    if constexpr (PX <= 128) return cfg_xs_sz<PX, 2>();
+    if ((e = cfg_xs_sz<PX, 0, false>()) != cudaSuccess || (e = cfg_xs_sz<PX, 0, true>()) != cudaSuccess) return e;
+    if ((e = cfg_xs_sz<PX, 1, true>()) != cudaSuccess) return e;
+    if constexpr (PX <= 128) return cfg_xs_sz<PX, 2, true>();
     return cudaSuccess;
 }
 

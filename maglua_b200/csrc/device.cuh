@@ -109,6 +109,54 @@ __device__ __forceinline__ float ml(float a, float b) { return __fmul_rn(a, b); 
 __device__ __forceinline__ double ml(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float ad(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double ad(double a, double b) { return __dadd_rn(a, b); }
+// Two FP32 values side by side: the packed instructions of sm_100 (one issue
+// for two roundings, each that of the single operation).  The assembler
+// contracts a packed product and the packed sum it feeds, so sums of products
+// are written as fm, and ad takes no fresh product.
+struct p2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ p2 pk(float a, float b)
+{
+    p2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 up(p2 a)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+    return r;
+}
+__device__ __forceinline__ p2 fm(p2 a, p2 b, p2 c)
+{
+    p2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ p2 ml(p2 a, p2 b)
+{
+    p2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ p2 ad(p2 a, p2 b)
+{
+    p2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ p2 operator-(p2 a)
+{
+    const float2 u = up(a);
+    return pk(-u.x, -u.y);
+}
+// a constant in every lane of V
+template <typename V, typename R> __device__ __forceinline__ V bc(R a);
+template <> __device__ __forceinline__ float bc<float, float>(float a) { return a; }
+template <> __device__ __forceinline__ double bc<double, double>(double a) { return a; }
+template <> __device__ __forceinline__ p2 bc<p2, float>(float a) { return pk(a, a); }
+
 // a b - c d and a0 b0 + a1 b1 + a2 b2
 template <typename R> __device__ __forceinline__ R crs(R a, R b, R c, R d) { return fm(a, b, -ml(c, d)); }
 template <typename R> __device__ __forceinline__ R dot3(R a0, R b0, R a1, R b1, R a2, R b2)

@@ -146,7 +146,7 @@ struct Tpl {
     static constexpr int V = N / 8 < 1 ? 1 : (N / 8 > 32 ? 32 : N / 8);
 };
 
-// One radix-R Stockham stage (R = 2 or 4) of a line of N points: thread tl
+// One radix-R Stockham stage (R = 2, 4 or 8) of a line of N points: thread tl
 // of the line's TPL threads handles butterflies j = tl + TPL m.  tw is the
 // N-entry table exp(-2 pi i k / N) (conjugated for SIGN = +1).  C is float2
 // or double2.
@@ -171,8 +171,7 @@ __device__ __forceinline__ void sm_stage(const C* src, C* dst, int tl, const C* 
             }
             v[r] = x;
         }
-        if (R == 4) RegFFT<4, SIGN, C>::run(v);
-        else RegFFT<2, SIGN, C>::run(v);
+        RegFFT<R, SIGN, C>::run(v);
         const int idxD = (j - jm) * R + jm;
 #pragma unroll
         for (int r = 0; r < R; r++) dst[idxD + r * NS] = v[r];
@@ -184,10 +183,16 @@ __device__ __forceinline__ void sm_stage(const C* src, C* dst, int tl, const C* 
 template <int N, int SIGN, int TPL, int NS, typename C>
 struct SmStages {
     static_assert(TPL <= 32 && 32 % TPL == 0, "a line's threads must lie in one warp");
-    // radix-4 while four more points fit, a final radix-2 when log2(N) is odd
+    // radix-4 while four more points fit, a final radix-2 when log2(N) is odd;
+    // 512 points in three radix-8 stages (five passes through shared memory
+    // would be four of radix 4 and one of 2)
     __device__ __forceinline__ static C* run(C* a, C* b, int tl, const C* tw, bool act)
     {
-        if (NS * 4 <= N) {
+        if (N == 512 && NS * 8 <= N) {
+            if (act) sm_stage<N, 8, NS, SIGN, TPL, C>(a, b, tl, tw);
+            __syncwarp();
+            return SmStages<N, SIGN, TPL, (NS * 8 <= N ? NS * 8 : N), C>::run(b, a, tl, tw, act);
+        } else if (NS * 4 <= N) {
             if (act) sm_stage<N, 4, NS, SIGN, TPL, C>(a, b, tl, tw);
             __syncwarp();
             return SmStages<N, SIGN, TPL, (NS * 4 <= N ? NS * 4 : N), C>::run(b, a, tl, tw, act);

@@ -28,26 +28,30 @@ __device__ __forceinline__ FastKT<R> fastk_resolved(const FastKT<R>& F)
 // Cubic anisotropy field of one axis set at the reduced moment (sx, sy, sz)
 // = S / ms (M/cpu/anisotropy/..._cubic.cpp:308-390): axes n[0..2], n[3..5],
 // n[6..8], constants K[0..2]; quirk keeps (n2s2 + n3s3) in the first K1 term.
-template <typename R>
-__device__ __forceinline__ void cubic_field(R sx, R sy, R sz, const R* n, const R* K, int quirk, R& hx, R& hy,
-                                            R& hz)
+// V: R, or p2 (two sites).
+template <typename R, typename V = R>
+__device__ __forceinline__ void cubic_field(V sx, V sy, V sz, const R* n, const R* K, int quirk, V& hx, V& hy, V& hz)
 {
-    const R n1s = dot3(n[0], sx, n[1], sy, n[2], sz);
-    const R n2s = dot3(n[3], sx, n[4], sy, n[5], sz);
-    const R n3s = dot3(n[6], sx, n[7], sy, n[8], sz);
-    const R n1s2 = ml(n1s, n1s), n2s2 = ml(n2s, n2s), n3s2 = ml(n3s, n3s);
-    const R n1s3 = ml(n1s2, n1s), n2s3 = ml(n2s2, n2s), n3s3 = ml(n3s2, n3s);
-    const R n1s4 = ml(n1s2, n1s2), n2s4 = ml(n2s2, n2s2), n3s4 = ml(n3s2, n3s2);
-    const R q = quirk ? n3s3 : n3s2;
-    const R k1 = ml((R)2, K[0]), k2 = ml((R)2, K[1]), k3 = ml((R)4, K[2]);
-    const R a1 = ml(ml(k1, n1s), ad(n2s2, q)), a2 = ml(ml(k1, n2s), ad(n1s2, n3s2)), a3 = ml(ml(k1, n3s), ad(n1s2, n2s2));
-    const R p = ml(k2, ml(ml(n1s, n2s), n3s));
-    const R b1 = ml(p, ml(n2s, n3s)), b2 = ml(p, ml(n1s, n3s)), b3 = ml(p, ml(n1s, n2s));
-    const R c1 = ml(ml(k3, n1s3), ad(n2s4, n3s4)), c2 = ml(ml(k3, n2s3), ad(n1s4, n3s4)), c3 = ml(ml(k3, n3s3), ad(n1s4, n2s4));
-    const R s1 = ad(ad(a1, b1), c1), s2 = ad(ad(a2, b2), c2), s3 = ad(ad(a3, b3), c3);
-    hx = dot3(n[0], s1, n[3], s2, n[6], s3);
-    hy = dot3(n[1], s1, n[4], s2, n[7], s3);
-    hz = dot3(n[2], s1, n[5], s2, n[8], s3);
+    const auto B = [](R a) { return bc<V, R>(a); };
+    const V n1s = dot3(B(n[0]), sx, B(n[1]), sy, B(n[2]), sz);
+    const V n2s = dot3(B(n[3]), sx, B(n[4]), sy, B(n[5]), sz);
+    const V n3s = dot3(B(n[6]), sx, B(n[7]), sy, B(n[8]), sz);
+    const V n1s2 = ml(n1s, n1s), n2s2 = ml(n2s, n2s), n3s2 = ml(n3s, n3s);
+    const V n1s3 = ml(n1s2, n1s), n2s3 = ml(n2s2, n2s), n3s3 = ml(n3s2, n3s);
+    const V n3s4 = ml(n3s2, n3s2), n2s4 = ml(n2s2, n2s2);
+    const V q = quirk ? n3s3 : n3s2;
+    const V k1 = B(ml((R)2, K[0])), k2 = B(ml((R)2, K[1])), k3 = B(ml((R)4, K[2]));
+    const V p = ml(k2, ml(ml(n1s, n2s), n3s));
+    // every sum a fused multiply-add of its own (the packed forms are
+    // contracted otherwise)
+    const V c1 = ml(ml(k3, n1s3), fm(n2s2, n2s2, n3s4)), c2 = ml(ml(k3, n2s3), fm(n1s2, n1s2, n3s4)),
+            c3 = ml(ml(k3, n3s3), fm(n1s2, n1s2, n2s4));
+    const V s1 = fm(ml(k1, n1s), fm(n2s, n2s, q), fm(p, ml(n2s, n3s), c1));
+    const V s2 = fm(ml(k1, n2s), fm(n1s, n1s, n3s2), fm(p, ml(n1s, n3s), c2));
+    const V s3 = fm(ml(k1, n3s), fm(n1s, n1s, n2s2), fm(p, ml(n1s, n2s), c3));
+    hx = dot3(B(n[0]), s1, B(n[3]), s2, B(n[6]), s3);
+    hy = dot3(B(n[1]), s1, B(n[4]), s2, B(n[7]), s3);
+    hz = dot3(B(n[2]), s1, B(n[5]), s2, B(n[8]), s3);
 }
 
 // ------------------------------------------------------------------ fused step
@@ -63,8 +67,6 @@ __device__ __forceinline__ void cubic_field(R sx, R sy, R sz, const R* n, const 
 // reciprocal square root and sine/cosine in the state precision
 __device__ __forceinline__ float fs_rsqrt(float v) { return rsqrtf(v); }
 __device__ __forceinline__ double fs_rsqrt(double v) { return rsqrt(v); }
-__device__ __forceinline__ void fs_sincos(float a, float* s, float* c) { sincosf(a, s, c); }
-__device__ __forceinline__ void fs_sincos(double a, double* s, double* c) { sincos(a, s, c); }
 
 // The spins come through ld(c, j) (component c of site j): global loads, or
 // shared-memory copies of some rows (the fused x pass).
@@ -81,6 +83,155 @@ __device__ __forceinline__ float3 thermal_normal3(const FastKT<R>& F, int i)
 {
     const uint64_t ctr = F.counter + (F.dctr ? *F.dctr : 0ull);
     return philox_normal3(F.seed, ctr, (uint32_t)i, 0x6d6c6232u);
+}
+
+// sine and cosine of the half rotation angle; in FP32 small angles by their
+// Taylor series (|th| <= 0.1: truncation below 1e-10, under FP32 rounding),
+// else (and always in FP64) sine and cosine
+template <typename V>
+__device__ __forceinline__ void taylor_sincos(V th, V& sn, V& cs)
+{
+    const auto B = [](float a) { return bc<V, float>(a); };
+    const V t2 = ml(th, th), n2 = -t2, one = B(1.f);
+    const V a = fm(n2, B(1.0f / 42.0f), one), b = fm(ml(n2, B(1.0f / 20.0f)), a, one);
+    sn = ml(th, fm(ml(n2, B(1.0f / 6.0f)), b, one));
+    const V c = fm(n2, B(1.0f / 56.0f), one), d = fm(ml(n2, B(1.0f / 30.0f)), c, one);
+    const V e = fm(ml(n2, B(1.0f / 12.0f)), d, one);
+    cs = fm(ml(n2, B(0.5f)), e, one);
+}
+__device__ __forceinline__ void half_sincos(float th, float& sn, float& cs)
+{
+    if (fabsf(th) <= 0.1f) taylor_sincos<float>(th, sn, cs);
+    else sincosf(th, &sn, &cs);
+}
+__device__ __forceinline__ void half_sincos(double th, double& sn, double& cs) { sincos(th, &sn, &cs); }
+__device__ __forceinline__ void half_sincos(p2 th, p2& sn, p2& cs)
+{
+    const float2 t = up(th);
+    if (fmaxf(fabsf(t.x), fabsf(t.y)) <= 0.1f) {
+        taylor_sincos<p2>(th, sn, cs);
+    } else {
+        float s0, c0, s1, c1;
+        half_sincos(t.x, s0, c0);
+        half_sincos(t.y, s1, c1);
+        sn = pk(s0, s1);
+        cs = pk(c0, c1);
+    }
+}
+__device__ __forceinline__ p2 fs_rsqrt(p2 v)
+{
+    const float2 u = up(v);
+    return pk(rsqrtf(u.x), rsqrtf(u.y));
+}
+// lanes of a where the lane of m is positive (not zero), else of b
+__device__ __forceinline__ float where_pos(float m, float a, float b) { return m > 0.f ? a : b; }
+__device__ __forceinline__ double where_pos(double m, double a, double b) { return m > 0.0 ? a : b; }
+__device__ __forceinline__ p2 where_pos(p2 m, p2 a, p2 b)
+{
+    const float2 u = up(m), x = up(a), y = up(b);
+    return pk(u.x > 0.f ? x.x : y.x, u.y > 0.f ? x.y : y.y);
+}
+__device__ __forceinline__ float where_nz(float m, float a, float b) { return m != 0.f ? a : b; }
+__device__ __forceinline__ double where_nz(double m, double a, double b) { return m != 0.0 ? a : b; }
+__device__ __forceinline__ p2 where_nz(p2 m, p2 a, p2 b)
+{
+    const float2 u = up(m), x = up(a), y = up(b);
+    return pk(u.x != 0.f ? x.x : y.x, u.y != 0.f ? x.y : y.y);
+}
+// 0 in every lane? (x 0 is 0 for a finite x, else not a number)
+__device__ __forceinline__ bool all_zero(float a) { return a == 0.f; }
+__device__ __forceinline__ bool all_zero(double a) { return a == 0.0; }
+__device__ __forceinline__ bool all_zero(p2 a)
+{
+    const float2 u = up(a);
+    return u.x == 0.f && u.y == 0.f;
+}
+
+// The rest of a site's step, after the Zeeman and exchange fields H: anisotropy,
+// thermal (nrm: its standard normals), the addend A, the LLG update.  V: R for
+// one site, p2 for two, each lane the same operations.
+template <int LT, bool ANI, bool TH, bool ADD, typename R, typename V>
+__device__ __forceinline__ void fused_update(const FastKT<R>& F, V Sx, V Sy, V Sz, V Hx, V Hy, V Hz, V nrmx, V nrmy,
+                                             V nrmz, V Ax, V Ay, V Az, V& rx, V& ry, V& rz)
+{
+    const auto B = [](R a) { return bc<V, R>(a); };
+    if (ANI) {
+        if (F.ani == 2) {
+            // one uniform cubic axis set
+            V cx, cy, cz;
+            const V im = B(F.cub_ims);
+            cubic_field<R, V>(ml(Sx, im), ml(Sy, im), ml(Sz, im), F.cub_n, F.cub_K, F.cub_quirk, cx, cy, cz);
+            Hx = ad(Hx, cx); Hy = ad(Hy, cy); Hz = ad(Hz, cz);
+        } else {
+            const V ax = B(F.axis[0]), ay = B(F.axis[1]), az = B(F.axis[2]);
+            const V v = ml(B(F.ani_c), dot3(Sx, ax, Sy, ay, Sz, az));
+            Hx = fm(v, ax, Hx); Hy = fm(v, ay, Hy); Hz = fm(v, az, Hz);
+        }
+    }
+    if (ADD) {
+        const V w = B(F.addw);
+        Hx = fm(w, Ax, Hx); Hy = fm(w, Ay, Hy); Hz = fm(w, Az, Hz);
+    }
+    // the field without the thermal part, for the terms that leave it out
+    V gx = Hx, gy = Hy, gz = Hz;
+    if (TH) {
+        const V sg = B(F.sigma);
+        Hx = fm(sg, nrmx, Hx); Hy = fm(sg, nrmy, Hy); Hz = fm(sg, nrmz, Hz);
+        if (!F.tof) { gx = Hx; gy = Hy; gz = Hz; }
+    }
+    V nx_ = Sx, ny_ = Sy, nz_ = Sz;
+    if (LT == LLG_CART) {
+        if (!F.dt_zero) {
+            // dM = -p gaa M x H - d (a/ms) gaa M x (M x h), h = H - Hth
+            const V mhx = crs(Sy, gz, Sz, gy), mhy = crs(Sz, gx, Sx, gz), mhz = crs(Sx, gy, Sy, gx);
+            const V mmx = crs(Sy, mhz, Sz, mhy), mmy = crs(Sz, mhx, Sx, mhz), mmz = crs(Sx, mhy, Sy, mhx);
+            const V MHx = crs(Sy, Hz, Sz, Hy), MHy = crs(Sz, Hx, Sx, Hz), MHz = crs(Sx, Hy, Sy, Hx);
+            const V dt = B(F.dt), cp = B(F.c_prec), cd = B(F.c_damp);
+            nx_ = fm(dt, crs(cp, MHx, cd, mmx), Sx);
+            ny_ = fm(dt, crs(cp, MHy, cd, mmy), Sy);
+            nz_ = fm(dt, crs(cp, MHz, cd, mmz), Sz);
+        }
+    } else {
+        V Hpx, Hpy, Hpz;
+        const V cd = B(F.c_damp);
+        if (F.tof) {
+            const V shx = crs(Sy, gz, Sz, gy), shy = crs(Sz, gx, Sx, gz), shz = crs(Sx, gy, Sy, gx);
+            const V pr = B(F.precess);
+            Hpx = fm(pr, Hx, ml(cd, shx));
+            Hpy = fm(pr, Hy, ml(cd, shy));
+            Hpz = fm(pr, Hz, ml(cd, shz));
+        } else {
+            const V shx = crs(Sy, Hz, Sz, Hy), shy = crs(Sz, Hx, Sx, Hz), shz = crs(Sx, Hy, Sy, Hx);
+            Hpx = fm(cd, shx, Hx); Hpy = fm(cd, shy, Hy); Hpz = fm(cd, shz, Hz);
+        }
+        const V HL2 = dot3(Hpx, Hpx, Hpy, Hpy, Hpz, Hpz);
+        const V iHL = fs_rsqrt(HL2);
+        const V th = ml(B(F.c_rot), ml(HL2, iHL));
+        V sn, cs;
+        half_sincos(th, sn, cs);
+        const V k = ml(sn, iHL);
+        const V qw = cs, qx = ml(k, Hpx), qy = ml(k, Hpy), qz = ml(k, Hpz);
+        const V nw = dot3(qx, Sx, qy, Sy, qz, Sz);   // -tw
+        const V tx = fm(qw, Sx, crs(qy, Sz, qz, Sy));
+        const V ty = fm(qw, Sy, crs(qz, Sx, qx, Sz));
+        const V tz = fm(qw, Sz, crs(qx, Sy, qy, Sx));
+        // no rotation without a field
+        nx_ = where_pos(HL2, fm(qw, tx, fm(nw, qx, crs(tz, qy, ty, qz))), Sx);
+        ny_ = where_pos(HL2, fm(qw, ty, fm(nw, qy, crs(tx, qz, tz, qx))), Sy);
+        nz_ = where_pos(HL2, fm(qw, tz, fm(nw, qz, crs(ty, qx, tx, qy))), Sz);
+    }
+    if (F.renorm) {
+        const V mm = dot3(nx_, nx_, ny_, ny_, nz_, nz_);
+        const V inv = ml(B(F.ms), fs_rsqrt(mm));
+        nx_ = where_nz(mm, ml(nx_, inv), nx_);
+        ny_ = where_nz(mm, ml(ny_, inv), ny_);
+        nz_ = where_nz(mm, ml(nz_, inv), nz_);
+    }
+    rx = nx_; ry = ny_; rz = nz_;
+    if (F.status) {
+        const V z = B((R)0);
+        if (!all_zero(fm(nx_, z, fm(ny_, z, ml(nz_, z))))) atomicOr(F.status, 1u);
+    }
 }
 
 template <int LT, bool EXS, bool ANI, bool TH, bool ADD, typename R, class LD>
@@ -121,91 +272,9 @@ __device__ __forceinline__ void fused_site_ld(const FastKT<R>& F, int NX, int NY
         }
         Hx = ad(Hx, ex); Hy = ad(Hy, ey); Hz = ad(Hz, ez);
     }
-    if (ANI) {
-        if (F.ani == 2) {
-            // one uniform cubic axis set
-            R cx, cy, cz;
-            cubic_field<R>(ml(Sx, F.cub_ims), ml(Sy, F.cub_ims), ml(Sz, F.cub_ims), F.cub_n, F.cub_K, F.cub_quirk, cx,
-                           cy, cz);
-            Hx = ad(Hx, cx); Hy = ad(Hy, cy); Hz = ad(Hz, cz);
-        } else {
-            const R v = ml(F.ani_c, dot3(Sx, F.axis[0], Sy, F.axis[1], Sz, F.axis[2]));
-            Hx = fm(v, F.axis[0], Hx); Hy = fm(v, F.axis[1], Hy); Hz = fm(v, F.axis[2], Hz);
-        }
-    }
-    R Tx = 0, Ty = 0, Tz = 0;
-    if (TH) {
-        const float3 nrm = pre ? *pre : thermal_normal3(F, i);
-        Tx = ml(F.sigma, (R)nrm.x); Ty = ml(F.sigma, (R)nrm.y); Tz = ml(F.sigma, (R)nrm.z);
-        Hx = ad(Hx, Tx); Hy = ad(Hy, Ty); Hz = ad(Hz, Tz);
-    }
-    if (ADD) {
-        Hx = fm(F.addw, Ax, Hx); Hy = fm(F.addw, Ay, Hy); Hz = fm(F.addw, Az, Hz);
-    }
-    R nx_, ny_, nz_;
-    if (LT == LLG_CART) {
-        if (F.dt_zero) { nx_ = Sx; ny_ = Sy; nz_ = Sz; }
-        else {
-            // h = H - Hth; dM = -p gaa M x H - d (a/ms) gaa M x (M x h)
-            const R hx = F.tof ? ad(Hx, -Tx) : Hx, hy = F.tof ? ad(Hy, -Ty) : Hy, hz = F.tof ? ad(Hz, -Tz) : Hz;
-            const R mhx = crs(Sy, hz, Sz, hy), mhy = crs(Sz, hx, Sx, hz), mhz = crs(Sx, hy, Sy, hx);
-            const R mmx = crs(Sy, mhz, Sz, mhy), mmy = crs(Sz, mhx, Sx, mhz), mmz = crs(Sx, mhy, Sy, mhx);
-            const R MHx = crs(Sy, Hz, Sz, Hy), MHy = crs(Sz, Hx, Sx, Hz), MHz = crs(Sx, Hy, Sy, Hx);
-            nx_ = fm(F.dt, crs(F.c_prec, MHx, F.c_damp, mmx), Sx);
-            ny_ = fm(F.dt, crs(F.c_prec, MHy, F.c_damp, mmy), Sy);
-            nz_ = fm(F.dt, crs(F.c_prec, MHz, F.c_damp, mmz), Sz);
-        }
-    } else {
-        R Hpx, Hpy, Hpz;
-        if (F.tof) {
-            const R hx = ad(Hx, -Tx), hy = ad(Hy, -Ty), hz = ad(Hz, -Tz);
-            const R shx = crs(Sy, hz, Sz, hy), shy = crs(Sz, hx, Sx, hz), shz = crs(Sx, hy, Sy, hx);
-            Hpx = fm(F.precess, Hx, ml(F.c_damp, shx));
-            Hpy = fm(F.precess, Hy, ml(F.c_damp, shy));
-            Hpz = fm(F.precess, Hz, ml(F.c_damp, shz));
-        } else {
-            const R shx = crs(Sy, Hz, Sz, Hy), shy = crs(Sz, Hx, Sx, Hz), shz = crs(Sx, Hy, Sy, Hx);
-            Hpx = fm(F.c_damp, shx, Hx); Hpy = fm(F.c_damp, shy, Hy); Hpz = fm(F.c_damp, shz, Hz);
-        }
-        const R HL2 = dot3(Hpx, Hpx, Hpy, Hpy, Hpz, Hpz);
-        if (HL2 > (R)0) {
-            const R iHL = fs_rsqrt(HL2);
-            const R HL = ml(HL2, iHL);
-            // half rotation angle; in FP32 small angles by their Taylor
-            // series (|th| <= 0.1: truncation below 1e-10, under FP32
-            // rounding), else (and always in FP64) sine and cosine
-            const R th = ml(F.c_rot, HL);
-            R sn, cs;
-            if (sizeof(R) == 4 && fabs(th) <= (R)0.1) {
-                const R t2 = ml(th, th);
-                const R a = fm(-t2, (R)(1.0f / 42.0f), (R)1), b = fm(ml(-t2, (R)(1.0f / 20.0f)), a, (R)1);
-                sn = ml(th, fm(ml(-t2, (R)(1.0f / 6.0f)), b, (R)1));
-                const R c = fm(-t2, (R)(1.0f / 56.0f), (R)1), d = fm(ml(-t2, (R)(1.0f / 30.0f)), c, (R)1);
-                const R e = fm(ml(-t2, (R)(1.0f / 12.0f)), d, (R)1);
-                cs = fm(ml(-t2, (R)0.5f), e, (R)1);
-            } else {
-                fs_sincos(th, &sn, &cs);
-            }
-            const R k = ml(sn, iHL);
-            const R qw = cs, qx = ml(k, Hpx), qy = ml(k, Hpy), qz = ml(k, Hpz);
-            const R tw = -dot3(qx, Sx, qy, Sy, qz, Sz);
-            const R tx = fm(qw, Sx, crs(qy, Sz, qz, Sy));
-            const R ty = fm(qw, Sy, crs(qz, Sx, qx, Sz));
-            const R tz = fm(qw, Sz, crs(qx, Sy, qy, Sx));
-            nx_ = fm(qw, tx, fm(-tw, qx, crs(tz, qy, ty, qz)));
-            ny_ = fm(qw, ty, fm(-tw, qy, crs(tx, qz, tz, qx)));
-            nz_ = fm(qw, tz, fm(-tw, qz, crs(ty, qx, tx, qy)));
-        } else { nx_ = Sx; ny_ = Sy; nz_ = Sz; }
-    }
-    if (F.renorm) {
-        const R mm = dot3(nx_, nx_, ny_, ny_, nz_, nz_);
-        if (mm != (R)0) {
-            const R inv = ml(F.ms, fs_rsqrt(mm));
-            nx_ = ml(nx_, inv); ny_ = ml(ny_, inv); nz_ = ml(nz_, inv);
-        }
-    }
-    rx = nx_; ry = ny_; rz = nz_;
-    if (F.status && !(isfinite(nx_) && isfinite(ny_) && isfinite(nz_))) atomicOr(F.status, 1u);
+    float3 nrm = make_float3(0.f, 0.f, 0.f);
+    if (TH) nrm = pre ? *pre : thermal_normal3(F, i);
+    fused_update<LT, ANI, TH, ADD, R, R>(F, Sx, Sy, Sz, Hx, Hy, Hz, (R)nrm.x, (R)nrm.y, (R)nrm.z, Ax, Ay, Az, rx, ry, rz);
 }
 
 template <int LT, bool EXS, bool ANI, bool TH, bool ADD, typename R = float>
@@ -218,3 +287,59 @@ __device__ __forceinline__ void fused_site_v(const FastKT<R>& F, int NX, int NY,
     fused_site_ld<LT, EXS, ANI, TH, ADD, R>(F, NX, NY, NZ, x, y, z, i, g, Ax, Ay, Az, rx, ry, rz, pre);
 }
 
+// Two sites of a FP32 lattice at once, i and i + NX: rows y and y + 1 of one
+// layer (y + 1 < NY), addends A packed (row y, row y + 1).  Every lane repeats
+// fused_site_v's operations (an absent neighbour or an unused direction adds
+// 0 times the site itself there instead of nothing), two per packed
+// instruction; the rows are each other's y neighbours, and the neighbours'
+// offsets serve both.  Byte offsets are 32 bits: at most 2^30 sites.
+template <int LT, bool ANI, bool TH>
+__device__ __forceinline__ void fused_pair(const FastK& F, int NX, int NY, int NZ, int x, int y, int z, int i,
+                                           const float* __restrict__ sx, const float* __restrict__ sy,
+                                           const float* __restrict__ sz, const p2 A[3], const p2 nrm[3], p2 r[3])
+{
+    const auto ld = [](const float* s, unsigned off) {
+        return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(s) + off));
+    };
+    const int nxy = NX * NY;
+    const unsigned o0 = 4u * (unsigned)i, o1 = o0 + 4u * (unsigned)NX;
+    // offsets in bytes (0: absent) and weights of the neighbours
+    int dxp = 4, dxm = -4, dyp = 4 * NX, dym = -4 * NX, dzp = 4 * nxy, dzm = -4 * nxy;
+    float jxp = F.J[0], jxm = F.J[1], jyp = F.J[2], jym = F.J[3], jzp = F.J[4], jzm = F.J[5];
+    if (x + 1 >= NX) { dxp = F.pbc[0] ? 4 - 4 * NX : 0; jxp = F.pbc[0] ? jxp : 0.f; }
+    if (x == 0) { dxm = F.pbc[0] ? 4 * NX - 4 : 0; jxm = F.pbc[0] ? jxm : 0.f; }
+    if (y + 2 >= NY) { dyp = F.pbc[1] ? 4 * NX - 4 * nxy : 0; jyp = F.pbc[1] ? jyp : 0.f; }
+    if (y == 0) { dym = F.pbc[1] ? 4 * nxy - 4 * NX : 0; jym = F.pbc[1] ? jym : 0.f; }
+    if (z + 1 >= NZ) { dzp = F.pbc[2] ? 4 * nxy - 4 * nxy * NZ : 0; jzp = F.pbc[2] ? jzp : 0.f; }
+    if (z == 0) { dzm = F.pbc[2] ? 4 * nxy * NZ - 4 * nxy : 0; jzm = F.pbc[2] ? jzm : 0.f; }
+    const float* s[3] = {sx, sy, sz};
+    float own[3][2], nb[3][10];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        own[c][0] = ld(s[c], o0);
+        own[c][1] = ld(s[c], o1);
+        nb[c][0] = ld(s[c], o0 + dxp); nb[c][1] = ld(s[c], o1 + dxp);
+        nb[c][2] = ld(s[c], o0 + dxm); nb[c][3] = ld(s[c], o1 + dxm);
+        nb[c][4] = ld(s[c], o1 + dyp);
+        nb[c][5] = ld(s[c], o0 + dym);
+        nb[c][6] = ld(s[c], o0 + dzp); nb[c][7] = ld(s[c], o1 + dzp);
+        nb[c][8] = ld(s[c], o0 + dzm); nb[c][9] = ld(s[c], o1 + dzm);
+    }
+    const p2 wx0 = pk(jxp, jxp), wx1 = pk(jxm, jxm), wy0 = pk(F.J[2], jyp), wy1 = pk(jym, F.J[3]);
+    const p2 wz0 = pk(jzp, jzp), wz1 = pk(jzm, jzm);
+    p2 S[3], H[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        S[c] = pk(own[c][0], own[c][1]);
+        p2 e = pk(0.f, 0.f);
+        if (F.J[0] != 0.f) e = fm(wx0, pk(nb[c][0], nb[c][1]), e);
+        if (F.J[1] != 0.f) e = fm(wx1, pk(nb[c][2], nb[c][3]), e);
+        if (F.J[2] != 0.f) e = fm(wy0, pk(own[c][1], nb[c][4]), e);
+        if (F.J[3] != 0.f) e = fm(wy1, pk(nb[c][5], own[c][0]), e);
+        if (F.J[4] != 0.f) e = fm(wz0, pk(nb[c][6], nb[c][7]), e);
+        if (F.J[5] != 0.f) e = fm(wz1, pk(nb[c][8], nb[c][9]), e);
+        H[c] = ad(pk(F.B[c], F.B[c]), e);
+    }
+    fused_update<LT, ANI, TH, true, float, p2>(F, S[0], S[1], S[2], H[0], H[1], H[2], nrm[0], nrm[1], nrm[2], A[0], A[1],
+                                               A[2], r[0], r[1], r[2]);
+}

@@ -91,6 +91,7 @@ cudaError_t launch_conv_fast_fyz(const ConvK& c, const FftLen L[3], const float2
 cudaError_t launch_conv_fast_ix(const ConvK& c, const FftLen L[3], const float2* tw, float2* spec, float* h[3],
                                 cudaStream_t st);
 bool xstep_ok(const ConvK& c, const FastK& F);
+bool xstep_pairs(const ConvK& c);
 // Inverse x pass + fused step (+ forward x pass of the new spins when fwd).
 cudaError_t launch_xstep(const ConvK& c, const FftLen L[3], const float2* tw, float2* spec, const FastK& F,
                          bool fwd, const float* s[3], float* h[3], float* o[3], cudaStream_t st);

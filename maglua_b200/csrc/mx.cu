@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(256, Occ<R, BIG>::X) k_mx_ix(const __grid_cons
 
 // ------------------------------------------------------------------ fused x pass of a step
 // The CTA's rows through the inverse x transform (-> their dipole field,
-// written to its slot), the field terms and LLG update of their sites (-> the
+// written to its slot unless hx is null), the field terms and LLG update of their sites (-> the
 // new spins; neighbours read from the current spin arrays, which no CTA
 // writes) and the forward x transform of the new spins (-> the next step's
 // spectrum rows, the ones the CTA itself read).  site(i, x, y, z, A) returns
@@ -520,7 +520,7 @@ __device__ __forceinline__ void step_rows(const MxX& m, typename CT<R>::T* __res
             int z = zr0, y = yr0 + row;
             while (y >= m.ny) { y -= m.ny; z++; }
             const int i = (rc.row0 + row) * m.nx + x;
-            hx[i] = Ad.x; hy[i] = Ad.y; hz[i] = Ad.z;
+            if (hx) { hx[i] = Ad.x; hy[i] = Ad.y; hz[i] = Ad.z; }
             o = site(i, x, y, z, Ad);
             ox[i] = o.x; oy[i] = o.y; oz[i] = o.z;
         }
