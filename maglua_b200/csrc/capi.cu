@@ -1690,6 +1690,16 @@ void flush_pending(mlb_system* s)
                                 h, s->st));
 }
 
+// Layer scales of a LongRange2D, the operator's global scale included.
+void lr2d_scales(const mlb_op* op, LR2DScale& sc)
+{
+    memset(&sc, 0, sizeof(sc));
+    for (int z = 0; z < op->nz; z++) {
+        sc.src[z] = op->lr2_src[z];
+        sc.dst[z] = op->lr2_dst[z] * op->gs;
+    }
+}
+
 void op_apply(mlb_op* op, mlb_system* s)
 {
     check_dims(op, s);
@@ -1782,11 +1792,7 @@ void op_apply(mlb_op* op, mlb_system* s)
         if (s->dry) return;
         LR2DPlan& P = *op->lr2;
         LR2DScale sc;
-        memset(&sc, 0, sizeof(sc));
-        for (int z = 0; z < op->nz; z++) {
-            sc.src[z] = op->lr2_src[z];
-            sc.dst[z] = op->lr2_dst[z] * op->gs;
-        }
+        lr2d_scales(op, sc);
         const void* sp[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
         if (!P.k.mx) {
             CK(mlb::launch_lr2d(P.k, P.L, P.tw.p, sp, P.spec.p, P.Q.p, sc, sl.h, s->rb, s->st));
@@ -5564,11 +5570,153 @@ void rk_row(mlb_rk* r, mlb_system* src, const std::vector<double>& f, mlb_system
         if (i <= (int)f.size() && f[i - 1] != 0.0) llg_apply(r->l, dst, f[i - 1], r->k[i - 2], dst, 1);
 }
 
+// The stages of a step on ss as fused passes: every stage's field (inverse x
+// pass and local terms) with the updates of all rows it contributes to in one
+// kernel (rk_rows), next to its (y,z) pass.  Each row takes its updates in the
+// order of rk_row.  Taken for uniform parameters, distinct operators in slots
+// of their own, one of them a convolution whose x passes are fused; false (and
+// nothing launched) otherwise.  The base system's new spins go to its other
+// buffer, so the fields of the step's start stay as they were recorded.
+template <typename R>
+bool rk_stages(mlb_rk* r, mlb_system* ss, bool keep_field)
+{
+    const int nst = (int)r->bt.size();
+    mlb_op* conv = nullptr;
+    std::set<int> kinds;
+    std::set<std::string> slots;
+    for (mlb_op* o : r->ops) {
+        const bool cv = is_conv(o->kind) || is_lr2d(o->kind);
+        if (o->kind == MLB_OP_THERMAL || (cv && conv) || !kinds.insert(o->kind).second) return false;
+        std::string n = o->slot;
+        for (char& ch : n) ch = (char)tolower(ch);
+        if (n == "total" || n == "thermal" || !slots.insert(n).second) return false;
+        if (cv) conv = o;
+    }
+    if (!conv || ss->sur || ss->dry || nst > MLB_RK_ROWS) return false;
+    for (mlb_system* k : r->k)
+        if (k->st != ss->st || k->rb != ss->rb || k->n != ss->n || k->alpha != ss->alpha || k->gamma != ss->gamma || k->sa || k->sg)
+            return false;
+    // the host's part of the start's field; the plan is built if need be
+    ss->dry = true;
+    try {
+        rk_field(r, ss);
+    } catch (...) {
+        ss->dry = false;
+        throw;
+    }
+    ss->dry = false;
+    ConvPlan* P = conv_of(conv);
+    if (P->k.general && !is_lr2d(conv->kind)) return false;
+    if (!P->k.mx && !(ss->rb == 4 && mlb::conv_fast_ok(P->k))) return false;
+    TermsK T;
+    long long gen;
+    double dt_sys;
+    build_sum_terms(ss, ss->slots[0].sum_list, T, gen, dt_sys, false, -1);
+    FastKT<R> F;
+    const int si = slot_find(ss, conv->slot.c_str());
+    if (gen != ss->gen || T.nadd != 1 || T.add[0][0] != ss->slots[si].h[0]) return false;
+    if (!fast_fused_t<R>(ss, T, r->l, ss->dt, dt_sys, F)) return false;
+    const bool pow2 = sizeof(R) == 4 && !P->x_mx;
+    if (pow2 ? !mlb::xstep_pairs(P->k) || P->k.Px < 32 : !P->x_mx) return false;
+    const bool cart = r->l->kind != MLB_LLG_QUATERNION;
+    const int cur = ss->cur, nb = 1 - cur;
+    nm_guard(ss, nb);
+    std::vector<bool> started(nst, false);
+    auto buf = [&](int row, int c) -> R* {   // running value of a row
+        return static_cast<R*>(row == nst - 1 ? ss->sp[nb][c] : r->k[row]->sp[r->k[row]->cur][c]);
+    };
+    for (int row = 0; row + 1 < nst; row++) {
+        mlb_system* k = r->k[row];
+        k->dt = ss->dt;
+        reset_fields(k);
+        k->spec_token = 0;
+        nm_guard(k, k->cur);
+    }
+    for (int i = 0; i < nst; i++) {
+        const void* sv[3];
+        const R* s[3];
+        R* o[3];
+        for (int c = 0; c < 3; c++) {
+            sv[c] = i == 0 ? ss->sp[cur][c] : r->k[i - 1]->sp[r->k[i - 1]->cur][c];
+            s[c] = static_cast<const R*>(sv[c]);
+            o[c] = buf(i, c);
+        }
+        RkRows<R> rows;
+        memset(&rows, 0, sizeof(rows));
+        for (int row = i; row < nst; row++) {
+            const std::vector<double>& f = r->bt[row];
+            const double w = i < (int)f.size() ? f[i] : 0.0;
+            // row i is the next stage's spins whatever its last weight
+            if (w == 0.0 && row != i) continue;
+            auto& e = rows.row[rows.n++];
+            for (int c = 0; c < 3; c++) {
+                e.base[c] = started[row] ? buf(row, c) : (i == 0 ? nullptr : static_cast<const R*>(ss->sp[cur][c]));
+                e.dst[c] = buf(row, c);
+            }
+            e.fresh = !started[row] && i > 0;
+            const double dt = w * ss->dt;
+            e.dt = (R)dt;
+            e.c_rot = (R)(0.5 * ss->gamma * dt / (1.0 + ss->alpha * ss->alpha));
+            started[row] = true;
+        }
+        const bool last = i == nst - 1;
+        const bool keep = i == 0 && keep_field;
+        R* h[3] = {nullptr, nullptr, nullptr};
+        for (int c = 0; c < 3 && keep; c++) h[c] = static_cast<R*>(ss->slots[si].h[c]);
+        // the (y,z) pass; the first stage's forward x pass before it
+        if (is_lr2d(conv->kind)) {
+            LR2DPlan& Q = *conv->lr2;
+            LR2DScale sc;
+            lr2d_scales(conv, sc);
+            if (i == 0) launch_x(*P, P->k, sv, P->spec.p, nullptr, true, ss->st);
+            CK(mlb::launch_mx_lr2d(P->k, P->mx.yz, P->L, P->tw.p, P->spec.p, Q.Q.p, sc, ss->rb, ss->st));
+        } else if (P->k.mx) {
+            if (i == 0) launch_x(*P, P->k, sv, P->spec.p, nullptr, true, ss->st);
+            launch_yz(*P, P->k, P->spec.p, ss->st);
+        } else {
+            const float* sf[3] = {static_cast<const float*>(sv[0]), static_cast<const float*>(sv[1]),
+                                  static_cast<const float*>(sv[2])};
+            CK(mlb::launch_conv_fast_fyz(P->k, P->L, reinterpret_cast<const float2*>(P->tw.p), sf,
+                                         reinterpret_cast<float2*>(P->spec.p),
+                                         reinterpret_cast<const float*>(P->ten6.p), i == 0, ss->st));
+        }
+        if constexpr (sizeof(R) == 4) {
+            if (pow2) {
+                CK(mlb::launch_xrk(P->k, P->L, P->tw.p, P->spec.p, F, rows, !last, s, h, o, ss->st));
+                continue;
+            }
+        }
+        CK(mlb::launch_mx_rk<R>(P->mx.x, P->L, P->tw.p, P->spec.p, F, rows, s, h, o, ss->st));
+    }
+    P->spec_token = 0;
+    ss->spec_token = 0;
+    ss->cur = nb;
+    ss->gen++;
+    // the times rk_row's updates of ss add up to
+    const std::vector<double>& f = r->bt[nst - 1];
+    for (size_t i = 0; i < f.size(); i++)
+        if (i == 0 || f[i] != 0.0) {
+            const double dt = f[i] * ss->dt;
+            if (!cart || dt != 0.0) ss->time = ss->time + dt;
+        }
+    return true;
+}
+
 // sfunc (RungeKutta.lua:194-213) on the base system ss (the script's
 // ss_input, default the system the scheme was made for)
 void rk_step(mlb_rk* r, mlb_system* ss, bool skip_temperature)
 {
     const int nstep = (int)r->bt.size();
+    const bool kick = r->temp && !skip_temperature;
+    if (ss->rb == 4 ? rk_stages<float>(r, ss, !kick) : rk_stages<double>(r, ss, !kick)) {
+        if (kick) {
+            reset_fields(ss);
+            op_apply(r->temp, ss);
+            sum_fields(ss);
+            llg_apply(r->l, ss, 1.0, ss, ss, 0);
+        }
+        return;
+    }
     rk_field(r, ss);
     for (int i = 1; i <= nstep - 1; i++) {
         mlb_system* d = r->k[i - 1];   // ss_k[i+1]

@@ -1346,6 +1346,39 @@ __global__ void __launch_bounds__(XSCfg<PX, false, SZ>::NT, XSCfg<PX, false, SZ>
         });
 }
 
+// A stage of a Runge-Kutta scheme: the inverse x pass of the stage's field, its
+// local terms and the rows it contributes to, two sites at a time; forward x
+// pass of row 0, the next stage's spins (fwd).  Bound like k_xstep by the
+// instructions of its sites; CTAs of 512 sites (two per SM at 128 registers).
+// An RK4 step with a thermal kick of 256x256x8 as 11 kernels in place of 29
+// (fields evaluated to slots and one pass per row and stage): alone 300 -> 169
+// us, among others 211 -> 122.
+template <int PX, int LT, bool ANI, int SZ>
+__global__ void __launch_bounds__(XSCfg<PX, false, SZ>::NT, XSCfg<PX, false, SZ>::GOCC)
+    k_xrk(ConvK c, const __grid_constant__ FastK F, const __grid_constant__ RkRows<float> rows, int fwd,
+          const float2* __restrict__ tw, float2* __restrict__ spec, const float* sx, const float* sy, const float* sz,
+          float* hx, float* hy, float* hz, float* ox, float* oy, float* oz)
+{
+    xstep_body<PX, false, SZ, true>(
+        c, nullptr, nullptr, fwd, tw, spec, sx, sy, sz, hx, hy, hz, ox, oy, oz, [] {}, [](int, int, int, bool) {},
+        [&](int i, int, int x, int y, int z, float2 Ax, float2 Ay, float2 Az, float2& rx, float2& ry, float2& rz) {
+            p2 M[3], H[3], g[3], o[3];
+            const p2 n = pk(0.f, 0.f);
+            pair_near(F, c.nx, c.ny, c.nz, x, y, z, i, sx, sy, sz, M, H);
+            fused_field<ANI, false, true, float, p2>(F, M[0], M[1], M[2], H[0], H[1], H[2], n, n, n, pk(Ax.x, Ax.y),
+                                                     pk(Ay.x, Ay.y), pk(Az.x, Az.y), g[0], g[1], g[2]);
+            rk_rows<LT, float, p2>(
+                F, rows, M, H, [&](const float* b) { return pk(b[i], b[i + c.nx]); },
+                [&](float* d, p2 v) {
+                    const float2 u = up(v);
+                    d[i] = u.x;
+                    d[i + c.nx] = u.y;
+                },
+                o);
+            rx = up(o[0]); ry = up(o[1]); rz = up(o[2]);
+        });
+}
+
 // Packed ensemble: tile b covers sites [bstart[b], bstart[b] + blockDim) of
 // packed replica brep[b]; rinfo[r] = {nx, ny, nz, first packed site}.  CTAs
 // walk the tile table with stride gridDim.x (persistent when the grid is
@@ -1828,6 +1861,51 @@ cudaError_t launch_xstep(const ConvK& c, const FftLen L[3], const float2* tw, fl
     return cudaErrorInvalidValue;
 }
 
+template <int PX, int LT, bool ANI, int SZ>
+static cudaError_t xrk_sz(const ConvK& c, const FastK& F, const RkRows<float>& rows, int fwd, const float2* tw,
+                          float2* spec, const float* const s[3], float* const h[3], float* const o[3], cudaStream_t st)
+{
+    using X = XSCfg<PX, false, SZ>;
+    return launch_pdl(k_xrk<PX, LT, ANI, SZ>, dim3((c.nz * c.ny + X::ROWS - 1) / X::ROWS), dim3(X::NT), (size_t)X::SMEM,
+                      st, c, F, rows, fwd, tw, spec, s[0], s[1], s[2], h[0], h[1], h[2], o[0], o[1], o[2]);
+}
+template <int PX, int LT, bool ANI>
+static cudaError_t xrk_px(const ConvK& c, const FastK& F, const RkRows<float>& rows, int fwd, const float2* tw,
+                          float2* spec, const float* const s[3], float* const h[3], float* const o[3], cudaStream_t st)
+{
+    const int sz = xs_size<PX>(c);
+    if constexpr (PX <= 128)
+        if (sz == 2) return xrk_sz<PX, LT, ANI, 2>(c, F, rows, fwd, tw, spec, s, h, o, st);
+    return xrk_sz<PX, LT, ANI, 1>(c, F, rows, fwd, tw, spec, s, h, o, st);
+}
+template <int LT, bool ANI>
+static cudaError_t xrk_any(const ConvK& c, const FastK& F, const RkRows<float>& rows, int fwd, const float2* tw,
+                           float2* spec, const float* const s[3], float* const h[3], float* const o[3], cudaStream_t st)
+{
+    switch (c.Px) {
+    case 32: return xrk_px<32, LT, ANI>(c, F, rows, fwd, tw, spec, s, h, o, st);
+    case 64: return xrk_px<64, LT, ANI>(c, F, rows, fwd, tw, spec, s, h, o, st);
+    case 128: return xrk_px<128, LT, ANI>(c, F, rows, fwd, tw, spec, s, h, o, st);
+    case 256: return xrk_px<256, LT, ANI>(c, F, rows, fwd, tw, spec, s, h, o, st);
+    case 512: return xrk_px<512, LT, ANI>(c, F, rows, fwd, tw, spec, s, h, o, st);
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_xrk(const ConvK& c, const FftLen L[3], const void* tw, void* spec, const FastK& F,
+                       const RkRows<float>& rows, bool fwd, const float* const s[3], float* const h[3],
+                       float* const o[3], cudaStream_t st)
+{
+    Prof pf("k_xrk", st);
+    const float2* t = static_cast<const float2*>(tw) + L[0].tw_off;
+    float2* sp = static_cast<float2*>(spec);
+    if (F.llg_type == LLG_CART)
+        return F.ani ? xrk_any<LLG_CART, true>(c, F, rows, fwd, t, sp, s, h, o, st)
+                     : xrk_any<LLG_CART, false>(c, F, rows, fwd, t, sp, s, h, o, st);
+    return F.ani ? xrk_any<LLG_QUAT, true>(c, F, rows, fwd, t, sp, s, h, o, st)
+                 : xrk_any<LLG_QUAT, false>(c, F, rows, fwd, t, sp, s, h, o, st);
+}
+
 bool xgstep_ok(const ConvK& c)
 {
     return c.nrep == 1 && (c.Px == 32 || c.Px == 64 || c.Px == 128 || c.Px == 256 || c.Px == 512);
@@ -1889,10 +1967,24 @@ static cudaError_t cfg_xs_sz()
         return e;
     return cudaSuccess;
 }
+template <int PX, int SZ>
+static cudaError_t cfg_xrk()
+{
+    const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const int m = XSCfg<PX, false, SZ>::SMEM;
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(k_xrk<PX, LLG_CART, false, SZ>, a, m)) || (e = cudaFuncSetAttribute(k_xrk<PX, LLG_CART, true, SZ>, a, m)) ||
+        (e = cudaFuncSetAttribute(k_xrk<PX, LLG_QUAT, false, SZ>, a, m)))
+        return e;
+    return cudaFuncSetAttribute(k_xrk<PX, LLG_QUAT, true, SZ>, a, m);
+}
 template <int PX>
 static cudaError_t cfg_xs()
 {
     cudaError_t e;
+    if ((e = cfg_xrk<PX, 1>()) != cudaSuccess) return e;
+    if constexpr (PX <= 128)
+        if ((e = cfg_xrk<PX, 2>()) != cudaSuccess) return e;
     if ((e = cfg_xs_sz<PX, 0, false>()) != cudaSuccess || (e = cfg_xs_sz<PX, 0, true>()) != cudaSuccess) return e;
     if ((e = cfg_xs_sz<PX, 1, true>()) != cudaSuccess) return e;
     if constexpr (PX <= 128) return cfg_xs_sz<PX, 2, true>();

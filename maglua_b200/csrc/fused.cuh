@@ -147,12 +147,13 @@ __device__ __forceinline__ bool all_zero(p2 a)
     return u.x == 0.f && u.y == 0.f;
 }
 
-// The rest of a site's step, after the Zeeman and exchange fields H: anisotropy,
-// thermal (nrm: its standard normals), the addend A, the LLG update.  V: R for
-// one site, p2 for two, each lane the same operations.
-template <int LT, bool ANI, bool TH, bool ADD, typename R, typename V>
-__device__ __forceinline__ void fused_update(const FastKT<R>& F, V Sx, V Sy, V Sz, V Hx, V Hy, V Hz, V nrmx, V nrmy,
-                                             V nrmz, V Ax, V Ay, V Az, V& rx, V& ry, V& rz)
+// Adds to the Zeeman and exchange fields H of a spin S its anisotropy, the addend
+// A and the thermal field (nrm: its standard normals); g: the field the terms
+// without the thermal part see.  V: R for one site, p2 for two, each lane the
+// same operations.
+template <bool ANI, bool TH, bool ADD, typename R, typename V>
+__device__ __forceinline__ void fused_field(const FastKT<R>& F, V Sx, V Sy, V Sz, V& Hx, V& Hy, V& Hz, V nrmx, V nrmy,
+                                            V nrmz, V Ax, V Ay, V Az, V& gx, V& gy, V& gz)
 {
     const auto B = [](R a) { return bc<V, R>(a); };
     if (ANI) {
@@ -172,21 +173,40 @@ __device__ __forceinline__ void fused_update(const FastKT<R>& F, V Sx, V Sy, V S
         const V w = B(F.addw);
         Hx = fm(w, Ax, Hx); Hy = fm(w, Ay, Hy); Hz = fm(w, Az, Hz);
     }
-    // the field without the thermal part, for the terms that leave it out
-    V gx = Hx, gy = Hy, gz = Hz;
+    gx = Hx; gy = Hy; gz = Hz;
     if (TH) {
         const V sg = B(F.sigma);
         Hx = fm(sg, nrmx, Hx); Hy = fm(sg, nrmy, Hy); Hz = fm(sg, nrmz, Hz);
         if (!F.tof) { gx = Hx; gy = Hy; gz = Hz; }
     }
+}
+
+// Length restored to ms.
+template <typename R, typename V>
+__device__ __forceinline__ void fused_renorm(R ms, V& x, V& y, V& z)
+{
+    const V mm = dot3(x, x, y, y, z, z);
+    const V inv = ml(bc<V, R>(ms), fs_rsqrt(mm));
+    x = where_nz(mm, ml(x, inv), x);
+    y = where_nz(mm, ml(y, inv), y);
+    z = where_nz(mm, ml(z, inv), z);
+}
+
+// The LLG update of the spin S by the torque of the spin M in the field H (g
+// without its thermal part) over dt (c_rot: its half angle per field).
+template <int LT, typename R, typename V>
+__device__ __forceinline__ void fused_llg(const FastKT<R>& F, R dt_, R c_rot, V Sx, V Sy, V Sz, V Mx, V My, V Mz, V Hx,
+                                          V Hy, V Hz, V gx, V gy, V gz, V& rx, V& ry, V& rz)
+{
+    const auto B = [](R a) { return bc<V, R>(a); };
     V nx_ = Sx, ny_ = Sy, nz_ = Sz;
     if (LT == LLG_CART) {
         if (!F.dt_zero) {
             // dM = -p gaa M x H - d (a/ms) gaa M x (M x h), h = H - Hth
-            const V mhx = crs(Sy, gz, Sz, gy), mhy = crs(Sz, gx, Sx, gz), mhz = crs(Sx, gy, Sy, gx);
-            const V mmx = crs(Sy, mhz, Sz, mhy), mmy = crs(Sz, mhx, Sx, mhz), mmz = crs(Sx, mhy, Sy, mhx);
-            const V MHx = crs(Sy, Hz, Sz, Hy), MHy = crs(Sz, Hx, Sx, Hz), MHz = crs(Sx, Hy, Sy, Hx);
-            const V dt = B(F.dt), cp = B(F.c_prec), cd = B(F.c_damp);
+            const V mhx = crs(My, gz, Mz, gy), mhy = crs(Mz, gx, Mx, gz), mhz = crs(Mx, gy, My, gx);
+            const V mmx = crs(My, mhz, Mz, mhy), mmy = crs(Mz, mhx, Mx, mhz), mmz = crs(Mx, mhy, My, mhx);
+            const V MHx = crs(My, Hz, Mz, Hy), MHy = crs(Mz, Hx, Mx, Hz), MHz = crs(Mx, Hy, My, Hx);
+            const V dt = B(dt_), cp = B(F.c_prec), cd = B(F.c_damp);
             nx_ = fm(dt, crs(cp, MHx, cd, mmx), Sx);
             ny_ = fm(dt, crs(cp, MHy, cd, mmy), Sy);
             nz_ = fm(dt, crs(cp, MHz, cd, mmz), Sz);
@@ -195,7 +215,7 @@ __device__ __forceinline__ void fused_update(const FastKT<R>& F, V Sx, V Sy, V S
         V Hpx, Hpy, Hpz;
         const V cd = B(F.c_damp);
         if (F.tof) {
-            const V shx = crs(Sy, gz, Sz, gy), shy = crs(Sz, gx, Sx, gz), shz = crs(Sx, gy, Sy, gx);
+            const V shx = crs(My, gz, Mz, gy), shy = crs(Mz, gx, Mx, gz), shz = crs(Mx, gy, My, gx);
             const V pr = B(F.precess);
             Hpx = fm(pr, Hx, ml(cd, shx));
             Hpy = fm(pr, Hy, ml(cd, shy));
@@ -206,7 +226,7 @@ __device__ __forceinline__ void fused_update(const FastKT<R>& F, V Sx, V Sy, V S
         }
         const V HL2 = dot3(Hpx, Hpx, Hpy, Hpy, Hpz, Hpz);
         const V iHL = fs_rsqrt(HL2);
-        const V th = ml(B(F.c_rot), ml(HL2, iHL));
+        const V th = ml(B(c_rot), ml(HL2, iHL));
         V sn, cs;
         half_sincos(th, sn, cs);
         const V k = ml(sn, iHL);
@@ -220,13 +240,7 @@ __device__ __forceinline__ void fused_update(const FastKT<R>& F, V Sx, V Sy, V S
         ny_ = where_pos(HL2, fm(qw, ty, fm(nw, qy, crs(tx, qz, tz, qx))), Sy);
         nz_ = where_pos(HL2, fm(qw, tz, fm(nw, qz, crs(ty, qx, tx, qy))), Sz);
     }
-    if (F.renorm) {
-        const V mm = dot3(nx_, nx_, ny_, ny_, nz_, nz_);
-        const V inv = ml(B(F.ms), fs_rsqrt(mm));
-        nx_ = where_nz(mm, ml(nx_, inv), nx_);
-        ny_ = where_nz(mm, ml(ny_, inv), ny_);
-        nz_ = where_nz(mm, ml(nz_, inv), nz_);
-    }
+    if (F.renorm) fused_renorm<R, V>(F.ms, nx_, ny_, nz_);
     rx = nx_; ry = ny_; rz = nz_;
     if (F.status) {
         const V z = B((R)0);
@@ -234,14 +248,22 @@ __device__ __forceinline__ void fused_update(const FastKT<R>& F, V Sx, V Sy, V S
     }
 }
 
-template <int LT, bool EXS, bool ANI, bool TH, bool ADD, typename R, class LD>
-__device__ __forceinline__ void fused_site_ld(const FastKT<R>& F, int NX, int NY, int NZ, int x, int y, int z, int i,
-                                              const LD& ld, R Ax, R Ay, R Az, R& rx, R& ry, R& rz,
-                                              const float3* pre = nullptr)
+// The rest of a site's step after the Zeeman and exchange fields H.
+template <int LT, bool ANI, bool TH, bool ADD, typename R, typename V>
+__device__ __forceinline__ void fused_update(const FastKT<R>& F, V Sx, V Sy, V Sz, V Hx, V Hy, V Hz, V nrmx, V nrmy,
+                                             V nrmz, V Ax, V Ay, V Az, V& rx, V& ry, V& rz)
+{
+    V gx, gy, gz;
+    fused_field<ANI, TH, ADD, R, V>(F, Sx, Sy, Sz, Hx, Hy, Hz, nrmx, nrmy, nrmz, Ax, Ay, Az, gx, gy, gz);
+    fused_llg<LT, R, V>(F, F.dt, F.c_rot, Sx, Sy, Sz, Sx, Sy, Sz, Hx, Hy, Hz, gx, gy, gz, rx, ry, rz);
+}
+
+// Zeeman and (EXS) exchange fields H of site i.
+template <bool EXS, typename R, class LD>
+__device__ __forceinline__ void fused_near(const FastKT<R>& F, int NX, int NY, int NZ, int x, int y, int z, int i,
+                                           const LD& ld, R& Hx, R& Hy, R& Hz)
 {
     const int nxy = NX * NY;
-    const R Sx = ld(0, i), Sy = ld(1, i), Sz = ld(2, i);
-    R Hx, Hy, Hz;
     if (F.Bdev) { Hx = (R)F.Bdev[0]; Hy = (R)F.Bdev[1]; Hz = (R)F.Bdev[2]; }
     else { Hx = F.B[0]; Hy = F.B[1]; Hz = F.B[2]; }
     if (EXS) {
@@ -272,6 +294,16 @@ __device__ __forceinline__ void fused_site_ld(const FastKT<R>& F, int NX, int NY
         }
         Hx = ad(Hx, ex); Hy = ad(Hy, ey); Hz = ad(Hz, ez);
     }
+}
+
+template <int LT, bool EXS, bool ANI, bool TH, bool ADD, typename R, class LD>
+__device__ __forceinline__ void fused_site_ld(const FastKT<R>& F, int NX, int NY, int NZ, int x, int y, int z, int i,
+                                              const LD& ld, R Ax, R Ay, R Az, R& rx, R& ry, R& rz,
+                                              const float3* pre = nullptr)
+{
+    const R Sx = ld(0, i), Sy = ld(1, i), Sz = ld(2, i);
+    R Hx, Hy, Hz;
+    fused_near<EXS, R>(F, NX, NY, NZ, x, y, z, i, ld, Hx, Hy, Hz);
     float3 nrm = make_float3(0.f, 0.f, 0.f);
     if (TH) nrm = pre ? *pre : thermal_normal3(F, i);
     fused_update<LT, ANI, TH, ADD, R, R>(F, Sx, Sy, Sz, Hx, Hy, Hz, (R)nrm.x, (R)nrm.y, (R)nrm.z, Ax, Ay, Az, rx, ry, rz);
@@ -293,10 +325,9 @@ __device__ __forceinline__ void fused_site_v(const FastKT<R>& F, int NX, int NY,
 // 0 times the site itself there instead of nothing), two per packed
 // instruction; the rows are each other's y neighbours, and the neighbours'
 // offsets serve both.  Byte offsets are 32 bits: at most 2^30 sites.
-template <int LT, bool ANI, bool TH>
-__device__ __forceinline__ void fused_pair(const FastK& F, int NX, int NY, int NZ, int x, int y, int z, int i,
-                                           const float* __restrict__ sx, const float* __restrict__ sy,
-                                           const float* __restrict__ sz, const p2 A[3], const p2 nrm[3], p2 r[3])
+__device__ __forceinline__ void pair_near(const FastK& F, int NX, int NY, int NZ, int x, int y, int z, int i,
+                                          const float* __restrict__ sx, const float* __restrict__ sy,
+                                          const float* __restrict__ sz, p2 S[3], p2 H[3])
 {
     const auto ld = [](const float* s, unsigned off) {
         return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(s) + off));
@@ -327,7 +358,6 @@ __device__ __forceinline__ void fused_pair(const FastK& F, int NX, int NY, int N
     }
     const p2 wx0 = pk(jxp, jxp), wx1 = pk(jxm, jxm), wy0 = pk(F.J[2], jyp), wy1 = pk(jym, F.J[3]);
     const p2 wz0 = pk(jzp, jzp), wz1 = pk(jzm, jzm);
-    p2 S[3], H[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         S[c] = pk(own[c][0], own[c][1]);
@@ -340,6 +370,42 @@ __device__ __forceinline__ void fused_pair(const FastK& F, int NX, int NY, int N
         if (F.J[5] != 0.f) e = fm(wz1, pk(nb[c][8], nb[c][9]), e);
         H[c] = ad(pk(F.B[c], F.B[c]), e);
     }
+}
+
+template <int LT, bool ANI, bool TH>
+__device__ __forceinline__ void fused_pair(const FastK& F, int NX, int NY, int NZ, int x, int y, int z, int i,
+                                           const float* __restrict__ sx, const float* __restrict__ sy,
+                                           const float* __restrict__ sz, const p2 A[3], const p2 nrm[3], p2 r[3])
+{
+    p2 S[3], H[3];
+    pair_near(F, NX, NY, NZ, x, y, z, i, sx, sy, sz, S, H);
     fused_update<LT, ANI, TH, true, float, p2>(F, S[0], S[1], S[2], H[0], H[1], H[2], nrm[0], nrm[1], nrm[2], A[0], A[1],
                                                A[2], r[0], r[1], r[2]);
+}
+
+// ------------------------------------------------------------------ Runge-Kutta stages
+// The rows of a scheme a stage contributes to: row r advances by this stage's
+// torque over dt (c_rot) from its running value (base; null: the stage's own
+// spin M; fresh: from a copy of the base system's spin, which an update over
+// no time leaves with its length restored) and is kept in dst.
+template <int LT, typename R, typename V, class Load, class Store>
+__device__ __forceinline__ void rk_rows(const FastKT<R>& F, const RkRows<R>& rows, const V M[3], const V H[3],
+                                        const Load& load, const Store& store, V first[3])
+{
+#pragma unroll 1
+    for (int r = 0; r < rows.n; r++) {
+        const auto& w = rows.row[r];
+        V b[3] = {M[0], M[1], M[2]}, o[3];
+        if (w.base[0]) {
+            for (int c = 0; c < 3; c++) b[c] = load(w.base[c]);
+            if (w.fresh && F.renorm) fused_renorm<R, V>(F.ms, b[0], b[1], b[2]);
+        }
+        fused_llg<LT, R, V>(F, w.dt, w.c_rot, b[0], b[1], b[2], M[0], M[1], M[2], H[0], H[1], H[2], H[0], H[1], H[2], o[0],
+                            o[1], o[2]);
+        if (r == 0) {
+            for (int c = 0; c < 3; c++) first[c] = o[c];
+        } else {
+            for (int c = 0; c < 3; c++) store(w.dst[c], o[c]);
+        }
+    }
 }

@@ -222,6 +222,20 @@ struct FastKT {
 // FP32 state (every fused kernel); FastKT<double> for FP64 state
 typedef FastKT<float> FastK;
 
+// Rows of a Runge-Kutta scheme that a stage advances (rk_rows): row 0 is
+// written by the pass itself.
+#define MLB_RK_ROWS 8
+template <typename R>
+struct RkRows {
+    int n;
+    struct {
+        const R* base[3];
+        R* dst[3];
+        R dt, c_rot;
+        int fresh;
+    } row[MLB_RK_ROWS];
+};
+
 // ------------------------------------------------------------- learned surrogate
 // Linear spectral-conv network on the in-plane grid (ny x nx) with the
 // (component, z) pairs as channels: ch = c * nz + z, C = 3 nz real channels

@@ -171,6 +171,13 @@ cudaError_t launch_mx_lr2d(const ConvK& c, const MxYZ& y, const FftLen L[3], con
 template <typename R>
 cudaError_t launch_mx_step(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FastKT<R>& F,
                            const R* const s[3], R* const h[3], R* const o[3], cudaStream_t st);
+// The same for a stage of a Runge-Kutta scheme: s the stage's spins, o row 0.
+template <typename R>
+cudaError_t launch_mx_rk(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FastKT<R>& F,
+                         const RkRows<R>& rows, const R* const s[3], R* const h[3], R* const o[3], cudaStream_t st);
+cudaError_t launch_xrk(const ConvK& c, const FftLen L[3], const void* tw, void* spec, const FastK& F,
+                       const RkRows<float>& rows, bool fwd, const float* const s[3], float* const h[3],
+                       float* const o[3], cudaStream_t st);
 cudaError_t launch_mx_gstep(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FusedK& P, double addw,
                             double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], int rb, cudaStream_t st);
 cudaError_t mx_configure();

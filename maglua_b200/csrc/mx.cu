@@ -553,6 +553,28 @@ __global__ void __launch_bounds__(256, Occ<R, BIG>::X) k_mx_step(const __grid_co
     });
 }
 
+// A stage of a Runge-Kutta scheme (rk_rows).
+template <typename R, int LT, bool ANI, bool BIG>
+__global__ void __launch_bounds__(256, Occ<R, BIG>::X)
+    k_mx_rk(const __grid_constant__ MxX m, const __grid_constant__ FastKT<R> F, const __grid_constant__ RkRows<R> rows,
+            const typename CT<R>::T* __restrict__ tw, typename CT<R>::T* __restrict__ spec, const R* sx, const R* sy,
+            const R* sz, R* hx, R* hy, R* hz, R* ox, R* oy, R* oz)
+{
+    mx::load_tables<typename CT<R>::T>(m.ax, tw, m.at);
+    pdl_trigger();
+    pdl_wait();
+    mx::step_rows<R, BIG>(m, spec, hx, hy, hz, ox, oy, oz, [&](int i, int x, int y, int z, V3<R> A) {
+        const GlobalSpins<R> ld{{sx, sy, sz}};
+        const R M[3] = {ld(0, i), ld(1, i), ld(2, i)};
+        R H[3], g[3], o[3];
+        fused_near<true, R>(F, m.nx, m.ny, m.nz, x, y, z, i, ld, H[0], H[1], H[2]);
+        fused_field<ANI, false, true, R, R>(F, M[0], M[1], M[2], H[0], H[1], H[2], (R)0, (R)0, (R)0, A.x, A.y, A.z, g[0],
+                                            g[1], g[2]);
+        rk_rows<LT, R, R>(F, rows, M, H, [&](const R* b) { return b[i]; }, [&](R* d, R v) { d[i] = v; }, o);
+        return v3<R>(o[0], o[1], o[2]);
+    });
+}
+
 // Per-site parameters, pathway lists, further addends (FusedK): P.terms
 // without the dipole addend, whose weight is addw.
 template <typename R, bool BIG>
@@ -1157,6 +1179,34 @@ template cudaError_t launch_mx_step<double>(const MxX&, const FftLen[3], const v
                                             const double* const[3], double* const[3], double* const[3], cudaStream_t);
 
 template <typename R>
+using RkKernel = void (*)(MxX, FastKT<R>, RkRows<R>, const typename CT<R>::T*, typename CT<R>::T*, const R*, const R*,
+                          const R*, R*, R*, R*, R*, R*, R*);
+template <typename R, bool BIG>
+static RkKernel<R> rk_kernel_b(int llg, bool ani)
+{
+    if (llg == LLG_CART) return ani ? k_mx_rk<R, LLG_CART, true, BIG> : k_mx_rk<R, LLG_CART, false, BIG>;
+    return ani ? k_mx_rk<R, LLG_QUAT, true, BIG> : k_mx_rk<R, LLG_QUAT, false, BIG>;
+}
+
+template <typename R>
+cudaError_t launch_mx_rk(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FastKT<R>& F,
+                         const RkRows<R>& rows, const R* const s[3], R* const h[3], R* const o[3], cudaStream_t st)
+{
+    typedef typename CT<R>::T C;
+    Prof pf("k_xrk", st);
+    const auto k = x.ax.big ? rk_kernel_b<R, true>(F.llg_type, F.ani != 0) : rk_kernel_b<R, false>(F.llg_type, F.ani != 0);
+    return launch_pdl(k, dim3((x.nr + x.rows - 1) / x.rows), dim3(256), mx_smem_x(x.ax, 3 * x.rows / 2, sizeof(R)), st, x,
+                      F, rows, static_cast<const C*>(tw) + L[0].tw_off, static_cast<C*>(spec), s[0], s[1], s[2], h[0],
+                      h[1], h[2], o[0], o[1], o[2]);
+}
+template cudaError_t launch_mx_rk<float>(const MxX&, const FftLen[3], const void*, void*, const FastKT<float>&,
+                                         const RkRows<float>&, const float* const[3], float* const[3], float* const[3],
+                                         cudaStream_t);
+template cudaError_t launch_mx_rk<double>(const MxX&, const FftLen[3], const void*, void*, const FastKT<double>&,
+                                          const RkRows<double>&, const double* const[3], double* const[3],
+                                          double* const[3], cudaStream_t);
+
+template <typename R>
 static cudaError_t mx_gstep_t(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FusedK& P, double addw,
                               double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], cudaStream_t st)
 {
@@ -1203,6 +1253,8 @@ static cudaError_t mx_configure_t()
         if ((e = mx_max_smem(yz_kernel_b<R, BIG>(nz))) != cudaSuccess) return e;
     for (int q = 0; q < 8; q++)
         if ((e = mx_max_smem(step_kernel_b<R, BIG>(q & 1 ? LLG_CART : LLG_QUAT, q & 2, q & 4))) != cudaSuccess) return e;
+    for (int q = 0; q < 4; q++)
+        if ((e = mx_max_smem(rk_kernel_b<R, BIG>(q & 1 ? LLG_CART : LLG_QUAT, q & 2))) != cudaSuccess) return e;
     if ((e = mx_max_smem(k_mx_lr2d<R, BIG>)) != cudaSuccess) return e;
     return mx_max_smem(k_mx_gstep<R, BIG>);
 }
