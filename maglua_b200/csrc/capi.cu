@@ -2656,6 +2656,7 @@ void plan_launch(mlb_plan* p, int nsteps)
 struct EnsClass {
     int nx, ny, nz, nrep;
     long long base;             // first packed site of the class
+    int rep0 = 0;               // first packed replica of the class
     mlb_op* dip = nullptr;      // tensor spectrum holder for this size
     bool fast = true;           // power-of-two fast passes (else the generic ones, replica by replica)
     int yz_variant = 0;         // tuned (y,z) pass of the fast path (ConvK::yz_variant)
@@ -2691,7 +2692,11 @@ struct mlb_ensemble {
     int grid = 0;                     // fused-kernel CTAs (autotuned; < nblk: persistent)
     bool tuned = false;
     std::string tune_log;
-    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    // by spin buffer; with fused x passes 2 and 3 the steps that find the spins'
+    // x spectra carried from the step before
+    cudaGraphExec_t exec[4] = {nullptr, nullptr, nullptr, nullptr};
+    bool fused_x = false;             // every class runs k_xens
+    bool carry = false;               // the classes' spectra hold the current spins
     double time = 0.0;
     uint64_t counter = 0;
     // per packed replica: temperature, applied field at the next step and
@@ -2717,10 +2722,11 @@ std::mutex g_ens_tune_mu;
 
 void ens_free_graphs(mlb_ensemble* e)
 {
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < 4; q++) {
         if (e->exec[q]) cudaGraphExecDestroy(e->exec[q]);
         e->exec[q] = nullptr;
     }
+    e->carry = false;
 }
 
 void ens_block_table(mlb_ensemble* e, int bs)
@@ -2855,7 +2861,9 @@ EnsLaunch ens_launch(mlb_ensemble* e, int q)
 // One step on spin buffer q: every class's dipole passes on a branch of its
 // own (the branches run concurrently in the captured graph), joined before
 // the fused step kernel over all replicas.
-void ens_enqueue_step(mlb_ensemble* e, int q)
+// With fused x passes (e->fused_x) a class' branch is its forward x pass
+// (unless carry), its (y,z) pass and k_xens.
+void ens_enqueue_step(mlb_ensemble* e, int q, bool carry)
 {
     const float* s[3] = {e->sp[q][0], e->sp[q][1], e->sp[q][2]};
     float* o[3] = {e->sp[1 - q][0], e->sp[1 - q][1], e->sp[1 - q][2]};
@@ -2864,19 +2872,27 @@ void ens_enqueue_step(mlb_ensemble* e, int q)
         const bool branch = e->cls.size() > 1;
         if (branch) CK(cudaEventRecord(e->fork, e->st));
         for (EnsClass& c : e->cls) {
-            if (branch) {
-                CK(cudaStreamWaitEvent(c.st, e->fork, 0));
-                ens_class_conv(e, c, s, c.st);
-                CK(cudaEventRecord(c.done, c.st));
+            cudaStream_t st = branch ? c.st : e->st;
+            if (branch) CK(cudaStreamWaitEvent(st, e->fork, 0));
+            if (e->fused_x) {
+                ConvPlan& P = *c.dip->plan;
+                const void* cs[3] = {s[0] + c.base, s[1] + c.base, s[2] + c.base};
+                if (!carry) launch_x(P, P.k, cs, P.spec.p, nullptr, true, st);
+                launch_yz(P, P.k, P.spec.p, st);
+                XEns E{};
+                E.rep0 = c.rep0; E.base = (int)c.base;
+                E.rB = e->d_rB[q]; E.rBn = e->d_rB[1 - q]; E.rdB = e->d_rdB; E.rsig = e->d_rsig;
+                CK(mlb::launch_xens(P.k, P.L, P.tw.p, P.spec.p, ens_fastk(e), E, s, o, st));
             } else {
-                ens_class_conv(e, c, s, e->st);
+                ens_class_conv(e, c, s, st);
             }
+            if (branch) CK(cudaEventRecord(c.done, st));
         }
         if (branch)
             for (EnsClass& c : e->cls) CK(cudaStreamWaitEvent(e->st, c.done, 0));
         for (int q3 = 0; q3 < 3; q3++) add[q3] = e->H[q3];
     }
-    CK(mlb::launch_fused_ens(ens_fastk(e), ens_launch(e, q), s, add, o, e->st));
+    if (!e->fused_x) CK(mlb::launch_fused_ens(ens_fastk(e), ens_launch(e, q), s, add, o, e->st));
     CK(mlb::launch_advance_step(e->dstep, e->dstep, e->st));
 }
 
@@ -3099,15 +3115,18 @@ void ens_prepare(mlb_ensemble* e)
             P.spec.alloc((size_t)P.k.Kx * 3 * k.nz * k.ny * P.k.nrep * sizeof(float2));
         }
     }
+    e->fused_x = c.g != 0.0 && c.J != 0.0;
+    for (EnsClass& k : e->cls)
+        e->fused_x = e->fused_x && k.fast && k.dip && k.dip->plan->k.ls && mlb::xens_ok(k.dip->plan->k);
     if (!e->tuned) ens_autotune(e);
     CK(cudaStreamSynchronize(e->st));
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < (e->fused_x ? 4 : 2); q++) {
         cudaGraph_t graph = nullptr;
         CK(cudaStreamBeginCapture(e->st, cudaStreamCaptureModeThreadLocal));
         bool ok = true;
         std::string why;
         try {
-            ens_enqueue_step(e, q);
+            ens_enqueue_step(e, q & 1, q >= 2);
         } catch (Err& er) {
             ok = false;
             why = er.msg;
@@ -5011,7 +5030,7 @@ int mlb_ensemble_create(int nrep, const int* dims, mlb_ensemble** out)
         e->rinfo_h.resize(nrep);
         int packed = 0;
         std::vector<int> first(e->cls.size(), 0);
-        for (size_t k = 0; k < e->cls.size(); k++) { first[k] = packed; packed += e->cls[k].nrep; }
+        for (size_t k = 0; k < e->cls.size(); k++) { first[k] = e->cls[k].rep0 = packed; packed += e->cls[k].nrep; }
         for (int r = 0; r < nrep; r++) {
             const int k = cls_of[r];
             const int p = first[k] + fill[k];
@@ -5118,6 +5137,7 @@ int mlb_ensemble_set_spins(mlb_ensemble* e, int rep, const double* x, const doub
         ens_download_fields(e);
         e->ms = m0;
         e->have_ms = true;
+        e->carry = false;
         CK(cudaStreamSynchronize(e->st));
         for (int c = 0; c < 3; c++) {
             f[c].resize(n);
@@ -5154,7 +5174,8 @@ int mlb_ensemble_run(mlb_ensemble* e, int nsteps)
         CK(cudaMemcpyAsync(e->dstep, &h, sizeof(h), cudaMemcpyHostToDevice, e->st));
         const bool cart = e->cfg.llg != MLB_LLG_QUATERNION;
         for (int k = 0; k < nsteps; k++) {
-            CK(cudaGraphLaunch(e->exec[e->cur], e->st));
+            CK(cudaGraphLaunch(e->exec[e->cur + (e->carry ? 2 : 0)], e->st));
+            e->carry = e->fused_x;
             e->cur = 1 - e->cur;
             if (!cart || e->cfg.dt != 0.0) e->time = e->time + e->cfg.dt;
         }

@@ -72,20 +72,21 @@ struct XCfg {
 // fr::line_fft (Split<N>::T lanes x Split<N>::E points, one warp-synchronous
 // exchange through ex, E (T + 1) elements per line), in place on a
 // natural-order line: the lanes have read the whole line before any of them
-// writes it back.
+// writes it back; SELF: the line's own buffer serves for the exchange.
 template <int N>
 struct XReg {
     static constexpr bool OK = N >= 32 && N <= 256;
     static constexpr int T = fr::Split<N>::T, E = fr::Split<N>::E, EX = E * (T + 1);
 };
-template <int N, int SIGN>
+template <int N, int SIGN, bool SELF = false>
 __device__ __forceinline__ void xreg_line(float2* line, float2* ex, int t, unsigned mask, const float2* tw)
 {
     constexpr int T = XReg<N>::T, E = XReg<N>::E;
     float2 v[E];
 #pragma unroll
     for (int j = 0; j < E; j++) v[j] = line[t + T * j];
-    fr::line_fft<N, SIGN, float2>(v, ex, t, mask, tw);
+    if (SELF) __syncwarp(mask);
+    fr::line_fft<N, SIGN, float2>(v, SELF ? line : ex, t, mask, tw);
 #pragma unroll
     for (int r = 0; r < E; r++) line[fr::out_index<N>(t, r)] = v[r];
 }
@@ -93,14 +94,17 @@ __device__ __forceinline__ void xreg_line(float2* line, float2* ex, int t, unsig
 // The CTA's nl lines (line l at base + l ls) in place, line l by threads
 // T l .. T l + T - 1.  Every thread of the CTA calls this; the CTA is
 // synchronised after the transforms.
-template <int N, int SIGN>
+// ex: exchange buffers of XReg<N>::EX elements per line; SELF: the lines
+// themselves (ls >= XReg<N>::EX).
+template <int N, int SIGN, bool SELF = false>
 __device__ __forceinline__ void xreg_lines(float2* base, int ls, int nl, float2* ex, const float2* tw)
 {
     constexpr int T = XReg<N>::T;
     const int l = threadIdx.x / T, t = threadIdx.x % T;
     if (l < nl) {
         const unsigned mask = ((1u << T) - 1u) << ((threadIdx.x & 31) & ~(T - 1));
-        xreg_line<N, SIGN>(base + (size_t)l * ls, ex + (size_t)l * XReg<N>::EX, t, mask, tw);
+        float2* ln = base + (size_t)l * ls;
+        xreg_line<N, SIGN, SELF>(ln, SELF ? nullptr : ex + (size_t)l * XReg<N>::EX, t, mask, tw);
     }
     __syncthreads();
 }
@@ -1036,35 +1040,43 @@ __global__ void __launch_bounds__(256) k_fused_fast(FastKT<R> F0, const R* __res
 // 64 registers, for lattices that fill the chip with such CTAs; 1: 512 sites on
 // 256 threads, 2: 128 sites on 128 threads (two rows at least), for smaller
 // ones (xs_size): a lattice of 128 x 128 x 4 is 32 CTAs of share 0, and the
-// step is one CTA's chain.  Lines are transformed alike at every share, so
-// results do not depend on it.
+// step is one CTA's chain; 3 (TIGHT): lines for 192 lanes on 256 threads, where
+// many CTAs share an SM (packed replicas).  Lines are transformed alike at every
+// share, so results do not depend on it.
+// TIGHT keeps one buffer, exchanged, replaced by the new spins and transformed
+// back in place, so that four CTAs fit an SM, and walks the sites alone rather
+// than the padded line (open replicas are half padding).  A periodic film has no
+// padding and its trip count is then known to the compiler: 256x256x8 takes
+// 21.05 us a step in the form of share 0 and 21.9 in this one.
 template <int PX, bool TH = false, int SZ = 0>
 struct XSCfg {
-    static constexpr int NT = SZ == 0 ? (XReg<PX>::OK ? 512 : 384) : (SZ == 1 ? 256 : 128);
+    static constexpr int NT = SZ == 0 ? (XReg<PX>::OK ? 512 : 384) : (SZ == 2 ? 128 : 256);
     static constexpr int TPL = fr::Tpl<PX>::V;
     static constexpr int SMALL = (SZ == 1 ? 512 : 128) / PX;
-    static constexpr int ROWS = SZ == 0 ? 2 * (384 / TPL) / 3 : (SMALL < 2 ? 2 : SMALL);
+    static constexpr int ROWS = SZ == 0 ? 2 * (384 / TPL) / 3 : (SZ == 3 ? 128 / XReg<PX>::T : (SMALL < 2 ? 2 : SMALL));
     static constexpr int L = 3 * ROWS / 2;              // complex lines
     static constexpr int R2 = ROWS / 2;
     static constexpr int KX = PX / 2 + 1;
-    // line stride in shared memory: one complex past the line, so that the
-    // same k of consecutive lines falls in different banks
-    static constexpr int LS = PX + 1;
+    static constexpr bool TIGHT = SZ == 3;
+    // line stride in shared memory, odd: the same k of consecutive lines
+    // falls in different banks
+    static constexpr int LS = (TIGHT && XReg<PX>::EX > PX ? XReg<PX>::EX : PX) | 1;
     static constexpr int LINE = L * LS;
     static constexpr int SPEC = 3 * ROWS * KX;
-    static constexpr int BUF = LINE > SPEC ? LINE : SPEC;
+    static constexpr int BUF = !TIGHT && SPEC > LINE ? SPEC : LINE;
+    static constexpr int NBUF = TIGHT ? 1 : 2;
     // thermal: the rows' normals, drawn while the spectrum loads are in
-    // flight, [3][ROWS][PX] floats (where two CTAs per SM still fit)
-    static constexpr bool PRE = TH && PX <= 256;
-    static constexpr int NOISE = PRE ? 3 * ROWS * PX : 0;
+    // flight, [3][R2][PX] pairs (where the CTAs of OCC still fit)
+    static constexpr bool PRE = TH && PX <= 256 && !TIGHT;
+    static constexpr int NOISE = PRE ? 3 * R2 * PX : 0;
     // 32- to 256-point lines: register four-step transforms, one exchange buffer per line
-    static constexpr int EX = XReg<PX>::OK ? L * XReg<PX>::EX : 0;
-    static constexpr int SMEM = (PX + 2 * BUF + EX) * 8 + NOISE * 4;
+    static constexpr int EX = XReg<PX>::OK && !TIGHT ? L * XReg<PX>::EX : 0;
+    static constexpr int SMEM = (PX + NBUF * BUF + EX + NOISE) * 8;
     static_assert(ROWS % 2 == 0, "line layout");
     static_assert(XReg<PX>::OK ? L * XReg<PX>::T <= NT : L * TPL <= NT, "lines per CTA");
     // CTAs per SM: 64 registers per thread; the general form's 96 or so
-    static constexpr int OCC = SZ == 0 ? 2 : (SZ == 1 ? 4 : 8);
-    static constexpr int GOCC = SZ == 0 ? 1 : (SZ == 1 ? 2 : 4);
+    static constexpr int OCC = SZ == 0 ? 2 : (SZ == 2 ? 8 : 4);
+    static constexpr int GOCC = SZ == 0 ? 1 : (SZ == 2 ? 4 : 2);
 };
 
 // The body of the fused x pass: begin() runs once the previous kernel's
@@ -1085,13 +1097,35 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
     constexpr int KX = X::KX, NT = X::NT, ROWS = X::ROWS, R2 = X::R2, LS = X::LS;
     extern __shared__ float2 sm[];
     float2* twl = sm;               // [PX]
-    float2* A = twl + PX;           // [L][LS] lines
-    float2* B = A + X::BUF;         // [L][LS] scratch
-    float2* EXB = B + X::BUF;       // [L][XReg<PX>::EX] exchange buffers (XReg<PX>::OK)
+    float2* A = twl + PX;                       // [L][LS] lines
+    float2* B = X::TIGHT ? A : A + X::BUF;      // [L][LS] scratch
+    float2* EXB = B + X::BUF;                   // [L][XReg<PX>::EX] exchange buffers (XReg<PX>::OK)
     const int nx = c.nx, ny = c.ny, nz = c.nz;
     const int nr = nz * ny;                     // rows (z, y), flattened
     const int row0 = blockIdx.x * ROWS;
     const int rows_here = min(ROWS, nr - row0);
+    // items of the site step: (row pair, x) of the padded lines, or of the
+    // sites alone (TIGHT), then divided by multiplication
+    constexpr int IP = (R2 * PX + NT - 1) / NT;
+    const int npair = R2 * nx;
+    const unsigned mnx = nx > 1 ? 0xffffffffu / (unsigned)nx + 1u : 0u;
+    const auto items = [&](auto&& f) {
+        if constexpr (X::TIGHT) {
+#pragma unroll 1
+            for (int idx = threadIdx.x; idx < npair; idx += NT) {
+                const int p = mnx ? (int)__umulhi((unsigned)idx, mnx) : idx;
+                f(p, idx - p * nx, true);
+            }
+        } else {
+#pragma unroll 1
+            for (int it = 0; it < IP; it++) {
+                const int idx = threadIdx.x + it * NT;
+                if (idx >= R2 * PX) break;
+                const int p = idx / PX, x = idx % PX;
+                f(p, x, x < nx);
+            }
+        }
+    };
     for (int k = threadIdx.x; k < PX; k += NT) twl[k] = tw[k];
     pdl_trigger();
     pdl_wait();
@@ -1151,16 +1185,10 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
         }
         // the normals of this thread's sites in the step below, while the
         // loads are in flight
-        constexpr int IP = (R2 * PX + NT - 1) / NT;
-        if (X::PRE) {
-#pragma unroll 1
-            for (int it = 0; it < IP; it++) {
-                const int idx = threadIdx.x + it * NT;
-                if (idx >= R2 * PX) break;
-                const int p = idx / PX, x = idx % PX;
-                if (2 * p < rows_here && x < nx) pre(p, x, (row0 + 2 * p) * nx + x, 2 * p + 1 < rows_here);
-            }
-        }
+        if (X::PRE)
+            items([&](int p, int x, bool in) {
+                if (2 * p < rows_here && in) pre(p, x, (row0 + 2 * p) * nx + x, 2 * p + 1 < rows_here);
+            });
 #pragma unroll
         for (int it = 0; it < IS; it++) {
             const int idx = threadIdx.x + it * NT;
@@ -1179,32 +1207,35 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
     const int l = threadIdx.x / X::TPL, tl = threadIdx.x % X::TPL;
     const float2* R;
     if constexpr (XReg<PX>::OK) {
-        xreg_lines<PX, +1>(A, LS, X::L, EXB, twl);
+        xreg_lines<PX, +1, X::TIGHT>(A, LS, X::L, EXB, twl);
         R = A;
     } else {
         R = fr::sm_fft<PX, +1, X::TPL, float2, LS>(A, B, l, tl, twl, l < X::L);
     }
-    float2* W = (R == A) ? B : A;   // free buffer: the new spins' lines (FWD)
+    // the new spins' lines (FWD): the free buffer, or (TIGHT) each where its
+    // item read the field
+    float2* W = (R == A) ? B : A;
     // 2. field of the rows to the slot (unless a later step of the same launch
     // overwrites it: hx null), then the step of every site: one (row pair, x)
     // per item, the pair's two rows the real and imaginary parts of one line
     // element
-    constexpr int IP = (R2 * PX + NT - 1) / NT;
     // (z, y) of the CTA's first row; a later row's by counting forward (no
     // division per site)
     const int zr0 = row0 / ny, yr0 = row0 - zr0 * ny;
-#pragma unroll 1
-    for (int it = 0; it < IP; it++) {
-        const int idx = threadIdx.x + it * NT;
-        if (idx >= R2 * PX) break;
-        const int p = idx / PX, x = idx % PX;
+    if (X::TIGHT && fwd && nx < PX) {   // zero padding of the new lines
+        for (int idx = threadIdx.x; idx < 3 * R2 * (PX - nx); idx += NT) {
+            const int l = idx % (3 * R2);
+            W[l * LS + nx + idx / (3 * R2)] = make_float2(0.f, 0.f);
+        }
+    }
+    items([&](int p, int x, bool in) {
         const float2 Ax2 = R[(0 * R2 + p) * LS + x], Ay2 = R[(1 * R2 + p) * LS + x], Az2 = R[(2 * R2 + p) * LS + x];
         float2 o0 = make_float2(0.f, 0.f), o1 = o0, o2 = o0;
         int zz = zr0, y = yr0 + 2 * p;
         while (y >= ny) { y -= ny; zz++; }
         if constexpr (PAIR) {
             // ny is even: the pair lies in one layer, and both rows exist
-            if (2 * p < rows_here && x < nx) {
+            if (2 * p < rows_here && in) {
                 const int i = (row0 + 2 * p) * nx + x;
                 if (hx) {
                     hx[i] = Ax2.x; hy[i] = Ay2.x; hz[i] = Az2.x;
@@ -1219,7 +1250,7 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
             for (int h = 0; h < 2; h++) {
                 const int row = 2 * p + h;
                 if (h && ++y >= ny) { y -= ny; zz++; }
-                if (row < rows_here && x < nx) {
+                if (row < rows_here && in) {
                     const float Ax = h ? Ax2.y : Ax2.x, Ay = h ? Ay2.y : Ay2.x, Az = h ? Az2.y : Az2.x;
                     const size_t i = (size_t)(row0 + row) * nx + x;
                     if (hx) { hx[i] = Ax; hy[i] = Ay; hz[i] = Az; }
@@ -1232,7 +1263,7 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
             }
         }
         if (fwd) { W[(0 * R2 + p) * LS + x] = o0; W[(1 * R2 + p) * LS + x] = o1; W[(2 * R2 + p) * LS + x] = o2; }
-    }
+    });
     if (!fwd) {
         tl_end(tls);
         return;
@@ -1241,7 +1272,7 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
     // 3. forward transform of the new spins' lines, split into the two rows
     const float2* Q;
     if constexpr (XReg<PX>::OK) {
-        xreg_lines<PX, -1>(W, LS, X::L, EXB, twl);
+        xreg_lines<PX, -1, X::TIGHT>(W, LS, X::L, EXB, twl);
         Q = W;
     } else {
         Q = fr::sm_fft<PX, -1, X::TPL, float2, LS>(W, const_cast<float2*>(R), l, tl, twl, l < X::L);
@@ -1277,7 +1308,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC)
     using X = XSCfg<PX, TH, SZ>;
     constexpr int NP = X::R2 * PX;
     extern __shared__ float2 sm[];
-    float2* noise = sm + PX + 2 * X::BUF + X::EX;   // [3][R2][PX] row pairs (X::PRE)
+    float2* noise = sm + PX + X::NBUF * X::BUF + X::EX;   // [3][R2][PX] row pairs (X::PRE)
     // the step block's values are the previous kernel's: resolved after the wait
     FastK F;
     const auto begin = [&] { F = fastk_resolved(F0); };
@@ -1343,6 +1374,58 @@ __global__ void __launch_bounds__(XSCfg<PX, false, SZ>::NT, XSCfg<PX, false, SZ>
             }
             const V3<float> o = step_site<float>(P, F, spin_at<float>(P.sys, i), ms, i);
             rx = o.x; ry = o.y; rz = o.z;
+        });
+}
+
+// The fused x pass of one size class of a packed ensemble: blockIdx.y the
+// replica of the class, packed replica E.rep0 + blockIdx.y, its sites from
+// E.base + blockIdx.y n on; each with its own applied field and thermal
+// deviation (the CTA of its first rows writes the next step's field).  Noise is
+// drawn by packed site, as in k_fused_ens.
+// Bound by issue and the barriers between its phases.  It replaces the inverse
+// x pass, the field slot, the fused step and the next step's forward x pass:
+// 512 open replicas of 16x16x16 to 64x64x4 (3.6 M sites), thermal,
+// 382 -> 308 us a step.
+template <int PX, int LT, bool ANI, bool TH, int SZ>
+__global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC)
+    k_xens(ConvK c, FastK F0, XEns E, const float2* __restrict__ tw, float2* __restrict__ spec,
+           const float* __restrict__ sx, const float* __restrict__ sy, const float* __restrict__ sz,
+           float* __restrict__ ox, float* __restrict__ oy, float* __restrict__ oz)
+{
+    using X = XSCfg<PX, TH, SZ>;
+    constexpr int NP = X::R2 * PX;
+    extern __shared__ float2 sm[];
+    float2* noise = sm + PX + X::NBUF * X::BUF + X::EX;   // [3][R2][PX] row pairs (X::PRE)
+    const int n = c.nx * c.ny * c.nz, rep = E.rep0 + blockIdx.y, off = E.base + blockIdx.y * n;
+    FastK F;
+    const auto begin = [&] {
+        F = fastk_resolved(F0);
+        F.B[0] = (float)E.rB[3 * rep]; F.B[1] = (float)E.rB[3 * rep + 1]; F.B[2] = (float)E.rB[3 * rep + 2];
+        if (TH) F.sigma = E.rsig[rep];
+        if (blockIdx.x == 0 && threadIdx.x < 3)
+            E.rBn[3 * rep + threadIdx.x] = E.rB[3 * rep + threadIdx.x] + E.rdB[3 * rep + threadIdx.x];
+    };
+    const float *s0 = sx + off, *s1 = sy + off, *s2 = sz + off;
+    xstep_body<PX, TH, SZ, true>(
+        c, nullptr, nullptr, 1, tw, spec + (size_t)blockIdx.y * c.Kx * 3 * c.nz * c.ny, s0, s1, s2, nullptr, nullptr,
+        nullptr, ox + off, oy + off, oz + off, begin,
+        [&](int p, int x, int i, bool) {
+            const float3 g = thermal_normal3(F, off + i), k = thermal_normal3(F, off + i + c.nx);
+            float2* q = noise + p * PX + x;
+            q[0] = make_float2(g.x, k.x); q[NP] = make_float2(g.y, k.y); q[2 * NP] = make_float2(g.z, k.z);
+        },
+        [&](int i, int p, int x, int y, int z, float2 Ax, float2 Ay, float2 Az, float2& rx, float2& ry, float2& rz) {
+            const p2 A[3] = {pk(Ax.x, Ax.y), pk(Ay.x, Ay.y), pk(Az.x, Az.y)};
+            p2 nn[3] = {pk(0.f, 0.f), pk(0.f, 0.f), pk(0.f, 0.f)}, r[3];
+            if (TH && !X::PRE) {
+                const float3 g = thermal_normal3(F, off + i), k = thermal_normal3(F, off + i + c.nx);
+                nn[0] = pk(g.x, k.x); nn[1] = pk(g.y, k.y); nn[2] = pk(g.z, k.z);
+            } else if (TH) {
+                const float2* q = noise + p * PX + x;
+                nn[0] = pk(q[0].x, q[0].y); nn[1] = pk(q[NP].x, q[NP].y); nn[2] = pk(q[2 * NP].x, q[2 * NP].y);
+            }
+            fused_pair<LT, ANI, TH>(F, c.nx, c.ny, c.nz, x, y, z, i, s0, s1, s2, A, nn, r);
+            rx = up(r[0]); ry = up(r[1]); rz = up(r[2]);
         });
 }
 
@@ -1861,6 +1944,68 @@ cudaError_t launch_xstep(const ConvK& c, const FftLen L[3], const float2* tw, fl
     return cudaErrorInvalidValue;
 }
 
+// Lines of 32 to 256 points (the normals of 512-point ones do not fit), rows in pairs
+bool xens_ok(const ConvK& c)
+{
+    return (c.Px == 32 || c.Px == 64 || c.Px == 128 || c.Px == 256) && xstep_pairs(c);
+}
+
+template <int PX, int LT, bool ANI, bool TH>
+static cudaError_t xens_t(const ConvK& c, const FastK& F, const XEns& E, const float2* tw, float2* spec,
+                          const float* const s[3], float* const o[3], cudaStream_t st)
+{
+    constexpr int SZ = 3;
+    using X = XSCfg<PX, TH, SZ>;
+    return launch_pdl(k_xens<PX, LT, ANI, TH, SZ>, dim3((c.nz * c.ny + X::ROWS - 1) / X::ROWS, c.nrep), dim3(X::NT),
+                      (size_t)X::SMEM, st, c, F, E, tw, spec, s[0], s[1], s[2], o[0], o[1], o[2]);
+}
+template <int PX>
+static cudaError_t xens_px(const ConvK& c, const FastK& F, const XEns& E, const float2* tw, float2* spec,
+                           const float* const s[3], float* const o[3], cudaStream_t st)
+{
+    if (F.llg_type == LLG_CART) {
+        if (F.ani) return F.th ? xens_t<PX, LLG_CART, true, true>(c, F, E, tw, spec, s, o, st)
+                               : xens_t<PX, LLG_CART, true, false>(c, F, E, tw, spec, s, o, st);
+        return F.th ? xens_t<PX, LLG_CART, false, true>(c, F, E, tw, spec, s, o, st)
+                    : xens_t<PX, LLG_CART, false, false>(c, F, E, tw, spec, s, o, st);
+    }
+    if (F.ani) return F.th ? xens_t<PX, LLG_QUAT, true, true>(c, F, E, tw, spec, s, o, st)
+                           : xens_t<PX, LLG_QUAT, true, false>(c, F, E, tw, spec, s, o, st);
+    return F.th ? xens_t<PX, LLG_QUAT, false, true>(c, F, E, tw, spec, s, o, st)
+                : xens_t<PX, LLG_QUAT, false, false>(c, F, E, tw, spec, s, o, st);
+}
+
+cudaError_t launch_xens(const ConvK& c, const FftLen L[3], const void* tw, void* spec, const FastK& F, const XEns& E,
+                        const float* const s[3], float* const o[3], cudaStream_t st)
+{
+    Prof pf("k_xens", st);
+    const float2* t = static_cast<const float2*>(tw) + L[0].tw_off;
+    float2* sp = static_cast<float2*>(spec);
+    switch (c.Px) {
+    case 32: return xens_px<32>(c, F, E, t, sp, s, o, st);
+    case 64: return xens_px<64>(c, F, E, t, sp, s, o, st);
+    case 128: return xens_px<128>(c, F, E, t, sp, s, o, st);
+    case 256: return xens_px<256>(c, F, E, t, sp, s, o, st);
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <int PX, bool TH>
+static cudaError_t cfg_xens()
+{
+    const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const auto co = cudaFuncAttributePreferredSharedMemoryCarveout;
+    const int m = XSCfg<PX, TH, 3>::SMEM, mx = (int)cudaSharedmemCarveoutMaxShared;
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(k_xens<PX, LLG_CART, false, TH, 3>, a, m)) || (e = cudaFuncSetAttribute(k_xens<PX, LLG_CART, true, TH, 3>, a, m)) ||
+        (e = cudaFuncSetAttribute(k_xens<PX, LLG_QUAT, false, TH, 3>, a, m)) || (e = cudaFuncSetAttribute(k_xens<PX, LLG_QUAT, true, TH, 3>, a, m)))
+        return e;
+    if ((e = cudaFuncSetAttribute(k_xens<PX, LLG_CART, false, TH, 3>, co, mx)) || (e = cudaFuncSetAttribute(k_xens<PX, LLG_CART, true, TH, 3>, co, mx)) ||
+        (e = cudaFuncSetAttribute(k_xens<PX, LLG_QUAT, false, TH, 3>, co, mx)))
+        return e;
+    return cudaFuncSetAttribute(k_xens<PX, LLG_QUAT, true, TH, 3>, co, mx);
+}
+
 template <int PX, int LT, bool ANI, int SZ>
 static cudaError_t xrk_sz(const ConvK& c, const FastK& F, const RkRows<float>& rows, int fwd, const float2* tw,
                           float2* spec, const float* const s[3], float* const h[3], float* const o[3], cudaStream_t st)
@@ -1983,6 +2128,8 @@ static cudaError_t cfg_xs()
 {
     cudaError_t e;
     if ((e = cfg_xrk<PX, 1>()) != cudaSuccess) return e;
+    if constexpr (PX <= 256)
+        if ((e = cfg_xens<PX, false>()) != cudaSuccess || (e = cfg_xens<PX, true>()) != cudaSuccess) return e;
     if constexpr (PX <= 128)
         if ((e = cfg_xrk<PX, 2>()) != cudaSuccess) return e;
     if ((e = cfg_xs_sz<PX, 0, false>()) != cudaSuccess || (e = cfg_xs_sz<PX, 0, true>()) != cudaSuccess) return e;

@@ -286,3 +286,12 @@ struct EnsLaunch {
     const double* rdB;
     const float* rsig;
 };
+// One size class of a packed ensemble in its fused x pass: first packed replica
+// and site; the per-replica arrays as in EnsLaunch.
+struct XEns {
+    int rep0, base;
+    const double* rB;
+    double* rBn;
+    const double* rdB;
+    const float* rsig;
+};

@@ -175,6 +175,10 @@ cudaError_t launch_mx_step(const MxX& x, const FftLen L[3], const void* tw, void
 template <typename R>
 cudaError_t launch_mx_rk(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FastKT<R>& F,
                          const RkRows<R>& rows, const R* const s[3], R* const h[3], R* const o[3], cudaStream_t st);
+// The fused x pass of a size class of a packed ensemble (c.nrep replicas).
+bool xens_ok(const ConvK& c);
+cudaError_t launch_xens(const ConvK& c, const FftLen L[3], const void* tw, void* spec, const FastK& F, const XEns& E,
+                        const float* const s[3], float* const o[3], cudaStream_t st);
 cudaError_t launch_xrk(const ConvK& c, const FftLen L[3], const void* tw, void* spec, const FastK& F,
                        const RkRows<float>& rows, bool fwd, const float* const s[3], float* const h[3],
                        float* const o[3], cudaStream_t st);
