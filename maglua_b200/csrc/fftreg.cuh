@@ -44,7 +44,8 @@ struct RegFFT {
         RegFFT<E / 2, SIGN, C>::run(od);
 #pragma unroll
         for (int k = 0; k < E / 2; k++) {
-            const C t = cmul(od[k], w64<C>(k * (64 / E), SIGN));
+            // 1 and -i need no multiplication
+            const C t = k == 0 ? od[0] : (k == E / 4 ? cmul_i(od[k], SIGN) : cmul(od[k], w64<C>(k * (64 / E), SIGN)));
             v[k] = cadd(ev[k], t);
             v[k + E / 2] = csub(ev[k], t);
         }
