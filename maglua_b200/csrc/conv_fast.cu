@@ -839,6 +839,102 @@ __global__ void __launch_bounds__(SPZ_NT, SplitOcc<C>::Z) k_sz_fast(ConvK c, con
     }
 }
 
+// The z pass with a column's three components in one group's registers: lane t
+// ends the forward transform with the frequencies t + T m, which is the order in
+// which the backward one begins, so the tensor multiply needs no exchange and the
+// CTA no barrier; HZ: nz <= PZ / 2, the padding is neither loaded, transformed
+// nor stored.  Lanes of mirrored columns share tensor rows within a load.
+// k_sz_fast, which puts each spectrum in order in shared memory and loads every
+// tensor row per point and value, spends 176 shared accesses per lane and line
+// where this one takes 64, and remains for lines whose registers do not fit
+// (512 points, FP64 from 128).  Bound by issue (the transforms): 128^3 open
+// (129 x 256 columns of 256 points), 122 -> 89 us.
+template <int PZ, typename C>
+struct SZR {
+    static constexpr int NT = PZ == 8 ? 64 : 128;   // columns divide any Py >= 32
+    static constexpr int T = fr::Split<PZ>::T, E = fr::Split<PZ>::E;
+    static constexpr int COLS = NT / T;   // ky columns per CTA
+    static constexpr int EX = E * (T + 1);
+    // 3 E complex values per lane
+    static constexpr bool OK = 3 * E * sizeof(C) <= 96 * 4;
+    static constexpr size_t SMEM = (size_t)(PZ + COLS * EX) * sizeof(C);
+};
+template <int PZ, bool QT, bool HZ, typename C>
+__global__ void __launch_bounds__(SZR<PZ, C>::NT, 384 / SZR<PZ, C>::NT) k_sz_reg(ConvK c, const C* __restrict__ twz, C* __restrict__ s2,
+                                                      const decltype(C().x)* __restrict__ ten6)
+{
+    typedef decltype(C().x) R;
+    using Z = SZR<PZ, C>;
+    constexpr int T = Z::T, E = Z::E, COLS = Z::COLS, QZ = PZ / 2 + 1;
+    extern __shared__ __align__(16) unsigned char smraw_szr[];
+    C* twl = reinterpret_cast<C*>(smraw_szr);
+    const int nz = c.nz, Py = c.Py, kx = blockIdx.x, b = blockIdx.y;
+    if (threadIdx.x == 0) {
+        // the columns' tensor rows (constant across steps) start towards L2
+        const R* Tb;
+        unsigned bytes;
+        if (QT) {
+            Tb = ten6 + ((size_t)kx * (Py / 2 + 1) + b * (COLS / 2)) * QZ * 6;
+            bytes = (unsigned)((COLS / 2) * QZ * 6 * sizeof(R));
+        } else {
+            Tb = ten6 + ((size_t)kx * Py + b * COLS) * PZ * 6;
+            bytes = (unsigned)(COLS * PZ * 6 * sizeof(R));
+        }
+        if ((((uintptr_t)Tb) & 15) == 0 && (bytes & 15) == 0)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(Tb), "r"(bytes) : "memory");
+    }
+    for (int k = threadIdx.x; k < PZ; k += Z::NT) twl[k] = twz[k];
+    pdl_trigger();
+    pdl_wait();
+    if (c.run_if && *c.run_if == 0) return;
+    __syncthreads();
+    const int cl = threadIdx.x / T, t = threadIdx.x % T;
+    const unsigned mask = group_mask(T);
+    C* exl = twl + PZ + (size_t)cl * Z::EX;
+    const int ky = sz_column<COLS>(b, cl, Py, QT);
+    C* colp = s2 + ((size_t)kx * Py + ky) * 3 * nz;
+    C v[3][E];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int j = 0; j < (HZ ? E / 2 : E); j++) {
+            const int z = t + T * j;
+            v[a][j] = z < nz ? colp[a * nz + z] : cmk<C>(0, 0);
+        }
+#pragma unroll
+    for (int a = 0; a < 3; a++) fr::line_fft<PZ, -1, C, HZ>(v[a], exl, t, mask, twl);
+    // tensor rows [kx][ky][kz][6] (a quarter tensor: ky <= Py/2, kz <= PZ/2,
+    // mirrored with the parity signs of XY, XZ, YZ)
+    const R gg = (R)c.g, sy = QT && ky > Py / 2 ? (R)-1 : (R)1;
+    const R* Tc = ten6 + (QT ? ((size_t)kx * (Py / 2 + 1) + (ky <= Py / 2 ? ky : Py - ky)) * QZ : ((size_t)kx * Py + ky) * PZ) * 6;
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        const int kz = fr::out_index<PZ>(t, r);
+        const bool up = QT && kz > PZ / 2;
+        const C* Tp = reinterpret_cast<const C*>(Tc + (up ? PZ - kz : kz) * 6);
+        const C ta = __ldg(Tp), tb = __ldg(Tp + 1), tc = __ldg(Tp + 2);
+        const R sz = up ? (R)-1 : (R)1;
+        const R t0 = ta.x, t1 = sy * ta.y, t2 = sz * tb.x, t3 = tb.y, t4 = sy * sz * tc.x, t5 = tc.y;
+        const C s0 = v[0][r], s1 = v[1][r], s2v = v[2][r];
+        v[0][r] = cmk<C>(gg * (t0 * s0.x + t1 * s1.x + t2 * s2v.x), gg * (t0 * s0.y + t1 * s1.y + t2 * s2v.y));
+        v[1][r] = cmk<C>(gg * (t1 * s0.x + t3 * s1.x + t4 * s2v.x), gg * (t1 * s0.y + t3 * s1.y + t4 * s2v.y));
+        v[2][r] = cmk<C>(gg * (t2 * s0.x + t4 * s1.x + t5 * s2v.x), gg * (t2 * s0.y + t4 * s1.y + t5 * s2v.y));
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        C u[E];   // element r = q T + k2 is frequency t + T (q + (E / T) k2)
+#pragma unroll
+        for (int r = 0; r < E; r++) u[r / T + (E / T) * (r % T)] = v[a][r];
+        fr::line_fft<PZ, +1, C>(u, exl, t, mask, twl);
+#pragma unroll
+        for (int r = 0; r < E; r++) {
+            if (HZ && E * (r % T) >= PZ / 2) continue;   // z >= PZ / 2
+            const int z = fr::out_index<PZ>(t, r);
+            if (z < nz) colp[a * nz + z] = u[r];
+        }
+    }
+}
+
 template <int PY, typename C = float2>
 __global__ void __launch_bounds__(SPL_NT, SplitOcc<C>::YI) k_syi_fast(ConvK c, const C* __restrict__ twy,
                                                                      const C* __restrict__ s2, C* __restrict__ spec)
@@ -905,19 +1001,31 @@ static cudaError_t launch_split_t(const ConvK& c, const C* twy, const C* twz, C*
                                   cudaStream_t st)
 {
     using Y = SPY<PY, C>;
-    using Z = SPZ<PZ, C>;
     C* s2 = static_cast<C*>(c.spec2);
     const dim3 gy(c.Kx, 3, (c.nz + Y::LN - 1) / Y::LN);
     cudaError_t e = mlb::launch_pdl(k_sy_fast<PY, C>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy, (const C*)spec, s2);
     if (e != cudaSuccess) return e;
-    if (c.quarter && c.Py % Z::COLS == 0)
-        e = mlb::launch_pdl(k_sz_fast<PZ, true, C>, dim3(c.Kx, c.Py / Z::COLS), dim3(SPZ_NT), Z::SMEM, st, c, twz, s2,
-                            ten6);
-    else if (c.quarter)
-        e = cudaErrorInvalidValue;
-    else
-        e = mlb::launch_pdl(k_sz_fast<PZ, false, C>, dim3(c.Kx, (c.Py + Z::COLS - 1) / Z::COLS), dim3(SPZ_NT), Z::SMEM,
-                            st, c, twz, s2, ten6);
+    if constexpr (SZR<PZ, C>::OK) {
+        using Q = SZR<PZ, C>;
+        const dim3 gz(c.Kx, c.Py / Q::COLS);
+        const bool hz = c.nz <= PZ / 2;
+        if (c.quarter)
+            e = hz ? mlb::launch_pdl(k_sz_reg<PZ, true, true, C>, gz, dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6)
+                   : mlb::launch_pdl(k_sz_reg<PZ, true, false, C>, gz, dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6);
+        else
+            e = hz ? mlb::launch_pdl(k_sz_reg<PZ, false, true, C>, gz, dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6)
+                   : mlb::launch_pdl(k_sz_reg<PZ, false, false, C>, gz, dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6);
+    } else {
+        using Z = SPZ<PZ, C>;
+        if (c.quarter && c.Py % Z::COLS == 0)
+            e = mlb::launch_pdl(k_sz_fast<PZ, true, C>, dim3(c.Kx, c.Py / Z::COLS), dim3(SPZ_NT), Z::SMEM, st, c, twz, s2,
+                                ten6);
+        else if (c.quarter)
+            e = cudaErrorInvalidValue;
+        else
+            e = mlb::launch_pdl(k_sz_fast<PZ, false, C>, dim3(c.Kx, (c.Py + Z::COLS - 1) / Z::COLS), dim3(SPZ_NT),
+                                Z::SMEM, st, c, twz, s2, ten6);
+    }
     if (e != cudaSuccess) return e;
     return mlb::launch_pdl(k_syi_fast<PY, C>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy, (const C*)s2, spec);
 }
@@ -976,8 +1084,11 @@ static cudaError_t cfg_split_c()
         if ((e = cudaFuncSetAttribute(k_sy_fast<P, C>, a, (int)SPY<P, C>::SMEM)) != cudaSuccess) return e;
         if ((e = cudaFuncSetAttribute(k_syi_fast<P, C>, a, (int)SPY<P, C>::SMEM)) != cudaSuccess) return e;
     }
-    if ((e = cudaFuncSetAttribute(k_sz_fast<P, true, C>, a, (int)SPZ<P, C>::SMEM)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_sz_fast<P, false, C>, a, (int)SPZ<P, C>::SMEM);
+    if constexpr (!SZR<P, C>::OK) {
+        if ((e = cudaFuncSetAttribute(k_sz_fast<P, true, C>, a, (int)SPZ<P, C>::SMEM)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(k_sz_fast<P, false, C>, a, (int)SPZ<P, C>::SMEM)) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 template <int P>

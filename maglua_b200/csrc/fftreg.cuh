@@ -33,15 +33,16 @@ __device__ __forceinline__ double2 w64<double2>(int k, int sign)
     return make_double2(w.x, sign > 0 ? -w.y : w.y);
 }
 
-template <int E, int SIGN, typename C>
+// HZ: the inputs from E/2 on are zero and not read.
+template <int E, int SIGN, typename C, bool HZ = false>
 struct RegFFT {
     __device__ __forceinline__ static void run(C* v)
     {
         C ev[E / 2], od[E / 2];
 #pragma unroll
-        for (int i = 0; i < E / 2; i++) { ev[i] = v[2 * i]; od[i] = v[2 * i + 1]; }
-        RegFFT<E / 2, SIGN, C>::run(ev);
-        RegFFT<E / 2, SIGN, C>::run(od);
+        for (int i = 0; i < (HZ ? E / 4 : E / 2); i++) { ev[i] = v[2 * i]; od[i] = v[2 * i + 1]; }
+        RegFFT<E / 2, SIGN, C, HZ>::run(ev);
+        RegFFT<E / 2, SIGN, C, HZ>::run(od);
 #pragma unroll
         for (int k = 0; k < E / 2; k++) {
             // 1 and -i need no multiplication
@@ -51,23 +52,35 @@ struct RegFFT {
         }
     }
 };
-template <int SIGN, typename C>
-struct RegFFT<1, SIGN, C> {
+template <int SIGN, typename C, bool HZ>
+struct RegFFT<1, SIGN, C, HZ> {
     __device__ __forceinline__ static void run(C*) {}
 };
-template <int SIGN, typename C>
-struct RegFFT<2, SIGN, C> {
+template <int SIGN, typename C, bool HZ>
+struct RegFFT<2, SIGN, C, HZ> {
     __device__ __forceinline__ static void run(C* v)
     {
+        if (HZ) {
+            v[1] = v[0];
+            return;
+        }
         const C a = v[0], b = v[1];
         v[0] = cadd(a, b);
         v[1] = csub(a, b);
     }
 };
-template <int SIGN, typename C>
-struct RegFFT<4, SIGN, C> {
+template <int SIGN, typename C, bool HZ>
+struct RegFFT<4, SIGN, C, HZ> {
     __device__ __forceinline__ static void run(C* v)
     {
+        if (HZ) {
+            const C a = v[0], b = v[1], ib = cmul_i(v[1], SIGN);
+            v[0] = cadd(a, b);
+            v[1] = cadd(a, ib);
+            v[2] = csub(a, b);
+            v[3] = csub(a, ib);
+            return;
+        }
         const C a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
         const C b0 = cadd(v[1], v[3]), b1 = cmul_i(csub(v[1], v[3]), SIGN);
         v[0] = cadd(a0, b0);
@@ -90,12 +103,13 @@ struct Split {
 //   out: lane t holds X[k1 + E k2] for k1 in {t, t + T, ...} (E/T values of k1)
 //        and k2 < T, in out[q * T + k2] with k1 = t + q T.
 // ex is this line's shared-memory exchange buffer of E*(T+1) elements; the lanes
-// of the group synchronise with __syncwarp(mask).
-template <int N, int SIGN, typename C>
+// of the group synchronise with __syncwarp(mask).  HZ: the line's upper half is
+// zero, v[j] for j >= E/2 is not read.
+template <int N, int SIGN, typename C, bool HZ = false>
 __device__ __forceinline__ void line_fft(C* v, C* ex, int t, unsigned mask, const C* twN)
 {
     constexpr int T = Split<N>::T, E = Split<N>::E;
-    RegFFT<E, SIGN, C>::run(v);
+    RegFFT<E, SIGN, C, HZ>::run(v);
     if (T > 1) {
 #pragma unroll
         for (int k1 = 1; k1 < E; k1++) {
