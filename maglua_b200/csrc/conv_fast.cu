@@ -78,17 +78,21 @@ struct XReg {
     static constexpr bool OK = N >= 32 && N <= 256;
     static constexpr int T = fr::Split<N>::T, E = fr::Split<N>::E, EX = E * (T + 1);
 };
-template <int N, int SIGN, bool SELF = false>
+// HZ: the data end before N / 2; the zeros behind them are not read (SIGN < 0)
+// or what would be written there is left out (SIGN > 0).
+template <int N, int SIGN, bool SELF = false, bool HZ = false>
 __device__ __forceinline__ void xreg_line(float2* line, float2* ex, int t, unsigned mask, const float2* tw)
 {
     constexpr int T = XReg<N>::T, E = XReg<N>::E;
+    constexpr bool HI = HZ && SIGN < 0, HO = HZ && SIGN > 0;
     float2 v[E];
 #pragma unroll
-    for (int j = 0; j < E; j++) v[j] = line[t + T * j];
+    for (int j = 0; j < (HI ? E / 2 : E); j++) v[j] = line[t + T * j];
     if (SELF) __syncwarp(mask);
-    fr::line_fft<N, SIGN, float2>(v, SELF ? line : ex, t, mask, tw);
+    fr::line_fft<N, SIGN, float2, HI>(v, SELF ? line : ex, t, mask, tw);
 #pragma unroll
-    for (int r = 0; r < E; r++) line[fr::out_index<N>(t, r)] = v[r];
+    for (int r = 0; r < E; r++)
+        if (!HO || E * (r % T) < N / 2) line[fr::out_index<N>(t, r)] = v[r];
 }
 
 // The CTA's nl lines (line l at base + l ls) in place, line l by threads
@@ -96,7 +100,7 @@ __device__ __forceinline__ void xreg_line(float2* line, float2* ex, int t, unsig
 // synchronised after the transforms.
 // ex: exchange buffers of XReg<N>::EX elements per line; SELF: the lines
 // themselves (ls >= XReg<N>::EX).
-template <int N, int SIGN, bool SELF = false>
+template <int N, int SIGN, bool SELF = false, bool HZ = false>
 __device__ __forceinline__ void xreg_lines(float2* base, int ls, int nl, float2* ex, const float2* tw)
 {
     constexpr int T = XReg<N>::T;
@@ -104,7 +108,7 @@ __device__ __forceinline__ void xreg_lines(float2* base, int ls, int nl, float2*
     if (l < nl) {
         const unsigned mask = ((1u << T) - 1u) << ((threadIdx.x & 31) & ~(T - 1));
         float2* ln = base + (size_t)l * ls;
-        xreg_line<N, SIGN, SELF>(ln, SELF ? nullptr : ex + (size_t)l * XReg<N>::EX, t, mask, tw);
+        xreg_line<N, SIGN, SELF, HZ>(ln, SELF ? nullptr : ex + (size_t)l * XReg<N>::EX, t, mask, tw);
     }
     __syncthreads();
 }
@@ -643,7 +647,8 @@ __global__ void __launch_bounds__(YZC<PY, PZ>::NT, 1) k_yz_col3(ConvK c, const f
 //   k_sy_fast   CTA (kx, comp, LN data layers): y transforms of the layers'
 //               rows, zero-padded to PY; transposed in shared memory so that
 //               each ky stores LN consecutive z;
-//   k_sz_fast   CTA (kx, COLS ky columns): z transforms of the columns' three
+//   k_sz_fast   (or k_sz_reg: in registers throughout)
+//               CTA (kx, COLS ky columns): z transforms of the columns' three
 //               components, zero-padded to PZ; 3x3 tensor multiply (ky-major
 //               real tensor, scaled by the strength); inverse z transforms,
 //               data layers back to S2;
@@ -679,12 +684,18 @@ __device__ __forceinline__ unsigned group_mask(int T)
     return T >= 32 ? 0xffffffffu : (((1u << T) - 1u) << (((threadIdx.x & 31) / T) * T));
 }
 
-// FP32 lines fit two CTAs per SM; FP64 lines hold twice the registers
-template <typename C> struct SplitOcc { static constexpr int Y = 2, YI = 3, Z = 3; };
-template <> struct SplitOcc<double2> { static constexpr int Y = 1, YI = 1, Z = 2; };
+// CTAs per SM.  The y passes wait for memory: lanes of 16 points (PY <= 256) fit
+// 64 registers, four CTAs; with the zero half left out (HZ), at 128^3 open, 53 ->
+// 42 us forward and 56 -> 51 us backward.  FP64 lines hold twice the registers.
+template <typename C, int PY = 512>
+struct SplitOcc {
+    static constexpr int Y = PY <= 256 ? 4 : 2, YI = PY <= 256 ? 4 : 3, Z = 3;
+};
+template <int PY> struct SplitOcc<double2, PY> { static constexpr int Y = 1, YI = 1, Z = 2; };
 
-template <int PY, typename C = float2>
-__global__ void __launch_bounds__(SPL_NT, SplitOcc<C>::Y) k_sy_fast(ConvK c, const C* __restrict__ twy,
+// HZ: ny <= PY / 2, the zeros behind the rows are neither loaded nor transformed.
+template <int PY, bool HZ, typename C = float2>
+__global__ void __launch_bounds__(SPL_NT, SplitOcc<C, PY>::Y) k_sy_fast(ConvK c, const C* __restrict__ twy,
                                                                    const C* __restrict__ spec, C* __restrict__ s2)
 {
     using Y = SPY<PY, C>;
@@ -707,11 +718,11 @@ __global__ void __launch_bounds__(SPL_NT, SplitOcc<C>::Y) k_sy_fast(ConvK c, con
     if (act) {
         const C* src = spec + (((size_t)kx * 3 + comp) * nz + z0 + lr) * ny;
 #pragma unroll
-        for (int j = 0; j < E; j++) {
+        for (int j = 0; j < (HZ ? E / 2 : E); j++) {
             const int y = t + T * j;
             v[j] = y < ny ? src[y] : cmk<C>(0, 0);
         }
-        fr::line_fft<PY, -1, C>(v, buf + (size_t)lr * Y::EX, t, group_mask(T), twl);
+        fr::line_fft<PY, -1, C, HZ>(v, buf + (size_t)lr * Y::EX, t, group_mask(T), twl);
     }
     __syncthreads();   // exchange buffers -> transpose buffer
     if (act) {
@@ -842,8 +853,8 @@ __global__ void __launch_bounds__(SPZ_NT, SplitOcc<C>::Z) k_sz_fast(ConvK c, con
 // The z pass with a column's three components in one group's registers: lane t
 // ends the forward transform with the frequencies t + T m, which is the order in
 // which the backward one begins, so the tensor multiply needs no exchange and the
-// CTA no barrier; HZ: nz <= PZ / 2, the padding is neither loaded, transformed
-// nor stored.  Lanes of mirrored columns share tensor rows within a load.
+// CTA no barrier.  nz <= PZ / 2 (z is always padded): the zeros are neither
+// loaded, transformed nor stored.  Lanes of mirrored columns share tensor rows within a load.
 // k_sz_fast, which puts each spectrum in order in shared memory and loads every
 // tensor row per point and value, spends 176 shared accesses per lane and line
 // where this one takes 64, and remains for lines whose registers do not fit
@@ -859,7 +870,7 @@ struct SZR {
     static constexpr bool OK = 3 * E * sizeof(C) <= 96 * 4;
     static constexpr size_t SMEM = (size_t)(PZ + COLS * EX) * sizeof(C);
 };
-template <int PZ, bool QT, bool HZ, typename C>
+template <int PZ, bool QT, typename C>
 __global__ void __launch_bounds__(SZR<PZ, C>::NT, 384 / SZR<PZ, C>::NT) k_sz_reg(ConvK c, const C* __restrict__ twz, C* __restrict__ s2,
                                                       const decltype(C().x)* __restrict__ ten6)
 {
@@ -897,12 +908,12 @@ __global__ void __launch_bounds__(SZR<PZ, C>::NT, 384 / SZR<PZ, C>::NT) k_sz_reg
 #pragma unroll
     for (int a = 0; a < 3; a++)
 #pragma unroll
-        for (int j = 0; j < (HZ ? E / 2 : E); j++) {
+        for (int j = 0; j < E / 2; j++) {
             const int z = t + T * j;
             v[a][j] = z < nz ? colp[a * nz + z] : cmk<C>(0, 0);
         }
 #pragma unroll
-    for (int a = 0; a < 3; a++) fr::line_fft<PZ, -1, C, HZ>(v[a], exl, t, mask, twl);
+    for (int a = 0; a < 3; a++) fr::line_fft<PZ, -1, C, true>(v[a], exl, t, mask, twl);
     // tensor rows [kx][ky][kz][6] (a quarter tensor: ky <= Py/2, kz <= PZ/2,
     // mirrored with the parity signs of XY, XZ, YZ)
     const R gg = (R)c.g, sy = QT && ky > Py / 2 ? (R)-1 : (R)1;
@@ -928,15 +939,16 @@ __global__ void __launch_bounds__(SZR<PZ, C>::NT, 384 / SZR<PZ, C>::NT) k_sz_reg
         fr::line_fft<PZ, +1, C>(u, exl, t, mask, twl);
 #pragma unroll
         for (int r = 0; r < E; r++) {
-            if (HZ && E * (r % T) >= PZ / 2) continue;   // z >= PZ / 2
+            if (E * (r % T) >= PZ / 2) continue;   // z >= PZ / 2
             const int z = fr::out_index<PZ>(t, r);
             if (z < nz) colp[a * nz + z] = u[r];
         }
     }
 }
 
-template <int PY, typename C = float2>
-__global__ void __launch_bounds__(SPL_NT, SplitOcc<C>::YI) k_syi_fast(ConvK c, const C* __restrict__ twy,
+// HZ: the outputs from PY / 2 on are left out.
+template <int PY, bool HZ, typename C = float2>
+__global__ void __launch_bounds__(SPL_NT, SplitOcc<C, PY>::YI) k_syi_fast(ConvK c, const C* __restrict__ twy,
                                                                      const C* __restrict__ s2, C* __restrict__ spec)
 {
     using Y = SPY<PY, C>;
@@ -977,6 +989,7 @@ __global__ void __launch_bounds__(SPL_NT, SplitOcc<C>::YI) k_syi_fast(ConvK c, c
         C* dst = spec + (((size_t)kx * 3 + comp) * nz + z0 + lr) * ny;
 #pragma unroll
         for (int r = 0; r < E; r++) {
+            if (HZ && E * (r % T) >= PY / 2) continue;
             const int y = fr::out_index<PY>(t, r);
             if (y < ny) dst[y] = v[r];
         }
@@ -989,7 +1002,7 @@ template <typename C>
 static bool split_fast_ok_t(const ConvK& c)
 {
     auto p2 = [](int v, int lo) { return v >= lo && v <= 512 && (v & (v - 1)) == 0; };
-    if (c.nrep != 1 || !p2(c.Py, 32) || !p2(c.Pz, 8)) return false;
+    if (c.nrep != 1 || !p2(c.Py, 32) || !p2(c.Pz, 8) || 2 * c.nz > c.Pz) return false;
     const int T = c.Pz <= 4 ? 1 : (c.Pz <= 32 ? (c.Pz <= 8 ? 2 : 4) : (c.Pz <= 128 ? 8 : 16));
     const int COLS = (SPZ_NT / T) / 3;
     return c.Py % COLS == 0;
@@ -1002,32 +1015,24 @@ static cudaError_t launch_split_t(const ConvK& c, const C* twy, const C* twz, C*
 {
     using Y = SPY<PY, C>;
     C* s2 = static_cast<C*>(c.spec2);
+    const bool hy = c.ny <= PY / 2;
     const dim3 gy(c.Kx, 3, (c.nz + Y::LN - 1) / Y::LN);
-    cudaError_t e = mlb::launch_pdl(k_sy_fast<PY, C>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy, (const C*)spec, s2);
+    cudaError_t e = mlb::launch_pdl(hy ? k_sy_fast<PY, true, C> : k_sy_fast<PY, false, C>, gy, dim3(SPL_NT), Y::SMEM, st,
+                                    c, twy, (const C*)spec, s2);
     if (e != cudaSuccess) return e;
     if constexpr (SZR<PZ, C>::OK) {
         using Q = SZR<PZ, C>;
-        const dim3 gz(c.Kx, c.Py / Q::COLS);
-        const bool hz = c.nz <= PZ / 2;
-        if (c.quarter)
-            e = hz ? mlb::launch_pdl(k_sz_reg<PZ, true, true, C>, gz, dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6)
-                   : mlb::launch_pdl(k_sz_reg<PZ, true, false, C>, gz, dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6);
-        else
-            e = hz ? mlb::launch_pdl(k_sz_reg<PZ, false, true, C>, gz, dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6)
-                   : mlb::launch_pdl(k_sz_reg<PZ, false, false, C>, gz, dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6);
+        e = mlb::launch_pdl(c.quarter ? k_sz_reg<PZ, true, C> : k_sz_reg<PZ, false, C>, dim3(c.Kx, c.Py / Q::COLS),
+                            dim3(Q::NT), Q::SMEM, st, c, twz, s2, ten6);
     } else {
         using Z = SPZ<PZ, C>;
-        if (c.quarter && c.Py % Z::COLS == 0)
-            e = mlb::launch_pdl(k_sz_fast<PZ, true, C>, dim3(c.Kx, c.Py / Z::COLS), dim3(SPZ_NT), Z::SMEM, st, c, twz, s2,
-                                ten6);
-        else if (c.quarter)
-            e = cudaErrorInvalidValue;
-        else
-            e = mlb::launch_pdl(k_sz_fast<PZ, false, C>, dim3(c.Kx, (c.Py + Z::COLS - 1) / Z::COLS), dim3(SPZ_NT),
-                                Z::SMEM, st, c, twz, s2, ten6);
+        if (c.quarter && c.Py % Z::COLS != 0) return cudaErrorInvalidValue;
+        e = mlb::launch_pdl(c.quarter ? k_sz_fast<PZ, true, C> : k_sz_fast<PZ, false, C>,
+                            dim3(c.Kx, (c.Py + Z::COLS - 1) / Z::COLS), dim3(SPZ_NT), Z::SMEM, st, c, twz, s2, ten6);
     }
     if (e != cudaSuccess) return e;
-    return mlb::launch_pdl(k_syi_fast<PY, C>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy, (const C*)s2, spec);
+    return mlb::launch_pdl(hy ? k_syi_fast<PY, true, C> : k_syi_fast<PY, false, C>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy,
+                           (const C*)s2, spec);
 }
 
 template <int PY, typename C>
@@ -1071,8 +1076,8 @@ static cudaError_t launch_split_y_t(const ConvK& c, const float2* twy, float2* s
     float2* s2 = static_cast<float2*>(c.spec2);
     const dim3 gy(c.Kx, 3, (c.nz + Y::LN - 1) / Y::LN);
     if (fwd)
-        return mlb::launch_pdl(k_sy_fast<PY, float2>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy, (const float2*)spec, s2);
-    return mlb::launch_pdl(k_syi_fast<PY, float2>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy, (const float2*)s2, spec);
+        return mlb::launch_pdl(k_sy_fast<PY, false, float2>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy, (const float2*)spec, s2);
+    return mlb::launch_pdl(k_syi_fast<PY, false, float2>, gy, dim3(SPL_NT), Y::SMEM, st, c, twy, (const float2*)s2, spec);
 }
 
 template <int P, typename C>
@@ -1081,8 +1086,8 @@ static cudaError_t cfg_split_c()
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e;
     if constexpr (P >= 32) {
-        if ((e = cudaFuncSetAttribute(k_sy_fast<P, C>, a, (int)SPY<P, C>::SMEM)) != cudaSuccess) return e;
-        if ((e = cudaFuncSetAttribute(k_syi_fast<P, C>, a, (int)SPY<P, C>::SMEM)) != cudaSuccess) return e;
+        for (auto* k : {k_sy_fast<P, false, C>, k_sy_fast<P, true, C>, k_syi_fast<P, false, C>, k_syi_fast<P, true, C>})
+            if ((e = cudaFuncSetAttribute(k, a, (int)SPY<P, C>::SMEM)) != cudaSuccess) return e;
     }
     if constexpr (!SZR<P, C>::OK) {
         if ((e = cudaFuncSetAttribute(k_sz_fast<P, true, C>, a, (int)SPZ<P, C>::SMEM)) != cudaSuccess) return e;
@@ -1195,7 +1200,7 @@ struct XSCfg {
 // of the CTA (sites i and, if both, i + nx) while the spectrum loads are in
 // flight; site(i, row, x, y, z, A..., r...) gives the new spin of site i in the
 // dipole field A, or with PAIR site(i, p, ...) those of i and i + nx.
-template <int PX, bool TH, int SZ, bool PAIR, class Begin, class Pre, class Site>
+template <int PX, bool TH, int SZ, bool PAIR, bool HZ, class Begin, class Pre, class Site>
 __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cur, DevStep* adv_next, int fwd,
                                            const float2* __restrict__ tw, float2* __restrict__ spec,
                                            const float* __restrict__ sx, const float* __restrict__ sy,
@@ -1217,7 +1222,8 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
     const int rows_here = min(ROWS, nr - row0);
     // items of the site step: (row pair, x) of the padded lines, or of the
     // sites alone (TIGHT), then divided by multiplication
-    constexpr int IP = (R2 * PX + NT - 1) / NT;
+    constexpr int XW = HZ ? PX / 2 : PX;
+    constexpr int IP = (R2 * XW + NT - 1) / NT;
     const int npair = R2 * nx;
     const unsigned mnx = nx > 1 ? 0xffffffffu / (unsigned)nx + 1u : 0u;
     const auto items = [&](auto&& f) {
@@ -1231,8 +1237,8 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
 #pragma unroll 1
             for (int it = 0; it < IP; it++) {
                 const int idx = threadIdx.x + it * NT;
-                if (idx >= R2 * PX) break;
-                const int p = idx / PX, x = idx % PX;
+                if (idx >= R2 * XW) break;
+                const int p = idx / XW, x = idx % XW;
                 f(p, x, x < nx);
             }
         }
@@ -1318,7 +1324,7 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
     const int l = threadIdx.x / X::TPL, tl = threadIdx.x % X::TPL;
     const float2* R;
     if constexpr (XReg<PX>::OK) {
-        xreg_lines<PX, +1, X::TIGHT>(A, LS, X::L, EXB, twl);
+        xreg_lines<PX, +1, X::TIGHT, HZ>(A, LS, X::L, EXB, twl);
         R = A;
     } else {
         R = fr::sm_fft<PX, +1, X::TPL, float2, LS>(A, B, l, tl, twl, l < X::L);
@@ -1333,8 +1339,8 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
     // (z, y) of the CTA's first row; a later row's by counting forward (no
     // division per site)
     const int zr0 = row0 / ny, yr0 = row0 - zr0 * ny;
-    if (X::TIGHT && fwd && nx < PX) {   // zero padding of the new lines
-        for (int idx = threadIdx.x; idx < 3 * R2 * (PX - nx); idx += NT) {
+    if (X::TIGHT && fwd && nx < XW) {   // zero padding of the new lines
+        for (int idx = threadIdx.x; idx < 3 * R2 * (XW - nx); idx += NT) {
             const int l = idx % (3 * R2);
             W[l * LS + nx + idx / (3 * R2)] = make_float2(0.f, 0.f);
         }
@@ -1383,7 +1389,7 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
     // 3. forward transform of the new spins' lines, split into the two rows
     const float2* Q;
     if constexpr (XReg<PX>::OK) {
-        xreg_lines<PX, -1, X::TIGHT>(W, LS, X::L, EXB, twl);
+        xreg_lines<PX, -1, X::TIGHT, HZ>(W, LS, X::L, EXB, twl);
         Q = W;
     } else {
         Q = fr::sm_fft<PX, -1, X::TPL, float2, LS>(W, const_cast<float2*>(R), l, tl, twl, l < X::L);
@@ -1407,7 +1413,7 @@ __device__ __forceinline__ void xstep_body(const ConvK& c, const DevStep* adv_cu
 
 // PAIR: two sites at a time (fused_pair), for an even number of rows per layer
 // and at most 2^30 sites.
-template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR>
+template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR, bool HZ>
 __global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC) k_xstep(ConvK c, FastK F0,
                                                   int fwd, const float2* __restrict__ tw,
                                                   float2* __restrict__ spec, const float* __restrict__ sx,
@@ -1431,7 +1437,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC)
         q[0] = make_float2(g.x, k.x); q[NP] = make_float2(g.y, k.y); q[2 * NP] = make_float2(g.z, k.z);
     };
     if constexpr (PAIR) {
-        xstep_body<PX, TH, SZ, true>(
+        xstep_body<PX, TH, SZ, true, HZ>(
             c, F0.adv_cur, F0.adv_next, fwd, tw, spec, sx, sy, sz, hx, hy, hz, ox, oy, oz, begin, pre,
             [&](int i, int p, int x, int y, int z, float2 Ax, float2 Ay, float2 Az, float2& rx, float2& ry, float2& rz) {
                 const p2 A[3] = {pk(Ax.x, Ax.y), pk(Ay.x, Ay.y), pk(Az.x, Az.y)};
@@ -1447,7 +1453,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC)
                 rx = up(r[0]); ry = up(r[1]); rz = up(r[2]);
             });
     } else {
-        xstep_body<PX, TH, SZ, false>(
+        xstep_body<PX, TH, SZ, false, HZ>(
             c, F0.adv_cur, F0.adv_next, fwd, tw, spec, sx, sy, sz, hx, hy, hz, ox, oy, oz, begin, pre,
             [&](int i, int row, int x, int y, int z, float Ax, float Ay, float Az, float& rx, float& ry, float& rz) {
                 float3 g;
@@ -1472,7 +1478,7 @@ __global__ void __launch_bounds__(XSCfg<PX, false, SZ>::NT, XSCfg<PX, false, SZ>
                                                             float* __restrict__ hx, float* __restrict__ hy,
                                                             float* __restrict__ hz)
 {
-    xstep_body<PX, false, SZ, false>(
+    xstep_body<PX, false, SZ, false, false>(
         c, cur, next, 1, tw, spec, static_cast<const float*>(P.sys.x), static_cast<const float*>(P.sys.y),
         static_cast<const float*>(P.sys.z), hx, hy, hz, static_cast<float*>(P.ox), static_cast<float*>(P.oy),
         static_cast<float*>(P.oz), [] {}, [](int, int, int, bool) {},
@@ -1496,8 +1502,8 @@ __global__ void __launch_bounds__(XSCfg<PX, false, SZ>::NT, XSCfg<PX, false, SZ>
 // Bound by issue and the barriers between its phases.  It replaces the inverse
 // x pass, the field slot, the fused step and the next step's forward x pass:
 // 512 open replicas of 16x16x16 to 64x64x4 (3.6 M sites), thermal,
-// 382 -> 308 us a step.
-template <int PX, int LT, bool ANI, bool TH, int SZ>
+// 382 -> 308 us a step (301 -> 296 by the padded ends left out, HZ).
+template <int PX, int LT, bool ANI, bool TH, int SZ, bool HZ>
 __global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC)
     k_xens(ConvK c, FastK F0, XEns E, const float2* __restrict__ tw, float2* __restrict__ spec,
            const float* __restrict__ sx, const float* __restrict__ sy, const float* __restrict__ sz,
@@ -1517,7 +1523,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC)
             E.rBn[3 * rep + threadIdx.x] = E.rB[3 * rep + threadIdx.x] + E.rdB[3 * rep + threadIdx.x];
     };
     const float *s0 = sx + off, *s1 = sy + off, *s2 = sz + off;
-    xstep_body<PX, TH, SZ, true>(
+    xstep_body<PX, TH, SZ, true, HZ>(
         c, nullptr, nullptr, 1, tw, spec + (size_t)blockIdx.y * c.Kx * 3 * c.nz * c.ny, s0, s1, s2, nullptr, nullptr,
         nullptr, ox + off, oy + off, oz + off, begin,
         [&](int p, int x, int i, bool) {
@@ -1553,7 +1559,7 @@ __global__ void __launch_bounds__(XSCfg<PX, false, SZ>::NT, XSCfg<PX, false, SZ>
           const float2* __restrict__ tw, float2* __restrict__ spec, const float* sx, const float* sy, const float* sz,
           float* hx, float* hy, float* hz, float* ox, float* oy, float* oz)
 {
-    xstep_body<PX, false, SZ, true>(
+    xstep_body<PX, false, SZ, true, false>(
         c, nullptr, nullptr, fwd, tw, spec, sx, sy, sz, hx, hy, hz, ox, oy, oz, [] {}, [](int, int, int, bool) {},
         [&](int i, int, int x, int y, int z, float2 Ax, float2 Ay, float2 Az, float2& rx, float2& ry, float2& rz) {
             p2 M[3], H[3], g[3], o[3];
@@ -2001,25 +2007,36 @@ static int xs_size(const ConvK& c)
     return 2;
 }
 
-template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR>
+template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR, bool HZ>
 static cudaError_t xstep_sz(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
                             const float* s[3], float* h[3], float* o[3], cudaStream_t st)
 {
     using X = XSCfg<PX, TH, SZ>;
     dim3 grid((c.nz * c.ny + X::ROWS - 1) / X::ROWS, 1, 1);
-    return launch_pdl(k_xstep<PX, LT, ANI, TH, SZ, PAIR>, grid, dim3(X::NT), (size_t)X::SMEM, st, c, F, fwd, tw, spec,
+    return launch_pdl(k_xstep<PX, LT, ANI, TH, SZ, PAIR, HZ>, grid, dim3(X::NT), (size_t)X::SMEM, st, c, F, fwd, tw, spec,
                       s[0], s[1], s[2], h[0], h[1], h[2], o[0], o[1], o[2]);
 }
+template <int PX, int LT, bool ANI, bool TH, bool HZ>
+static cudaError_t xstep_z(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
+                           const float* s[3], float* h[3], float* o[3], cudaStream_t st)
+{
+    const int sz = xs_size<PX>(c);
+    if (sz == 0) return xstep_sz<PX, LT, ANI, TH, 0, true, HZ>(c, F, fwd, tw, spec, s, h, o, st);
+    if constexpr (PX <= 128)
+        if (sz == 2) return xstep_sz<PX, LT, ANI, TH, 2, true, HZ>(c, F, fwd, tw, spec, s, h, o, st);
+    return xstep_sz<PX, LT, ANI, TH, 1, true, HZ>(c, F, fwd, tw, spec, s, h, o, st);
+}
+// Rows that end in the first half of their lines (an open x) take HZ: half of
+// the site loop's items and of the transforms' padded ends are never there.
+// k_xstep of 128^3 open 102 -> 90 us.
 template <int PX, int LT, bool ANI, bool TH>
 static cudaError_t xstep_t(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
                            const float* s[3], float* h[3], float* o[3], cudaStream_t st)
 {
-    if (!xstep_pairs(c)) return xstep_sz<PX, LT, ANI, TH, 0, false>(c, F, fwd, tw, spec, s, h, o, st);
-    const int sz = xs_size<PX>(c);
-    if (sz == 0) return xstep_sz<PX, LT, ANI, TH, 0, true>(c, F, fwd, tw, spec, s, h, o, st);
-    if constexpr (PX <= 128)
-        if (sz == 2) return xstep_sz<PX, LT, ANI, TH, 2, true>(c, F, fwd, tw, spec, s, h, o, st);
-    return xstep_sz<PX, LT, ANI, TH, 1, true>(c, F, fwd, tw, spec, s, h, o, st);
+    if (!xstep_pairs(c)) return xstep_sz<PX, LT, ANI, TH, 0, false, false>(c, F, fwd, tw, spec, s, h, o, st);
+    if constexpr (XReg<PX>::OK)
+        if (c.nx <= PX / 2) return xstep_z<PX, LT, ANI, TH, true>(c, F, fwd, tw, spec, s, h, o, st);
+    return xstep_z<PX, LT, ANI, TH, false>(c, F, fwd, tw, spec, s, h, o, st);
 }
 template <int PX, int LT>
 static cudaError_t xstep_lt(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec,
@@ -2067,8 +2084,9 @@ static cudaError_t xens_t(const ConvK& c, const FastK& F, const XEns& E, const f
 {
     constexpr int SZ = 3;
     using X = XSCfg<PX, TH, SZ>;
-    return launch_pdl(k_xens<PX, LT, ANI, TH, SZ>, dim3((c.nz * c.ny + X::ROWS - 1) / X::ROWS, c.nrep), dim3(X::NT),
-                      (size_t)X::SMEM, st, c, F, E, tw, spec, s[0], s[1], s[2], o[0], o[1], o[2]);
+    return launch_pdl(c.nx <= PX / 2 ? k_xens<PX, LT, ANI, TH, SZ, true> : k_xens<PX, LT, ANI, TH, SZ, false>,
+                      dim3((c.nz * c.ny + X::ROWS - 1) / X::ROWS, c.nrep), dim3(X::NT), (size_t)X::SMEM, st, c, F, E, tw,
+                      spec, s[0], s[1], s[2], o[0], o[1], o[2]);
 }
 template <int PX>
 static cudaError_t xens_px(const ConvK& c, const FastK& F, const XEns& E, const float2* tw, float2* spec,
@@ -2101,20 +2119,17 @@ cudaError_t launch_xens(const ConvK& c, const FftLen L[3], const void* tw, void*
     return cudaErrorInvalidValue;
 }
 
-template <int PX, bool TH>
+template <int PX, bool TH, bool HZ>
 static cudaError_t cfg_xens()
 {
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     const auto co = cudaFuncAttributePreferredSharedMemoryCarveout;
     const int m = XSCfg<PX, TH, 3>::SMEM, mx = (int)cudaSharedmemCarveoutMaxShared;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_xens<PX, LLG_CART, false, TH, 3>, a, m)) || (e = cudaFuncSetAttribute(k_xens<PX, LLG_CART, true, TH, 3>, a, m)) ||
-        (e = cudaFuncSetAttribute(k_xens<PX, LLG_QUAT, false, TH, 3>, a, m)) || (e = cudaFuncSetAttribute(k_xens<PX, LLG_QUAT, true, TH, 3>, a, m)))
-        return e;
-    if ((e = cudaFuncSetAttribute(k_xens<PX, LLG_CART, false, TH, 3>, co, mx)) || (e = cudaFuncSetAttribute(k_xens<PX, LLG_CART, true, TH, 3>, co, mx)) ||
-        (e = cudaFuncSetAttribute(k_xens<PX, LLG_QUAT, false, TH, 3>, co, mx)))
-        return e;
-    return cudaFuncSetAttribute(k_xens<PX, LLG_QUAT, true, TH, 3>, co, mx);
+    for (auto* k : {k_xens<PX, LLG_CART, false, TH, 3, HZ>, k_xens<PX, LLG_CART, true, TH, 3, HZ>,
+                    k_xens<PX, LLG_QUAT, false, TH, 3, HZ>, k_xens<PX, LLG_QUAT, true, TH, 3, HZ>})
+        if ((e = cudaFuncSetAttribute(k, a, m)) || (e = cudaFuncSetAttribute(k, co, mx))) return e;
+    return cudaSuccess;
 }
 
 template <int PX, int LT, bool ANI, int SZ>
@@ -2202,25 +2217,26 @@ cudaError_t launch_xgstep(const ConvK& c, const FftLen L[3], const float2* tw, f
     return cudaErrorInvalidValue;
 }
 
-template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR>
+template <int PX, int LT, bool ANI, bool TH, int SZ, bool PAIR, bool HZ>
 static cudaError_t cfg_xs1()
 {
-    const auto k = k_xstep<PX, LT, ANI, TH, SZ, PAIR>;
+    const auto k = k_xstep<PX, LT, ANI, TH, SZ, PAIR, HZ>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, XSCfg<PX, TH, SZ>::SMEM);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
 }
-template <int PX, int SZ, bool PAIR>
+template <int PX, int SZ, bool PAIR, bool HZ = false>
 static cudaError_t cfg_xs_sz()
 {
     cudaError_t e =
         cudaFuncSetAttribute(k_xgstep<PX, SZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, XSCfg<PX, false, SZ>::SMEM);
     if (e != cudaSuccess) return e;
-    if ((e = cfg_xs1<PX, LLG_CART, false, false, SZ, PAIR>()) || (e = cfg_xs1<PX, LLG_CART, false, true, SZ, PAIR>()) ||
-        (e = cfg_xs1<PX, LLG_CART, true, false, SZ, PAIR>()) || (e = cfg_xs1<PX, LLG_CART, true, true, SZ, PAIR>()) ||
-        (e = cfg_xs1<PX, LLG_QUAT, false, false, SZ, PAIR>()) || (e = cfg_xs1<PX, LLG_QUAT, false, true, SZ, PAIR>()) ||
-        (e = cfg_xs1<PX, LLG_QUAT, true, false, SZ, PAIR>()) || (e = cfg_xs1<PX, LLG_QUAT, true, true, SZ, PAIR>()))
+    if ((e = cfg_xs1<PX, LLG_CART, false, false, SZ, PAIR, HZ>()) || (e = cfg_xs1<PX, LLG_CART, false, true, SZ, PAIR, HZ>()) ||
+        (e = cfg_xs1<PX, LLG_CART, true, false, SZ, PAIR, HZ>()) || (e = cfg_xs1<PX, LLG_CART, true, true, SZ, PAIR, HZ>()) ||
+        (e = cfg_xs1<PX, LLG_QUAT, false, false, SZ, PAIR, HZ>()) || (e = cfg_xs1<PX, LLG_QUAT, false, true, SZ, PAIR, HZ>()) ||
+        (e = cfg_xs1<PX, LLG_QUAT, true, false, SZ, PAIR, HZ>()) || (e = cfg_xs1<PX, LLG_QUAT, true, true, SZ, PAIR, HZ>()))
         return e;
+    if constexpr (PAIR && !HZ && XReg<PX>::OK) return cfg_xs_sz<PX, SZ, true, true>();
     return cudaSuccess;
 }
 template <int PX, int SZ>
@@ -2240,7 +2256,9 @@ static cudaError_t cfg_xs()
     cudaError_t e;
     if ((e = cfg_xrk<PX, 1>()) != cudaSuccess) return e;
     if constexpr (PX <= 256)
-        if ((e = cfg_xens<PX, false>()) != cudaSuccess || (e = cfg_xens<PX, true>()) != cudaSuccess) return e;
+        if ((e = cfg_xens<PX, false, false>()) || (e = cfg_xens<PX, true, false>()) || (e = cfg_xens<PX, false, true>()) ||
+            (e = cfg_xens<PX, true, true>()))
+            return e;
     if constexpr (PX <= 128)
         if ((e = cfg_xrk<PX, 2>()) != cudaSuccess) return e;
     if ((e = cfg_xs_sz<PX, 0, false>()) != cudaSuccess || (e = cfg_xs_sz<PX, 0, true>()) != cudaSuccess) return e;
