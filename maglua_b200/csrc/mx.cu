@@ -888,22 +888,28 @@ static double mx_best(int n, int total, bool f64, std::vector<int>& out)
 }
 
 // Wavefronts of the axis' shared-memory accesses with padding shift sh: the
-// first warps of every stage, elements of eb bytes.
-static int mx_conflicts(const MxAxis& ax, int sh, int nl, int eb)
+// first warps of every stage, elements of eb bytes; counted up to `limit`.
+static int mx_conflicts(const MxAxis& ax, int sh, int nl, int eb, int limit)
 {
-    const int lanes = 128 / eb, LS = ax.n + (ax.n >> sh);
-    int sum = 0;
+    const int lanes = 128 / eb, LS = (ax.n + (ax.n >> sh)) | 1;
+    int sum = 0, line[128], at[128];
     for (int i = 0; i < ax.nst; i++) {
         const MxStage& s = ax.s[i];
         const int total = std::min(nl * s.nb, 128);
+        for (int t = 0; t < total; t++) {
+            const int q = t % s.nb;
+            line[t] = t / s.nb * LS;
+            at[t] = (q / s.m) * s.m * s.R + q % s.m;
+        }
         for (int w = 0; w < total; w += lanes)
-            for (int r = 0; r < s.R; r++) {
+            for (int r = 0, rm = 0; r < s.R; r++, rm += s.m) {
                 int hit[16] = {0}, worst = 0;
                 for (int t = w; t < std::min(w + lanes, total); t++) {
-                    const int l = t / s.nb, q = t % s.nb, p = (q / s.m) * s.m * s.R + q % s.m + r * s.m;
-                    worst = std::max(worst, ++hit[(l * (LS | 1) + p + (p >> sh)) % lanes]);
+                    const int p = at[t] + rm;
+                    worst = std::max(worst, ++hit[(line[t] + p + (p >> sh)) & (lanes - 1)]);
                 }
                 sum += worst;
+                if (sum >= limit) return limit;
             }
     }
     return sum;
@@ -911,8 +917,10 @@ static int mx_conflicts(const MxAxis& ax, int sh, int nl, int eb)
 
 // The stages of an axis of n points of which a CTA holds nl lines, their
 // padding, and the place of each frequency after the forward transform (into
-// *at); false when n has a prime factor above 31.
-static bool mx_axis(int n, int nl, bool f64, MxAxis& ax, std::vector<int>* at)
+// *at); false when n has a prime factor above 31.  prev: the axis of the same
+// length and type for prev_nl lines, taken over if the search would be the same.
+static bool mx_axis(int n, int nl, bool f64, MxAxis& ax, std::vector<int>* at, const MxAxis* prev = nullptr,
+                    int prev_nl = 0)
 {
     std::vector<int> r;
     if (mx_best(n, nl * n, f64, r) >= 1e300 || (int)r.size() > MX_MAX_STAGES) return false;
@@ -926,7 +934,17 @@ static bool mx_axis(int n, int nl, bool f64, MxAxis& ax, std::vector<int>* at)
     std::sort(r.begin(), r.end());
     int best = 1 << 30;
     MxAxis t = ax;
-    do {
+    bool same = prev && prev->nst == ax.nst;
+    if (same) {
+        std::vector<int> pr;
+        for (int i = 0; i < prev->nst; i++) pr.push_back(prev->s[i].R);
+        std::sort(pr.begin(), pr.end());
+        same = pr == r && std::all_of(r.begin(), r.end(), [&](int R) {
+            return std::min(nl * (n / R), 128) == std::min(prev_nl * (n / R), 128);
+        });
+    }
+    if (same) ax = *prev;
+    else do {
         if (ax.big && r.back() <= 16) continue;
         int len = n;   // points of a block
         for (int i = 0; i < t.nst; i++) {
@@ -940,7 +958,7 @@ static bool mx_axis(int n, int nl, bool f64, MxAxis& ax, std::vector<int>* at)
             len = s.m;
         }
         for (int sh : {3, 4, 5, 30}) {
-            const int c = mx_conflicts(t, sh, nl, f64 ? 16 : 8);
+            const int c = mx_conflicts(t, sh, nl, f64 ? 16 : 8, best);
             if (c < best) {
                 best = c;
                 ax = t;
@@ -983,9 +1001,11 @@ bool mx_plan_x(const ConvK& c, int rb, MxX& x, std::vector<int>& at)
     const int nr = c.nz * c.ny;
     double best = 1e300;
     int rows = 0;
+    MxAxis prev;
     for (int r = 2; r <= 32; r += 2) {
         MxAxis ax;
-        if (!mx_axis(c.Px, 3 * r / 2, f64, ax, nullptr)) return false;
+        if (!mx_axis(c.Px, 3 * r / 2, f64, ax, nullptr, r > 2 ? &prev : nullptr, 3 * (r - 2) / 2)) return false;
+        prev = ax;
         const size_t sm = mx_smem_x(ax, 3 * r / 2, rb);
         if (sm > MX_SMEM) break;
         const int regs = f64 ? (ax.big ? 1 : 2) : (ax.big ? 2 : 3);
