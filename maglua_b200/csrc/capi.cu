@@ -278,7 +278,7 @@ struct mlb_system {
     bool defer_x = false;
     mlb_op* pend_op = nullptr;      // operator whose inverse x pass is pending
     int pend_si = -1;               // and its slot
-    bool cap_carry = false;         // capture: assume SPEC holds the current spins' x transform
+    mlb_op* cap_carry_op = nullptr; // capture: its SPEC holds the step's spins' x transform (until it is applied)
     bool cap_inner = false;         // capture: not the last step of its graph
     mlb_op* cap_xstep = nullptr;    // capture: the convolution whose x pass the captured step fused
     unsigned long long* cap_tl = nullptr;   // capture: device timeline stamps of a timing plan
@@ -1690,6 +1690,18 @@ void flush_pending(mlb_system* s)
                                 h, s->st));
 }
 
+// Whether op's SPEC already holds the forward x transform of the current spins,
+// left there by the step before.  A captured step knows it of one operator, and
+// of its first application only: the (y,z) pass overwrites the spectrum, as the
+// cleared token says of a step that is not captured.
+bool take_carry(mlb_system* s, mlb_op* op, const ConvPlan& P)
+{
+    if (!s->capturing) return s->spec_token != 0 && s->spec_token == P.spec_token;
+    if (s->cap_carry_op != op) return false;
+    s->cap_carry_op = nullptr;
+    return true;
+}
+
 // Layer scales of a LongRange2D, the operator's global scale included.
 void lr2d_scales(const mlb_op* op, LR2DScale& sc)
 {
@@ -1801,7 +1813,7 @@ void op_apply(mlb_op* op, mlb_system* s)
         // inside a whole step: the inverse x pass waits for the LLG update,
         // the forward one ran in the step before
         const bool defer = s->defer_x;
-        const bool carry = defer && (s->capturing ? s->cap_carry : (s->spec_token != 0 && s->spec_token == P.spec_token));
+        const bool carry = defer && take_carry(s, op, P);
         if (!carry) launch_x(P, P.k, sp, P.spec.p, sl.h, true, s->st);
         CK(mlb::launch_mx_lr2d(P.k, P.mx.yz, P.L, P.tw.p, P.spec.p, P.Q.p, sc, s->rb, s->st));
         if (!s->capturing) P.spec_token = 0;
@@ -1832,7 +1844,7 @@ void op_apply(mlb_op* op, mlb_system* s)
         const void* spv[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
         if (s->defer_x && P.k.nrep == 1 && !P.k.general && (P.k.mx || (s->rb == 4 && mlb::conv_fast_ok(P.k)))) {
             // forward x pass only when SPEC does not already hold it
-            const bool carry = s->capturing ? s->cap_carry : (s->spec_token != 0 && s->spec_token == P.spec_token);
+            const bool carry = take_carry(s, op, P);
             ConvK kk = P.k;
             kk.tl = s->capturing ? s->cap_tl : nullptr;
             if (P.k.mx) {
@@ -2473,7 +2485,7 @@ void plan_capture(mlb_plan* p)
         for (int q = 0; q < 4; q++) {
             if (q >= 2 && !p->carry_op) break;   // no fused x pass: no carried variant
             s->cur = q & 1;
-            s->cap_carry = q >= 2;
+            s->cap_carry_op = q >= 2 ? p->carry_op : nullptr;
             cudaGraph_t graph = nullptr;
             CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
             s->capturing = true;
@@ -2490,7 +2502,7 @@ void plan_capture(mlb_plan* p)
             }
             mlb::prof_set_capture_sink(nullptr);
             s->capturing = false;
-            s->cap_carry = false;
+            s->cap_carry_op = nullptr;
             s->cap_tl = nullptr;
             if (q < 2) {
                 // the carried variants exist only when both parities end in the fused x pass
@@ -2523,7 +2535,7 @@ void plan_capture(mlb_plan* p)
                 bool ok = true;
                 try {
                     for (int j = 0; j < kMultiSteps && ok; j++) {
-                        s->cap_carry = true;
+                        s->cap_carry_op = p->carry_op;
                         s->cap_inner = j < kMultiSteps - 1;
                         s->cap_xstep = nullptr;
                         do_step(s, p->ops.data(), nops, p->l);
@@ -2534,7 +2546,7 @@ void plan_capture(mlb_plan* p)
                     ok = false;
                 }
                 s->capturing = false;
-                s->cap_carry = false;
+                s->cap_carry_op = nullptr;
                 s->cap_inner = false;
                 cudaError_t e = cudaStreamEndCapture(s->st, &graph);
                 if (ok && e == cudaSuccess) e = cudaGraphInstantiate(&p->multi[q], graph, 0);
@@ -2555,7 +2567,7 @@ void plan_capture(mlb_plan* p)
     } catch (...) {
         s->dry = false;
         s->capturing = false;
-        s->cap_carry = false;
+        s->cap_carry_op = nullptr;
         s->cap_inner = false;
         s->cap_tl = nullptr;
         mlb::prof_set_capture_sink(nullptr);

@@ -1,0 +1,117 @@
+"""Captured steps with more than one long-range operator, or with one operator
+listed twice: the spectrum a step carries into the next is its last operator's
+alone, so every captured step (single, carried, several to a launch) equals the
+single calls bit for bit.  The field slots of the last step equal theirs too."""
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import random_spins
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 11   # an uncarried step, single carried ones, two launches of several steps
+
+
+@pytest.fixture(scope="module")
+def M():
+    import maglua_b200 as M
+    M.init(0)
+    return M
+
+
+def _dipole(M, ss, g, slot=None, trunc=8):
+    dip = M.Dipole(ss)
+    dip.setStrength(g)
+    dip.setTruncation(trunc)
+    if slot:
+        dip.setSlotName(slot)
+    return dip
+
+
+def _layers(M, ss):
+    nx, ny, nz = ss.nx(), ss.ny(), ss.nz()
+    r = np.random.default_rng(5)
+    op = M.LongRange2D(ss)
+    op.setNewDataRequired(False)
+    for i in range(nz):
+        for j in range(nz):
+            for ab in ("XX", "XY", "XZ", "YX", "YY", "YZ", "ZX", "ZY", "ZZ"):
+                op.setTensorArray(i + 1, j + 1, ab, 0.3 * r.normal(size=nx * ny) / np.sqrt(nx * ny))
+    return op
+
+
+def _magnetostatic(M, ss):
+    op = M.Magnetostatic(ss)
+    op.setStrength(0.05)
+    op.setTruncation(4)
+    return op
+
+
+def _operators(M, ss, kind):
+    if kind == "two dipoles":
+        return [_dipole(M, ss, 0.1, "near", 3), _dipole(M, ss, 0.06, "far", 9)]
+    if kind == "twice":
+        return [_dipole(M, ss, 0.1)] * 2
+    make = {"dipole": lambda: _dipole(M, ss, 0.1), "layers": lambda: _layers(M, ss),
+            "magnetostatic": lambda: _magnetostatic(M, ss)}
+    return [make[name]() for name in kind.split(",")]
+
+
+def _build(M, dims, precision, kind, per_site=False, T=0.0, llg="Quaternion"):
+    n = int(np.prod(dims))
+    ss = M.SpinSystem(*dims, precision=precision)
+    ss.setSpinArrays(*random_spins(n, 31), np.ones(n))
+    ss.setAlpha(0.1)
+    ss.setTimeStep(0.01)
+    ex = M.Exchange(ss)
+    ex.addPaths(*O.nn_paths(*dims, pbc=(1, 1, 0)))
+    ani = M.Anisotropy(ss)
+    r = np.random.default_rng(8)
+    ani.addMany(np.arange(n), np.tile([0, 0, 1.0], (n, 1)), r.uniform(0.1, 0.3, n) if per_site else np.full(n, 0.2))
+    z = M.AppliedField(ss)
+    z.set(0.2, 0, 0)
+    ops = [ex, ani, z]
+    if T > 0:
+        th = M.Thermal(ss, M.Random.Philox(3))
+        th.setTemperature(T)
+        ops.append(th)
+    return ss, ops + _operators(M, ss, kind), M.LLG.new(llg)
+
+
+def _calls(ss, ops, llg, n):
+    for _ in range(n):
+        ss.resetFields()
+        for op in ops:
+            op.apply(ss)
+        ss.sumFields()
+        llg.apply(ss)
+
+
+def _compare(M, a, ops_a, b, ops_b, what):
+    np.testing.assert_array_equal(np.stack(a.spinArrays()[:3]), np.stack(b.spinArrays()[:3]), err_msg=what)
+    for name in {op.slotName() for op in ops_a}:
+        np.testing.assert_array_equal(np.stack(a.fieldArrays(name)), np.stack(b.fieldArrays(name)),
+                                      err_msg=what + " field " + name)
+
+
+KINDS = ["dipole,layers", "layers,dipole", "dipole,magnetostatic", "magnetostatic,dipole", "two dipoles", "twice"]
+# rows in pairs and lines of a power of two; any length; odd rows
+DIMS = [(64, 32, 2), (30, 14, 3), (32, 9, 2)]
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("dims", DIMS)
+@pytest.mark.parametrize("kind", KINDS)
+def test_captured_steps_equal_single_calls(M, kind, dims, precision):
+    ref, ops_r, llg = _build(M, dims, precision, kind)
+    _calls(ref, ops_r, llg, STEPS)
+    ss, ops, llg = _build(M, dims, precision, kind)
+    M.run(ss, ops, llg, STEPS)
+    _compare(M, ref, ops_r, ss, ops, "run")
+    ss, ops, llg = _build(M, dims, precision, kind)
+    plan = M.Plan(ss, ops, llg)
+    plan.launch(STEPS - 2)
+    plan.launch(1)
+    plan.launch(1)
+    _compare(M, ref, ops_r, ss, ops, "plan")
