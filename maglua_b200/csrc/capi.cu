@@ -2618,6 +2618,11 @@ void plan_launch(mlb_plan* p, int nsteps)
     }
     s->dstep_known = true;
     ConvPlan* CP = p->carry_op ? conv_of(p->carry_op) : nullptr;
+    // the graphs move the spins and overwrite their operators' spectra: what an
+    // earlier step left carried there is gone, but for CP's
+    for (mlb_op* o : p->ops)
+        if ((is_conv(o->kind) || is_lr2d(o->kind)) && o != p->carry_op) conv_of(o)->spec_token = 0;
+    if (!CP) s->spec_token = 0;
     for (int k = 0; k < nsteps; k++) {
         const bool carry = CP && s->spec_token != 0 && s->spec_token == CP->spec_token;
         if (carry && p->multi[s->cur] && nsteps - k >= kMultiSteps) {

@@ -115,3 +115,60 @@ def test_captured_steps_equal_single_calls(M, kind, dims, precision):
     plan.launch(1)
     plan.launch(1)
     _compare(M, ref, ops_r, ss, ops, "plan")
+
+
+# (plan, steps) in turn: a plan whose steps end in the fused x pass, then one without a
+# convolution, with the same operator and another one that comes last, or with
+# its operators in the other order (no fused x pass), then the first again
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("dims", DIMS[:2])
+@pytest.mark.parametrize("between", ["none", "near,far", "far,near"])
+def test_plans_in_turn(M, between, dims, precision):
+    turns = [("near", 3), (between, 2), ("near", 5), (between, 1), ("near", 2)]
+    res = []
+    for captured in (False, True):
+        ss, ops, llg = _build(M, dims, precision, "two dipoles")
+        base, near, far = ops[:-2], ops[-2], ops[-1]
+        lists = {"none": [], "near": [near], "near,far": [near, far], "far,near": [far, near]}
+        near.apply(ss)   # its slot comes first in the sum
+        ss.resetFields()
+        plans = {name: M.Plan(ss, base + lists[name], llg) for name in ("near", between)}
+        for name, n in turns:
+            if captured:
+                plans[name].launch(n)
+            else:
+                _calls(ss, base + lists[name], llg, n)
+        # a short run takes up what the last plan left
+        if captured:
+            plans[between].launch(2)
+            M.run(ss, base + [near], llg, 2)
+        else:
+            _calls(ss, base + lists[between], llg, 2)
+            _calls(ss, base + [near], llg, 2)
+        res.append(np.stack(ss.spinArrays()[:3]))
+    np.testing.assert_array_equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("dims,precision", [((64, 32, 2), "f32"), ((30, 14, 3), "f64")])
+def test_operator_shared_by_two_systems(M, dims, precision):
+    """A plan of another system runs the shared operator in between."""
+    res = []
+    for captured in (False, True):
+        ss, ops, llg = _build(M, dims, precision, "two dipoles")
+        other, ops2, _ = _build(M, dims, precision, "two dipoles")
+        base, near, far = ops[:-2], ops[-2], ops[-1]
+        mine = M.Plan(ss, base + [near], llg)
+        theirs = M.Plan(other, base + [near, far], llg)
+        for k in range(3):
+            if captured:
+                mine.launch(3)
+                ss.synchronize()
+                theirs.launch(2)
+            else:
+                _calls(ss, base + [near], llg, 3)
+                ss.synchronize()
+                _calls(other, base + [near, far], llg, 2)
+            other.synchronize()
+        res.append((np.stack(ss.spinArrays()[:3]), np.stack(other.spinArrays()[:3])))
+    np.testing.assert_array_equal(res[0][0], res[1][0])
+    np.testing.assert_array_equal(res[0][1], res[1][1])
