@@ -171,6 +171,8 @@ struct ConvPlan {
     bool x_mx = false;   // the x passes are mx.cu's too
     double max_imag = 0; // largest |Im| of the FP64 tensor transform (6-component)
     int device = -1;     // CUDA device the arrays above live on
+    // the system whose stream used the spectra last (claim_spec); may be gone
+    mlb_system* user = nullptr;
     // SPEC holds the forward x transform of the spins of the system whose
     // spec_token equals this one (set by the fused x pass; 0 = none)
     unsigned long long spec_token = 0;
@@ -1672,6 +1674,31 @@ void sur_advance(mlb_system* s);
 // The plan of a convolution operator (built).
 ConvPlan* conv_of(mlb_op* op) { return is_lr2d(op->kind) ? static_cast<ConvPlan*>(op->lr2.get()) : op->plan.get(); }
 
+// Before the stream of s uses a convolution's spectra: it waits for what another
+// system's stream still does with them (an operator serves any number of
+// systems, each on a stream of its own).  Graphs claim them where they are
+// launched; a caller's own capture cannot wait for what lies outside it.
+void claim_spec(mlb_op* op, mlb_system* s)
+{
+    if (s->capturing || !(is_conv(op->kind) || is_lr2d(op->kind))) return;
+    ConvPlan& P = *conv_of(op);
+    mlb_system* u = P.user;
+    P.user = s;
+    // a freed system, or a system whose stream changed, waited for its stream
+    if (!u || u == s || !g_systems.count(u) || u->st == s->st) return;
+    for (cudaStream_t st : {u->st, s->st}) {
+        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(st, &c));
+        if (c != cudaStreamCaptureStatusNone) return;
+    }
+    cudaEvent_t ev;
+    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    cudaError_t e = cudaEventRecord(ev, u->st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s->st, ev, 0);
+    cudaEventDestroy(ev);
+    CK(e);
+}
+
 // Run a deferred inverse x pass on its own (the step took another path).
 void flush_pending(mlb_system* s)
 {
@@ -1802,6 +1829,7 @@ void op_apply(mlb_op* op, mlb_system* s)
         slot_alloc(s, sl);
         sl.state = ST_DATA;
         if (s->dry) return;
+        claim_spec(op, s);
         LR2DPlan& P = *op->lr2;
         LR2DScale sc;
         lr2d_scales(op, sc);
@@ -1840,6 +1868,7 @@ void op_apply(mlb_op* op, mlb_system* s)
         P.k.g = conv_scale(op, P.k);
         sl.state = ST_DATA;
         if (s->dry) return;
+        claim_spec(op, s);
         if (s->sur && sur_hook(op, s, sl)) return;
         const void* spv[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
         if (s->defer_x && P.k.nrep == 1 && !P.k.general && (P.k.mx || (s->rb == 4 && mlb::conv_fast_ok(P.k)))) {
@@ -2620,8 +2649,10 @@ void plan_launch(mlb_plan* p, int nsteps)
     ConvPlan* CP = p->carry_op ? conv_of(p->carry_op) : nullptr;
     // the graphs move the spins and overwrite their operators' spectra: what an
     // earlier step left carried there is gone, but for CP's
-    for (mlb_op* o : p->ops)
+    for (mlb_op* o : p->ops) {
+        claim_spec(o, s);
         if ((is_conv(o->kind) || is_lr2d(o->kind)) && o != p->carry_op) conv_of(o)->spec_token = 0;
+    }
     if (!CP) s->spec_token = 0;
     for (int k = 0; k < nsteps; k++) {
         const bool carry = CP && s->spec_token != 0 && s->spec_token == CP->spec_token;
@@ -5659,6 +5690,7 @@ bool rk_stages(mlb_rk* r, mlb_system* ss, bool keep_field)
     const bool cart = r->l->kind != MLB_LLG_QUATERNION;
     const int cur = ss->cur, nb = 1 - cur;
     nm_guard(ss, nb);
+    claim_spec(conv, ss);
     std::vector<bool> started(nst, false);
     auto buf = [&](int row, int c) -> R* {   // running value of a row
         return static_cast<R*>(row == nst - 1 ? ss->sp[nb][c] : r->k[row]->sp[r->k[row]->cur][c]);
@@ -5795,6 +5827,7 @@ void rk_step_graph(mlb_rk* r)
     std::vector<HostState> saved;
     for (mlb_system* x : sys) saved.push_back(save_state(x, all));
     for (mlb_system* x : sys) nm_guard(x, -1);   // no waits on outside events inside the capture
+    for (mlb_op* o : r->ops) claim_spec(o, ss);
     cudaStream_t st = ss->st;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));

@@ -172,3 +172,48 @@ def test_operator_shared_by_two_systems(M, dims, precision):
         res.append((np.stack(ss.spinArrays()[:3]), np.stack(other.spinArrays()[:3])))
     np.testing.assert_array_equal(res[0][0], res[1][0])
     np.testing.assert_array_equal(res[0][1], res[1][1])
+
+
+@pytest.mark.parametrize("precision,make", [("f32", "dipole"), ("f64", "dipole"), ("f32", "layers")])
+@pytest.mark.parametrize("dims", [(256, 128, 4), (150, 100, 3)])
+def test_operator_applied_to_many_systems(M, dims, precision, make):
+    """The systems run on streams of their own; the operator's one spectrum serves
+    them in turn (SpinOperation::apply(SpinSystem**, n))."""
+    n = int(np.prod(dims))
+    systems = []
+    for k in range(6):
+        ss = M.SpinSystem(*dims, precision=precision)
+        ss.setSpinArrays(*random_spins(n, 70 + k), np.ones(n))
+        ss.setAlpha(0.1)
+        ss.setTimeStep(0.01)
+        systems.append(ss)
+    op = _dipole(M, systems[0], 0.1, trunc=5) if make == "dipole" else _layers(M, systems[0])
+    name = op.slotName()
+    want = []
+    for ss in systems:
+        ss.resetFields()
+        op.apply(ss)
+        ss.synchronize()
+        want.append(np.stack(ss.fieldArrays(name)))
+    for attempt in range(3):
+        for ss in systems:
+            ss.resetFields()
+        op.apply(systems)
+        for ss, w in zip(systems, want):
+            np.testing.assert_array_equal(np.stack(ss.fieldArrays(name)), w)
+    # and their captured steps, launched one after the other
+    llg = M.LLG.new("Quaternion")
+    start = [np.stack(ss.spinArrays()[:3]) for ss in systems]
+    res = []
+    for wait in (True, False):
+        for ss, s in zip(systems, start):
+            ss.setSpinArrays(*s, np.ones(n))
+        plans = [M.Plan(ss, [op], llg) for ss in systems]
+        for k in range(4):
+            for ss, p in zip(systems, plans):
+                p.launch(2)
+                if wait:
+                    ss.synchronize()
+        res.append([np.stack(ss.spinArrays()[:3]) for ss in systems])
+    for a, b in zip(*res):
+        np.testing.assert_array_equal(a, b)
