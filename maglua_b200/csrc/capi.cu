@@ -103,6 +103,24 @@ struct DBuf {
     }
 };
 
+// Host data to the device in the order of stream st (a pageable source is staged
+// before the call returns).  Not by cudaMemcpy: its copy, on the legacy stream,
+// may still be on its way when it returns, and the systems' streams do not wait for
+// that stream.
+void upload(void* dst, const void* src, size_t bytes, cudaStream_t st)
+{
+    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+}
+
+// The same for data that every stream may read: written when nothing in flight
+// reads what it replaces, and there when the call returns.
+void upload_all(void* dst, const void* src, size_t bytes)
+{
+    CK(cudaDeviceSynchronize());
+    upload(dst, src, bytes, nullptr);
+    CK(cudaStreamSynchronize(nullptr));
+}
+
 bool name_eq(const std::string& a, const char* b) { return strcasecmp(a.c_str(), b) == 0; }
 
 // ------------------------------------------------------------------ FFT plans
@@ -574,9 +592,9 @@ void compile_exchange(mlb_op* op)
             val[q] = op->eJ[p];
         }
         op->eptr.alloc(n + 1); op->ecol.alloc(np); op->eval.alloc(np);
-        CK(cudaMemcpy(op->eptr.p, cnt.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(op->ecol.p, col.data(), sizeof(int) * np, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(op->eval.p, val.data(), sizeof(double) * np, cudaMemcpyHostToDevice));
+        upload_all(op->eptr.p, cnt.data(), sizeof(int) * (n + 1));
+        upload_all(op->ecol.p, col.data(), sizeof(int) * np);
+        upload_all(op->eval.p, val.data(), sizeof(double) * np);
         k.ptr = op->eptr.p; k.col = op->ecol.p; k.val = op->eval.p;
     } else {
         k.mode = EX_NONE;
@@ -620,9 +638,9 @@ void compile_aniso(mlb_op* op)
             for (int a = 0; a < nk; a++) kk[q * nk + a] = op->apar[j * npar + nax + a] * gs;
         }
         op->aptr.alloc(n + 1); op->aaxes.alloc(ax.size()); op->aK.alloc(kk.size());
-        CK(cudaMemcpy(op->aptr.p, cnt.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(op->aaxes.p, ax.data(), sizeof(double) * ax.size(), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(op->aK.p, kk.data(), sizeof(double) * kk.size(), cudaMemcpyHostToDevice));
+        upload_all(op->aptr.p, cnt.data(), sizeof(int) * (n + 1));
+        upload_all(op->aaxes.p, ax.data(), sizeof(double) * ax.size());
+        upload_all(op->aK.p, kk.data(), sizeof(double) * kk.size());
     }
     if (op->kind == MLB_OP_ANISOTROPY) {
         AniK k{};
@@ -660,7 +678,7 @@ void compile_thermal_scale(mlb_op* op)
     if (!op->tscale_dirty) return;
     const int n = op->nx * op->ny * op->nz;
     op->dscale.alloc(n);
-    CK(cudaMemcpy(op->dscale.p, op->tscale.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+    upload_all(op->dscale.p, op->tscale.data(), sizeof(double) * n);
     op->tscale_dirty = false;
 }
 
@@ -1013,14 +1031,14 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
     }
     if (rb == 8) {
         P->tw.alloc(sizeof(double2) * twd.size());
-        CK(cudaMemcpy(P->tw.p, twd.data(), sizeof(double2) * twd.size(), cudaMemcpyHostToDevice));
+        upload(P->tw.p, twd.data(), sizeof(double2) * twd.size(), st);
     } else {
         P->tw.alloc(sizeof(float2) * twf.size());
-        CK(cudaMemcpy(P->tw.p, twf.data(), sizeof(float2) * twf.size(), cudaMemcpyHostToDevice));
+        upload(P->tw.p, twf.data(), sizeof(float2) * twf.size(), st);
     }
     DBuf<double2> twdd;
     twdd.alloc(twd.size());
-    CK(cudaMemcpy(twdd.p, twd.data(), sizeof(double2) * twd.size(), cudaMemcpyHostToDevice));
+    upload(twdd.p, twd.data(), sizeof(double2) * twd.size(), st);
 
     const int ncomp = k.general ? 9 : 6;
     const size_t plane = (size_t)Px * Py * Pz;
@@ -1056,7 +1074,7 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
             if (op->t9[q].size() != plane) continue;
             for (size_t i = 0; i < plane; i++) h[q * plane + i] = make_double2(op->t9[q][i], 0.0);
         }
-        CK(cudaMemcpy(W.p, h.data(), sizeof(double2) * h.size(), cudaMemcpyHostToDevice));
+        upload(W.p, h.data(), sizeof(double2) * h.size(), st);
     } else {
         // host tensor (user-set LongRange, or an edited Dipole tensor), z offset
         // k = source - target at padded index (zsign*k mod Pz)
@@ -1076,7 +1094,7 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
                         h[q * plane + ((size_t)zi * Py + j) * Px + i] = make_double2(op->t6[qq][src], 0.0);
                     }
             }
-        CK(cudaMemcpy(W.p, h.data(), sizeof(double2) * h.size(), cudaMemcpyHostToDevice));
+        upload(W.p, h.data(), sizeof(double2) * h.size(), st);
     }
     // x and y transforms; then the layer tensor, if a pass that sums over the
     // layers takes the size and the tensor has the parities it relies on (to
@@ -1090,7 +1108,7 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
         at.resize(Px, 0);
         at.insert(at.end(), at_y.begin(), at_y.end());
         P->at.alloc(at.size());
-        CK(cudaMemcpy(P->at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice));
+        upload(P->at.p, at.data(), sizeof(int) * at.size(), st);
         P->mx.x.at = P->at.p;
         DBuf<unsigned long long> stat;
         stat.alloc(2);
@@ -1385,14 +1403,14 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
     }
     if (rb == 8) {
         P->tw.alloc(sizeof(double2) * twd.size());
-        CK(cudaMemcpy(P->tw.p, twd.data(), sizeof(double2) * twd.size(), cudaMemcpyHostToDevice));
+        upload(P->tw.p, twd.data(), sizeof(double2) * twd.size(), st);
     } else {
         P->tw.alloc(sizeof(float2) * twf.size());
-        CK(cudaMemcpy(P->tw.p, twf.data(), sizeof(float2) * twf.size(), cudaMemcpyHostToDevice));
+        upload(P->tw.p, twf.data(), sizeof(float2) * twf.size(), st);
     }
     DBuf<double2> twdd;
     twdd.alloc(twd.size());
-    CK(cudaMemcpy(twdd.p, twd.data(), sizeof(double2) * twd.size(), cudaMemcpyHostToDevice));
+    upload(twdd.p, twd.data(), sizeof(double2) * twd.size(), st);
     ensure_t2(op);
     const size_t plane = (size_t)nx * ny;
     const int npair = nz * nz;
@@ -1405,7 +1423,7 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
         at.resize(nx, 0);
         at.insert(at.end(), at_y.begin(), at_y.end());
         P->at.alloc(at.size());
-        CK(cudaMemcpy(P->at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice));
+        upload(P->at.p, at.data(), sizeof(int) * at.size(), st);
         P->mx.x.at = P->at.p;
         k.mx = 1;
     }
@@ -2276,30 +2294,30 @@ mlb_system* make_system(int nx, int ny, int nz, int rb)
     for (int b = 0; b < 2; b++)
         for (int c = 0; c < 3; c++) {
             CK(cudaMalloc(&s->sp[b][c], (size_t)rb * n));
-            CK(cudaMemset(s->sp[b][c], 0, (size_t)rb * n));
+            CK(cudaMemsetAsync(s->sp[b][c], 0, (size_t)rb * n, s->st));
         }
     CK(cudaMalloc(&s->ms, (size_t)rb * n));
-    CK(cudaMemset(s->ms, 0, (size_t)rb * n));
+    CK(cudaMemsetAsync(s->ms, 0, (size_t)rb * n, s->st));
     s->ms_host.assign(n, 0.0);
     s->ms_dirty = true;
     s->ms_token = ++g_ms_token;
     CK(cudaMalloc(&s->dstep, 2 * sizeof(DevStep)));
-    CK(cudaMemset(s->dstep, 0, 2 * sizeof(DevStep)));
+    CK(cudaMemsetAsync(s->dstep, 0, 2 * sizeof(DevStep), s->st));
     CK(cudaMalloc(&s->status, sizeof(unsigned)));
-    CK(cudaMemset(s->status, 0, sizeof(unsigned)));
+    CK(cudaMemsetAsync(s->status, 0, sizeof(unsigned), s->st));
     CK(cudaMallocHost(&s->nm_host, sizeof(double) * 30));
     // pinned memory is mapped for the device under unified addressing; the
     // call fails (host side) where it is not
     CK(cudaHostGetDevicePointer((void**)&s->nm_host_dev, s->nm_host, 0));
     CK(cudaMalloc(&s->nm_counter, sizeof(unsigned)));
-    CK(cudaMemset(s->nm_counter, 0, sizeof(unsigned)));
+    CK(cudaMemsetAsync(s->nm_counter, 0, sizeof(unsigned), s->st));
     s->red_nb = (int)std::min<long long>(1024, std::max<long long>(1, (n + 255) / 256));
     CK(cudaMalloc(&s->red, sizeof(double) * 6 * s->red_nb));
     CK(cudaMalloc(&s->redout, sizeof(double) * 8));
     CK(cudaMalloc(&s->red_a, sizeof(double) * 6 * s->red_nb));
     CK(cudaMalloc(&s->redout_a, sizeof(double) * 8));
     CK(cudaMalloc(&s->nm_counter_a, sizeof(unsigned)));
-    CK(cudaMemset(s->nm_counter_a, 0, sizeof(unsigned)));
+    CK(cudaMemsetAsync(s->nm_counter_a, 0, sizeof(unsigned), s->st));
     slot_register(s.get(), "Total");
     mlb_system* r = s.release();
     g_systems.insert(r);
@@ -2468,7 +2486,7 @@ void load_state(mlb_system* s, const std::vector<mlb_op*>& ops, const HostState&
 void plan_timeline_reset(mlb_plan* p)
 {
     const unsigned long long init[4] = {~0ull, 0ull, ~0ull, 0ull};
-    CK(cudaMemcpy(p->tl.p, init, sizeof(init), cudaMemcpyHostToDevice));
+    upload(p->tl.p, init, sizeof(init), p->s->st);
 }
 
 void plan_release(mlb_plan* p)
@@ -2790,8 +2808,8 @@ void ens_block_table(mlb_ensemble* e, int bs)
     e->brep = nullptr; e->bstart = nullptr;
     CK(cudaMalloc(&e->brep, sizeof(int) * br.size()));
     CK(cudaMalloc(&e->bstart, sizeof(int) * br.size()));
-    CK(cudaMemcpy(e->brep, br.data(), sizeof(int) * br.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(e->bstart, bstv.data(), sizeof(int) * bstv.size(), cudaMemcpyHostToDevice));
+    upload(e->brep, br.data(), sizeof(int) * br.size(), e->st);
+    upload(e->bstart, bstv.data(), sizeof(int) * bstv.size(), e->st);
     e->nblk = (int)br.size();
     e->bs = bs;
 }
@@ -2816,9 +2834,9 @@ void ens_upload_params(mlb_ensemble* e)
         if (e->rT[r] != 0.0 && c.gamma > 0)
             sig[r] = (float)std::sqrt((2.0 * c.alpha * e->rT[r]) / (e->ms * c.dt * c.gamma));
     CK(cudaStreamSynchronize(e->st));
-    CK(cudaMemcpy(e->d_rB[e->cur], e->rB.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(e->d_rdB, e->rdB.data(), sizeof(double) * 3 * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(e->d_rsig, sig.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
+    upload(e->d_rB[e->cur], e->rB.data(), sizeof(double) * 3 * n, e->st);
+    upload(e->d_rdB, e->rdB.data(), sizeof(double) * 3 * n, e->st);
+    upload(e->d_rsig, sig.data(), sizeof(float) * n, e->st);
     e->rpar_dirty = false;
 }
 
@@ -3227,6 +3245,7 @@ int mlb_init(int device)
         CK(mlb::mx_configure());
         CK(mlb::yz_ls_configure());
         CK(mlb::sur_configure());
+        CK(cudaDeviceSynchronize());   // the constant tables are there
     });
 }
 
@@ -3270,7 +3289,7 @@ int mlb_system_status(mlb_system* s, int clear, unsigned* flags)
         if (!s || !flags) fail(MLB_EINVAL, "null argument");
         CK(cudaStreamSynchronize(s->st));
         CK(cudaMemcpy(flags, s->status, sizeof(unsigned), cudaMemcpyDeviceToHost));
-        if (clear) CK(cudaMemset(s->status, 0, sizeof(unsigned)));
+        if (clear) CK(cudaMemsetAsync(s->status, 0, sizeof(unsigned), s->st));
     });
 }
 
@@ -4213,11 +4232,11 @@ int mlb_system_copy(mlb_system* dst, mlb_system* src, int with_fields)
         upload_site_array(dst, &dst->sg, nullptr);
         if (src->sa) {
             CK(cudaMalloc(&dst->sa, bytes));
-            CK(cudaMemcpy(dst->sa, src->sa, bytes, cudaMemcpyDeviceToDevice));
+            CK(cudaMemcpyAsync(dst->sa, src->sa, bytes, cudaMemcpyDeviceToDevice, src->st));
         }
         if (src->sg) {
             CK(cudaMalloc(&dst->sg, bytes));
-            CK(cudaMemcpy(dst->sg, src->sg, bytes, cudaMemcpyDeviceToDevice));
+            CK(cudaMemcpyAsync(dst->sg, src->sg, bytes, cudaMemcpyDeviceToDevice, src->st));
         }
         if (with_fields) {
             materialize_all(src);
@@ -4229,7 +4248,7 @@ int mlb_system_copy(mlb_system* dst, mlb_system* src, int with_fields)
                 if (x.state == ST_DATA) {
                     slot_alloc(dst, y);
                     for (int c = 0; c < 3; c++)
-                        CK(cudaMemcpy(y.h[c], x.h[c], bytes, cudaMemcpyDeviceToDevice));
+                        CK(cudaMemcpyAsync(y.h[c], x.h[c], bytes, cudaMemcpyDeviceToDevice, src->st));
                     y.state = ST_DATA;
                 }
             }
@@ -4529,7 +4548,7 @@ int mlb_thermal_inject(mlb_op* op, const double* nx, const double* ny, const dou
         const double* src[3] = {nx, ny, nz};
         for (int c = 0; c < 3; c++) {
             op->inj[c].alloc(n);
-            CK(cudaMemcpy(op->inj[c].p, src[c], sizeof(double) * n, cudaMemcpyHostToDevice));
+            upload_all(op->inj[c].p, src[c], sizeof(double) * n);
         }
         op->inject_pending = true;
     });
@@ -5092,22 +5111,22 @@ int mlb_ensemble_create(int nrep, const int* dims, mlb_ensemble** out)
         for (int b = 0; b < 2; b++)
             for (int c = 0; c < 3; c++) {
                 CK(cudaMalloc(&e->sp[b][c], sizeof(float) * e->ntot));
-                CK(cudaMemset(e->sp[b][c], 0, sizeof(float) * e->ntot));
+                CK(cudaMemsetAsync(e->sp[b][c], 0, sizeof(float) * e->ntot, e->st));
             }
         for (int c = 0; c < 3; c++) {
             CK(cudaMalloc(&e->H[c], sizeof(float) * e->ntot));
-            CK(cudaMemset(e->H[c], 0, sizeof(float) * e->ntot));
+            CK(cudaMemsetAsync(e->H[c], 0, sizeof(float) * e->ntot, e->st));
         }
         CK(cudaMalloc(&e->rinfo, sizeof(int4) * nrep));
-        CK(cudaMemcpy(e->rinfo, e->rinfo_h.data(), sizeof(int4) * nrep, cudaMemcpyHostToDevice));
+        upload(e->rinfo, e->rinfo_h.data(), sizeof(int4) * nrep, e->st);
         CK(cudaMalloc(&e->dstep, sizeof(DevStep)));
-        CK(cudaMemset(e->dstep, 0, sizeof(DevStep)));
+        CK(cudaMemsetAsync(e->dstep, 0, sizeof(DevStep), e->st));
         CK(cudaMalloc(&e->mom, sizeof(double) * 6 * nrep));
         CK(cudaMalloc(&e->status, sizeof(unsigned)));
-        CK(cudaMemset(e->status, 0, sizeof(unsigned)));
+        CK(cudaMemsetAsync(e->status, 0, sizeof(unsigned), e->st));
         for (int q = 0; q < 2; q++) {
             CK(cudaMalloc(&e->d_rB[q], sizeof(double) * 3 * nrep));
-            CK(cudaMemset(e->d_rB[q], 0, sizeof(double) * 3 * nrep));
+            CK(cudaMemsetAsync(e->d_rB[q], 0, sizeof(double) * 3 * nrep, e->st));
         }
         CK(cudaMalloc(&e->d_rdB, sizeof(double) * 3 * nrep));
         CK(cudaMalloc(&e->d_rsig, sizeof(float) * nrep));
@@ -5190,7 +5209,7 @@ int mlb_ensemble_set_spins(mlb_ensemble* e, int rep, const double* x, const doub
         for (int c = 0; c < 3; c++) {
             f[c].resize(n);
             for (int i = 0; i < n; i++) f[c][i] = (float)src[c][i];
-            CK(cudaMemcpy(e->sp[e->cur][c] + ri.w, f[c].data(), sizeof(float) * n, cudaMemcpyHostToDevice));
+            upload(e->sp[e->cur][c] + ri.w, f[c].data(), sizeof(float) * n, e->st);
         }
     });
 }
@@ -5270,7 +5289,7 @@ int mlb_ensemble_status(mlb_ensemble* e, int clear, unsigned* flags)
         if (!e || !flags) fail(MLB_EINVAL, "null argument");
         CK(cudaStreamSynchronize(e->st));
         CK(cudaMemcpy(flags, e->status, sizeof(unsigned), cudaMemcpyDeviceToHost));
-        if (clear) CK(cudaMemset(e->status, 0, sizeof(unsigned)));
+        if (clear) CK(cudaMemsetAsync(e->status, 0, sizeof(unsigned), e->st));
     });
 }
 
@@ -6122,8 +6141,8 @@ void sur_upload_w(mlb_surrogate* S, const std::vector<float>& w)
                 const size_t byte = (size_t)(co >> 3) * (CP / 8) * 128 + (ci >> 3) * 128 + (co & 7) * 16 + (ci & 7) * 2;
                 t[(size_t)o * CP * CP + byte / 2] = host_bf16(w[((size_t)o * C + co) * C + ci]);
             }
-    CK(cudaMemcpy(S->wc.p, t.data(), t.size() * 2, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(S->w.p, w.data(), sizeof(float) * w.size(), cudaMemcpyHostToDevice));
+    upload_all(S->wc.p, t.data(), t.size() * 2);
+    upload_all(S->w.p, w.data(), sizeof(float) * w.size());
 }
 
 void sur_check_err(mlb_surrogate* S)
@@ -6132,6 +6151,7 @@ void sur_check_err(mlb_surrogate* S)
     CK(cudaMemcpy(&e, S->err.p, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
         CK(cudaMemset(S->err.p, 0, sizeof(int)));
+        CK(cudaDeviceSynchronize());
         fail(MLB_ECUDA, "tensor-core completion wait gave up (results of that launch are invalid)");
     }
 }
@@ -6309,9 +6329,9 @@ int mlb_surrogate_create(mlb_op* op, int mx, int my, int rad, mlb_surrogate** ou
                 }
             }
         S->F.alloc(F.size());
-        CK(cudaMemcpy(S->F.p, F.data(), F.size() * 2, cudaMemcpyHostToDevice));
+        upload_all(S->F.p, F.data(), F.size() * 2);
         S->Fc.alloc(Fc.size() * 2);
-        CK(cudaMemcpy(S->Fc.p, Fc.data(), Fc.size() * 2, cudaMemcpyHostToDevice));
+        upload_all(S->Fc.p, Fc.data(), Fc.size() * 2);
         std::vector<float2> twy((size_t)my * ny);
         for (int j = 0; j < my; j++) {
             const int ky = j < my / 2 ? j : ny - my + j;
@@ -6321,7 +6341,7 @@ int mlb_surrogate_create(mlb_op* op, int mx, int my, int rad, mlb_surrogate** ou
             }
         }
         S->twy.alloc(twy.size());
-        CK(cudaMemcpy(S->twy.p, twy.data(), sizeof(float2) * twy.size(), cudaMemcpyHostToDevice));
+        upload_all(S->twy.p, twy.data(), sizeof(float2) * twy.size());
         S->Xp.alloc((size_t)k.nxc * mx * C * ny);
         S->Yh.alloc((size_t)mx * my * C);
         S->Gh.alloc((size_t)mx * my * C);
@@ -6354,7 +6374,7 @@ int mlb_surrogate_create(mlb_op* op, int mx, int my, int rad, mlb_surrogate** ou
         h.k = S->kint;
         h.eps = (float)S->eps;
         h.tol = (float)S->tol;
-        CK(cudaMemcpy(S->dev.p, &h, sizeof(h), cudaMemcpyHostToDevice));
+        upload_all(S->dev.p, &h, sizeof(h));
         CK(cudaDeviceSynchronize());
         *out = S.release();
     });
@@ -6391,7 +6411,7 @@ int mlb_surrogate_set_params(mlb_surrogate* s, const float* w, const float* r)
     return guard([&] {
         g_version++;
         if (w) sur_upload_w(s, std::vector<float>(w, w + s->nw));
-        if (r) CK(cudaMemcpy(s->r.p, r, sizeof(float) * s->nr, cudaMemcpyHostToDevice));
+        if (r) upload_all(s->r.p, r, sizeof(float) * s->nr);
         if (s->g_train == 0.0) s->g_train = s->op->g * s->op->gs;
         CK(cudaDeviceSynchronize());
     });
@@ -6412,7 +6432,7 @@ int mlb_surrogate_forward(mlb_surrogate* s, const float* const x[3], float* cons
 {
     return guard([&] {
         const size_t bytes = sizeof(float) * s->n;
-        for (int c = 0; c < 3; c++) CK(cudaMemcpy(s->m0[c].p, x[c], bytes, cudaMemcpyHostToDevice));
+        for (int c = 0; c < 3; c++) upload_all(s->m0[c].p, x[c], bytes);
         const float* a[3] = {s->m0[0].p, s->m0[1].p, s->m0[2].p};
         float* P[3] = {s->P[0].p, s->P[1].p, s->P[2].p};
         sur_forward(s, a, nullptr, 1, nullptr, P, nullptr, nullptr, 1.f, 0);
@@ -6428,8 +6448,8 @@ int mlb_surrogate_gradients(mlb_surrogate* s, const float* const x[3], const flo
     return guard([&] {
         const size_t bytes = sizeof(float) * s->n;
         for (int c = 0; c < 3; c++) {
-            CK(cudaMemcpy(s->m0[c].p, x[c], bytes, cudaMemcpyHostToDevice));
-            CK(cudaMemcpy(s->h0[c].p, t[c], bytes, cudaMemcpyHostToDevice));
+            upload_all(s->m0[c].p, x[c], bytes);
+            upload_all(s->h0[c].p, t[c], bytes);
         }
         const float* a[3] = {s->m0[0].p, s->m0[1].p, s->m0[2].p};
         const float* hx[3] = {s->h0[0].p, s->h0[1].p, s->h0[2].p};
