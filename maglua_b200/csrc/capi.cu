@@ -1147,6 +1147,9 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
         k.spec2 = P->spec2.p;
     }
     CK(cudaStreamSynchronize(st));
+    // captured steps hold the arrays of the plan that goes (a system of the other
+    // precision may have asked for this one)
+    if (op->plan) g_version++;
     op->plan = std::move(P);
     op->plan_dirty = false;
 }
@@ -1448,6 +1451,7 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
         P->spec2.alloc((size_t)k.Kx * ny * 3 * nz * cb);
         P->k.spec2 = P->spec2.p;
     }
+    if (op->lr2) g_version++;   // as in build_plan
     op->lr2 = std::move(P);
     op->lr2_compile = false;
 }

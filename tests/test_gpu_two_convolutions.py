@@ -217,3 +217,27 @@ def test_operator_applied_to_many_systems(M, dims, precision, make):
         res.append([np.stack(ss.spinArrays()[:3]) for ss in systems])
     for a, b in zip(*res):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("make", ["dipole", "layers"])
+@pytest.mark.parametrize("dims", DIMS[:2])
+def test_operator_shared_by_both_precisions(M, dims, make):
+    """The operator's spectrum is rebuilt whenever the precision changes; plans
+    captured on the one that went are captured again."""
+    res = []
+    for captured in (False, True):
+        systems = {p: _build(M, dims, p, make) for p in ("f32", "f64")}
+        op = systems["f32"][1][-1]
+        llg = M.LLG.new("Quaternion")
+        lists = {p: systems[p][1][:-1] + [op] for p in systems}
+        if captured:
+            plans = {p: M.Plan(systems[p][0], lists[p], llg) for p in systems}
+        for k in range(2):
+            for p in systems:
+                if captured:
+                    plans[p].launch(6)
+                else:
+                    _calls(systems[p][0], lists[p], llg, 6)
+        res.append([np.stack(systems[p][0].spinArrays()[:3]) for p in systems])
+    for a, b in zip(*res):
+        np.testing.assert_array_equal(a, b)
