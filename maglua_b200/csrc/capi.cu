@@ -377,14 +377,22 @@ struct mlb_llg {
     double precess = 1.0, damp = 1.0;
 };
 
-// A captured step: one graph per spin-buffer parity q and per carry c
-// (index q + 2 c); c = 1 when the convolution's SPEC already holds the
-// forward x transform of the current spins (left there by the previous
-// step's fused x pass), so the step starts at the (y,z) pass.
 // Carried steps captured in one graph by a plan (an even count: a graph
 // starts and ends on the same spin buffer).
 constexpr int kMultiSteps = 4;
+// A plan has that graph from its creation; one that is captured again, or for a
+// single run, from this many steps on.  Capturing it takes 140 us and saves 1 to 2.5
+// us a step: a run of 50 steps 838 us with it and 798 without (64x64x2 FP64), of 70
+// 1067 and 1063, of 100 1411 and 1433; 256x256x8 FP32 1378 and 1371, 1833 and 1865,
+// 2505 and 2604.
+constexpr int kMultiFrom = 64;
 
+// A captured step: one graph per spin-buffer parity q and per carry c (index q +
+// 2 c); c = 1 when the convolution's SPEC holds the forward x transform of the
+// current spins when the step starts, at its (y,z) pass.  A plan whose steps end in
+// the fused x pass, which leaves that transform to the next one, has the graphs of
+// c = 1 alone: a step that finds no carried spectrum launches its forward x pass
+// before them.  (Plans with event nodes or a device timeline have all four.)
 struct mlb_plan {
     mlb_system* s = nullptr;
     std::vector<mlb_op*> ops;
@@ -393,10 +401,13 @@ struct mlb_plan {
     bool timeline = false;          // device timeline of the fused (y,z) and x passes
     DBuf<unsigned long long> tl;    // its four stamps (ConvK::tl)
     cudaGraphExec_t exec[4] = {nullptr, nullptr, nullptr, nullptr};
-    // carried steady state: kMultiSteps consecutive steps in one graph per
-    // starting parity (null: none; plans with event nodes or a device
-    // timeline keep one step per graph)
-    cudaGraphExec_t multi[2] = {nullptr, nullptr};
+    // carried steady state: kMultiSteps consecutive steps in one graph, from spin
+    // buffer multi_q on (null: none; plans with event nodes or a device timeline
+    // keep one step per graph)
+    cudaGraphExec_t multi = nullptr;
+    int multi_q = 0;
+    bool multi_tried = false;
+    long long steps = 0;          // launched since the capture
     std::vector<mlb::ProfCaptured> ev[4];
     mlb_op* carry_op = nullptr;   // the convolution whose SPEC a step leaves carried (null: none)
     std::vector<mlb::ProfCaptured>* last = nullptr;
@@ -2495,10 +2506,10 @@ void plan_timeline_reset(mlb_plan* p)
 
 void plan_release(mlb_plan* p)
 {
-    for (int q = 0; q < 2; q++) {
-        if (p->multi[q]) cudaGraphExecDestroy(p->multi[q]);
-        p->multi[q] = nullptr;
-    }
+    if (p->multi) cudaGraphExecDestroy(p->multi);
+    p->multi = nullptr;
+    p->multi_tried = false;
+    p->steps = 0;
     for (int q = 0; q < 4; q++) {
         if (p->exec[q]) cudaGraphExecDestroy(p->exec[q]);
         p->exec[q] = nullptr;
@@ -2506,6 +2517,63 @@ void plan_release(mlb_plan* p)
         p->ev[q].clear();
     }
     p->last = nullptr;
+}
+
+// nsteps consecutive steps from spin buffer q into one graph, the first of them
+// with the spectrum of `carry` (null: none) carried into it, the others with what
+// the step before left: their host logic runs one after the other while the
+// stream is captured, so the dependent-launch edges are kept across the step
+// boundaries (the next step's first pass is scheduled while the last one drains).
+// False, and no graph, when a step does not end in the fused x pass of `carry`.
+bool plan_capture_steps(mlb_plan* p, int q, int nsteps, mlb_op* carry, const HostState& h0, std::vector<ProfCaptured>* ev,
+                        cudaGraphExec_t* exec)
+{
+    mlb_system* s = p->s;
+    s->cur = q;
+    cudaGraph_t graph = nullptr;
+    CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
+    s->capturing = true;
+    s->cap_tl = p->timeline ? p->tl.p : nullptr;
+    if (p->timing) mlb::prof_set_capture_sink(ev);
+    bool ok = true, fits = true;
+    std::string why;
+    try {
+        for (int j = 0; j < nsteps && fits; j++) {
+            s->cap_carry_op = carry;
+            s->cap_inner = j < nsteps - 1;
+            s->cap_xstep = nullptr;
+            do_step(s, p->ops.data(), (int)p->ops.size(), p->l);
+            fits = !carry || s->cap_xstep == carry;
+            advance_sweep(p->ops.data(), (int)p->ops.size());
+        }
+    } catch (Err& e) {
+        ok = false;
+        why = e.msg;
+    }
+    mlb::prof_set_capture_sink(nullptr);
+    s->capturing = false;
+    s->cap_carry_op = nullptr;
+    s->cap_inner = false;
+    s->cap_tl = nullptr;
+    cudaError_t e = cudaStreamEndCapture(s->st, &graph);
+    if (ok && e == cudaSuccess && fits) e = cudaGraphInstantiate(exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    load_state(s, p->ops, h0);
+    if (!ok || e != cudaSuccess) {
+        cudaGetLastError();
+        fail(MLB_ESTATE, "step capture failed: " + (ok ? std::string(cudaGetErrorString(e)) : why));
+    }
+    return fits;
+}
+
+// The convolution whose spectrum a step of these operators would leave to the next
+// one if it ends in a fused x pass: the last one.
+mlb_op* plan_last_conv(const mlb_plan* p)
+{
+    mlb_op* c = nullptr;
+    for (mlb_op* o : p->ops)
+        if (is_conv(o->kind) || is_lr2d(o->kind)) c = o;
+    return c;
 }
 
 // Capture one step for each spin-buffer parity.  A dry pass first runs the
@@ -2532,100 +2600,38 @@ void plan_capture(mlb_plan* p)
         if (!s->last_fused) fail(MLB_ESTATE, "step is not fusable");
         load_state(s, p->ops, h0);
         CK(cudaStreamSynchronize(s->st));
-        p->carry_op = nullptr;
-        for (int q = 0; q < 4; q++) {
-            if (q >= 2 && !p->carry_op) break;   // no fused x pass: no carried variant
-            s->cur = q & 1;
-            s->cap_carry_op = q >= 2 ? p->carry_op : nullptr;
-            cudaGraph_t graph = nullptr;
-            CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
-            s->capturing = true;
-            s->cap_xstep = nullptr;
-            s->cap_tl = p->timeline ? p->tl.p : nullptr;
-            if (p->timing) mlb::prof_set_capture_sink(&p->ev[q]);
-            bool ok = true;
-            std::string why;
-            try {
-                do_step(s, p->ops.data(), nops, p->l);
-            } catch (Err& e) {
-                ok = false;
-                why = e.msg;
-            }
-            mlb::prof_set_capture_sink(nullptr);
-            s->capturing = false;
-            s->cap_carry_op = nullptr;
-            s->cap_tl = nullptr;
-            if (q < 2) {
-                // the carried variants exist only when both parities end in the fused x pass
-                if (q == 0) p->carry_op = s->cap_xstep;
-                else if (p->carry_op != s->cap_xstep) p->carry_op = nullptr;
-            }
-            cudaError_t e = cudaStreamEndCapture(s->st, &graph);
-            if (!ok || e != cudaSuccess) {
-                if (graph) cudaGraphDestroy(graph);
-                cudaGetLastError();
-                fail(MLB_ESTATE, "step capture failed: " + (ok ? std::string(cudaGetErrorString(e)) : why));
-            }
-            e = cudaGraphInstantiate(&p->exec[q], graph, 0);
-            cudaGraphDestroy(graph);
-            if (e != cudaSuccess) fail(MLB_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-            load_state(s, p->ops, h0);
+        p->carry_op = plan_last_conv(p);
+        bool both = true;
+        for (int q = 0; q < 2 && both && p->carry_op; q++)
+            both = plan_capture_steps(p, q, 1, p->carry_op, h0, &p->ev[q + 2], &p->exec[q + 2]);
+        if (!both) {
+            plan_release(p);
+            p->carry_op = nullptr;
         }
-        // kMultiSteps carried steps in one graph: the host logic of the steps
-        // runs one after the other while the stream is captured, so the
-        // graph holds the single-step graphs' kernels in sequence with the
-        // dependent-launch edges kept across the step boundaries (the next
-        // step's first pass is scheduled while the last one drains).  A step
-        // that does not end in the fused x pass leaves the plan without it.
-        if (p->carry_op && !p->timing && !p->timeline) {
-            for (int q = 0; q < 2; q++) {
-                s->cur = q;
-                cudaGraph_t graph = nullptr;
-                CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
-                s->capturing = true;
-                bool ok = true;
-                try {
-                    for (int j = 0; j < kMultiSteps && ok; j++) {
-                        s->cap_carry_op = p->carry_op;
-                        s->cap_inner = j < kMultiSteps - 1;
-                        s->cap_xstep = nullptr;
-                        do_step(s, p->ops.data(), nops, p->l);
-                        ok = s->cap_xstep == p->carry_op;
-                        advance_sweep(p->ops.data(), nops);
-                    }
-                } catch (Err&) {
-                    ok = false;
-                }
-                s->capturing = false;
-                s->cap_carry_op = nullptr;
-                s->cap_inner = false;
-                cudaError_t e = cudaStreamEndCapture(s->st, &graph);
-                if (ok && e == cudaSuccess) e = cudaGraphInstantiate(&p->multi[q], graph, 0);
-                if (graph) cudaGraphDestroy(graph);
-                if (!ok || e != cudaSuccess) {
-                    cudaGetLastError();
-                    p->multi[q] = nullptr;
-                }
-                load_state(s, p->ops, h0);
-            }
-            if (!p->multi[0] || !p->multi[1]) {
-                for (int q = 0; q < 2; q++) {
-                    if (p->multi[q]) cudaGraphExecDestroy(p->multi[q]);
-                    p->multi[q] = nullptr;
-                }
-            }
-        }
+        if (!p->carry_op || p->timing || p->timeline)
+            for (int q = 0; q < 2; q++) plan_capture_steps(p, q, 1, nullptr, h0, &p->ev[q], &p->exec[q]);
     } catch (...) {
         s->dry = false;
-        s->capturing = false;
-        s->cap_carry_op = nullptr;
-        s->cap_inner = false;
-        s->cap_tl = nullptr;
-        mlb::prof_set_capture_sink(nullptr);
         load_state(s, p->ops, h0);
         throw;
     }
     p->version = g_version;
+}
+
+// The graph of several steps, from the current spin buffer on (launches start
+// there, and with an even number of steps end there).  A step that does not allow
+// it leaves the plan without.
+void plan_capture_multi(mlb_plan* p)
+{
+    if (p->multi_tried || !p->carry_op || p->timing || p->timeline) return;
+    p->multi_tried = true;
+    p->multi_q = p->s->cur;
+    const HostState h0 = save_state(p->s, p->ops);
+    try {
+        if (!plan_capture_steps(p, p->multi_q, kMultiSteps, p->carry_op, h0, nullptr, &p->multi)) p->multi = nullptr;
+    } catch (Err&) {
+        p->multi = nullptr;
+    }
 }
 
 void advance_host(mlb_plan* p)
@@ -2647,6 +2653,8 @@ void plan_launch(mlb_plan* p, int nsteps)
     if (nsteps <= 0) return;
     mlb_system* s = p->s;
     if (p->version != g_version) plan_capture(p);
+    p->steps += nsteps;
+    if (p->steps >= kMultiFrom) plan_capture_multi(p);
     DevStep h;
     memset(&h, 0, sizeof(h));
     for (mlb_op* o : p->ops) {
@@ -2677,12 +2685,17 @@ void plan_launch(mlb_plan* p, int nsteps)
     }
     if (!CP) s->spec_token = 0;
     for (int k = 0; k < nsteps; k++) {
-        const bool carry = CP && s->spec_token != 0 && s->spec_token == CP->spec_token;
-        if (carry && p->multi[s->cur] && nsteps - k >= kMultiSteps) {
+        bool carry = CP && s->spec_token != 0 && s->spec_token == CP->spec_token;
+        if (CP && !carry && !p->exec[s->cur]) {
+            const void* sp[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
+            launch_x(*CP, CP->k, sp, CP->spec.p, nullptr, true, s->st);
+            carry = true;
+        }
+        if (carry && p->multi && s->cur == p->multi_q && nsteps - k >= kMultiSteps) {
             // kMultiSteps carried steps in one launch; they write both spin
             // buffers
             nm_guard(s, -1);
-            CK(cudaGraphLaunch(p->multi[s->cur], s->st));
+            CK(cudaGraphLaunch(p->multi, s->st));
             p->last = nullptr;
             for (int j = 0; j < kMultiSteps; j++, k++) {
                 CP->spec_token = ++g_spec_token;
@@ -4984,6 +4997,7 @@ int mlb_plan_create(mlb_system* s, mlb_op* const* ops, int nops, mlb_llg* l, int
             plan_timeline_reset(p.get());
         }
         plan_capture(p.get());
+        plan_capture_multi(p.get());
         *out = p.release();
     });
 }
