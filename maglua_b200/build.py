@@ -6,13 +6,18 @@ import os
 import shutil
 import subprocess
 import sys
+import time
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmlb200.so")
-SOURCES = ["kernels.cu", "conv_fast.cu", "mx.cu", "yzls.cu", "surrogate.cu", "ewald.cu", "capi.cu"]
-HEADERS = ["device.cuh", "fftreg.cuh", "fused.cuh", "kparams.h", "launch.h", "terms.cuh", "umma.cuh"]
+# the long ones first
+SOURCES = ["conv_fast.cu", "mx_f64.cu", "mx_f64_big.cu", "mx_f32.cu", "mx_f32_big.cu", "yzls_f32.cu", "yzls_f64.cu",
+           "xstep_32.cu", "xstep_64.cu", "xstep_128.cu", "xstep_256.cu", "xstep_512.cu", "kernels.cu", "surrogate.cu",
+           "capi.cu", "ewald.cu", "mx.cu", "yzls.cu"]
+HEADERS = ["device.cuh", "fftreg.cuh", "fused.cuh", "kparams.h", "launch.h", "mx.cuh", "mxradix.h", "terms.cuh", "umma.cuh",
+           "xreg.cuh", "xstep.cuh", "yzls.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
@@ -40,14 +45,17 @@ def build(force=False, verbose=False):
     if not force and not _stale():
         return LIB
     objs, running = [], []
+    jobs = max(1, os.cpu_count() or 1)
     bdir = os.path.join(HERE, "_build")
     os.makedirs(bdir, exist_ok=True)
-    for src in SOURCES:   # the sources compile side by side
+    for src in SOURCES:   # side by side, one per core
         obj = os.path.join(bdir, src.replace(".cu", ".o"))
         cmd = [nvcc()] + ARCH + FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
             print(" ".join(cmd))
+        while sum(p.poll() is None for _, p in running) >= jobs:
+            time.sleep(0.05)
         running.append((cmd, subprocess.Popen(cmd)))
         objs.append(obj)
     failed = [cmd for cmd, p in running if p.wait() != 0]

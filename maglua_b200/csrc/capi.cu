@@ -381,11 +381,10 @@ struct mlb_llg {
 // starts and ends on the same spin buffer).
 constexpr int kMultiSteps = 4;
 // A plan has that graph from its creation; one that is captured again, or for a
-// single run, from this many steps on.  Capturing it takes 140 us and saves 1 to 2.5
-// us a step: a run of 50 steps 838 us with it and 798 without (64x64x2 FP64), of 70
-// 1067 and 1063, of 100 1411 and 1433; 256x256x8 FP32 1378 and 1371, 1833 and 1865,
-// 2505 and 2604.
-constexpr int kMultiFrom = 64;
+// single run, from this many steps on.  It saves 1 to 2 us a step, and capturing it
+// takes 25 to 140 us of host time, as the host is: it paid from 11 (256x256x8) to 43
+// steps (64x64x2 FP64) on, and on a slower host from 32 to 70.
+constexpr int kMultiFrom = 48;
 
 // A captured step: one graph per spin-buffer parity q and per carry c (index q +
 // 2 c); c = 1 when the convolution's SPEC holds the forward x transform of the
@@ -1020,6 +1019,17 @@ void build_magnetostatic_t6(mlb_op* op)
     op->t6_valid = true;
 }
 
+// The constant tables of the translation units that the plan's passes run from
+// (loading them, outside any capture).
+void plan_tables(const ConvPlan& P)
+{
+    const ConvK& k = P.k;
+    if (P.x_mx) CK(mlb::mx_init(P.mx.x.ax, P.rb));
+    else if (P.rb == 4) CK(mlb::xstep_init(k.Px));
+    if (k.ls) CK(mlb::yz_ls_init(P.rb));
+    else if (k.mx) CK(mlb::mx_init(P.mx.yz.ax, P.rb));
+}
+
 // Build or rebuild the tensor spectrum of op (FP64 on the GPU), stored at
 // rb bytes per real for the systems it is applied to.
 void build_plan(mlb_op* op, cudaStream_t st, int rb)
@@ -1158,6 +1168,7 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
         k.spec2 = P->spec2.p;
     }
     CK(cudaStreamSynchronize(st));
+    plan_tables(*P);
     // captured steps hold the arrays of the plan that goes (a system of the other
     // precision may have asked for this one)
     if (op->plan) g_version++;
@@ -1462,6 +1473,7 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
         P->spec2.alloc((size_t)k.Kx * ny * 3 * nz * cb);
         P->k.spec2 = P->spec2.p;
     }
+    plan_tables(*P);
     if (op->lr2) g_version++;   // as in build_plan
     op->lr2 = std::move(P);
     op->lr2_compile = false;
@@ -3192,6 +3204,7 @@ void ens_prepare(mlb_ensemble* e)
             ConvPlan& P = *k.dip->plan;
             // all replicas per launch: the power-of-two passes
             if (P.k.ls && x_pow2(P.k, 4, 16)) P.x_mx = false;
+            plan_tables(P);
             k.fast = P.k.mx ? P.k.ls && !P.x_mx : mlb::conv_fast_ok(P.k) && !P.k.split;
             P.k.g = c.g / ((double)P.k.Px * P.k.Py * (P.k.mx ? 1 : P.k.Pz));
             P.k.nrep = k.fast ? k.nrep : 1;
@@ -3258,9 +3271,6 @@ int mlb_init(int device)
         CK(cudaFree(0));
         CK(mlb::conv_configure());
         CK(mlb::fftreg_init());
-        CK(mlb::conv_fast_configure());
-        CK(mlb::mx_configure());
-        CK(mlb::yz_ls_configure());
         CK(mlb::sur_configure());
         CK(cudaDeviceSynchronize());   // the constant tables are there
     });

@@ -13,9 +13,23 @@
 namespace fr {
 
 // w_64^k = exp(-2 pi i k / 64); one copy per translation unit that includes
-// this header, filled by that unit's fftreg_init().
+// this header, filled by fill_tables() there.
 static __constant__ float2 c_w64[64];
 static __constant__ double2 c_w64d[64];   // the same in FP64, for double2 lines
+inline cudaError_t fill_tables(const void* w64, const void* w64d)
+{
+    float2 h[64];
+    double2 hd[64];
+    for (int k = 0; k < 64; k++) {
+        const double a = 2.0 * M_PI * k / 64.0;
+        h[k] = make_float2((float)cos(a), (float)(-sin(a)));
+        hd[k] = make_double2(cos(a), -sin(a));
+    }
+    cudaError_t e = cudaMemcpyToSymbol(w64, h, sizeof(h));
+    if (e != cudaSuccess || (e = cudaMemcpyToSymbol(w64d, hd, sizeof(hd))) != cudaSuccess) return e;
+    return cudaStreamSynchronize(nullptr);   // there for every stream
+}
+static inline cudaError_t fill_tables() { return fill_tables(&c_w64, &c_w64d); }
 
 template <typename C>
 __device__ __forceinline__ C w64(int k, int sign)

@@ -1228,6 +1228,57 @@ cudaError_t launch_fft3d_d(double2* W, int ncomp, int Px, int Py, int Pz, const 
     return cudaSuccess;
 }
 
+// T(kx, ky, dz) of six components from their FP64 transforms over x and y,
+// W[q][z][ky][kx] (z = dz mod Pz): tz[kx][dz][q][at[ky]], the real part or (XZ,
+// YZ) the imaginary part, ky at its place after the y transform.  stat: bits of the largest |W| and of the largest
+// deviation from the parities the layer sum relies on.
+template <typename R>
+__global__ void k_mx_pack(const double2* W, int Px, int Py, int Pz, int nz, int Kx, const int* at, R* tz,
+                          unsigned long long* stat)
+{
+    const long long total = (long long)Kx * nz * 6 * Py;
+    double big = 0, dev = 0;
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+         e += (long long)gridDim.x * blockDim.x) {
+        // kx fastest for the reads: the writes are Py apart
+        const int kx = (int)(e % Kx);
+        long long r = e / Kx;
+        const int ky = (int)(r % Py);
+        r /= Py;
+        const int q = (int)(r % 6), dz = (int)(r / 6);
+        const double2* Wq = W + (size_t)q * Px * Py * Pz;
+        const double2 v = Wq[((size_t)dz * Py + ky) * Px + kx];
+        const double2 u = Wq[((size_t)((Pz - dz) % Pz) * Py + ky) * Px + kx];
+        const bool odd = q == 2 || q == 4;
+        tz[(((size_t)kx * nz + dz) * 6 + q) * Py + at[ky]] = (R)(odd ? v.y : v.x);
+        big = fmax(big, fmax(fabs(v.x), fabs(v.y)));
+        dev = fmax(dev, odd ? fmax(fmax(fabs(v.x), fabs(u.x)), fabs(v.y + u.y))
+                            : fmax(fmax(fabs(v.y), fabs(u.y)), fabs(v.x - u.x)));
+    }
+    unsigned long long s[2] = {(unsigned long long)__double_as_longlong(big), (unsigned long long)__double_as_longlong(dev)};
+    for (int k = 0; k < 2; k++) {
+        unsigned long long x = s[k];
+        for (int o = 16; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
+        if ((threadIdx.x & 31) == 0 && x) atomicMax(stat + k, x);
+    }
+}
+
+size_t mx_tensor_bytes(const ConvK& c, int rb) { return (size_t)c.Kx * c.nz * 6 * c.Py * rb; }
+
+cudaError_t launch_mx_pack(const double2* W, const ConvK& c, const int* at, void* tz, unsigned long long* stat2, int rb,
+                           cudaStream_t st)
+{
+    const long long total = (long long)c.Kx * c.nz * 6 * c.Py;
+    const unsigned nb = (unsigned)std::min<long long>((total + 255) / 256, 148 * 8);
+    if (rb == 8)
+        k_mx_pack<double><<<nb, 256, 0, st>>>(W, c.Px, c.Py, c.Pz, c.nz, c.Kx, at, static_cast<double*>(tz),
+                                              stat2);
+    else
+        k_mx_pack<float><<<nb, 256, 0, st>>>(W, c.Px, c.Py, c.Pz, c.nz, c.Kx, at, static_cast<float*>(tz),
+                                             stat2);
+    return cudaGetLastError();
+}
+
 // LongRange2D tensor: Q[kx][ky][s][d][ab] = W_{(s d ab)}(kx, ky) / (nx ny) for
 // the layer pairs p0 .. p0 + np - 1 (p = s nz + d), W holding their
 // transforms [(p - p0) 9 + ab][ky][kx] over the full x length.  at (not null):

@@ -6,9 +6,53 @@
 #include "device.cuh"
 #include "kparams.h"
 
+#include <map>
+#include <mutex>
+#include <set>
+#include <utility>
 #include <vector>
 
 namespace mlb {
+// A kernel's limit of dynamic shared memory (and, max_carveout, the SM's whole
+// shared memory preferred over L1), set when its first launch on a device asks
+// for it.  Setting them for every instantiation when the library starts loads
+// them all: 250 to 340 ms where a program takes a handful.
+inline cudaError_t use_smem(const void* kern, size_t smem, bool max_carveout = false)
+{
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> allowed;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = allowed.find({kern, dev});
+    if (it != allowed.end() && it->second >= smem) return cudaSuccess;
+    if (smem > 48 * 1024 &&
+        (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        return e;
+    if (max_carveout &&
+        (e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  (int)cudaSharedmemCarveoutMaxShared)) != cudaSuccess)
+        return e;
+    allowed[{kern, dev}] = smem;
+    return cudaSuccess;
+}
+
+// f() once on each device (per call site: the lambda's type).
+template <class F>
+inline cudaError_t per_device(F&& f)
+{
+    static std::mutex mu;
+    static std::set<int> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count(dev)) return cudaSuccess;
+    if ((e = f()) == cudaSuccess) done.insert(dev);
+    return e;
+}
+
 // Launch with programmatic stream serialization: the kernel's CTAs may be
 // scheduled before the previous kernel of the stream has finished (they
 // wait in pdl_wait()), which hides the launch latency between the kernels
@@ -17,6 +61,10 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               Args... args)
 {
+    if (smem > 48 * 1024) {
+        const cudaError_t e = use_smem(reinterpret_cast<const void*>(kern), smem);
+        if (e != cudaSuccess) return e;
+    }
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -28,6 +76,15 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// The same for kernels whose CTAs share an SM best with all of its shared memory.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl_carved(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                     Args... args)
+{
+    const cudaError_t e = use_smem(reinterpret_cast<const void*>(kern), smem, true);
+    return e != cudaSuccess ? e : launch_pdl(kern, grid, block, smem, st, args...);
 }
 
 // Kernel timing: 1 = eager profiling (mlb_profile_begin/end), 2 = event
@@ -61,7 +118,6 @@ struct Prof {
     }
 };
 cudaError_t fftreg_init();
-cudaError_t conv_fast_configure();
 bool conv_fast_ok(const ConvK& c);
 // FP32 x passes alone (power-of-two Px 16..512): the forward transform of the
 // spins to SPEC (fwd) or the inverse to the field h.
@@ -90,6 +146,21 @@ cudaError_t launch_conv_fast_fyz(const ConvK& c, const FftLen L[3], const float2
                                  const float* ten6, bool with_fx, cudaStream_t st);
 cudaError_t launch_conv_fast_ix(const ConvK& c, const FftLen L[3], const float2* tw, float2* spec, float* h[3],
                                 cudaStream_t st);
+// The fused x pass for lines of PX points (xstep.cuh); init: its constant tables,
+// before its first launch and outside any capture (xstep_init: by length).
+template <int PX>
+struct XUnit {
+    static cudaError_t init();
+    static cudaError_t step(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec, const float* s[3],
+                            float* h[3], float* o[3], cudaStream_t st);
+    static cudaError_t gstep(const ConvK& c, const FusedK& P, double addw, double dt_sys, const DevStep* cur,
+                             DevStep* next, const float2* tw, float2* spec, float* const h[3], cudaStream_t st);
+    static cudaError_t ens(const ConvK& c, const FastK& F, const XEns& E, const float2* tw, float2* spec,
+                           const float* const s[3], float* const o[3], cudaStream_t st);
+    static cudaError_t rk(const ConvK& c, const FastK& F, const RkRows<float>& rows, int fwd, const float2* tw,
+                          float2* spec, const float* const s[3], float* const h[3], float* const o[3], cudaStream_t st);
+};
+cudaError_t xstep_init(int Px);
 bool xstep_ok(const ConvK& c, const FastK& F);
 bool xstep_pairs(const ConvK& c);
 // Inverse x pass + fused step (+ forward x pass of the new spins when fwd).
@@ -148,7 +219,16 @@ cudaError_t launch_mx_pack(const double2* W, const ConvK& c, const int* at, void
 bool yz_ls_plan(const ConvK& c, int rb, std::vector<int>& at);
 cudaError_t launch_yz_ls(const ConvK& c, const FftLen L[3], const void* tw, void* spec, const void* tz, int rb,
                          cudaStream_t st);
-cudaError_t yz_ls_configure();
+// the pass for lines of C (float2 or double2; yzls.cuh), and its constant tables (before
+// its first launch, outside any capture)
+template <typename C>
+struct YzUnit {
+    typedef decltype(C().x) R;
+    static cudaError_t init();
+    static bool takes(int Py, int nz);
+    static cudaError_t pass(const ConvK& c, const C* tw, C* spec, const R* tz, cudaStream_t st);
+};
+cudaError_t yz_ls_init(int rb);
 // Any-length passes (mx.cu): the plans of the x passes and of the (y,z) pass
 // (false: not a size they take) with the places of their frequencies, and the
 // passes.
@@ -184,7 +264,26 @@ cudaError_t launch_xrk(const ConvK& c, const FftLen L[3], const void* tw, void* 
                        float* const o[3], cudaStream_t st);
 cudaError_t launch_mx_gstep(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FusedK& P, double addw,
                             double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], int rb, cudaStream_t st);
-cudaError_t mx_configure();
+// The kernels for state precision R, BIG: with prime radices above 13 (mx.cuh); init:
+// their constant tables, before their first launch and outside any capture
+// (mx_init: those of an axis).
+template <typename R, bool BIG>
+struct MxUnit {
+    typedef typename CT<R>::T C;
+    static cudaError_t init();
+    static cudaError_t fx(const MxX& x, size_t smem, const C* tw, const void* const s[3], C* spec, cudaStream_t st);
+    static cudaError_t ix(const MxX& x, size_t smem, const C* tw, const C* spec, void* const h[3], cudaStream_t st);
+    static cudaError_t yz(const MxYZ& y, int Kx, size_t smem, const C* tw, C* spec, const R* tz, cudaStream_t st);
+    static cudaError_t lr2d(const MxYZ& y, int Kx, size_t smem, const LR2DScale& sc, int stream, const C* tw, C* spec,
+                            const C* Q, cudaStream_t st);
+    static cudaError_t step(const MxX& x, size_t smem, const C* tw, C* spec, const FastKT<R>& F, const R* const s[3],
+                            R* const h[3], R* const o[3], cudaStream_t st);
+    static cudaError_t rk(const MxX& x, size_t smem, const C* tw, C* spec, const FastKT<R>& F, const RkRows<R>& rows,
+                          const R* const s[3], R* const h[3], R* const o[3], cudaStream_t st);
+    static cudaError_t gstep(const MxX& x, size_t smem, const C* tw, C* spec, const FusedK& P, double addw,
+                             double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], cudaStream_t st);
+};
+cudaError_t mx_init(const MxAxis& ax, int rb);
 cudaError_t launch_tensor_lattice(int nx, int ny, int nz, const int gmax[4], const double ABC[9], int Px,
                                   int Py, int Pz, int zsign, double2* W, cudaStream_t st);
 cudaError_t launch_tensor_rings(int nx, int ny, int nz, int nrings, int lstep, const double ABC[9], int Px, int Py,

@@ -1,0 +1,2 @@
+#include "mx.cuh"
+template struct mlb::MxUnit<double, false>;
