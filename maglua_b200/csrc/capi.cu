@@ -2997,7 +2997,9 @@ void ens_enqueue_step(mlb_ensemble* e, int q, bool carry)
 // and the fused kernel's tile size and grid (one CTA per tile, or
 // persistent CTAs walking the tile table).  Each candidate is timed with
 // CUDA events on the ensemble's stream over repeated launches on the
-// current state (the passes write only H and the other spin buffer).  The
+// current state (the passes write only H and the other spin buffer).  Where
+// the step runs inside every class' x pass (fused_x) none of them is used, and
+// nothing is timed.  The
 // choices are kept per process and in a cache file keyed by the device and
 // the classes: MLB_TUNE_CACHE names the file ("off": none), else
 // $XDG_CACHE_HOME/maglua_b200/tune.txt or ~/.cache/maglua_b200/tune.txt.
@@ -3020,7 +3022,7 @@ std::string ens_tune_key(mlb_ensemble* e)
     CK(cudaGetDeviceProperties(&pr, dev));
     std::string k = std::string(pr.name) + "/" + std::to_string(pr.multiProcessorCount) + "/" +
                     (e->cfg.llg == MLB_LLG_QUATERNION ? "Q" : "C") + (e->cfg.g != 0.0 ? "D" : "-") +
-                    (ens_thermal(e) ? "T" : "-") + "/";
+                    (ens_thermal(e) ? "T" : "-") + (e->fused_x ? "X" : "") + "/";
     for (char& ch : k)
         if (ch == ' ') ch = '_';
     for (EnsClass& c : e->cls)
@@ -3111,7 +3113,13 @@ void ens_autotune(mlb_ensemble* e)
         e->tune_log = "tuner: cached choices for " + key + "\n";
     }
     const float* s[3] = {e->sp[e->cur][0], e->sp[e->cur][1], e->sp[e->cur][2]};
-    if (!have) {
+    if (!have && e->fused_x) {
+        e->tune_log = "tuner: " + key + "\n  fused step: inside every class' x pass (k_xens), CTAs of 256 threads\n"
+                      "  chosen: as such (nothing to time)\n";
+        t.bs = 256;
+        t.yz.assign(e->cls.size(), 0);
+        tune_file_store(key, t);
+    } else if (!have) {
         char buf[256];
         std::string log = "tuner: " + key + "\n";
         // (y,z) pass variant per fast class
@@ -3175,7 +3183,8 @@ void ens_autotune(mlb_ensemble* e)
         g_ens_tuned[key] = t;
     }
     for (size_t i = 0; i < e->cls.size(); i++) e->cls[i].yz_variant = i < t.yz.size() ? t.yz[i] : 0;
-    ens_block_table(e, t.bs);
+    if (e->fused_x) e->bs = t.bs;   // no tile table
+    else ens_block_table(e, t.bs);
     e->grid = t.grid;
     e->tuned = true;
 }
