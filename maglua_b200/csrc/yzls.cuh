@@ -1,5 +1,5 @@
 // yzls.cuh -- (y,z) pass of the dipole convolution with the sum over layers,
-// power-of-two Py 16..512, up to 8 layers or 16, FP32 and FP64.
+// power-of-two Py 16..512, up to 8 layers (to 64 rows up to 16), FP32 and FP64.
 //
 // One CTA per kx (and packed replica).  A line (component, layer) of Py = T E
 // points belongs to T lanes of a warp:
@@ -68,21 +68,22 @@ __device__ __forceinline__ void axpy(double2& acc, double w, double2 s)
     acc.y = fm(w, s.y, acc.y);
 }
 
-template <int PY, int NZ, typename C, bool SM>
+// NZ layers, or (UP) c.nz of them, up to NZ.
+template <int PY, int NZ, typename C, bool SM, bool UP = false>
 __global__ void __launch_bounds__(LS<PY, C, SM>::NT, LS<PY, C, SM>::MINB) k_yz_ls(ConvK c, const C* __restrict__ twy, C* __restrict__ spec,
                                                           const decltype(C().x)* __restrict__ tz)
 {
     typedef decltype(C().x) R;
     using Y = LS<PY, C, SM>;
-    constexpr int NT = Y::NT, T = Y::T, E = Y::E, LINE = Y::LINE, NI = Y::NI, nl = 3 * NZ;
+    constexpr int NT = Y::NT, T = Y::T, E = Y::E, LINE = Y::LINE, NI = Y::NI;
     extern __shared__ __align__(16) unsigned char smraw_ls[];
     C* twl = reinterpret_cast<C*>(smraw_ls);   // [PY]
     C* P = twl + PY;                           // [3 NZ][E][T + 1]
-    const int kx = blockIdx.x, ny = c.ny;
-    const R* Tk = tz + (size_t)kx * NZ * 6 * PY;
+    const int kx = blockIdx.x, ny = c.ny, nz = UP ? c.nz : NZ, nl = 3 * nz;
+    const R* Tk = tz + (size_t)kx * nz * 6 * PY;
     if (threadIdx.x == 0) {
         // this kx's tensor (constant between steps) starts towards L2
-        const unsigned bytes = (unsigned)(NZ * 6 * PY * sizeof(R));
+        const unsigned bytes = (unsigned)(nz * 6 * PY * sizeof(R));
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(Tk), "r"(bytes) : "memory");
     }
     for (int k = threadIdx.x; k < PY; k += NT) twl[k] = twy[k];
@@ -139,12 +140,13 @@ __global__ void __launch_bounds__(LS<PY, C, SM>::NT, LS<PY, C, SM>::MINB) k_yz_l
             R w[NZ], wn[NZ];
 #pragma unroll
             for (int d = 0; d < NZ; d++) {
-                w[d] = __ldg(Tk + (d * 6 + q) * PY + p);
+                w[d] = !UP || d < nz ? __ldg(Tk + (d * 6 + q) * PY + p) : (R)0;
                 wn[d] = odd ? -w[d] : w[d];
             }
 #pragma unroll
             for (int zs = 0; zs < NZ; zs++) {
-                const C m = col[(b * NZ + zs) * LINE];
+                if (UP && zs >= nz) break;
+                const C m = col[(b * nz + zs) * LINE];
                 const C s = odd ? cmk<C>(-m.y, m.x) : m;
 #pragma unroll
                 for (int zt = 0; zt < NZ; zt++) axpy(acc[i][zt], zt >= zs ? w[zt - zs] : wn[zs - zt], s);
@@ -158,7 +160,8 @@ __global__ void __launch_bounds__(LS<PY, C, SM>::NT, LS<PY, C, SM>::MINB) k_yz_l
         const int a = item / PY, p = item % PY;
         if (item >= 3 * PY) continue;
 #pragma unroll
-        for (int z = 0; z < NZ; z++) P[(a * NZ + z) * LINE + p + p / T] = cmk<C>(g * acc[i][z].x, g * acc[i][z].y);
+        for (int z = 0; z < NZ; z++)
+            if (!UP || z < nz) P[(a * nz + z) * LINE + p + p / T] = cmk<C>(g * acc[i][z].x, g * acc[i][z].y);
     }
     __syncthreads();
     for (int l = lr; l < nl && lr < Y::LPR; l += Y::LPR) {
@@ -193,6 +196,13 @@ __global__ void __launch_bounds__(LS<PY, C, SM>::NT, LS<PY, C, SM>::MINB) k_yz_l
 
 template <typename C> using Kern = void (*)(ConvK, const C*, C*, const decltype(C().x)*);
 
+// Up to 8 layers in planes of any width, 9 to 16 in planes of up to 64 rows: one kernel
+// for 16, and one that leaves out what is missing to 16 (64x64x12 11.3 us a step where
+// the z spectra took 14.9, 256x64x9 16.9 against 20.0, FP64 64x64x12 17.6 against
+// 48.7; all 16 by it 12.8 against 11.9).  Wider planes keep the z spectra: the kernel
+// would serve 128 and 256 rows too (64x128x9 24.8 -> 13.4, 256x256x16 54.6 -> 44.1), but
+// its small-CTA form does not fit the registers there (4.7 KB spilled), and at 512
+// rows it is slower (64x512x16 41 -> 48).
 template <int PY, typename C, bool SM>
 Kern<C> kern_py(int nz)
 {
@@ -205,10 +215,9 @@ Kern<C> kern_py(int nz)
     case 6: return k_yz_ls<PY, 6, C, SM>;
     case 7: return k_yz_ls<PY, 7, C, SM>;
     case 8: return k_yz_ls<PY, 8, C, SM>;
-    case 16:
-        if constexpr (PY <= 64) return k_yz_ls<PY, 16, C, SM>;
-        break;
     }
+    if constexpr (PY <= 64)
+        if (nz <= 16) return nz == 16 ? k_yz_ls<PY, 16, C, SM> : k_yz_ls<PY, 16, C, SM, true>;
     return nullptr;
 }
 
