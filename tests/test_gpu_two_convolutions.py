@@ -241,3 +241,17 @@ def test_operator_shared_by_both_precisions(M, dims, make):
         res.append([np.stack(systems[p][0].spinArrays()[:3]) for p in systems])
     for a, b in zip(*res):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("dims,precision,kind", [((64, 32, 2), "f32", "dipole,layers"), ((32, 9, 2), "f32", "layers"),
+                                                 ((30, 14, 3), "f32", "two dipoles"), ((30, 14, 3), "f64", "layers,dipole"),
+                                                 ((64, 32, 2), "f64", "dipole")])
+@pytest.mark.parametrize("llg,T", [("Quaternion", 0.0), ("Cartesian", 0.3)])
+def test_per_site_terms_beside_convolutions(M, dims, precision, kind, llg, T):
+    """The general step with its last convolution's x pass fused and other addends
+    in slots: a constant per site and noise beside them."""
+    ref, ops_r, l = _build(M, dims, precision, kind, per_site=True, T=T, llg=llg)
+    _calls(ref, ops_r, l, STEPS)
+    ss, ops, l = _build(M, dims, precision, kind, per_site=True, T=T, llg=llg)
+    M.run(ss, ops, l, STEPS)
+    _compare(M, ref, [o for o in ops_r if o.slotName() != "Thermal"], ss, ops, "run")
