@@ -34,7 +34,7 @@ if ROOT not in sys.path:
 NX, NY, NZ = 256, 256, 8
 J, K_ANI, G_DIP, BX = 1.0, 0.05, 0.02, 0.1
 TEMP, ALPHA, DT = 0.5, 0.05, 0.005
-WORKLOAD = "film 256x256x8, periodic x/y, open z (z padded to 16), J=1, K=0.05 z, g=0.02, B=0.1 x, T=0.5, alpha=0.05, dt=0.005, LLG.Quaternion"
+WORKLOAD = "film 256x256x8, periodic x/y, open z, J=1, K=0.05 z, g=0.02, B=0.1 x, T=0.5, alpha=0.05, dt=0.005, LLG.Quaternion"
 METRIC = "spin-steps/s"
 UNIT = "spin-steps/s"
 FLUSH_BYTES = 1 << 30
@@ -170,23 +170,22 @@ def _pow2_at_least(m):
 
 
 def ensemble_bytes(dims):
-    """Algorithmic bytes of one ensemble step by the per-site formula
-    B = 36 + 24 + (K/N)(24 + 48 * 2) per replica, K = (Px/2+1) Py Pz stored
-    k-points with every axis of an open replica padded to the power of two
-    at least 2n - 1 (z: 1 when nz = 1)."""
+    """Bytes that one ensemble step's passes cannot do without: the spins in and
+    out (24 B per site), the x spectra of the data rows in and out of the (y,z)
+    pass and of the fused x pass (96 B per stored kx and row, every axis of an
+    open replica padded to the power of two at least 2n - 1), and each size
+    class' layer tensor once (kx, ky, layer distance, 6 values)."""
     total = 0
     for nx, ny, nz in dims:
-        n = nx * ny * nz
-        Px, Py = _pow2_at_least(2 * nx - 1), _pow2_at_least(2 * ny - 1)
-        Pz = 1 if nz == 1 else _pow2_at_least(2 * nz - 1)
-        K = (Px // 2 + 1) * Py * Pz
-        total += 60 * n + K * (24 + 48 * 2)
+        total += 24 * nx * ny * nz + 96 * (_pow2_at_least(2 * nx - 1) // 2 + 1) * ny * nz
+    for nx, ny, nz in set(dims):
+        total += 24 * (_pow2_at_least(2 * nx - 1) // 2 + 1) * _pow2_at_least(2 * ny - 1) * nz
     return total
 
 
 def run_batched(M, torch, steps, warmup):
     """Configuration 3: the packed ensemble (one captured graph per step,
-    classes on concurrent branches, tuned tile/grid/(y,z) variant), the same
+    classes on concurrent branches, the step inside each class' x pass), the same
     replicas through the plain path one SpinSystem per replica, and the
     ensemble without the dipole (the bound any dipole surrogate works under)."""
     dims = ensemble_dims()
@@ -201,8 +200,8 @@ def run_batched(M, torch, steps, warmup):
             "sites": sites, "replicas": len(dims), "fused_block_size": info["block_size"],
             "step_roofline": {"algorithmic_bytes_per_step": nbytes, "achieved_gbs": nbytes / (ms * 1e-3) / 1e9,
                               "frac": nbytes / (ms * 1e-3) / 1e9 / peak, "peak": peak, "peak_kind": peak_kind,
-                              "how": "36 + 24 B per site + (24 + 96) B per stored k-point of each replica's padded "
-                                     "grid, over the event-timed step"},
+                              "how": "24 B per site + 96 B per stored kx and data row of each replica + the size "
+                                     "classes' layer tensors, over the event-timed step"},
             "config": e.configInfo(), "tune_log": e.tuneLog().strip().splitlines(),
             "workload": ENS_WORKLOAD,
             "plain_one_system_per_replica": {"value": sites / (plain_ms * 1e-3), "ms_per_step": plain_ms,
@@ -219,7 +218,7 @@ def run_batched(M, torch, steps, warmup):
 
 # ----------------------------------------------------------------- learned surrogate
 SUR_DIMS = (512, 512, 4)
-SUR_WORKLOAD = ("film 512x512x4, periodic x/y, open z (z padded to 8), J=1, K=0.02 z, g=0.05, T=0.1, "
+SUR_WORKLOAD = ("film 512x512x4, periodic x/y, open z, J=1, K=0.02 z, g=0.05, T=0.1, "
                 "alpha=0.02, dt=0.005, LLG.Quaternion; spins from a seeded random start relaxed 200 steps; "
                 "surrogate: linear spectral-conv net (BF16 tcgen05, 16x16 modes, radius-3 stencil) trained "
                 "online on the plain method over 8 seeded random-start runs")
@@ -551,8 +550,8 @@ def run_fp64_film(M, torch, steps=20):
     ms = a.elapsed_time(b) / steps
     n = NX * NY * NZ
     return {"workload": WORKLOAD + " in FP64", "value": n / (ms * 1e-3), "unit": UNIT, "ms_per_step": ms,
-            "how": "one captured step per graph launch, back to back, CUDA events; FP64 register split (y,z) "
-                   "passes, x passes and fused step"}
+            "how": "captured steps back to back (four to a graph), CUDA events; FP64 (y,z) pass with the layer "
+                   "sum and fused x pass"}
 
 
 # ----------------------------------------------------------------- LongRange2D / Dipole2D

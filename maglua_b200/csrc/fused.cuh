@@ -1,6 +1,7 @@
 // fused.cuh -- one site of the fused step (field terms + LLG update) for
-// uniform-parameter FP32 systems, shared by the fused-step kernels
-// (conv_fast.cu) and the surrogate's output kernel (surrogate.cu).
+// uniform-parameter systems, FP32 or FP64, or two FP32 sites in packed arithmetic;
+// shared by the fused-step kernels (conv_fast.cu), the fused x passes (xstep.cuh,
+// mx.cuh) and the Runge-Kutta stages there.
 #pragma once
 #include "device.cuh"
 #include "kparams.h"

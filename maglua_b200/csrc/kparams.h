@@ -1,6 +1,5 @@
 // kparams.h -- plain-old-data launch parameters shared by the host layer
-// (capi.cu) and the kernels (kernels.cu, conv_fast.cu).  Device pointers
-// only.
+// (capi.cu) and the kernels.  Device pointers only.
 #pragma once
 #include <stdint.h>
 

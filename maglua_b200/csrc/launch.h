@@ -1,4 +1,4 @@
-// launch.h -- host-callable launchers for the kernels in kernels.cu.
+// launch.h -- host-callable launchers of the kernels.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -29,7 +29,7 @@
 //
 // What bounds them: at 100 to 300 CTAs of one wave each, a CTA's own chain of
 // loads, stages and barriers (DRAM sees the tensor only); at a million sites
-// instruction issue (400x500x5: 830 instructions per site in k_mx_step).
+// instruction issue (400x500x5: 817 instructions per site in k_mx_step).
 // Measured, one step alone, before (mixed-radix stages with runtime divisions,
 // three components in turn, zero-padded z transforms, five kernels) and after:
 // 200x150x5 FP32 122 -> 23 us, 128x128x4 FP64 37.5 -> 24 us, 32x95x3 FP64 173 ->

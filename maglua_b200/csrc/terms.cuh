@@ -1,7 +1,7 @@
 // terms.cuh -- field terms and LLG update of one site in the general form
 // (per-site parameters, pathway lists, several addends), FP32 or FP64 state;
-// shared by the general step kernels (kernels.cu) and the fused x pass
-// (mx.cu).  Reference semantics are cited per function.
+// shared by the general step kernels (kernels.cu) and the fused x passes
+// (xstep.cuh, mx.cuh).  Reference semantics are cited per function.
 #pragma once
 #include "device.cuh"
 #include "fused.cuh"

@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(XSCfg<PX, TH, SZ>::NT, XSCfg<PX, TH, SZ>::OCC)
 // local terms and the rows it contributes to, two sites at a time; forward x
 // pass of row 0, the next stage's spins (fwd).  Bound like k_xstep by the
 // instructions of its sites; CTAs of 512 sites (two per SM at 128 registers).
-// An RK4 step with a thermal kick of 256x256x8 as 11 kernels in place of 29
+// An RK4 step with a thermal kick of 256x256x8 as 10 kernels in place of 29
 // (fields evaluated to slots and one pass per row and stage): alone 300 -> 169
 // us, among others 211 -> 122.
 template <int PX, int LT, bool ANI, int SZ>
