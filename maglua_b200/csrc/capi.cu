@@ -1719,10 +1719,28 @@ void sur_advance(mlb_system* s);
 // The plan of a convolution operator (built).
 ConvPlan* conv_of(mlb_op* op) { return is_lr2d(op->kind) ? static_cast<ConvPlan*>(op->lr2.get()) : op->plan.get(); }
 
+// Stream `then` waits for the work enqueued on `first` so far (not when one of
+// them is being captured: a capture cannot wait for what lies outside it).
+void order_streams(cudaStream_t first, cudaStream_t then)
+{
+    if (first == then) return;
+    for (cudaStream_t st : {first, then}) {
+        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(st, &c));
+        if (c != cudaStreamCaptureStatusNone) return;
+    }
+    cudaEvent_t ev;
+    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    cudaError_t e = cudaEventRecord(ev, first);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(then, ev, 0);
+    cudaEventDestroy(ev);
+    CK(e);
+}
+
 // Before the stream of s uses a convolution's spectra: it waits for what another
 // system's stream still does with them (an operator serves any number of
 // systems, each on a stream of its own).  Graphs claim them where they are
-// launched; a caller's own capture cannot wait for what lies outside it.
+// launched.
 void claim_spec(mlb_op* op, mlb_system* s)
 {
     if (s->capturing || !(is_conv(op->kind) || is_lr2d(op->kind))) return;
@@ -1730,18 +1748,8 @@ void claim_spec(mlb_op* op, mlb_system* s)
     mlb_system* u = P.user;
     P.user = s;
     // a freed system, or a system whose stream changed, waited for its stream
-    if (!u || u == s || !g_systems.count(u) || u->st == s->st) return;
-    for (cudaStream_t st : {u->st, s->st}) {
-        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-        CK(cudaStreamIsCapturing(st, &c));
-        if (c != cudaStreamCaptureStatusNone) return;
-    }
-    cudaEvent_t ev;
-    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    cudaError_t e = cudaEventRecord(ev, u->st);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s->st, ev, 0);
-    cudaEventDestroy(ev);
-    CK(e);
+    if (!u || u == s || !g_systems.count(u)) return;
+    order_streams(u->st, s->st);
 }
 
 // Run a deferred inverse x pass on its own (the step took another path).
@@ -2231,6 +2239,9 @@ void llg_apply(mlb_llg* l, mlb_system* from, double scale, mlb_system* dmdt, mlb
         nm_guard(to, to->cur);
         CK(mlb::launch_llg(sysk(from, from->cur), m, H, Ht, dmdt->sa, dmdt->sg, dmdt->alpha, dmdt->gamma,
                            llgk(l, dt, to->status), out, to->rb, to->st));
+        // the sources change after the update has read them
+        order_streams(to->st, from->st);
+        order_streams(to->st, dmdt->st);
     }
     if (cart) {
         if (dt != 0.0 && advance) to->time = from->time + dt;
@@ -2416,6 +2427,7 @@ void copy_spins(mlb_system* dst, mlb_system* src)
         dst->ms_dirty = true;
         dst->ms_token = src->ms_token;
     }
+    order_streams(dst->st, src->st);   // src changes after the copy has read it
 }
 
 // SpinSystem::diff (spinsystem.cpp:301-307): sum_i |a_i - b_i| per component
