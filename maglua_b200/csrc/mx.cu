@@ -1,5 +1,7 @@
 // mx.cu -- dipole convolution and fused step for lattice edges of any
-// (31-smooth) length, FP32 and FP64 state.
+// (31-smooth) length, FP32 and FP64 state, for tensors with the point-dipole
+// parities (others, user tensors and sheared cells among them, keep the passes of
+// kernels.cu).
 //
 //   k_mx_fx / k_mx_ix   x transforms of row pairs (two real rows per complex
 //                       line) to and from SPEC[kx][c][z][y];
