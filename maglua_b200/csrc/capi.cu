@@ -380,18 +380,24 @@ struct mlb_llg {
 // Carried steps captured in one graph by a plan (an even count: a graph
 // starts and ends on the same spin buffer).
 constexpr int kMultiSteps = 4;
-// A plan has that graph from its creation; one that is captured again, or for a
-// single run, from this many steps on.  It saves 1 to 2 us a step, and capturing it
+// A plan has that graph from its creation; one captured again after fewer steps, or
+// for a single run, from this many steps on.  It saves 1 to 2 us a step, and capturing it
 // takes 25 to 140 us of host time, as the host is: it paid from 11 (256x256x8) to 43
 // steps (64x64x2 FP64) on, and on a slower host from 32 to 70.
 constexpr int kMultiFrom = 48;
+// A plan captured again after this many steps gets all of its graphs (three more,
+// 75 to 225 us: about what the steps themselves took).
+constexpr int kRestFrom = 16;
 
 // A captured step: one graph per spin-buffer parity q and per carry c (index q +
 // 2 c); c = 1 when the convolution's SPEC holds the forward x transform of the
-// current spins when the step starts, at its (y,z) pass.  A plan whose steps end in
-// the fused x pass, which leaves that transform to the next one, has the graphs of
-// c = 1 alone: a step that finds no carried spectrum launches its forward x pass
-// before them.  (Plans with event nodes or a device timeline have all four.)
+// current spins when the step starts, at its (y,z) pass.  Where steps end in the
+// fused x pass, which leaves that transform to the next one, those of c = 1 serve
+// alone: a step that finds no carried spectrum launches the forward x pass before
+// them (4 to 6 us more than in one graph, which takes 25 to 75 us to capture).
+// mlb_run leaves it at that; a plan has all four from its creation, and gets them
+// again when it is captured again after kRestFrom steps or more: one whose
+// parameters change more often would pay for graphs it hardly launches.
 struct mlb_plan {
     mlb_system* s = nullptr;
     std::vector<mlb_op*> ops;
@@ -406,6 +412,7 @@ struct mlb_plan {
     cudaGraphExec_t multi = nullptr;
     int multi_q = 0;
     bool multi_tried = false;
+    bool kept = false;            // a plan of the caller's, not of a single run
     long long steps = 0;          // launched since the capture
     std::vector<mlb::ProfCaptured> ev[4];
     mlb_op* carry_op = nullptr;   // the convolution whose SPEC a step leaves carried (null: none)
@@ -2658,6 +2665,17 @@ void plan_capture_multi(mlb_plan* p)
     }
 }
 
+// The graphs that a kept plan has beside plan_capture's: steps that find no carried
+// spectrum, several steps at once.
+void plan_capture_rest(mlb_plan* p)
+{
+    if (!p->carry_op) return;
+    const HostState h0 = save_state(p->s, p->ops);
+    for (int q = 0; q < 2; q++)
+        if (!p->exec[q]) plan_capture_steps(p, q, 1, nullptr, h0, &p->ev[q], &p->exec[q]);
+    plan_capture_multi(p);
+}
+
 void advance_host(mlb_plan* p)
 {
     mlb_system* s = p->s;
@@ -2676,7 +2694,11 @@ void plan_launch(mlb_plan* p, int nsteps)
 {
     if (nsteps <= 0) return;
     mlb_system* s = p->s;
-    if (p->version != g_version) plan_capture(p);
+    if (p->version != g_version) {
+        const bool all = p->kept && p->steps >= kRestFrom;
+        plan_capture(p);
+        if (all) plan_capture_rest(p);
+    }
     p->steps += nsteps;
     if (p->steps >= kMultiFrom) plan_capture_multi(p);
     DevStep h;
@@ -5028,7 +5050,8 @@ int mlb_plan_create(mlb_system* s, mlb_op* const* ops, int nops, mlb_llg* l, int
             plan_timeline_reset(p.get());
         }
         plan_capture(p.get());
-        plan_capture_multi(p.get());
+        p->kept = true;
+        plan_capture_rest(p.get());
         *out = p.release();
     });
 }
