@@ -20,8 +20,16 @@ HEADERS = ["device.cuh", "fftreg.cuh", "fused.cuh", "kparams.h", "launch.h", "mx
            "xreg.cuh", "xstep.cuh", "yzls.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
+FLAGS = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
          "-I", os.path.join(ROOT, "include"), "-I", CSRC]
+
+
+def _lineinfo(src):
+    """Line tables, for profiles: three quarters of the size of the units that
+    hold many instances of one kernel, and most of the time their modules take
+    to load (mlb_init 230 ms with them), so there only on request."""
+    many = src.startswith(("xstep_", "mx_f", "yzls_f"))
+    return ["-lineinfo"] if not many or os.environ.get("MLB_LINEINFO") else []
 
 
 def nvcc():
@@ -50,7 +58,7 @@ def build(force=False, verbose=False):
     os.makedirs(bdir, exist_ok=True)
     for src in SOURCES:   # side by side, one per core
         obj = os.path.join(bdir, src.replace(".cu", ".o"))
-        cmd = [nvcc()] + ARCH + FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
+        cmd = [nvcc()] + ARCH + FLAGS + _lineinfo(src) + ["-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
             print(" ".join(cmd))

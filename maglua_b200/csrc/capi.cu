@@ -1026,17 +1026,6 @@ void build_magnetostatic_t6(mlb_op* op)
     op->t6_valid = true;
 }
 
-// The constant tables of the translation units that the plan's passes run from
-// (loading them, outside any capture).
-void plan_tables(const ConvPlan& P)
-{
-    const ConvK& k = P.k;
-    if (P.x_mx) CK(mlb::mx_init(P.mx.x.ax, P.rb));
-    else if (P.rb == 4) CK(mlb::xstep_init(k.Px));
-    if (k.ls) CK(mlb::yz_ls_init(P.rb));
-    else if (k.mx) CK(mlb::mx_init(P.mx.yz.ax, P.rb));
-}
-
 // Build or rebuild the tensor spectrum of op (FP64 on the GPU), stored at
 // rb bytes per real for the systems it is applied to.
 void build_plan(mlb_op* op, cudaStream_t st, int rb)
@@ -1175,7 +1164,6 @@ void build_plan(mlb_op* op, cudaStream_t st, int rb)
         k.spec2 = P->spec2.p;
     }
     CK(cudaStreamSynchronize(st));
-    plan_tables(*P);
     // captured steps hold the arrays of the plan that goes (a system of the other
     // precision may have asked for this one)
     if (op->plan) g_version++;
@@ -1480,7 +1468,6 @@ void build_lr2d(mlb_op* op, cudaStream_t st, int rb)
         P->spec2.alloc((size_t)k.Kx * ny * 3 * nz * cb);
         P->k.spec2 = P->spec2.p;
     }
-    plan_tables(*P);
     if (op->lr2) g_version++;   // as in build_plan
     op->lr2 = std::move(P);
     op->lr2_compile = false;
@@ -3247,7 +3234,6 @@ void ens_prepare(mlb_ensemble* e)
             ConvPlan& P = *k.dip->plan;
             // all replicas per launch: the power-of-two passes
             if (P.k.ls && x_pow2(P.k, 4, 16)) P.x_mx = false;
-            plan_tables(P);
             k.fast = P.k.mx ? P.k.ls && !P.x_mx : mlb::conv_fast_ok(P.k) && !P.k.split;
             P.k.g = c.g / ((double)P.k.Px * P.k.Py * (P.k.mx ? 1 : P.k.Pz));
             P.k.nrep = k.fast ? k.nrep : 1;
@@ -3314,6 +3300,9 @@ int mlb_init(int device)
         CK(cudaFree(0));
         CK(mlb::conv_configure());
         CK(mlb::fftreg_init());
+        CK(mlb::xstep_init());
+        CK(mlb::mx_init());
+        CK(mlb::yz_ls_init());
         CK(mlb::sur_configure());
         CK(cudaDeviceSynchronize());   // the constant tables are there
     });

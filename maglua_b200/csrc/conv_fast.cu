@@ -1381,16 +1381,11 @@ cudaError_t launch_conv_fast_ix(const ConvK& c, const FftLen L[3], const float2*
     return launch_x_any(c, tw + L[0].tw_off, nullptr, spec, h, st, false);
 }
 
-cudaError_t xstep_init(int Px)
+cudaError_t xstep_init()
 {
-    switch (Px) {
-    case 32: return XUnit<32>::init();
-    case 64: return XUnit<64>::init();
-    case 128: return XUnit<128>::init();
-    case 256: return XUnit<256>::init();
-    case 512: return XUnit<512>::init();
-    }
-    return cudaSuccess;
+    cudaError_t e;
+    if ((e = XUnit<32>::init()) || (e = XUnit<64>::init()) || (e = XUnit<128>::init()) || (e = XUnit<256>::init())) return e;
+    return XUnit<512>::init();
 }
 
 bool xstep_ok(const ConvK& c, const FastK& F)

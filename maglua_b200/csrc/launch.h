@@ -8,7 +8,6 @@
 
 #include <map>
 #include <mutex>
-#include <set>
 #include <utility>
 #include <vector>
 
@@ -36,21 +35,6 @@ inline cudaError_t use_smem(const void* kern, size_t smem, bool max_carveout = f
         return e;
     allowed[{kern, dev}] = smem;
     return cudaSuccess;
-}
-
-// f() once on each device (per call site: the lambda's type).
-template <class F>
-inline cudaError_t per_device(F&& f)
-{
-    static std::mutex mu;
-    static std::set<int> done;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done.count(dev)) return cudaSuccess;
-    if ((e = f()) == cudaSuccess) done.insert(dev);
-    return e;
 }
 
 // Launch with programmatic stream serialization: the kernel's CTAs may be
@@ -146,8 +130,8 @@ cudaError_t launch_conv_fast_fyz(const ConvK& c, const FftLen L[3], const float2
                                  const float* ten6, bool with_fx, cudaStream_t st);
 cudaError_t launch_conv_fast_ix(const ConvK& c, const FftLen L[3], const float2* tw, float2* spec, float* h[3],
                                 cudaStream_t st);
-// The fused x pass for lines of PX points (xstep.cuh); init: its constant tables,
-// before its first launch and outside any capture (xstep_init: by length).
+// The fused x pass for lines of PX points (xstep.cuh); init: its constant tables
+// (loads the module; when the library starts, outside any capture).
 template <int PX>
 struct XUnit {
     static cudaError_t init();
@@ -160,7 +144,7 @@ struct XUnit {
     static cudaError_t rk(const ConvK& c, const FastK& F, const RkRows<float>& rows, int fwd, const float2* tw,
                           float2* spec, const float* const s[3], float* const h[3], float* const o[3], cudaStream_t st);
 };
-cudaError_t xstep_init(int Px);
+cudaError_t xstep_init();
 bool xstep_ok(const ConvK& c, const FastK& F);
 bool xstep_pairs(const ConvK& c);
 // Inverse x pass + fused step (+ forward x pass of the new spins when fwd).
@@ -219,8 +203,7 @@ cudaError_t launch_mx_pack(const double2* W, const ConvK& c, const int* at, void
 bool yz_ls_plan(const ConvK& c, int rb, std::vector<int>& at);
 cudaError_t launch_yz_ls(const ConvK& c, const FftLen L[3], const void* tw, void* spec, const void* tz, int rb,
                          cudaStream_t st);
-// the pass for lines of C (float2 or double2; yzls.cuh), and its constant tables (before
-// its first launch, outside any capture)
+// the pass for lines of C (float2 or double2; yzls.cuh), and its constant tables
 template <typename C>
 struct YzUnit {
     typedef decltype(C().x) R;
@@ -228,7 +211,7 @@ struct YzUnit {
     static bool takes(int Py, int nz);
     static cudaError_t pass(const ConvK& c, const C* tw, C* spec, const R* tz, cudaStream_t st);
 };
-cudaError_t yz_ls_init(int rb);
+cudaError_t yz_ls_init();
 // Any-length passes (mx.cu): the plans of the x passes and of the (y,z) pass
 // (false: not a size they take) with the places of their frequencies, and the
 // passes.
@@ -265,8 +248,7 @@ cudaError_t launch_xrk(const ConvK& c, const FftLen L[3], const void* tw, void* 
 cudaError_t launch_mx_gstep(const MxX& x, const FftLen L[3], const void* tw, void* spec, const FusedK& P, double addw,
                             double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], int rb, cudaStream_t st);
 // The kernels for state precision R, BIG: with prime radices above 13 (mx.cuh); init:
-// their constant tables, before their first launch and outside any capture
-// (mx_init: those of an axis).
+// their constant tables.
 template <typename R, bool BIG>
 struct MxUnit {
     typedef typename CT<R>::T C;
@@ -283,7 +265,7 @@ struct MxUnit {
     static cudaError_t gstep(const MxX& x, size_t smem, const C* tw, C* spec, const FusedK& P, double addw,
                              double dt_sys, const DevStep* cur, DevStep* next, void* const h[3], cudaStream_t st);
 };
-cudaError_t mx_init(const MxAxis& ax, int rb);
+cudaError_t mx_init();
 cudaError_t launch_tensor_lattice(int nx, int ny, int nz, const int gmax[4], const double ABC[9], int Px,
                                   int Py, int Pz, int zsign, double2* W, cudaStream_t st);
 cudaError_t launch_tensor_rings(int nx, int ny, int nz, int nrings, int lstep, const double ABC[9], int Px, int Py,

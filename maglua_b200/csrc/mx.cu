@@ -374,9 +374,11 @@ cudaError_t launch_mx_gstep(const MxX& x, const FftLen L[3], const void* tw, voi
                                       static_cast<float2*>(spec), P, addw, dt_sys, cur, next, h, st));
 }
 
-cudaError_t mx_init(const MxAxis& ax, int rb)
+cudaError_t mx_init()
 {
-    return rb == 8 ? MX_UNIT(double, ax, init()) : MX_UNIT(float, ax, init());
+    cudaError_t e;
+    if ((e = MxUnit<float, false>::init()) || (e = MxUnit<float, true>::init()) || (e = MxUnit<double, false>::init())) return e;
+    return MxUnit<double, true>::init();
 }
 
 } // namespace mlb

@@ -1,6 +1,6 @@
 // mx.cuh -- the kernels of mx.cu, one translation unit per state precision and with or
-// without prime radices above 13 (mx_f32.cu, mx_f32_big.cu and so on): a program loads
-// those it takes.
+// without prime radices above 13 (mx_f32.cu, mx_f32_big.cu and so on), which compile
+// side by side.
 #pragma once
 #include "device.cuh"
 #include "fused.cuh"
@@ -760,20 +760,18 @@ namespace mlb {
 template <typename R, bool BIG>
 cudaError_t MxUnit<R, BIG>::init()
 {
-    return per_device([] {
-        static float2 hf[mx::NW];
-        static double2 hd[mx::NW];
-        for (int r = 1; r <= mx::MAXR; r++)
-            for (int k = 0; k < r; k++) {
-                const double a = 2.0 * M_PI * k / r;
-                hd[r * (r - 1) / 2 + k] = make_double2(cos(a), -sin(a));
-                hf[r * (r - 1) / 2 + k] = make_float2((float)cos(a), (float)-sin(a));
-            }
-        cudaError_t e;
-        if ((e = cudaMemcpyToSymbol(mx::c_wf, hf, sizeof(hf))) != cudaSuccess) return e;
-        if ((e = cudaMemcpyToSymbol(mx::c_wd, hd, sizeof(hd))) != cudaSuccess) return e;
-        return cudaStreamSynchronize(nullptr);   // there for every stream
-    });
+    static float2 hf[mx::NW];
+    static double2 hd[mx::NW];
+    for (int r = 1; r <= mx::MAXR; r++)
+        for (int k = 0; k < r; k++) {
+            const double a = 2.0 * M_PI * k / r;
+            hd[r * (r - 1) / 2 + k] = make_double2(cos(a), -sin(a));
+            hf[r * (r - 1) / 2 + k] = make_float2((float)cos(a), (float)-sin(a));
+        }
+    cudaError_t e;
+    if ((e = cudaMemcpyToSymbol(mx::c_wf, hf, sizeof(hf))) != cudaSuccess) return e;
+    if ((e = cudaMemcpyToSymbol(mx::c_wd, hd, sizeof(hd))) != cudaSuccess) return e;
+    return cudaStreamSynchronize(nullptr);   // there for every stream
 }
 
 static dim3 mx_grid(const MxX& x) { return dim3((x.nr + x.rows - 1) / x.rows); }

@@ -1,8 +1,7 @@
 // xstep.cuh -- the fused x pass of a step for power-of-two FP32 lines, in the forms
 // of a step with uniform parameters (k_xstep), of the general step (k_xgstep), of a
 // packed ensemble's size class (k_xens) and of a Runge-Kutta stage (k_xrk).  One
-// translation unit per line length (xstep_32.cu and so on): a program loads the
-// modules of the lengths it takes, and they compile side by side.
+// translation unit per line length (xstep_32.cu and so on), which compile side by side.
 #pragma once
 #include "device.cuh"
 #include "fftreg.cuh"
@@ -591,7 +590,7 @@ static cudaError_t xgstep_px(const ConvK& c, const FusedK& P, double addw, doubl
 template <int PX>
 cudaError_t XUnit<PX>::init()
 {
-    return per_device([] { return fr::fill_tables(); });
+    return fr::fill_tables();
 }
 template <int PX>
 cudaError_t XUnit<PX>::step(const ConvK& c, const FastK& F, int fwd, const float2* tw, float2* spec, const float* s[3],

@@ -44,6 +44,10 @@ cudaError_t launch_yz_ls(const ConvK& c, const FftLen L[3], const void* tw, void
                                 static_cast<const float*>(tz), st);
 }
 
-cudaError_t yz_ls_init(int rb) { return rb == 8 ? YzUnit<double2>::init() : YzUnit<float2>::init(); }
+cudaError_t yz_ls_init()
+{
+    const cudaError_t e = YzUnit<float2>::init();
+    return e != cudaSuccess ? e : YzUnit<double2>::init();
+}
 
 } // namespace mlb

@@ -267,7 +267,7 @@ constexpr size_t LS_SMEM = 227 * 1024;
 template <typename C>
 cudaError_t YzUnit<C>::init()
 {
-    return per_device([] { return fr::fill_tables(); });
+    return fr::fill_tables();
 }
 template <typename C>
 bool YzUnit<C>::takes(int Py, int nz)

@@ -1,7 +1,6 @@
-"""mlb_init loads what every program needs; the passes of one line length, precision
-or ensemble are loaded when a plan first takes them.  Seen by the device memory
-that init takes in a fresh process: 46 MB when it set the limits of every kernel
-(250 ms), 2 MB now."""
+"""mlb_init loads the library's modules, not every kernel in them: a kernel is loaded
+by its first launch.  Seen by the device memory that init takes in a fresh process:
+46 MB when it set the limits of every kernel, 2 MB now."""
 import os
 import subprocess
 import sys
