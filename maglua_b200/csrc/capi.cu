@@ -1776,6 +1776,13 @@ bool take_carry(mlb_system* s, mlb_op* op, const ConvPlan& P)
     return true;
 }
 
+// Whether a plan's inverse x pass can wait for the LLG update of a step (defer_x).
+bool conv_defers(const mlb_op* op, const ConvPlan& P)
+{
+    if (is_lr2d(op->kind)) return P.k.mx;
+    return P.k.nrep == 1 && !P.k.general && (P.k.mx || (P.rb == 4 && mlb::conv_fast_ok(P.k)));
+}
+
 // Layer scales of a LongRange2D, the operator's global scale included.
 void lr2d_scales(const mlb_op* op, LR2DScale& sc)
 {
@@ -1918,7 +1925,7 @@ void op_apply(mlb_op* op, mlb_system* s)
         claim_spec(op, s);
         if (s->sur && sur_hook(op, s, sl)) return;
         const void* spv[3] = {s->sp[s->cur][0], s->sp[s->cur][1], s->sp[s->cur][2]};
-        if (s->defer_x && P.k.nrep == 1 && !P.k.general && (P.k.mx || (s->rb == 4 && mlb::conv_fast_ok(P.k)))) {
+        if (s->defer_x && conv_defers(op, P)) {
             // forward x pass only when SPEC does not already hold it
             const bool carry = take_carry(s, op, P);
             ConvK kk = P.k;
@@ -2584,14 +2591,14 @@ bool plan_capture_steps(mlb_plan* p, int q, int nsteps, mlb_op* carry, const Hos
     return fits;
 }
 
-// The convolution whose spectrum a step of these operators would leave to the next
-// one if it ends in a fused x pass: the last one.
+// The convolution (its plan built) whose spectrum a step of these operators would
+// leave to the next one if it ends in a fused x pass: the last one.
 mlb_op* plan_last_conv(const mlb_plan* p)
 {
     mlb_op* c = nullptr;
     for (mlb_op* o : p->ops)
         if (is_conv(o->kind) || is_lr2d(o->kind)) c = o;
-    return c;
+    return c && conv_defers(c, *conv_of(c)) ? c : nullptr;
 }
 
 // Capture one step for each spin-buffer parity.  A dry pass first runs the

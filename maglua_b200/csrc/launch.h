@@ -16,6 +16,9 @@ namespace mlb {
 // shared memory preferred over L1), set when its first launch on a device asks
 // for it.  Setting them for every instantiation when the library starts loads
 // them all: 250 to 340 ms where a program takes a handful.
+// Beyond SMEM_FREE it has to be set: the 48 KB that need no limit hold the kernel's
+// static shared memory too (up to 1 KB in these).
+constexpr size_t SMEM_FREE = 40 * 1024;
 inline cudaError_t use_smem(const void* kern, size_t smem, bool max_carveout = false)
 {
     static std::mutex mu;
@@ -26,7 +29,7 @@ inline cudaError_t use_smem(const void* kern, size_t smem, bool max_carveout = f
     std::lock_guard<std::mutex> lk(mu);
     auto it = allowed.find({kern, dev});
     if (it != allowed.end() && it->second >= smem) return cudaSuccess;
-    if (smem > 48 * 1024 &&
+    if (smem > SMEM_FREE &&
         (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
         return e;
     if (max_carveout &&
@@ -45,7 +48,7 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               Args... args)
 {
-    if (smem > 48 * 1024) {
+    if (smem > SMEM_FREE) {
         const cudaError_t e = use_smem(reinterpret_cast<const void*>(kern), smem);
         if (e != cudaSuccess) return e;
     }
