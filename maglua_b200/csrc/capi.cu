@@ -303,6 +303,10 @@ struct mlb_system {
     mlb_op* cap_xstep = nullptr;    // capture: the convolution whose x pass the captured step fused
     unsigned long long* cap_tl = nullptr;   // capture: device timeline stamps of a timing plan
     unsigned long long spec_token = 0;   // matches ConvPlan::spec_token while that holds
+    cudaEvent_t order_ev = nullptr;      // order_streams: recorded on this system's stream
+    // graphs that a run or a plan gave up, each destroyed once its last launch
+    // (before the event) has run
+    std::vector<std::pair<cudaEvent_t, cudaGraphExec_t>> retired;
 };
 
 struct mlb_op {
@@ -423,6 +427,7 @@ struct mlb_plan {
 namespace {
 
 void nm_guard(mlb_system* s, int q);
+void purge_retired(mlb_system* s, bool all);
 
 std::set<mlb_system*> g_systems;
 unsigned long long g_ms_token = 0;
@@ -1713,22 +1718,19 @@ void sur_advance(mlb_system* s);
 // The plan of a convolution operator (built).
 ConvPlan* conv_of(mlb_op* op) { return is_lr2d(op->kind) ? static_cast<ConvPlan*>(op->lr2.get()) : op->plan.get(); }
 
-// Stream `then` waits for the work enqueued on `first` so far (not when one of
-// them is being captured: a capture cannot wait for what lies outside it).
-void order_streams(cudaStream_t first, cudaStream_t then)
+// The stream of `then` waits for the work enqueued on that of `first` so far (not
+// when one of them is being captured: a capture cannot wait for what lies outside it).
+void order_streams(mlb_system* first, mlb_system* then)
 {
-    if (first == then) return;
-    for (cudaStream_t st : {first, then}) {
+    if (first->st == then->st) return;
+    for (cudaStream_t st : {first->st, then->st}) {
         cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
         CK(cudaStreamIsCapturing(st, &c));
         if (c != cudaStreamCaptureStatusNone) return;
     }
-    cudaEvent_t ev;
-    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    cudaError_t e = cudaEventRecord(ev, first);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(then, ev, 0);
-    cudaEventDestroy(ev);
-    CK(e);
+    if (!first->order_ev) CK(cudaEventCreateWithFlags(&first->order_ev, cudaEventDisableTiming));
+    CK(cudaEventRecord(first->order_ev, first->st));
+    CK(cudaStreamWaitEvent(then->st, first->order_ev, 0));
 }
 
 // Before the stream of s uses a convolution's spectra: it waits for what another
@@ -1743,7 +1745,7 @@ void claim_spec(mlb_op* op, mlb_system* s)
     P.user = s;
     // a freed system, or a system whose stream changed, waited for its stream
     if (!u || u == s || !g_systems.count(u)) return;
-    order_streams(u->st, s->st);
+    order_streams(u, s);
 }
 
 // Run a deferred inverse x pass on its own (the step took another path).
@@ -2241,8 +2243,8 @@ void llg_apply(mlb_llg* l, mlb_system* from, double scale, mlb_system* dmdt, mlb
         CK(mlb::launch_llg(sysk(from, from->cur), m, H, Ht, dmdt->sa, dmdt->sg, dmdt->alpha, dmdt->gamma,
                            llgk(l, dt, to->status), out, to->rb, to->st));
         // the sources change after the update has read them
-        order_streams(to->st, from->st);
-        order_streams(to->st, dmdt->st);
+        order_streams(to, from);
+        order_streams(to, dmdt);
     }
     if (cart) {
         if (dt != 0.0 && advance) to->time = from->time + dt;
@@ -2368,6 +2370,8 @@ void free_system(mlb_system* s)
     if (!s) return;
     g_systems.erase(s);
     cudaStreamSynchronize(s->st);
+    purge_retired(s, true);
+    if (s->order_ev) cudaEventDestroy(s->order_ev);
     for (int b = 0; b < 2; b++)
         for (int c = 0; c < 3; c++) cudaFree(s->sp[b][c]);
     cudaFree(s->ms);
@@ -2428,7 +2432,7 @@ void copy_spins(mlb_system* dst, mlb_system* src)
         dst->ms_dirty = true;
         dst->ms_token = src->ms_token;
     }
-    order_streams(dst->st, src->st);   // src changes after the copy has read it
+    order_streams(dst, src);   // src changes after the copy has read it
 }
 
 // SpinSystem::diff (spinsystem.cpp:301-307): sum_i |a_i - b_i| per component
@@ -2529,15 +2533,51 @@ void plan_timeline_reset(mlb_plan* p)
     upload(p->tl.p, init, sizeof(init), p->s->st);
 }
 
+// Destroys the retired graphs that have run (all: waited for).
+void purge_retired(mlb_system* s, bool all)
+{
+    size_t kept = 0;
+    for (auto& g : s->retired) {
+        if (!all && cudaEventQuery(g.first) == cudaErrorNotReady) {
+            s->retired[kept++] = g;
+            continue;
+        }
+        cudaGraphExecDestroy(g.second);
+        cudaEventDestroy(g.first);
+    }
+    s->retired.resize(kept);
+    cudaGetLastError();
+}
+
+// A graph launched on the stream of s that is no longer needed.
+void retire_graph(mlb_system* s, cudaGraphExec_t& g)
+{
+    if (!g) return;
+    cudaEvent_t ev = nullptr;
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess && cudaEventRecord(ev, s->st) == cudaSuccess) {
+        s->retired.push_back({ev, g});
+    } else {
+        if (ev) cudaEventDestroy(ev);
+        cudaStreamSynchronize(s->st);
+        cudaGraphExecDestroy(g);
+    }
+    g = nullptr;
+}
+
 void plan_release(mlb_plan* p)
 {
-    if (p->multi) cudaGraphExecDestroy(p->multi);
-    p->multi = nullptr;
+    const bool alive = g_systems.count(p->s) != 0;   // else its stream has been waited for
+    auto drop = [&](cudaGraphExec_t& g) {
+        if (alive) retire_graph(p->s, g);
+        else if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    };
+    if (alive) purge_retired(p->s, false);
+    drop(p->multi);
     p->multi_tried = false;
     p->steps = 0;
     for (int q = 0; q < 4; q++) {
-        if (p->exec[q]) cudaGraphExecDestroy(p->exec[q]);
-        p->exec[q] = nullptr;
+        drop(p->exec[q]);
         for (ProfCaptured& r : p->ev[q]) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
         p->ev[q].clear();
     }
@@ -2845,6 +2885,7 @@ std::mutex g_ens_tune_mu;
 
 void ens_free_graphs(mlb_ensemble* e)
 {
+    if (e->exec[0]) cudaStreamSynchronize(e->st);   // their last launches have run
     for (int q = 0; q < 4; q++) {
         if (e->exec[q]) cudaGraphExecDestroy(e->exec[q]);
         e->exec[q] = nullptr;
@@ -3649,9 +3690,9 @@ static void netmoment_enqueue(mlb_system* s, double m, int d, cudaStream_t st)
     double* redout = d ? s->redout_a : s->redout;
     unsigned* counter = d ? s->nm_counter_a : s->nm_counter;
     if (!s->nm_exec[q][d] || s->nm_m[q][d] != m) {
-        if (s->nm_exec[q][d]) { cudaGraphExecDestroy(s->nm_exec[q][d]); s->nm_exec[q][d] = nullptr; }
         CK(cudaStreamSynchronize(s->st));
         if (s->nm_st) CK(cudaStreamSynchronize(s->nm_st));
+        if (s->nm_exec[q][d]) { cudaGraphExecDestroy(s->nm_exec[q][d]); s->nm_exec[q][d] = nullptr; }
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
         // one kernel: the last block writes the sums into the pinned slot
@@ -5942,8 +5983,7 @@ void rk_step_graph(mlb_rk* r)
         cudaGraphExecUpdateResultInfo info;
         if (cudaGraphExecUpdate(r->exec, g, &info) != cudaSuccess) {
             cudaGetLastError();
-            cudaGraphExecDestroy(r->exec);
-            r->exec = nullptr;
+            retire_graph(ss, r->exec);
         }
     }
     cudaError_t ie = cudaSuccess;
@@ -6041,7 +6081,8 @@ int mlb_rk_destroy(mlb_rk* r)
 {
     return guard([&] {
         if (!r) return;
-        if (r->exec) cudaGraphExecDestroy(r->exec);
+        if (g_systems.count(r->ss)) retire_graph(r->ss, r->exec);
+        else if (r->exec) cudaGraphExecDestroy(r->exec);
         for (mlb_system* c : r->k) free_system(c);
         delete r;
     });

@@ -59,3 +59,20 @@ def test_reader_behind_its_queue(M, how):
         src.synchronize()
         res.append(np.stack(dst.spinArrays()[:3]))
     np.testing.assert_array_equal(res[0], res[1])
+
+
+def test_short_runs_in_turn(M):
+    """Two systems with one operator, a hundred runs of three steps each and none
+    waited for: the graphs of a run outlive it until they have run."""
+    res = []
+    for wait in (True, False):
+        a, ops, llg = _system(M, 1)
+        b, _, _ = _system(M, 2)
+        for k in range(100):
+            for ss in (a, b):
+                M.run(ss, ops, llg, 3)
+                if wait:
+                    ss.synchronize()
+        res.append([np.stack(ss.spinArrays()[:3]) for ss in (a, b)])
+    for x, y in zip(*res):
+        np.testing.assert_array_equal(x, y)
